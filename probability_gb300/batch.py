@@ -20,7 +20,7 @@ import numpy as np
 import torch
 
 from probability_gb300 import _native, _util, targets
-from probability_gb300.mcmc.nuts import NUTSKernelResults
+from probability_gb300.mcmc.nuts import NUTSKernelResults, last_leaf_iterations
 
 FAMILY_MVN, FAMILY_HIER = 1, 2
 P = ctypes.c_void_p
@@ -166,8 +166,12 @@ class BatchedNoUTurnSampler:
     self._handle = h
     _native.check(_native.lib().gbm_nuts_set_graphs(h, int(bool(use_graphs))),
                   'gbm_nuts_set_graphs')
-    self.last_leaf_iterations = 0
     self.inverse_mass = None
+
+  @property
+  def last_leaf_iterations(self):
+    """Leaf iterations of the last one_step or run_free (waits for it)."""
+    return last_leaf_iterations(self._handle)
 
   def set_inverse_mass(self, inverse_mass):
     """Diagonal inverse mass matrix (the preconditioning of
@@ -220,10 +224,10 @@ class BatchedNoUTurnSampler:
     eps = self._eps(pkr.step_size)
     nq, ng = torch.empty_like(q), torch.empty_like(q)
     f64 = lambda: torch.empty(C, dtype=torch.float64, device=dev)
-    u8 = lambda: torch.empty(C, dtype=torch.uint8, device=dev)
+    flag = lambda: torch.empty(C, dtype=torch.bool, device=dev)
     nl, lar, energy = f64(), f64(), f64()
     lf = torch.empty(C, dtype=torch.int32, device=dev)
-    acc, rmd, div = u8(), u8(), u8()
+    acc, rmd, div = flag(), flag(), flag()
     Pt = _native.ptr
     b._enter()
     _native.check(_native.lib().gbm_nuts_one_step(
@@ -231,13 +235,10 @@ class BatchedNoUTurnSampler:
         1, _native.seed_words(seed), Pt(nq), Pt(nl), Pt(ng), Pt(lar), Pt(lf), Pt(acc), Pt(rmd),
         Pt(div), Pt(energy), None), 'gbm_nuts_one_step')
     b._leave()
-    n = ctypes.c_int64()
-    _native.lib().gbm_nuts_last_leaf_iterations(self._handle, ctypes.byref(n))
-    self.last_leaf_iterations = int(n.value)
     return nq, NUTSKernelResults(
         target_log_prob=nl, grads_target_log_prob=ng, step_size=eps, log_accept_ratio=lar,
-        leapfrogs_taken=lf, is_accepted=acc.bool(), reach_max_depth=rmd.bool(),
-        has_divergence=div.bool(), energy=energy, seed=_util.seed_tensor(seed))
+        leapfrogs_taken=lf, is_accepted=acc, reach_max_depth=rmd,
+        has_divergence=div, energy=energy, seed=_util.seed_tensor(seed))
 
   def run_free(self, current_state, kernel_results, transitions_per_chain, seed,
                  first_step=0, max_leaf_iterations=1 << 40):
@@ -257,7 +258,6 @@ class BatchedNoUTurnSampler:
                      first_step, transitions_per_chain, max_leaf_iterations, (q.numel(),))
     finally:
       b._leave()
-    self.last_leaf_iterations = run.leaf_iterations
     return run
 
 

@@ -32,6 +32,7 @@
 
 #include "engine.h"
 #include "gb300_mcmc.h"
+#include "nuts_chain.h"
 
 namespace gbm {
 namespace {
@@ -416,6 +417,7 @@ class BatchTarget final : public Target {
     C_ = chains;
     E_ = elems;
     dim = dmax;
+    set_chain_models(ctx);
     coff_.reserve(sizeof(int64_t) * C_);
     cdim_.reserve(sizeof(int) * C_);
     GBM_CUDA(cudaMemcpyAsync(coff_.ptr, coff.data(), sizeof(int64_t) * C_,
@@ -446,6 +448,9 @@ class BatchTarget final : public Target {
   int64_t ragged_chains() const override { return C_; }
   int64_t ragged_elements() const override { return E_; }
   int launches_per_eval(int64_t) const override { return 3; }
+  const ChainModels* chain_models() const override {
+    return models_.ptr ? &chain_models_ : nullptr;
+  }
 
   // All chains (the direct log_prob_and_grad call): q, grad ragged.
   void eval(const float* q, int, const int*, int, double* logp, float* grad, int, void*,
@@ -500,6 +505,35 @@ class BatchTarget final : public Target {
   struct Owned {
     DeviceBuffer a, b;
   };
+
+  // The hierarchical members whose chains fit a warp's registers.
+  void set_chain_models(gbm_context* ctx) {
+    const std::vector<double> table = chain_log_table();
+    table_.reserve(sizeof(double) * table.size());
+    std::vector<HierModel> models(T_);
+    std::vector<int> model_of(C_, -1);
+    int max_dim = 0, held = 0;
+    for (int t = 0; t < T_; ++t) {
+      const BDesc& d = hdesc_[t];
+      if (d.family != kBatchHier || d.dim > kChainMaxDim) continue;
+      models[t] = HierModel{d.y, d.sigma, d.mu_scale, d.tau_scale, d.hconst, table_.as<double>()};
+      std::fill(model_of.begin() + d.c_begin, model_of.begin() + d.c_end, t);
+      max_dim = std::max(max_dim, d.dim);
+      held += d.c_end - d.c_begin;
+    }
+    if (held == 0) return;
+    GBM_CUDA(cudaMemcpyAsync(table_.ptr, table.data(), sizeof(double) * table.size(),
+                             cudaMemcpyHostToDevice, ctx->stream));
+    models_.reserve(sizeof(HierModel) * T_);
+    model_of_.reserve(sizeof(int) * C_);
+    GBM_CUDA(cudaMemcpyAsync(models_.ptr, models.data(), sizeof(HierModel) * T_,
+                             cudaMemcpyHostToDevice, ctx->stream));
+    GBM_CUDA(cudaMemcpyAsync(model_of_.ptr, model_of.data(), sizeof(int) * C_,
+                             cudaMemcpyHostToDevice, ctx->stream));
+    GBM_CUDA(cudaStreamSynchronize(ctx->stream));   // the vectors are this call's
+    chain_models_ = ChainModels{models_.as<HierModel>(), model_of_.as<int>(), max_dim,
+                                held == C_};
+  }
 
   void upload() {
     GBM_CUDA(cudaMemcpyAsync(desc_.ptr, hdesc_.data(), sizeof(BDesc) * T_,
@@ -559,7 +593,8 @@ class BatchTarget final : public Target {
   int chosen_[kClasses] = {0, 0, 0, 0};
   std::vector<BDesc> hdesc_;
   std::vector<std::unique_ptr<Owned>> owned_;
-  DeviceBuffer desc_, coff_, cdim_, u_, part_, sched_, all_;
+  DeviceBuffer desc_, coff_, cdim_, u_, part_, sched_, all_, models_, model_of_, table_;
+  ChainModels chain_models_{};
 };
 
 }  // namespace

@@ -530,8 +530,11 @@ int gbm_nuts_run_free(gbm_nuts* k, int64_t chains, const float* state,
 
 int gbm_nuts_last_leaf_iterations(const gbm_nuts* k, int64_t* out) {
   if (!k || !out) return invalid("gbm_nuts_last_leaf_iterations: NULL argument");
-  *out = k->last_leaf_iterations;
-  return GBM_OK;
+  return guarded([&] {
+    DeviceGuard g(k->ctx->device);
+    *out = gbm::nuts_last_leaf_iterations(const_cast<gbm_nuts*>(k));
+    return GBM_OK;
+  });
 }
 
 static int check_loop_args(int64_t chains, int64_t max_chains, int64_t first_step,

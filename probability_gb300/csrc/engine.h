@@ -64,6 +64,26 @@ struct DeviceBuffer {
   template <class T> T* as() const { return static_cast<T*>(ptr); }
 };
 
+// A non-centred hierarchical normal whose whole chains a warp can run
+// (nuts_chain.cu): y, sigma [J] on the device.
+struct HierModel {
+  const float* y;
+  const float* sigma;
+  float mu_scale, tau_scale;
+  double konst;             // constant part of the log-density
+  const double* neg_log_c;  // chain_log_table() on the device
+};
+
+// The chains of a target that nuts_chain.cu runs: models on the device, the
+// model of each chain (-1: evaluated by the batched path; NULL: model 0 for
+// every chain), the longest vector among them, and whether they are all.
+struct ChainModels {
+  const HierModel* models;
+  const int* model_of;
+  int max_dim;
+  bool all;
+};
+
 // A built-in model family: batched log-density + gradient over a dense batch.
 // Rows 0..n-1 of `q` (row stride ldq floats) are states; n is read on the
 // device from *n_dev (so samplers can compact active chains without a host
@@ -88,6 +108,8 @@ struct Target {
   virtual const int* ragged_dims() const { return nullptr; }
   virtual int64_t ragged_chains() const { return 0; }
   virtual int64_t ragged_elements() const { return 0; }
+  // Chains that run whole in one warp (nuts_chain.cu); nullptr: none.
+  virtual const ChainModels* chain_models() const { return nullptr; }
   // Ragged evaluation in place: the chains act_idx[0 .. *act_count) (sorted),
   // states and gradients at their element offsets, logp indexed by chain.
   virtual void eval_active(const float* q, const int* act_idx, const int* act_count,

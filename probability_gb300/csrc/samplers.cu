@@ -19,6 +19,8 @@
 #include <cstring>
 #include <vector>
 
+#include "nuts_chain.h"
+#include "nuts_layout.cuh"
 #include "rng.cuh"
 #include "samplers.h"
 
@@ -34,31 +36,11 @@ __device__ __forceinline__ int warp_id() {
   return (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
 }
 
-__device__ __forceinline__ float eps_of(const float* eps, int per_chain, int c) {
-  return per_chain ? eps[c] : eps[0];
-}
-
-// Layout helpers (uniform or ragged, see NutsDev).
-__device__ __forceinline__ size_t voff(const NutsDev& w, int c) {
-  return w.ragged ? (size_t)w.coff[c] : (size_t)c * w.D;
-}
-__device__ __forceinline__ int vdim(const NutsDev& w, int c) {
-  return w.ragged ? w.cdim[c] : w.D;
-}
-// Start of U-turn slot i of chain c.
-__device__ __forceinline__ size_t soff(const NutsDev& w, int c, int i) {
-  return w.ragged ? (size_t)w.coff[c] * w.slots + (size_t)i * w.cdim[c]
-                  : ((size_t)c * w.slots + i) * w.D;
-}
 // Start of chain c (at batch position j) in the gradient batch qw / gw.
 __device__ __forceinline__ size_t boff(const NutsDev& w, int c, int j) {
   return w.ragged ? (size_t)w.coff[c] : (size_t)j * w.D;
 }
 __device__ __forceinline__ int lwi(const NutsDev& w, int c, int j) { return w.ragged ? c : j; }
-// Inverse mass of element d of the chain whose vector starts at o (1: identity).
-__device__ __forceinline__ float imass(const NutsDev& w, size_t o, int d) {
-  return w.inv_mass ? (w.im_per_chain ? w.inv_mass[o + d] : w.inv_mass[d]) : 1.f;
-}
 
 // --------------------------------------------------------------------------
 // Active-chain compaction: idx[0..count) = chains with (flags & bit), sorted.
@@ -221,9 +203,14 @@ __device__ void nuts_chain_init(const NutsDev& w, int c, int lane, const float* 
 
 __global__ void nuts_init_kernel(NutsDev w, const float* __restrict__ q,
                                  const double* __restrict__ l, const float* __restrict__ g,
-                                 const float* __restrict__ eps_in, int eps_per_chain, uint2 key) {
+                                 const float* __restrict__ eps_in, int eps_per_chain, uint2 key,
+                                 const int* __restrict__ model_of) {
   const int c = warp_id(), lane = threadIdx.x & 31;
   if (c >= w.C) return;
+  if (model_of && model_of[c] >= 0) {
+    if (lane == 0) w.flags[c] = kElsewhere;
+    return;
+  }
   nuts_chain_init(w, c, lane, q, l, g, eps_of(eps_in, eps_per_chain, c), key);
 }
 
@@ -525,7 +512,7 @@ __device__ void nuts_chain_finalize(const NutsDev& w, int c, int lane, const Nut
 
 __global__ void nuts_finalize_kernel(NutsDev w, NutsOutputs out, int unrolled) {
   const int c = warp_id(), lane = threadIdx.x & 31;
-  if (c >= w.C) return;
+  if (c >= w.C || (w.flags[c] & kElsewhere)) return;
   nuts_chain_finalize(w, c, lane, out, unrolled);
 }
 
@@ -537,9 +524,14 @@ __global__ void nuts_finalize_kernel(NutsDev w, NutsOutputs out, int unrolled) {
 // --------------------------------------------------------------------------
 __global__ void nuts_free_start_kernel(NutsDev w, FreeDev f, const float* __restrict__ q,
                                       const double* __restrict__ l,
-                                      const float* __restrict__ g) {
+                                      const float* __restrict__ g,
+                                      const int* __restrict__ model_of) {
   const int c = warp_id(), lane = threadIdx.x & 31;
   if (c >= w.C) return;
+  if (model_of && model_of[c] >= 0) {
+    if (lane == 0) w.flags[c] = kElsewhere;
+    return;
+  }
   const size_t o = voff(w, c);
   const int D = vdim(w, c);
   for (int d = lane; d < D; d += 32) {
@@ -929,6 +921,15 @@ void nuts_setup(gbm_nuts* k) {
   w.flags = reinterpret_cast<uint8_t*>(base + off_b);
   w.eps = reinterpret_cast<float*>(base + off_e);
   GBM_CUDA(cudaMemsetAsync(base, 0, bytes, k->ctx->stream));
+  const size_t leaves = (size_t)1 << k->max_tree_depth;
+  std::vector<int> tab(3 * leaves + kMaxDepth, 0);
+  std::copy(k->write_instr.begin(), k->write_instr.end(), tab.begin());
+  std::copy(k->read_lo.begin(), k->read_lo.end(), tab.begin() + leaves);
+  std::copy(k->read_hi.begin(), k->read_hi.end(), tab.begin() + 2 * leaves);
+  k->tables.reserve(sizeof(int) * tab.size());
+  GBM_CUDA(cudaMemcpyAsync(k->tables.ptr, tab.data(), sizeof(int) * tab.size(),
+                           cudaMemcpyHostToDevice, k->ctx->stream));
+  GBM_CUDA(cudaStreamSynchronize(k->ctx->stream));   // tab is freed on return
   k->target_ws.reserve(k->target->impl->workspace_bytes(C));
   for (auto& ev : k->poll_events) GBM_CUDA(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
   k->key_dev.reserve(sizeof(uint2));
@@ -985,6 +986,30 @@ void nuts_profile_flush(gbm_nuts* k) {
   k->prof_used = 0;
 }
 
+// The chains that run whole in a warp (nuts_chain.cu), unless the caller wants
+// every batched gradient timed or several leapfrog steps per leaf.
+static const ChainModels* whole_chains(const gbm_nuts* k) {
+  if (k->profiling || k->unrolled_leapfrog_steps != 1) return nullptr;
+  return k->target->impl->chain_models();
+}
+
+static void set_tables(const gbm_nuts* k, FreeDev* f) {
+  const int leaves = 1 << k->max_tree_depth;
+  f->wtab = k->tables.as<int>();
+  f->rlo = f->wtab + leaves;
+  f->rhi = f->rlo + leaves;
+  f->max_depth = k->max_tree_depth;
+  f->max_energy_diff = k->max_energy_diff;
+}
+
+// Leaves of depth `depth` the batched loop launches when the longest subtree
+// has `most` leaves: batches of 8, ended by a count seen one batch late.
+static int64_t batched_leaves(int depth, int64_t most) {
+  if (most == 0) return 0;
+  const int64_t b = std::max<int64_t>(2, (most + 7) / 8 + 1);
+  return std::min<int64_t>((int64_t)1 << depth, 8 * b);
+}
+
 void nuts_one_step(gbm_nuts* k, int64_t chains, const float* q, const double* l, const float* g,
                    const float* eps, int eps_per_chain, uint2 key, const NutsOutputs& out) {
   gbm_context* ctx = k->target->ctx;
@@ -994,12 +1019,39 @@ void nuts_one_step(gbm_nuts* k, int64_t chains, const float* q, const double* l,
   w.inv_mass = k->inv_mass;
   w.im_per_chain = k->im_per_chain;
   int* host_flags = ctx->host_flags;
+  const ChainModels* cm = whole_chains(k);
+  int64_t per_depth[kMaxDepth] = {};   // leaves launched by the batched loop
+  if (cm) {
+    FreeDev f{};
+    set_tables(k, &f);
+    f.eps_in = eps;
+    f.eps_per_chain = eps_per_chain;
+    f.seed = key;
+    f.kmax = 1;
+    GBM_CUDA(cudaMemsetAsync(k->leaf_max(), 0, sizeof(int) * kMaxDepth, s));
+    nuts_chain_launch(w, f, *cm, q, l, g, &out, INT64_MAX, nullptr, k->leaf_max(), s);
+    k->prof_launches += 1;
+  }
+  // Leaf iterations are counted as the batched loop counts them: the longest
+  // subtree of each depth decides, whichever way its chain was run.
+  auto count_leaves = [&] {
+    k->leaf_count_pending = cm != nullptr;
+    k->last_leaf_iterations = 0;
+    for (int d = 0; d < k->max_tree_depth; ++d) {
+      k->leaves_per_depth[d] = per_depth[d];
+      k->last_leaf_iterations += per_depth[d];
+    }
+  };
+  if (cm && cm->all) {
+    count_leaves();
+    return;
+  }
   const int wb = warp_blocks(chains), tb = 256;
   const uint2* keyp = k->key_dev.as<uint2>();
   set_key_kernel<<<1, 1, 0, s>>>(k->key_dev.as<uint2>(), key);
-  nuts_init_kernel<<<wb, 32 * kWarpsPerBlock, 0, s>>>(w, q, l, g, eps, eps_per_chain, key);
+  nuts_init_kernel<<<wb, 32 * kWarpsPerBlock, 0, s>>>(w, q, l, g, eps, eps_per_chain, key,
+                                                      cm ? cm->model_of : nullptr);
   GBM_CUDA(cudaGetLastError());
-  k->last_leaf_iterations = 0;
   // One leaf: half kick + drift, gradient, final kick and tree bookkeeping,
   // then the next active list (on stream ls: the caller's, or the capture
   // stream while a graph is recorded).
@@ -1071,12 +1123,12 @@ void nuts_one_step(gbm_nuts* k, int64_t chains, const float* q, const double* l,
         k->prof_launches += (int64_t)nl * (2 + active_launches(w.C) +
                                            k->unrolled_leapfrog_steps * (
             k->target->impl->launches_per_eval(chains) + 1) - 1);
-        k->last_leaf_iterations += nl;
+        per_depth[depth] += nl;
         leaf += nl - 1;
         continue;
       }
       leaf_step(depth, leaf, false, s);
-      ++k->last_leaf_iterations;
+      ++per_depth[depth];
     }
     nuts_depth_end_kernel<<<wb, 32 * kWarpsPerBlock, 0, s>>>(w, key, depth);
     GBM_CUDA(cudaGetLastError());
@@ -1085,6 +1137,21 @@ void nuts_one_step(gbm_nuts* k, int64_t chains, const float* q, const double* l,
   nuts_finalize_kernel<<<wb, 32 * kWarpsPerBlock, 0, s>>>(w, out, k->unrolled_leapfrog_steps);
   GBM_CUDA(cudaGetLastError());
   k->prof_launches += 2;
+  count_leaves();
+}
+
+int64_t nuts_last_leaf_iterations(gbm_nuts* k) {
+  if (k->leaf_count_pending) {
+    int most[kMaxDepth];
+    cudaStream_t s = k->ctx->stream;
+    GBM_CUDA(cudaMemcpyAsync(most, k->leaf_max(), sizeof(most), cudaMemcpyDeviceToHost, s));
+    GBM_CUDA(cudaStreamSynchronize(s));
+    k->last_leaf_iterations = 0;
+    for (int d = 0; d < k->max_tree_depth; ++d)
+      k->last_leaf_iterations += std::max(k->leaves_per_depth[d], batched_leaves(d, most[d]));
+    k->leaf_count_pending = false;
+  }
+  return k->last_leaf_iterations;
 }
 
 int64_t nuts_run_free(gbm_nuts* k, int64_t chains, const float* q, const double* l,
@@ -1098,43 +1165,49 @@ int64_t nuts_run_free(gbm_nuts* k, int64_t chains, const float* q, const double*
   w.inv_mass = k->inv_mass;
   w.im_per_chain = k->im_per_chain;
   const int C = (int)chains;
-  const int leaves = 1 << k->max_tree_depth;
-  // Per-chain loop state and the leaf tables (device), carved from free_mem.
-  const size_t tab = ((size_t)leaves * 3 * sizeof(int) + 255) / 256 * 256;
-  const size_t per = ((size_t)C * (3 * sizeof(int) + sizeof(uint2) + 1) + 255) / 256 * 256;
-  if (k->free_mem.bytes < tab + per) {
-    GBM_CUDA(cudaStreamSynchronize(s));
-    k->free_mem.reserve(tab + per);
-  }
-  char* base = k->free_mem.as<char>();
-  int* tabs = reinterpret_cast<int*>(base);
-  std::vector<int> host_tab(3 * leaves);
-  std::copy(k->write_instr.begin(), k->write_instr.end(), host_tab.begin());
-  std::copy(k->read_lo.begin(), k->read_lo.end(), host_tab.begin() + leaves);
-  std::copy(k->read_hi.begin(), k->read_hi.end(), host_tab.begin() + 2 * leaves);
-  GBM_CUDA(cudaMemcpyAsync(tabs, host_tab.data(), sizeof(int) * 3 * leaves,
-                           cudaMemcpyHostToDevice, s));
-  GBM_CUDA(cudaStreamSynchronize(s));   // host_tab is freed on return
-  f.wtab = tabs;
-  f.rlo = tabs + leaves;
-  f.rhi = tabs + 2 * leaves;
-  char* pc = base + tab;
-  f.key = reinterpret_cast<uint2*>(pc);
-  f.t = reinterpret_cast<int*>(pc + sizeof(uint2) * C);
-  f.depth = f.t + C;
-  f.leaf = f.t + 2 * C;
-  f.phase = reinterpret_cast<uint8_t*>(f.t + 3 * C);
   f.eps_in = eps;
   f.eps_per_chain = eps_per_chain;
   f.seed = seed;
   f.first = first_step;
   f.kmax = kmax;
-  f.max_depth = k->max_tree_depth;
-  f.max_energy_diff = k->max_energy_diff;
+  set_tables(k, &f);
+  k->leaf_count_pending = false;
+  int* host_flags = ctx->host_flags;
+  const ChainModels* cm = whole_chains(k);
+  int64_t chain_iters = 0;   // iterations the batched loop would take for the whole chains
+  auto run_whole = [&](int32_t* done) {
+    GBM_CUDA(cudaMemsetAsync(k->leaf_max(), 0, sizeof(int), s));
+    nuts_chain_launch(w, f, *cm, q, l, g, nullptr, max_leaf_iterations, done, k->leaf_max(), s);
+    k->prof_launches += 1;
+    GBM_CUDA(cudaMemcpyAsync(host_flags, k->leaf_max(), sizeof(int), cudaMemcpyDeviceToHost, s));
+    GBM_CUDA(cudaStreamSynchronize(s));
+    // Batches of 8 iterations; the running count is read at the start of a
+    // batch's last iteration and seen one batch late.
+    chain_iters = std::min<int64_t>(8 * ((int64_t)host_flags[0] / 8 + 2), max_leaf_iterations);
+  };
+  if (cm && cm->all) {
+    run_whole(transitions_done);
+    k->last_leaf_iterations = chain_iters;
+    return chain_iters;
+  }
+  // Per-chain loop state, carved from free_mem.
+  const size_t per = (size_t)C * (3 * sizeof(int) + sizeof(uint2) + 1);
+  if (k->free_mem.bytes < per) {
+    GBM_CUDA(cudaStreamSynchronize(s));
+    k->free_mem.reserve(per);
+  }
+  char* pc = k->free_mem.as<char>();
+  f.key = reinterpret_cast<uint2*>(pc);
+  f.t = reinterpret_cast<int*>(pc + sizeof(uint2) * C);
+  f.depth = f.t + C;
+  f.leaf = f.t + 2 * C;
+  f.phase = reinterpret_cast<uint8_t*>(f.t + 3 * C);
   const int wb = warp_blocks(chains);
-  nuts_free_start_kernel<<<wb, 32 * kWarpsPerBlock, 0, s>>>(w, f, q, l, g);
+  nuts_free_start_kernel<<<wb, 32 * kWarpsPerBlock, 0, s>>>(w, f, q, l, g,
+                                                            cm ? cm->model_of : nullptr);
   GBM_CUDA(cudaGetLastError());
   k->prof_launches += 1;
+  if (cm) run_whole(f.t);
   auto iteration = [&](cudaStream_t ls, bool capturing) {
     build_active(w, kRunning, ls);
     nuts_free_prepare_kernel<<<wb, 32 * kWarpsPerBlock, 0, ls>>>(w, f);
@@ -1158,7 +1231,6 @@ int64_t nuts_run_free(gbm_nuts* k, int64_t chains, const float* q, const double*
     GBM_CUDA(cudaGraphInstantiate(&exec, graph, 0));
     GBM_CUDA(cudaGraphDestroy(graph));
   }
-  int* host_flags = ctx->host_flags;
   int64_t iters = 0;
   int64_t b = 0;
   try {
@@ -1198,8 +1270,8 @@ int64_t nuts_run_free(gbm_nuts* k, int64_t chains, const float* q, const double*
     nuts_free_done_kernel<<<(C + 255) / 256, 256, 0, s>>>(f, C, transitions_done);
     GBM_CUDA(cudaGetLastError());
   }
-  k->last_leaf_iterations = iters;
-  return iters;
+  k->last_leaf_iterations = std::max(iters, chain_iters);
+  return k->last_leaf_iterations;
 }
 
 void hmc_setup(gbm_hmc* k) {

@@ -18,6 +18,7 @@ enum ChainFlag : uint8_t {
   kSubNotDiv = 16,  // subtree-level not_divergence
   kForward = 32,    // direction of the current subtree
   kRunning = 64,    // free-running loop: the chain has transitions left
+  kElsewhere = 128, // nuts_chain.cu runs this chain: the batched kernels leave it alone
 };
 
 // Free-running NUTS (every chain at its own transition, depth and leaf):
@@ -54,6 +55,8 @@ struct FreeDev {
   int64_t mom_base;
   size_t tr_estride;        // state elements per transition
 };
+
+constexpr int kMaxDepth = 16;   // largest max_tree_depth
 
 // Device pointers of the NUTS workspace (passed to kernels by value).
 // Uniform layout: chain c's D-vector starts at c * D.  Ragged layout (many
@@ -159,6 +162,8 @@ struct gbm_hmc;
 
 namespace gbm {
 void nuts_setup(gbm_nuts* k);
+// Leaf iterations of the last transition or run (waits for it if need be).
+int64_t nuts_last_leaf_iterations(gbm_nuts* k);
 void nuts_one_step(gbm_nuts* k, int64_t chains, const float* q, const double* l, const float* g,
                    const float* eps, int eps_per_chain, uint2 key, const NutsOutputs& out);
 void hmc_setup(gbm_hmc* k);
@@ -221,7 +226,9 @@ struct gbm_nuts {
   cudaStream_t graph_stream = nullptr;   // capture stream (graphs launch on the caller's)
   std::map<int64_t, cudaGraphExec_t> graphs;   // (chains, depth, first leaf)
   gbm::DeviceBuffer key_dev;   // uint2
-  gbm::DeviceBuffer free_mem;  // free-running loop: per-chain state and leaf tables
+  gbm::DeviceBuffer free_mem;  // free-running loop: per-chain state
+  gbm::DeviceBuffer tables;    // write slot, read range per leaf (3 x 2^max_depth ints), then
+                               // leaf counts of whole-chain launches [kMaxDepth]
   // sample_chain runs the draws after adaptation (fixed step size, no
   // thinning) free-running: per chain the same transitions, without waiting
   // for the batch's longest trajectory.
@@ -230,6 +237,11 @@ struct gbm_nuts {
   int64_t graph_launches = 0;
   // Counters for the last transition (host-visible after one_step returns).
   int64_t last_leaf_iterations = 0;
+  // A whole-chain transition's count is on the device (leaf_max) until it is
+  // asked for; the batched loop's leaves per depth wait here.
+  bool leaf_count_pending = false;
+  int64_t leaves_per_depth[gbm::kMaxDepth] = {};
+  int* leaf_max() const { return tables.as<int>() + (size_t(3) << max_tree_depth); }
   // Optional profiling: CUDA events bracket every batched target evaluation.
   bool profiling = false;
   std::vector<cudaEvent_t> prof_events;  // pairs (start, end)

@@ -21,6 +21,7 @@
 #include <memory>
 
 #include "engine.h"
+#include "nuts_chain.h"
 
 namespace gbm {
 namespace {
@@ -204,8 +205,23 @@ class Hier final : public Target {
     GBM_CUDA(cudaMemcpyAsync(y_.ptr, y, sizeof(float) * J, cudaMemcpyDeviceToDevice, ctx->stream));
     GBM_CUDA(cudaMemcpyAsync(s_.ptr, sigma, sizeof(float) * J, cudaMemcpyDeviceToDevice,
                              ctx->stream));
+    if (dim <= kChainMaxDim) {
+      const std::vector<double> table = chain_log_table();
+      table_.reserve(sizeof(double) * table.size());
+      GBM_CUDA(cudaMemcpyAsync(table_.ptr, table.data(), sizeof(double) * table.size(),
+                               cudaMemcpyHostToDevice, ctx->stream));
+      const HierModel m{y_.as<float>(), s_.as<float>(), mu_scale,
+                        tau_scale,      const_term,     table_.as<double>()};
+      model_.reserve(sizeof(m));
+      GBM_CUDA(cudaMemcpyAsync(model_.ptr, &m, sizeof(m), cudaMemcpyHostToDevice, ctx->stream));
+      GBM_CUDA(cudaStreamSynchronize(ctx->stream));   // m, table are this call's
+      chain_models_ = ChainModels{model_.as<HierModel>(), nullptr, (int)dim, true};
+    }
   }
   size_t workspace_bytes(int64_t) const override { return 256; }
+  const ChainModels* chain_models() const override {
+    return model_.ptr ? &chain_models_ : nullptr;
+  }
   void eval(const float* q, int ldq, const int* n_dev, int cap, double* logp, float* grad,
             int ldg, void*, cudaStream_t s) override {
     hier_kernel<<<(cap + 7) / 8, 256, 0, s>>>(q, ldq, n_dev, (int)J_, y_.as<float>(),
@@ -221,7 +237,8 @@ class Hier final : public Target {
   int64_t J_;
   float mu_scale_, tau_scale_;
   double const_;
-  DeviceBuffer y_, s_;
+  DeviceBuffer y_, s_, model_, table_;
+  ChainModels chain_models_{};
 };
 
 }  // namespace

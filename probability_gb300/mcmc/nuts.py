@@ -59,6 +59,16 @@ def generate_efficient_write_read_instruction(instruction_array):
   return write, np.asarray(read)
 
 
+def last_leaf_iterations(handle):
+  """gbm_nuts_last_leaf_iterations of a sampler handle (None: 0)."""
+  if handle is None:
+    return 0
+  n = ctypes.c_int64()
+  _native.check(_native.lib().gbm_nuts_last_leaf_iterations(handle, ctypes.byref(n)),
+                'gbm_nuts_last_leaf_iterations')
+  return int(n.value)
+
+
 FreeRun = collections.namedtuple(
     'FreeRun', ['all_states', 'trace', 'transitions_done', 'leaf_iterations'])
 
@@ -76,8 +86,8 @@ def run_free(handle, q, kr, step_size, per_chain, seed, first_step, transitions_
   tr = dict(target_log_prob=torch.empty((K, C), dtype=torch.float64, device=dev),
             log_accept_ratio=torch.empty((K, C), dtype=torch.float64, device=dev),
             leapfrogs_taken=torch.zeros((K, C), dtype=torch.int32, device=dev),
-            is_accepted=torch.zeros((K, C), dtype=torch.uint8, device=dev),
-            has_divergence=torch.zeros((K, C), dtype=torch.uint8, device=dev))
+            is_accepted=torch.zeros((K, C), dtype=torch.bool, device=dev),
+            has_divergence=torch.zeros((K, C), dtype=torch.bool, device=dev))
   states = torch.empty((K, E), dtype=torch.float32, device=dev)
   done = torch.empty(C, dtype=torch.int32, device=dev)
   l0 = _util.as_tensor(kr.target_log_prob, torch.float64, dev).reshape(C).contiguous()
@@ -89,8 +99,6 @@ def run_free(handle, q, kr, step_size, per_chain, seed, first_step, transitions_
       int(first_step), K, int(max_leaf_iterations), P(done), P(states),
       P(tr['target_log_prob']), P(tr['log_accept_ratio']), P(tr['leapfrogs_taken']),
       P(tr['is_accepted']), P(tr['has_divergence']), ctypes.byref(iters)), 'gbm_nuts_run_free')
-  for k in ('is_accepted', 'has_divergence'):
-    tr[k] = tr[k].bool()
   return FreeRun(states.reshape((K,) + tuple(state_shape)), tr, done, int(iters.value))
 
 
@@ -118,7 +126,6 @@ class NoUTurnSampler(kernel_base.TransitionKernel):
         experimental_shard_axis_names=experimental_shard_axis_names, name=name)
     self._handle = None
     self._capacity = 0
-    self.last_leaf_iterations = 0
 
   target_log_prob_fn = property(lambda self: self._parameters['target_log_prob_fn'])
   step_size = property(lambda self: self._parameters['step_size'])
@@ -129,6 +136,11 @@ class NoUTurnSampler(kernel_base.TransitionKernel):
   name = property(lambda self: self._parameters['name'])
   write_instruction = property(lambda self: self._write_instruction)
   read_instruction = property(lambda self: self._read_instruction)
+
+  @property
+  def last_leaf_iterations(self):
+    """Leaf iterations of the last one_step or run_free (waits for it)."""
+    return last_leaf_iterations(self._handle)
 
   @property
   def is_calibrated(self):
@@ -165,23 +177,25 @@ class NoUTurnSampler(kernel_base.TransitionKernel):
     nq = torch.empty_like(q)
     ng = torch.empty_like(q)
     f64 = lambda: torch.empty(C, dtype=torch.float64, device=dev)
-    u8 = lambda: torch.empty(C, dtype=torch.uint8, device=dev)
+    flag = lambda: torch.empty(C, dtype=torch.bool, device=dev)   # the engine writes 0 / 1 bytes
     nl, lar, energy = f64(), f64(), f64()
     lf = torch.empty(C, dtype=torch.int32, device=dev)
-    acc, rmd, div = u8(), u8(), u8()
+    acc, rmd, div = flag(), flag(), flag()
     P = _native.ptr
     _native.check(_native.lib().gbm_nuts_one_step(
         self._handle, C, P(q), P(l0), P(g0), P(eps), per_chain, _native.seed_words(seed),
         P(nq), P(nl), P(ng), P(lar), P(lf), P(acc), P(rmd), P(div), P(energy), None),
         'gbm_nuts_one_step')
-    n = ctypes.c_int64()
-    _native.lib().gbm_nuts_last_leaf_iterations(self._handle, ctypes.byref(n))
-    self.last_leaf_iterations = int(n.value)
+    # The transition may still be running: a caller on another stream than the
+    # target's gets its buffers back only when it has ended.
+    ctx = self._target._ctx
+    if ctx.stream != torch.cuda.current_stream(dev):
+      ctx.synchronize()
     unflat = lambda t: _util.unflatten_state(t, layout, is_list)
     kr = NUTSKernelResults(
         target_log_prob=nl, grads_target_log_prob=unflat(ng), step_size=pkr.step_size,
-        log_accept_ratio=lar, leapfrogs_taken=lf, is_accepted=acc.bool(),
-        reach_max_depth=rmd.bool(), has_divergence=div.bool(), energy=energy,
+        log_accept_ratio=lar, leapfrogs_taken=lf, is_accepted=acc,
+        reach_max_depth=rmd, has_divergence=div, energy=energy,
         seed=_util.seed_tensor(seed))
     return unflat(nq), kr
 
@@ -203,7 +217,6 @@ class NoUTurnSampler(kernel_base.TransitionKernel):
     run = run_free(self._handle, q.contiguous().reshape(-1), kernel_results, eps.contiguous(),
                    per_chain, _util.sanitize_seed(seed), first_step, transitions_per_chain,
                    max_leaf_iterations, (C, D))
-    self.last_leaf_iterations = run.leaf_iterations
     return run
 
   def bootstrap_results(self, init_state):

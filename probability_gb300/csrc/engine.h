@@ -150,14 +150,9 @@ std::unique_ptr<Target> make_transformed(gbm_context* ctx, Target* inner, const 
 std::unique_ptr<Target> make_logreg_large(gbm_context* ctx, const void* X, int x_dtype, int64_t n,
                                           int64_t d, const float* y, float prior_scale,
                                           bool mixed);
-// FP32 target for up to 128 features on the CUDA cores (row-pair layout,
-// bulk-copied tiles): what make_logreg_f16 does not take.  nullptr above that.
+// FP32 target for up to 128 features (row-pair layout, bulk-copied tiles);
+// nullptr above that.
 std::unique_ptr<Target> make_logreg_f32(gbm_context* ctx, const float* X, int64_t n, int64_t d,
-                                        const float* y, float prior_scale);
-// FP32 target for up to 128 features and many rows on the tensor cores (exact
-// leading products of FP16 splits); nullptr outside that and for columns whose
-// range the splits cannot hold.
-std::unique_ptr<Target> make_logreg_f16(gbm_context* ctx, const float* X, int64_t n, int64_t d,
                                         const float* y, float prior_scale);
 std::unique_ptr<Target> make_logreg_simt(gbm_context* ctx, const float* X, int64_t n,
                                          int64_t d, const float* y, float prior_scale);

@@ -248,9 +248,8 @@ __device__ __forceinline__ void tmem_ld_wait() {
 }
 
 // ---- MMA ---------------------------------------------------------------------
-// D[tmem] (+)= A[smem] * B[smem], kind::f16 (the instruction descriptor names
-// FP16 or BF16 inputs), FP32 accumulate.
-__device__ __forceinline__ void mma_16bit(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc,
+// D[tmem] (+)= A[smem] * B[smem], kind::f16 (BF16 inputs), FP32 accumulate.
+__device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc,
                                          uint32_t idesc, uint32_t accumulate) {
   asm volatile(
       "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
@@ -259,10 +258,9 @@ __device__ __forceinline__ void mma_16bit(uint32_t d_tmem, uint64_t adesc, uint6
       : "memory");
 }
 
-// D[tmem] (+)= A[tmem] * B[smem], kind::f16 (the instruction descriptor names
-// FP16 or BF16 inputs), FP32 accumulate:
+// D[tmem] (+)= A[tmem] * B[smem], kind::f16 (BF16 inputs), FP32 accumulate:
 // A (M x K) lives in TMEM, row m in lane m, two K elements per 32-bit column.
-__device__ __forceinline__ void mma_16bit_tmem_a(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc,
+__device__ __forceinline__ void mma_bf16_tmem_a(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc,
                                                 uint32_t idesc, uint32_t accumulate) {
   asm volatile(
       "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
@@ -318,13 +316,6 @@ __device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t addr, uint32_t lbo,
 __host__ __device__ constexpr uint32_t idesc_bf16_f32(int M, int N, bool a_mn, bool b_mn) {
   return (1u << 4) | (1u << 7) | (1u << 10) | ((a_mn ? 1u : 0u) << 15) |
          ((b_mn ? 1u : 0u) << 16) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
-}
-
-// The same with FP16 (format 0) or BF16 operands.
-__host__ __device__ constexpr uint32_t idesc_16bit_f32(int M, int N, bool a_mn, bool b_mn,
-                                                       bool bf16) {
-  return bf16 ? idesc_bf16_f32(M, N, a_mn, b_mn)
-              : idesc_bf16_f32(M, N, a_mn, b_mn) & ~((1u << 7) | (1u << 10));
 }
 
 // Byte offset of element (row, col) of a 128-byte-swizzled atom stack whose

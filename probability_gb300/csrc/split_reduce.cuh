@@ -4,12 +4,19 @@
 // Layout written by the partial kernels: lpart[S][n] (float64) and
 // gpart[S][n][D] (float32), where S = number of row splits for n chains:
 //   S = clamp(grid / ceil(n / ct), 1, ceil(N / nt)).
-// One warp per chain: each lane owns features lane + 32k (D <= DMAX) and adds
-// the splits in index order, U splits' loads in flight at a time; the
-// log-density terms (likelihood partials, prior, linear part) are combined
-// per lane and summed by one float64 warp reduction.  The order depends only
-// on S and D, so results are reproducible.
+// One block per chain: a thread of each 128 owns features thread + 128 k and
+// adds up to kOrdered splits in index order, 16 loads in flight; with more
+// splits, groups of 128 threads add a range of them each and the ranges are
+// added in order.  The log-density terms (likelihood partials, prior, linear
+// part) are combined per lane by the first warp and summed by one float64 warp
+// reduction.  The order depends only on S, D and the launch, so results are
+// reproducible.
 //
+// What bounds it: the latency of the partials' loads (L2), so the loads of a
+// chain are spread over threads instead of over rounds of one warp.  Measured
+// with the partial kernel: 12,007 x 173 BF16, 77 chains (94 splits) 37.2 us with
+// a warp per chain, 28.7 so; a leapfrog step of 1000 x 25, 64 chains 40.8 and
+// 38.2; 1024 chains (19 splits) the same (four groups there: 10 us more).
 // `lin` (optional, float64 [D]) adds lin . q_c to each chain's log-density:
 // the tensor-core kernels leave the linear part sum_r (y_r - 1/2) z_rc of the
 // Bernoulli log-likelihood to this pass as (X^T (y - 1/2)) . q_c, exact in
@@ -17,11 +24,14 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <algorithm>
+
 #include "common.cuh"
 
 namespace gbm {
 
-constexpr int kReduceWarps = 4;            // chains per CTA
+constexpr int kOrdered = 32;               // splits one thread adds
+constexpr int kReduceGroups = 4;           // groups of 128 threads when there may be more
 
 // Chains of one launch.  A launch covers at most grid * ct chains (one work
 // item per CTA); larger batches are evaluated as consecutive chunks of
@@ -51,7 +61,7 @@ constexpr int64_t kMinSplitRows = 64;
 
 namespace {
 
-__device__ __forceinline__ int split_count(int n, int ct, int nt, int grid, int N) {
+__host__ __device__ __forceinline__ int split_count(int n, int ct, int nt, int grid, int N) {
   const int tiles = (n + ct - 1) / ct;
   if (tiles == 0) return 0;
   int s = grid / tiles;
@@ -60,85 +70,99 @@ __device__ __forceinline__ int split_count(int n, int ct, int nt, int grid, int 
   return s > row_tiles ? row_tiles : s;
 }
 
-template <int DMAX>
-__global__ void __launch_bounds__(32 * kReduceWarps)
+// Sum of p[s * stride], s in [s0, s1), in order.
+__device__ __forceinline__ float sum_splits(const float* __restrict__ p, size_t stride, int s0,
+                                            int s1) {
+  constexpr int U = 16;
+  float acc = 0.f;
+  int s = s0;
+  for (; s + U <= s1; s += U) {
+    float v[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) v[u] = p[(size_t)(s + u) * stride];
+#pragma unroll
+    for (int u = 0; u < U; ++u) acc += v[u];
+  }
+  if (s < s1) {
+    float v[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) v[u] = s + u < s1 ? p[(size_t)(s + u) * stride] : 0.f;
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (s + u < s1) acc += v[u];
+  }
+  return acc;
+}
+
+__global__ void __launch_bounds__(128 * kReduceGroups)
 split_reduce_kernel(const double* __restrict__ lpart, const float* __restrict__ gpart,
                     const float* __restrict__ Q, int ldq, const int* __restrict__ n_dev,
                     int c_base, int c_lim, int ct, int nt, int grid, int N, int D,
                     float inv_var, double log_norm, const double* __restrict__ lin,
                     double* __restrict__ logp, float* __restrict__ grad, int ldg) {
-  constexpr int kK = DMAX / 32;               // features per lane
-  constexpr int U = DMAX <= 128 ? 8 : 4;      // splits in flight
+  __shared__ float range[kReduceGroups - 1][512];
   const int n = chunk_count(*n_dev, c_base, c_lim);
-  const int c = blockIdx.x * kReduceWarps + (threadIdx.x >> 5);
+  const int c = blockIdx.x;
   if (c >= n) return;
-  const int lane = threadIdx.x & 31;
   const int S = split_count(n, ct, nt, grid, N);
-  const size_t sstride = (size_t)n * D;
+  const size_t stride = (size_t)n * D;
   const float* p = gpart + (size_t)c * D;
-  float acc[kK];
-#pragma unroll
-  for (int k = 0; k < kK; ++k) acc[k] = 0.f;
-  int s = 0;
-  for (; s + U <= S; s += U) {
-    float v[U][kK];
-#pragma unroll
-    for (int u = 0; u < U; ++u)
-#pragma unroll
-      for (int k = 0; k < kK; ++k) {
-        const int d = lane + 32 * k;
-        v[u][k] = d < D ? p[(size_t)(s + u) * sstride + d] : 0.f;
-      }
-#pragma unroll
-    for (int u = 0; u < U; ++u)
-#pragma unroll
-      for (int k = 0; k < kK; ++k) acc[k] += v[u][k];
-  }
-  for (; s < S; ++s)
-#pragma unroll
-    for (int k = 0; k < kK; ++k) {
-      const int d = lane + 32 * k;
-      if (d < D) acc[k] += p[(size_t)s * sstride + d];
+  const float* q = Q + (size_t)c * ldq;
+  const int groups = S <= kOrdered ? 1 : (int)(blockDim.x >> 7);
+  const int group = threadIdx.x >> 7, first = threadIdx.x & 127;
+  if (group > 0) {
+    if (groups > 1) {
+      const int s0 = group * S / groups, s1 = (group + 1) * S / groups;
+      for (int d = first; d < D; d += 128) range[group - 1][d] = sum_splits(p + d, stride, s0, s1);
+      __syncthreads();
     }
+    return;
+  }
+  const int s1 = groups > 1 ? S / groups : S;
+  float acc[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k)
+    if (first + 128 * k < D) acc[k] = sum_splits(p + first + 128 * k, stride, 0, s1);
+  if (groups > 1) {
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      if (first + 128 * k < D)
+        for (int g = 0; g + 1 < groups; ++g) acc[k] += range[g][first + 128 * k];
+  }
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const int d = first + 128 * k;
+    if (d < D) grad[(size_t)c * ldg + d] = acc[k] - q[d] * inv_var;
+  }
+  if (threadIdx.x >= 32) return;
   // Per-lane log-density terms: likelihood partials of splits lane, lane + 32,
-  // ..., then lin . q - q.q / (2 s^2) over this lane's features.
+  // ..., then lin . q - q.q / (2 s^2) over features lane, lane + 32, ...
+  const int lane = threadIdx.x;
   double t = 0.0;
   for (int j = lane; j < S; j += 32) t += lpart[(size_t)j * n + c];
   double pr = 0.0, li = 0.0;
-#pragma unroll
-  for (int k = 0; k < kK; ++k) {
-    const int d = lane + 32 * k;
-    if (d < D) {
-      const float q = Q[(size_t)c * ldq + d];
-      const double qd = (double)q;
-      pr += qd * qd;
-      if (lin) li += lin[d] * qd;
-      grad[(size_t)c * ldg + d] = acc[k] - q * inv_var;
-    }
+  for (int d = lane; d < D; d += 32) {
+    const double qd = (double)q[d];
+    pr += qd * qd;
+    if (lin) li += lin[d] * qd;
   }
   t = warp_sum(t + li - 0.5 * (double)inv_var * pr);
   if (lane == 0) logp[c] = t + (double)D * log_norm;
 }
 
 // Q, logp and grad point at chain c_base of the batch; `cap` bounds this
-// chunk's chains (<= c_lim).
+// chunk's chains (<= c_lim); D <= 512.
 void launch_split_reduce(const double* lpart, const float* gpart, const float* Q, int ldq,
                          const int* n_dev, int c_base, int c_lim, int cap, int ct, int nt,
                          int grid, int N, int D, float inv_var, double log_norm,
                          const double* lin, double* logp, float* grad, int ldg, cudaStream_t s) {
-  const unsigned blocks = (unsigned)((cap + kReduceWarps - 1) / kReduceWarps);
-  if (D <= 128)
-    split_reduce_kernel<128><<<blocks, 32 * kReduceWarps, 0, s>>>(
-        lpart, gpart, Q, ldq, n_dev, c_base, c_lim, ct, nt, grid, N, D, inv_var, log_norm, lin,
-        logp, grad, ldg);
-  else if (D <= 256)
-    split_reduce_kernel<256><<<blocks, 32 * kReduceWarps, 0, s>>>(
-        lpart, gpart, Q, ldq, n_dev, c_base, c_lim, ct, nt, grid, N, D, inv_var, log_norm, lin,
-        logp, grad, ldg);
-  else
-    split_reduce_kernel<512><<<blocks, 32 * kReduceWarps, 0, s>>>(
-        lpart, gpart, Q, ldq, n_dev, c_base, c_lim, ct, nt, grid, N, D, inv_var, log_norm, lin,
-        logp, grad, ldg);
+  // Few chains make many splits: several threads per feature.  (A sampler's
+  // active chains are fewer than cap; one thread then adds more than kOrdered.)
+  const int threads = split_count(cap, ct, nt, grid, N) <= kOrdered ? 128 : 128 * kReduceGroups;
+  split_reduce_kernel<<<(unsigned)cap, threads, 0, s>>>(
+      lpart, gpart, Q, ldq, n_dev, c_base, c_lim, ct, nt, grid, N, D, inv_var, log_norm, lin, logp,
+      grad, ldg);
   GBM_CUDA(cudaGetLastError());
 }
 

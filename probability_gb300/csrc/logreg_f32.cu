@@ -28,13 +28,30 @@
 // row tile is one contiguous block moved by one bulk copy (cp.async.bulk)
 // into a double-buffered shared-memory stage.  X is read from HBM once per
 // chain tile (L2 serves the other chain tiles of the same rows).
+//
+// From kTcMinRows rows on, phase 2 runs on the tensor cores instead
+// (logreg_f32_tc_kernel), beside phase 1 of the next tile: the residuals go to
+// shared memory as FP16 hi + lo (of R 2^15) and X is kept as FP16 hi + lo
+// (of each feature scaled to the top of FP16's range) beside its FP32 form,
+//   G^T = R_lo^T X_hi + R_hi^T X_lo + R_hi^T X_hi  (M = 128 chains, K = 64 rows).
+// hi + lo carries a float to 2^-24 of itself; what is left out (lo.lo) is as
+// small.  The tensor cores truncate every addition to their FP32 accumulator,
+// so a turn of at most two tiles starts from zero, the small terms of a tile
+// first, and is then added in FP32 to the sum of the turns before: gradient
+// error against 64 bits 1.4e-7 at 1e5 x 100 x 1024 chains (phase 2 on the CUDA
+// cores: 2.9e-7).  Z, and with it the log-density, is phase 1's, bit for bit.
+#include <cuda.h>
+#include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cmath>
 #include <memory>
+#include <vector>
 
 #include "engine.h"
 #include "split_reduce.cuh"
+#include "tc_common.cuh"
 #include "tc_ptx.cuh"
 
 namespace gbm {
@@ -78,6 +95,127 @@ __device__ __forceinline__ float4 lds4(const float* p) {
 __device__ __forceinline__ float neg_copysign_f(float w, float z) {
   return __int_as_float((__float_as_int(w) & 0x7fffffff) |
                         (~__float_as_int(z) & (int)0x80000000));
+}
+
+// Phase 1 of one thread: z[i][c] = x_i . B_c over dk features (even) for its
+// four rows (row pairs xa and xa + pair) and eight chains (bp and bp + 64), K
+// in order.
+__device__ __forceinline__ void f32_phase1(float (&z)[4][8], const float* xa, int pair,
+                                           const float* bp, int dk) {
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int c = 0; c < 8; ++c) z[i][c] = 0.f;
+  const float* xb = xa + pair;
+  // Register double buffering: the next feature pair's six loads are in
+  // flight while this pair's 64 FMAs issue (the last iteration re-reads
+  // its own pair instead of reading past the tile).
+  float4 u = lds4(xa), v = lds4(xb);   // x(r0,d) x(r1,d) x(r0,d+1) x(r1,d+1); rows r2, r3
+  float4 b0 = lds4(bp), b1 = lds4(bp + 64), b2 = lds4(bp + kF32CT), b3 = lds4(bp + kF32CT + 64);
+#pragma unroll 2
+  for (int d = 0; d < dk; d += 2) {
+    const int dn = d + 2 < dk ? d + 2 : d;
+    const float4 un = lds4(xa + 2 * dn), vn = lds4(xb + 2 * dn);
+    const float4 b0n = lds4(bp + dn * kF32CT), b1n = lds4(bp + dn * kF32CT + 64);
+    const float4 b2n = lds4(bp + (dn + 1) * kF32CT), b3n = lds4(bp + (dn + 1) * kF32CT + 64);
+    const float xr0[4] = {u.x, u.y, v.x, v.y};
+    const float xr1[4] = {u.z, u.w, v.z, v.w};
+    const float bb0[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
+    const float bb1[8] = {b2.x, b2.y, b2.z, b2.w, b3.x, b3.y, b3.z, b3.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int c = 0; c < 8; ++c) z[i][c] = fmaf(xr1[i], bb1[c], fmaf(xr0[i], bb0[c], z[i][c]));
+    u = un; v = vn; b0 = b0n; b1 = b1n; b2 = b2n; b3 = b3n;
+  }
+}
+
+// Phase 1 of one thread over NT row tiles (`tile` floats apart): its four rows
+// of each and eight chains, two chains to an instruction (fma.rn.f32x2: the
+// same roundings); z[4 t + i] are row i of tile t.  With two tiles a fragment of
+// B^T feeds 16 rows' worth of loads' FMAs: 107 FMAs a clock and SM where the
+// 4 x 8 tile above gets 79 (of 128; measured in a loop of nothing else).
+template <int NT>
+__device__ __forceinline__ void f32_phase1_pairs(float2 (&z)[8][4], const float* xp, int pair,
+                                                 int tile, const float* bp, int dk) {
+#pragma unroll
+  for (int i = 0; i < 4 * NT; ++i)
+#pragma unroll
+    for (int c = 0; c < 4; ++c) z[i][c] = make_float2(0.f, 0.f);
+  float4 u[2 * NT], b[4], un[2 * NT], bn[4];
+  auto load = [&](int d, float4(&x)[2 * NT], float4(&q)[4]) {
+#pragma unroll
+    for (int t = 0; t < NT; ++t) {
+      x[2 * t] = lds4(xp + t * tile + 2 * d);
+      x[2 * t + 1] = lds4(xp + t * tile + pair + 2 * d);
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) q[j] = lds4(bp + (d + (j >> 1)) * kF32CT + (j & 1) * 64);
+  };
+  load(0, u, b);
+#pragma unroll 2
+  for (int d = 0; d < dk; d += 2) {
+    load(d + 2 < dk ? d + 2 : d, un, bn);
+#pragma unroll
+    for (int k = 0; k < 2 * NT; ++k)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {      // row 2 k + h of this thread's
+        const float xa = h ? u[k].y : u[k].x, xb = h ? u[k].w : u[k].z;
+        float2(&zr)[4] = z[2 * k + h];
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          zr[2 * j] = __ffma2_rn(make_float2(xa, xa), make_float2(b[j].x, b[j].y), zr[2 * j]);
+          zr[2 * j + 1] =
+              __ffma2_rn(make_float2(xa, xa), make_float2(b[j].z, b[j].w), zr[2 * j + 1]);
+        }
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          zr[2 * j] =
+              __ffma2_rn(make_float2(xb, xb), make_float2(b[2 + j].x, b[2 + j].y), zr[2 * j]);
+          zr[2 * j + 1] = __ffma2_rn(make_float2(xb, xb), make_float2(b[2 + j].z, b[2 + j].w),
+                                     zr[2 * j + 1]);
+        }
+      }
+#pragma unroll
+    for (int k = 0; k < 2 * NT; ++k) u[k] = un[k];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) b[j] = bn[j];
+  }
+}
+
+// Epilogue of one thread: adds its rows' -(|z|/2 + ln(1 + e^-|z|)) to each
+// chain's Kahan sum and passes R of row i to `store`.
+template <class Store>
+__device__ __forceinline__ void f32_epilogue(const float (&z)[4][8], const float (&yr)[4],
+                                             int nvalid, float (&lsum)[8], float (&lcomp)[8],
+                                             Store&& store) {
+  float sabs[8], prod[8];
+#pragma unroll
+  for (int c = 0; c < 8; ++c) { sabs[c] = 0.f; prod[c] = 1.f; }
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    float r[8];
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+      const float a = fabsf(z[i][c]);
+      const float e = tc::ex2_approx(a * kNegLog2e);       // e^-|z|
+      const float u1 = 1.f + e;
+      if (i < nvalid) {
+        sabs[c] += a;
+        prod[c] *= u1;
+      }
+      const float w = tc::rcp_approx(u1) - 0.5f;          // sigmoid(|z|) - 1/2
+      r[c] = yr[i] + neg_copysign_f(w, z[i][c]);
+    }
+    store(i, r);
+  }
+#pragma unroll
+  for (int c = 0; c < 8; ++c) {   // Kahan: lsum += -(sabs / 2 + ln prod)
+    const float v = -fmaf(kLn2f, tc::lg2_approx(prod[c]), 0.5f * sabs[c]) - lcomp[c];
+    const float t = lsum[c] + v;
+    lcomp[c] = (t - lsum[c]) - v;
+    lsum[c] = t;
+  }
 }
 
 template <int KD>
@@ -153,67 +291,16 @@ logreg_f32_kernel(const float* __restrict__ X2, const float* __restrict__ ym, in
     const float* xs = Xs + st * (L::kXStage / 4);
     // ---- phase 1: Z = X_tile B^T ----
     float z[4][8];
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-      for (int c = 0; c < 8; ++c) z[i][c] = 0.f;
-    const float* xa = xs + (2 * ty) * Dp * 2;        // row pair 2 ty (rows 4 ty, 4 ty + 1)
-    const float* xb = xa + Dp * 2;                   // row pair 2 ty + 1
-    const float* bp = Bt + 4 * tx;
-    // Register double buffering: the next feature pair's six loads are in
-    // flight while this pair's 64 FMAs issue (the last iteration re-reads
-    // its own pair instead of reading past the tile).
-    float4 u = lds4(xa), v = lds4(xb);   // x(r0,d) x(r1,d) x(r0,d+1) x(r1,d+1); rows r2, r3
-    float4 b0 = lds4(bp), b1 = lds4(bp + 64), b2 = lds4(bp + kF32CT), b3 = lds4(bp + kF32CT + 64);
-#pragma unroll 2
-    for (int d = 0; d < dk; d += 2) {
-      const int dn = d + 2 < dk ? d + 2 : d;
-      const float4 un = lds4(xa + 2 * dn), vn = lds4(xb + 2 * dn);
-      const float4 b0n = lds4(bp + dn * kF32CT), b1n = lds4(bp + dn * kF32CT + 64);
-      const float4 b2n = lds4(bp + (dn + 1) * kF32CT), b3n = lds4(bp + (dn + 1) * kF32CT + 64);
-      const float xr0[4] = {u.x, u.y, v.x, v.y};
-      const float xr1[4] = {u.z, u.w, v.z, v.w};
-      const float bb0[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
-      const float bb1[8] = {b2.x, b2.y, b2.z, b2.w, b3.x, b3.y, b3.z, b3.w};
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int c = 0; c < 8; ++c) z[i][c] = fmaf(xr1[i], bb1[c], fmaf(xr0[i], bb0[c], z[i][c]));
-      u = un; v = vn; b0 = b0n; b1 = b1n; b2 = b2n; b3 = b3n;
-    }
+    f32_phase1(z, xs + (2 * ty) * Dp * 2, Dp * 2, Bt + 4 * tx, dk);
     // ---- epilogue: log-likelihood sums and R ----
     const float4 yv = lds4(Ys + st * kF32RT + 4 * ty);
     const float yr[4] = {yv.x, yv.y, yv.z, yv.w};
     const int nvalid = N - (rt_begin + it) * kF32RT - 4 * ty;   // rows of mine that exist
-    float sabs[8], prod[8];
-#pragma unroll
-    for (int c = 0; c < 8; ++c) { sabs[c] = 0.f; prod[c] = 1.f; }
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      float r[8];
-#pragma unroll
-      for (int c = 0; c < 8; ++c) {
-        const float a = fabsf(z[i][c]);
-        const float e = tc::ex2_approx(a * kNegLog2e);       // e^-|z|
-        const float u1 = 1.f + e;
-        if (i < nvalid) {
-          sabs[c] += a;
-          prod[c] *= u1;
-        }
-        const float w = tc::rcp_approx(u1) - 0.5f;          // sigmoid(|z|) - 1/2
-        r[c] = yr[i] + neg_copysign_f(w, z[i][c]);
-      }
+    f32_epilogue(z, yr, nvalid, lsum, lcomp, [&](int i, const float(&r)[8]) {
       float* rrow = Rs + (4 * ty + i) * kF32CT;
       *reinterpret_cast<float4*>(rrow + 4 * tx) = make_float4(r[0], r[1], r[2], r[3]);
       *reinterpret_cast<float4*>(rrow + 64 + 4 * tx) = make_float4(r[4], r[5], r[6], r[7]);
-    }
-#pragma unroll
-    for (int c = 0; c < 8; ++c) {   // Kahan: lsum += -(sabs / 2 + ln prod)
-      const float v = -fmaf(kLn2f, tc::lg2_approx(prod[c]), 0.5f * sabs[c]) - lcomp[c];
-      const float t = lsum[c] + v;
-      lcomp[c] = (t - lsum[c]) - v;
-      lsum[c] = t;
-    }
+    });
     if (__syncthreads_or(!ok)) {   // R complete (and every thread's wait succeeded)
       failed = true;
       break;
@@ -290,6 +377,359 @@ logreg_f32_kernel(const float* __restrict__ X2, const float* __restrict__ ym, in
   }
 }
 
+// ---------------------------------------------------------------------------
+// Phase 2 on the tensor cores (see the head of this file).
+//
+// Two groups of four warps, a warp of each on every SM quarter, take the upper
+// and the lower 32 rows of each tile, and have their own stages, accumulators
+// and a service warp that loads their rows and issues their MMAs.  A group runs
+// phase 1 over the rows of two tiles (8 rows x 8 chains a thread), then the two
+// epilogues, while its next rows load and its MMAs (6 a tile) run.  Group 1
+// begins with a single tile, so that the groups are half a turn apart and one's
+// epilogue (MUFU and issue) fills what the other's phase 1 (FMA pipe) leaves.
+//
+// What bounds it: the FMA pipe in phase 1, half of the kernel (107 of 128 FMAs a
+// clock and SM), and the issue of the epilogues.  An evaluation at 1e5 rows, 1024
+// chains: 523 us at 100 features (both phases on the CUDA cores: 849; this
+// kernel with one group of eight warps, epilogues together: 547), 221 at 25
+// (344), 54 at 4 and 256 chains (72).
+// ---------------------------------------------------------------------------
+constexpr int kF32TcThreads = kF32Threads + 64;
+constexpr float kF16Scale = 32768.f;        // R' = 2^15 R
+constexpr int kF16Top = 14;                 // X' = X 2^(kF16Top - fexp) < 2^15
+constexpr int kHalf = kF32RT / 2;           // rows of a tile in each group
+constexpr int kRBox = kHalf * 128;          // [32 rows][128 B]: 64 chains
+constexpr int kXBox = 2 * kRBox;            // [2 tiles][32 rows][128 B]: 64 features
+
+template <int KD>
+struct F32TcLayout {
+  static constexpr int kDp = 16 * KD;
+  static constexpr int kNkb = (KD + 3) / 4;                  // 64-feature blocks
+  static constexpr int kGCols = KD <= 2 ? 32 : KD <= 4 ? 64 : 128;
+  static constexpr int kX16Group = 2 * kNkb * kXBox;         // hi, lo
+  static constexpr int kR16Group = 4 * kRBox;                // hi, lo of 2 x 64 chains
+  static constexpr int kXHalf = kHalf * kDp * 4;             // X2 of a tile's rows of a group
+  static constexpr int kX16 = 0;                              // [group]
+  static constexpr int kR16 = kX16 + 2 * kX16Group;           // [group]
+  static constexpr int kBt = kR16 + 2 * kR16Group;            // [Dp][128] float
+  static constexpr int kX = kBt + kDp * kF32CT * 4;           // [group][2 tiles]
+  static constexpr int kY = kX + 4 * kXHalf;                  // [group][2 tiles][32] float
+  static constexpr int kCtl = kY + 2 * kF32RT * 4;
+  static constexpr int kBytes = kCtl + 256 + 1024;
+  // After the loop: log-likelihood sums over R, the gradient tile over B^T and X2.
+  static_assert(16 * kF32CT * 8 <= 2 * kR16Group, "reduction scratch fits R");
+  static_assert(kF32CT * (kDp + 1) * 4 <= kY - kBt, "gradient tile fits B^T and X2");
+  static_assert(kBytes <= 232448, "shared memory over the sm_103a limit");
+};
+
+struct F32TcBars {
+  struct Group {
+    uint64_t x_full, x_free, x16_full, r_full, mma_done;
+  } group[2];
+};
+
+// Tiles of turn j of a group: [first, first + count).
+__device__ __forceinline__ int turn_first(int group, int j) {
+  return group == 0 || j == 0 ? 2 * j : 2 * j - 1;
+}
+__device__ __forceinline__ int turn_count(int group, int j, int T) {
+  const int left = T - turn_first(group, j);
+  const int most = group == 1 && j == 0 ? 1 : 2;
+  return left < most ? left : most;
+}
+
+template <int KD>
+__global__ void __launch_bounds__(kF32TcThreads, 1)
+logreg_f32_tc_kernel(const __grid_constant__ CUtensorMap himap,
+                     const __grid_constant__ CUtensorMap lomap, const float* __restrict__ X2,
+                     const float* __restrict__ ym, const float* __restrict__ gscale, int N, int D,
+                     const float* __restrict__ Q, int ldq, const int* __restrict__ n_dev,
+                     int c_base, int c_lim, int grid, double* __restrict__ lpart,
+                     float* __restrict__ gpart, int* __restrict__ err) {
+  using L = F32TcLayout<KD>;
+  constexpr int Dp = L::kDp;
+  extern __shared__ __align__(1024) unsigned char smem_raw[];
+  unsigned char* smem = reinterpret_cast<unsigned char*>(
+      (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  const int n = chunk_count(*n_dev, c_base, c_lim);
+  const int row_tiles = (N + kF32RT - 1) / kF32RT;
+  const int S = f32_splits(n, grid, row_tiles);
+  const int tiles = (n + kF32CT - 1) / kF32CT;
+  if (S == 0 || (int)blockIdx.x >= tiles * S) return;
+  const int tile = blockIdx.x % tiles, split = blockIdx.x / tiles;
+  const int c0 = tile * kF32CT;
+  const int rt_begin = (int)((long long)split * row_tiles / S);
+  const int rt_end = (int)((long long)(split + 1) * row_tiles / S);
+  const int T = rt_end - rt_begin;
+
+  float* Bt = reinterpret_cast<float*>(smem + L::kBt);
+  F32TcBars* all = reinterpret_cast<F32TcBars*>(smem + L::kCtl);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + L::kCtl + sizeof(F32TcBars));
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int group = warp < 8 ? warp >> 2 : warp - 8;
+  F32TcBars::Group* bars = &all->group[group];
+  unsigned char* X16 = smem + L::kX16 + group * L::kX16Group;
+  unsigned char* R16 = smem + L::kR16 + group * L::kR16Group;
+  float* Xs = reinterpret_cast<float*>(smem + L::kX + group * 2 * L::kXHalf);
+  float* Ys = reinterpret_cast<float*>(smem + L::kY) + group * kF32RT;
+  if (tid == 0) {
+    for (int i = 0; i < 2; ++i) {
+      F32TcBars::Group& b = all->group[i];
+      tc::mbar_init(&b.x_full, 1);
+      tc::mbar_init(&b.x_free, 4);
+      tc::mbar_init(&b.x16_full, 1);
+      tc::mbar_init(&b.r_full, 4);
+      tc::mbar_init(&b.mma_done, 1);
+    }
+    *abort_flag = 0;
+    tc::fence_mbar_init();
+  }
+  // TMEM: G of a group's turn (two groups), then the groups' sums.
+  if (warp == 8) tc::tmem_alloc(tmem_slot, 4 * L::kGCols);
+  // Chain states, transposed: Bt[d][c] = Q[c0 + c][d], zero outside (n, D).
+  // Lanes run over chains: conflict-free stores, and a row of Q stays in L1.
+  for (int i = tid; i < Dp * kF32CT; i += kF32TcThreads) {
+    const int c = i & (kF32CT - 1), d = i / kF32CT;
+    Bt[i] = (c0 + c < n && d < D) ? Q[(size_t)(c0 + c) * ldq + d] : 0.f;
+  }
+  tc::tc_fence_before();
+  __syncthreads();
+  tc::tc_fence_after();
+  const uint32_t tmem = *tmem_slot;
+  const uint32_t tg = tmem + group * L::kGCols, tsum = tmem + (2 + group) * L::kGCols;
+
+  if (warp >= 8) {
+    // ---------------- a group's loads and MMAs ----------------
+    if (lane == 0) {
+      // A turn's rows: 32 of each tile, X2 and y, and the FP16 form.
+      auto load_x = [&](int j) {
+        const int first = turn_first(group, j), count = turn_count(group, j, T);
+        tc::mbar_arrive_expect_tx(&bars->x_full, (uint32_t)(count * (L::kXHalf + kHalf * 4)));
+        for (int t = 0; t < count; ++t) {
+          const size_t r0 = (size_t)(rt_begin + first + t) * kF32RT + group * kHalf;
+          tc::bulk_load(Xs + t * (L::kXHalf / 4), X2 + r0 * Dp, (uint32_t)L::kXHalf, &bars->x_full);
+          tc::bulk_load(Ys + t * kHalf, ym + r0, (uint32_t)(kHalf * 4), &bars->x_full);
+        }
+      };
+      auto load_x16 = [&](int j) {
+        const int first = turn_first(group, j), count = turn_count(group, j, T);
+        tc::mbar_arrive_expect_tx(&bars->x16_full, (uint32_t)(count * 2 * L::kNkb * kRBox));
+        for (int t = 0; t < count; ++t) {
+          const int r0 = (rt_begin + first + t) * kF32RT + group * kHalf;
+#pragma unroll
+          for (int kb = 0; kb < L::kNkb; ++kb) {
+            tc::tma_load_2d(X16 + kb * kXBox + t * kRBox, &himap, kb * 64, r0, &bars->x16_full);
+            tc::tma_load_2d(X16 + (L::kNkb + kb) * kXBox + t * kRBox, &lomap, kb * 64, r0,
+                            &bars->x16_full);
+          }
+        }
+      };
+      if (T > 0) {
+        load_x(0);
+        load_x16(0);
+      }
+      int nx = T > 0, nx16 = nx;      // turns whose loads were issued
+      constexpr uint32_t idesc = tc::idesc_16bit_f32(128, Dp, true, true, false);
+      const uint64_t rd = tc::smem_desc_sw128(tc::smem_u32(R16), kRBox, 1024);
+      const uint64_t xd = tc::smem_desc_sw128(tc::smem_u32(X16), kXBox, 1024);
+      constexpr uint64_t kRlo = 2 * kRBox >> 4, kXlo = L::kNkb * kXBox >> 4;
+      bool ok = true;
+      int it = 0;
+      for (int j = 0; ok && turn_first(group, j) < T; ++j) {
+        const int count = turn_count(group, j, T);
+        const bool more = turn_first(group, j + 1) < T;
+        // Phase 1 of the turn is done: the next rows load during its epilogue.
+        if (more) {
+          ok = wait_or_abort(&bars->x_free, (uint32_t)j & 1, abort_flag);
+          if (!ok) break;
+          load_x(nx++);
+        }
+        ok = wait_or_abort(&bars->x16_full, (uint32_t)j & 1, abort_flag);
+        for (int t = 0; ok && t < count; ++t, ++it) {
+          ok = wait_or_abort(&bars->r_full, (uint32_t)it & 1, abort_flag);
+          if (!ok) break;
+          tc::tc_fence_after();
+          const uint64_t xt = xd + (uint64_t)((t * kRBox) >> 4);
+#pragma unroll
+          for (int ks = 0; ks < kHalf / 16; ++ks) {
+            const uint64_t o = (uint64_t)((ks * 2048) >> 4);
+            tc::mma_16bit(tg, rd + kRlo + o, xt + o, idesc, t > 0 || ks > 0 ? 1u : 0u);
+            tc::mma_16bit(tg, rd + o, xt + kXlo + o, idesc, 1u);
+          }
+#pragma unroll
+          for (int ks = 0; ks < kHalf / 16; ++ks) {
+            const uint64_t o = (uint64_t)((ks * 2048) >> 4);
+            tc::mma_16bit(tg, rd + o, xt + o, idesc, 1u);
+          }
+          tc::mma_commit(&bars->mma_done);
+        }
+        if (ok && more) {
+          ok = wait_or_abort(&bars->mma_done, (uint32_t)(it - 1) & 1, abort_flag);
+          if (ok) load_x16(nx16++);
+        }
+      }
+      if (!ok) {
+        tc::record_error(err, kF32TimeoutCode);
+        *abort_flag = 1;
+        // Let the MMAs and the copies still in flight end before the CTA exits.
+        if (it > 0) tc::mbar_wait(&bars->mma_done, (uint32_t)(it - 1) & 1, kWaitLimitNs);
+        if (nx > 0) tc::mbar_wait(&bars->x_full, (uint32_t)(nx - 1) & 1, kWaitLimitNs);
+        if (nx16 > 0) tc::mbar_wait(&bars->x16_full, (uint32_t)(nx16 - 1) & 1, kWaitLimitNs);
+      }
+    }
+    __syncwarp();
+  } else {
+    const int ty = tid >> 4, tx = tid & 15;   // rows 4 ty.., chains 4 tx.., 64 + 4 tx..
+    const int gy = ty & 7;                    // ty within the group
+    const int dk = (D + 1) & ~1;              // K extent of phase 1 (B^T rows >= D are zero)
+    const uint32_t quarter = (uint32_t)((warp & 3) * 32) << 16;
+    // Per chain: Kahan sum over tiles of -(sum |z|/2 + sum ln(1 + e^-|z|)).
+    float lsum[8], lcomp[8];
+#pragma unroll
+    for (int c = 0; c < 8; ++c) lsum[c] = lcomp[c] = 0.f;
+    bool ok = true, summed = false;
+    // Adds G of a turn to the sum of the turns before, which is kept in TMEM
+    // beside it: the registers for it would not be left.
+    auto drain = [&]() {
+      tc::tc_fence_after();
+#pragma unroll
+      for (int j = 0; j < 2 * KD; ++j) {
+        float v[8], sum[8];
+        tc::tmem_ld8(tg + quarter + 8 * j, v);
+        if (summed) tc::tmem_ld8(tsum + quarter + 8 * j, sum);
+        tc::tmem_ld_wait();
+        if (summed) {
+#pragma unroll
+          for (int e = 0; e < 8; ++e) v[e] += sum[e];
+        }
+        tc::tmem_st8(tsum + quarter + 8 * j, v);
+      }
+      tc::tmem_st_wait();
+      tc::tc_fence_before();
+      summed = true;
+    };
+    for (int j = 0; turn_first(group, j) < T && ok; ++j) {
+      const int first = turn_first(group, j), count = turn_count(group, j, T);
+      if (!warp_wait(&bars->x_full, (uint32_t)j & 1, abort_flag)) {
+        ok = false;
+        break;
+      }
+      // ---- phase 1: Z = X_tile B^T of the turn's tiles ----
+      float2 z[8][4];
+      const float* xp = Xs + (2 * gy) * Dp * 2;
+      if (count == 2)
+        f32_phase1_pairs<2>(z, xp, Dp * 2, L::kXHalf / 4, Bt + 4 * tx, dk);
+      else
+        f32_phase1_pairs<1>(z, xp, Dp * 2, L::kXHalf / 4, Bt + 4 * tx, dk);
+      float4 yv[2];
+      yv[0] = lds4(Ys + 4 * gy);
+      yv[1] = lds4(Ys + kHalf + 4 * gy);
+      __syncwarp();
+      if (lane == 0) tc::mbar_arrive(&bars->x_free);
+#pragma unroll
+      for (int t = 0; t < 2; ++t) {
+        const int it = first + t;
+        if (t == 1 && count == 1) break;
+        // The MMAs of the tile before are done: R is free, and with a new turn
+        // G of the last one is complete.
+        if (it > 0) {
+          if (!warp_wait(&bars->mma_done, (uint32_t)(it - 1) & 1, abort_flag)) {
+            ok = false;
+            break;
+          }
+          if (t == 0) drain();
+        }
+        // ---- epilogue: log-likelihood sums, R' in FP16 hi + lo ----
+        float zt[4][8];
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            zt[i][2 * c] = z[4 * t + i][c].x;
+            zt[i][2 * c + 1] = z[4 * t + i][c].y;
+          }
+        const float yr[4] = {yv[t].x, yv[t].y, yv[t].z, yv[t].w};
+        const int nvalid = N - (rt_begin + it) * kF32RT - 4 * ty;   // rows of mine that exist
+        f32_epilogue(zt, yr, nvalid, lsum, lcomp, [&](int i, const float(&r)[8]) {
+          const uint32_t off = tc::sw128_offset(4 * gy + i, 4 * tx);
+#pragma unroll
+          for (int b = 0; b < 2; ++b) {
+            uint32_t hi[2], lo[2];
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+              const float v0 = r[4 * b + 2 * e] * kF16Scale, v1 = r[4 * b + 2 * e + 1] * kF16Scale;
+              const __half2 h = __floats2half2_rn(v0, v1);
+              const float2 hf = __half22float2(h);
+              const __half2 l = __floats2half2_rn(v0 - hf.x, v1 - hf.y);
+              hi[e] = *reinterpret_cast<const uint32_t*>(&h);
+              lo[e] = *reinterpret_cast<const uint32_t*>(&l);
+            }
+            *reinterpret_cast<uint2*>(R16 + b * kRBox + off) = make_uint2(hi[0], hi[1]);
+            *reinterpret_cast<uint2*>(R16 + (2 + b) * kRBox + off) = make_uint2(lo[0], lo[1]);
+          }
+        });
+        tc::fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) tc::mbar_arrive(&bars->r_full);
+      }
+    }
+    if (ok && T > 0) {
+      ok = warp_wait(&bars->mma_done, (uint32_t)(T - 1) & 1, abort_flag);
+      if (ok) drain();
+    }
+    if (!ok) {
+      tc::record_error(err, kF32TimeoutCode);
+      *abort_flag = 1;
+    }
+    // Every warp is past its last read of B^T, X2 and R (or has given up), and
+    // both groups' sums are complete.
+    named_barrier(1, kF32Threads);
+    const bool good = *abort_flag == 0;
+    if (good) {
+      tc::tc_fence_after();
+      double* red = reinterpret_cast<double*>(smem + L::kR16);    // [16][128]
+#pragma unroll
+      for (int c = 0; c < 8; ++c) {
+        const int cc = c < 4 ? 4 * tx + c : 64 + 4 * tx + (c - 4);
+        red[ty * kF32CT + cc] = (double)lsum[c] - (double)lcomp[c];
+      }
+      // This group's half of the features of its lanes' chains.
+      const int gc = (warp & 3) * 32 + lane, gf = group * 8 * KD;
+#pragma unroll
+      for (int j = 0; j < KD; ++j) {
+        float v0[8], v1[8];
+        tc::tmem_ld8(tmem + 2 * L::kGCols + quarter + gf + 8 * j, v0);
+        tc::tmem_ld8(tmem + 3 * L::kGCols + quarter + gf + 8 * j, v1);
+        tc::tmem_ld_wait();
+#pragma unroll
+        for (int e = 0; e < 8; ++e) Bt[gc * (Dp + 1) + gf + 8 * j + e] = v0[e] + v1[e];
+      }
+    }
+    named_barrier(1, kF32Threads);
+    if (good) {
+      const double* red = reinterpret_cast<const double*>(smem + L::kR16);
+      if (tid < kF32CT && c0 + tid < n) {
+        double s = 0.0;
+#pragma unroll
+        for (int t = 0; t < 16; ++t) s += red[t * kF32CT + tid];
+        lpart[(size_t)split * n + c0 + tid] = s;
+      }
+      for (int cc = warp; cc < kF32CT; cc += kF32Threads / 32) {
+        if (c0 + cc >= n) break;
+        float* dst = gpart + ((size_t)split * n + c0 + cc) * D;
+        for (int d = lane; d < D; d += 32) dst[d] = Bt[cc * (Dp + 1) + d] * gscale[d];
+      }
+    }
+  }
+  tc::tc_fence_before();
+  __syncthreads();
+  if (warp == 8) {
+    tc::tc_fence_after();
+    tc::tmem_dealloc(tmem, 4 * L::kGCols);
+  }
+}
+
 // X [N][D] -> X2 [N2/2][Dp][2] (row pairs, zero padding) and ym = y - 1/2
 // (zero past N), N2 = N rounded up to whole row tiles.
 __global__ void f32_pack_kernel(const float* __restrict__ X, const float* __restrict__ y,
@@ -303,6 +743,71 @@ __global__ void f32_pack_kernel(const float* __restrict__ X, const float* __rest
   X2[((r >> 1) * Dp + d) * 2 + (r & 1)] = (r < N && d < D) ? X[r * D + d] : 0.f;
 }
 
+// ---- FP16 form of X ----
+__device__ __forceinline__ int float_exponent(unsigned bits) {
+  return (int)((bits >> 23) & 255u) - 127;
+}
+
+// Largest |x| of each column, as bits.
+__global__ void column_max_kernel(const float* __restrict__ X, int64_t N, int D, int64_t chunk,
+                                  unsigned* __restrict__ out) {
+  const int64_t r0 = (int64_t)blockIdx.x * chunk, r1 = r0 + chunk < N ? r0 + chunk : N;
+  for (int d = threadIdx.x; d < D; d += blockDim.x) {
+    unsigned m = 0;
+#pragma unroll 8
+    for (int64_t r = r0; r < r1; ++r) m = max(m, __float_as_uint(X[r * D + d]) & 0x7fffffffu);
+    if (m) atomicMax(&out[d], m);
+  }
+}
+
+// X [N][D] -> X' = X 2^(kF16Top - exponent of the column's largest) as FP16 hi
+// + lo [N][Dp], zero-padded; rows [b chunk, (b + 1) chunk) also sum X'^2 and
+// the square of what hi + lo leaves of it into part[b][d].
+__global__ void f16_pack_kernel(const float* __restrict__ X, int64_t N, int D, int Dp,
+                                int64_t chunk, const unsigned* __restrict__ max_bits,
+                                __half* __restrict__ hi, __half* __restrict__ lo,
+                                float2* __restrict__ part) {
+  const int64_t r0 = (int64_t)blockIdx.x * chunk, r1 = r0 + chunk < N ? r0 + chunk : N;
+  for (int d = threadIdx.x; d < Dp; d += blockDim.x) {
+    const int shift = d < D ? kF16Top - float_exponent(max_bits[d]) : 0;
+    float2 acc = make_float2(0.f, 0.f);
+#pragma unroll 4
+    for (int64_t r = r0; r < r1; ++r) {
+      const float v = d < D ? ldexpf(X[r * D + d], shift) : 0.f;
+      const __half h = __float2half_rn(v);
+      const float rest = v - __half2float(h);
+      const __half l = __float2half_rn(rest);
+      hi[r * Dp + d] = h;
+      lo[r * Dp + d] = l;
+      const float left = rest - __half2float(l);
+      acc.x = fmaf(v, v, acc.x);
+      acc.y = fmaf(left, left, acc.y);
+    }
+    if (d < D) part[(size_t)blockIdx.x * D + d] = acc;
+  }
+}
+
+// Sums of part over blocks: one block per feature, fixed order.
+__global__ void __launch_bounds__(128)
+column_rest_kernel(const float2* __restrict__ part, int nb, int D, double2* __restrict__ out) {
+  __shared__ double2 sh[128];
+  const int d = blockIdx.x, tid = threadIdx.x;
+  double2 acc = make_double2(0.0, 0.0);
+  for (int b = tid; b < nb; b += 128) {
+    acc.x += (double)part[(size_t)b * D + d].x;
+    acc.y += (double)part[(size_t)b * D + d].y;
+  }
+  sh[tid] = acc;
+  for (int o = 64; o > 0; o >>= 1) {
+    __syncthreads();
+    if (tid < o) {
+      sh[tid].x += sh[tid + o].x;
+      sh[tid].y += sh[tid + o].y;
+    }
+  }
+  if (tid == 0) out[d] = sh[0];
+}
+
 // lin[d] = sum_r (y_r - 1/2) X[r][d] in float64 and a fixed order: block b
 // sums rows [b chunk, (b + 1) chunk) into part[b][d]; blocks added in order.
 __global__ void f32_lin_partial(const float* __restrict__ X, const float* __restrict__ y,
@@ -311,6 +816,7 @@ __global__ void f32_lin_partial(const float* __restrict__ X, const float* __rest
   const int64_t r1 = r0 + chunk < N ? r0 + chunk : N;
   for (int d = threadIdx.x; d < D; d += blockDim.x) {
     double acc = 0.0;
+#pragma unroll 8
     for (int64_t r = r0; r < r1; ++r) acc += ((double)y[r] - 0.5) * (double)X[r * D + d];
     part[(size_t)blockIdx.x * D + d] = acc;
   }
@@ -330,7 +836,18 @@ void f32_set_smem() {
   GBM_CUDA(cudaFuncSetAttribute(logreg_f32_kernel<KD>,
                                 cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 F32Layout<KD>::kBytes));
+  GBM_CUDA(cudaFuncSetAttribute(logreg_f32_tc_kernel<KD>,
+                                cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                F32TcLayout<KD>::kBytes));
 }
+
+// Rows from which phase 2 runs on the tensor cores.  It is the faster one from
+// there on: 4096 rows x 10 features x 64 chains 26.2 us an evaluation (27.7 on
+// the CUDA cores), x 100 30.1 (35.2), 8192 x 4 x 1024 31.3 (35.0).  Below, where
+// an evaluation is launch latency for the most part (2000 x 100 x 64: 36
+// against 43 us), the gradient keeps its FP32 summation order: a sampler run
+// over a small data set repeats to the digit.
+constexpr int64_t kTcMinRows = 4096;
 
 class LogregF32 final : public Target {
  public:
@@ -365,6 +882,7 @@ class LogregF32 final : public Target {
     log_norm_ = -log((double)prior_scale) - 0.5 * log(2.0 * M_PI);
     grid_ = ctx->num_sms;
     err_dev_ = ctx->err_dev;
+    tc_ = n >= kTcMinRows && prepare_f16(ctx, X);
     switch (kd_) {
       case 1: f32_set_smem<1>(); break;
       case 2: f32_set_smem<2>(); break;
@@ -394,9 +912,14 @@ class LogregF32 final : public Target {
       const float* qc = q + (size_t)base * ldq;
       const int g = work_grid(grid_, std::min(lim, cap - base), kF32CT, N_, kMinSplitRows);
 #define GBM_F32_LAUNCH(KD_)                                                                \
-  logreg_f32_kernel<KD_><<<g, kF32Threads, F32Layout<KD_>::kBytes, s>>>(                    \
-      x2_.as<float>(), ym_.as<float>(), N, D, qc, ldq, n_dev, base, lim, g, lpart, gpart,     \
-      err_dev_)
+  if (tc_)                                                                                 \
+    logreg_f32_tc_kernel<KD_><<<g, kF32TcThreads, F32TcLayout<KD_>::kBytes, s>>>(             \
+        himap_, lomap_, x2_.as<float>(), ym_.as<float>(), gscale_, N, D, qc, ldq,  \
+        n_dev, base, lim, g, lpart, gpart, err_dev_);                                        \
+  else                                                                                     \
+    logreg_f32_kernel<KD_><<<g, kF32Threads, F32Layout<KD_>::kBytes, s>>>(                    \
+        x2_.as<float>(), ym_.as<float>(), N, D, qc, ldq, n_dev, base, lim, g, lpart, gpart,    \
+        err_dev_)
       switch (kd_) {
         case 1: GBM_F32_LAUNCH(1); break;
         case 2: GBM_F32_LAUNCH(2); break;
@@ -423,12 +946,68 @@ class LogregF32 final : public Target {
   }
 
  private:
+  // X as FP16 hi + lo of scaled features; false if a column does not fit that:
+  // infinities, NaN, exponents that the scaling cannot carry, or a range so
+  // wide that hi + lo leaves more than 2^-23 of it in root mean square (a normal
+  // sample: 2^-25); or if a label is so far outside [0, 1] that a residual,
+  // below |y - 1/2| + 1/2, could leave FP16's range (R' < 2^16).
+  bool prepare_f16(gbm_context* ctx, const float* X) {
+    cudaStream_t s = ctx->stream;
+    const int D = (int)D_, nb = 8 * ctx->num_sms;
+    const int64_t chunk = (N_ + nb - 1) / nb;
+    const size_t off_part = 1024;
+    const size_t off_sum = off_part + (sizeof(float2) * (size_t)nb * D + 255) / 256 * 256;
+    DeviceBuffer buf;
+    buf.reserve(off_sum + sizeof(double2) * D);
+    unsigned* mx = buf.as<unsigned>();
+    float2* part = reinterpret_cast<float2*>(buf.as<char>() + off_part);
+    double2* sum = reinterpret_cast<double2*>(buf.as<char>() + off_sum);
+    const size_t x16 = sizeof(__half) * (size_t)N_ * dp_;
+    x16_.reserve(2 * x16 + sizeof(float) * D);   // hi, lo (32-byte rows), scales
+    __half* hi = x16_.as<__half>();
+    __half* lo = hi + (size_t)N_ * dp_;
+    gscale_ = reinterpret_cast<float*>(x16_.as<char>() + 2 * x16);
+    GBM_CUDA(cudaMemsetAsync(mx, 0, sizeof(unsigned) * (D + 1), s));
+    column_max_kernel<<<nb, 128, 0, s>>>(X, N_, D, chunk, mx);
+    column_max_kernel<<<nb, 32, 0, s>>>(ym_.as<float>(), N_, 1, chunk, mx + D);
+    f16_pack_kernel<<<nb, 128, 0, s>>>(X, N_, D, dp_, chunk, mx, hi, lo, part);
+    column_rest_kernel<<<(unsigned)D, 128, 0, s>>>(part, nb, D, sum);
+    GBM_CUDA(cudaGetLastError());
+    std::vector<unsigned> hmax(D + 1);
+    std::vector<double2> hsum(D);
+    GBM_CUDA(cudaMemcpyAsync(hmax.data(), mx, sizeof(unsigned) * (D + 1), cudaMemcpyDeviceToHost, s));
+    GBM_CUDA(cudaMemcpyAsync(hsum.data(), sum, sizeof(double2) * D, cudaMemcpyDeviceToHost, s));
+    GBM_CUDA(cudaStreamSynchronize(s));
+    std::vector<float> gs(D, 0.f);   // from G' to G; a column of zeros stays zero
+    constexpr unsigned kLabelTop = 0x3fa00000u;   // 1.25f
+    bool fits = hmax[D] <= kLabelTop;
+    for (int i = 0; i < D; ++i) {
+      if (hmax[i] == 0) continue;
+      const int fexp = (int)((hmax[i] >> 23) & 255u) - 127;
+      fits = fits && fexp >= -60 && fexp <= 60 && hsum[i].y <= std::ldexp(hsum[i].x, -46);
+      gs[i] = std::ldexp(1.f, fexp - kF16Top - 15);
+    }
+    if (!fits) {
+      x16_.release();
+      return false;
+    }
+    GBM_CUDA(cudaMemcpyAsync(gscale_, gs.data(), sizeof(float) * D, cudaMemcpyHostToDevice, s));
+    GBM_CUDA(cudaStreamSynchronize(s));   // gs ends here
+    encode_rows(&himap_, hi, N_, dp_, kHalf);
+    encode_rows(&lomap_, lo, N_, dp_, kHalf);
+    return true;
+  }
+
   int64_t N_, D_, n2_ = 0;
   int kd_ = 1, dp_ = 16, grid_ = 0;
   float inv_var_ = 1.f;
   double log_norm_ = 0.0;
   int* err_dev_ = nullptr;
   DeviceBuffer x2_, ym_, lin_;
+  bool tc_ = false;            // phase 2 on the tensor cores
+  DeviceBuffer x16_;
+  float* gscale_ = nullptr;    // within x16_
+  CUtensorMap himap_, lomap_;
 };
 
 }  // namespace

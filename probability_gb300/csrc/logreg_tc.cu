@@ -45,6 +45,7 @@
 
 #include "engine.h"
 #include "split_reduce.cuh"
+#include "tc_common.cuh"
 #include "tc_ptx.cuh"
 
 namespace gbm {
@@ -53,16 +54,8 @@ namespace {
 constexpr int kRows = 128;                         // rows of X per tile
 // Threads of a CTA with EPI epilogue warps (plus the TMA and MMA warps).
 __host__ __device__ constexpr int tc_threads(int epi) { return 32 * (2 + epi); }
-constexpr uint64_t kWaitLimitNs = 2000000000ull;   // 2 s bound on every device wait
 constexpr float kNeg2Log2e = -2.8853900817779268f;  // -2 log2(e)
 constexpr float kLn2 = 0.6931471805599453f;
-
-enum TcError : int {
-  kTcOk = 0,
-  kTcTimeoutTma = 1,
-  kTcTimeoutMma = 2,
-  kTcTimeoutEpilogue = 3,
-};
 
 __host__ __device__ inline int tc_splits(int n, int ct, int grid, int row_tiles) {
   const int tiles = (n + ct - 1) / ct;
@@ -116,29 +109,6 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float a, float b) {
 // rows).
 __device__ __forceinline__ uint32_t residual_bf16x2(float h0, float h1, float ym) {
   return pack_bf16x2(fmaf(-0.5f, tc::tanh_approx(h0), ym), fmaf(-0.5f, tc::tanh_approx(h1), ym));
-}
-
-__device__ __forceinline__ void named_barrier(int id, int nthreads) {
-  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
-}
-
-// Wait that also gives up when another role has already aborted.
-__device__ __forceinline__ bool wait_or_abort(uint64_t* bar, uint32_t parity,
-                                              volatile int* abort_flag) {
-  if (tc::mbar_try_wait(bar, parity)) return true;
-  const uint64_t t0 = tc::globaltimer_ns();
-  while (true) {
-    if (tc::mbar_try_wait(bar, parity)) return true;
-    if (*abort_flag) return false;
-    if (tc::globaltimer_ns() - t0 > kWaitLimitNs) return false;
-  }
-}
-
-// wait_or_abort by every lane of a warp, with one outcome for the whole warp
-// (the .sync.aligned TMEM accesses that follow need a converged warp).
-__device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity,
-                                          volatile int* abort_flag) {
-  return __all_sync(0xffffffffu, wait_or_abort(bar, parity, abort_flag));
 }
 
 // XLO: X is FP32 data stored as X_hi + X_lo (both BF16); GEMM1 adds the
@@ -301,11 +271,11 @@ logreg_tc_kernel(const __grid_constant__ CUtensorMap xmap,
             const uint64_t a = tc::smem_desc_sw128(xa + kb * 16384 + k * 32, 16, 1024);
             const uint64_t bh = tc::smem_desc_sw128(bhi_a + kb * (CT * 128) + k * 32, 16, 1024);
             const uint64_t bl = tc::smem_desc_sw128(blo_a + kb * (CT * 128) + k * 32, 16, 1024);
-            tc::mma_bf16(tz, a, bh, idesc1, (kb | k) ? 1u : 0u);
-            tc::mma_bf16(tz, a, bl, idesc1, 1u);
+            tc::mma_16bit(tz, a, bh, idesc1, (kb | k) ? 1u : 0u);
+            tc::mma_16bit(tz, a, bl, idesc1, 1u);
             if constexpr (XLO) {
               const uint64_t al = tc::smem_desc_sw128(xla + kb * 16384 + k * 32, 16, 1024);
-              tc::mma_bf16(tz, al, bh, idesc1, 1u);
+              tc::mma_16bit(tz, al, bh, idesc1, 1u);
             }
           }
         }
@@ -333,7 +303,7 @@ logreg_tc_kernel(const __grid_constant__ CUtensorMap xmap,
           for (int ks = 0; ks < kRows / 16; ++ks) {
             const uint64_t a = tc::smem_desc_sw128(xa + mt * 32768 + ks * 2048, 16384, 1024);
             const uint64_t bd = tc::smem_desc_sw128(ra + ks * 2048, 16384, 1024);
-            tc::mma_bf16(tg + mt * CT, a, bd, idesc2, (it > 0 || ks > 0) ? 1u : 0u);
+            tc::mma_16bit(tg + mt * CT, a, bd, idesc2, (it > 0 || ks > 0) ? 1u : 0u);
           }
         }
         tc::mma_commit(&bars->x_empty[s]);
@@ -722,10 +692,10 @@ logreg_tct_kernel(const __grid_constant__ CUtensorMap xmap,
         for (int k = 0; k < 8; ++k) {
           if (k < ksteps) {
             const uint64_t bx = xs + (uint64_t)(((k >> 2) * 16384 + (k & 3) * 32) >> 4);
-            tc::mma_bf16_tmem_a(tz, tmem + kTBhi + k * 8, bx, idesc1, k > 0 ? 1u : 0u);
-            tc::mma_bf16_tmem_a(tz, tmem + kTBlo + k * 8, bx, idesc1, 1u);
+            tc::mma_16bit_tmem_a(tz, tmem + kTBhi + k * 8, bx, idesc1, k > 0 ? 1u : 0u);
+            tc::mma_16bit_tmem_a(tz, tmem + kTBlo + k * 8, bx, idesc1, 1u);
             if constexpr (XLO)
-              tc::mma_bf16_tmem_a(tz, tmem + kTBhi + k * 8, bx + (32768 >> 4), idesc1, 1u);
+              tc::mma_16bit_tmem_a(tz, tmem + kTBhi + k * 8, bx + (32768 >> 4), idesc1, 1u);
           }
         }
         tc::mma_commit(&bars->z_full[b]);
@@ -750,10 +720,10 @@ logreg_tct_kernel(const __grid_constant__ CUtensorMap xmap,
           // R_lo^T X_hi (+ R_hi^T X_lo for FP32 data).
           const uint32_t ra = tr + (ks >> 1) * 32 + (ks & 1) * 8;
           const uint64_t bx = xs + (uint64_t)((ks * 2048) >> 4);
-          tc::mma_bf16_tmem_a(tmem + kTG, ra, bx, idesc2, (it > 0 || ks > 0) ? 1u : 0u);
-          tc::mma_bf16_tmem_a(tmem + kTG, ra + 16, bx, idesc2, 1u);
+          tc::mma_16bit_tmem_a(tmem + kTG, ra, bx, idesc2, (it > 0 || ks > 0) ? 1u : 0u);
+          tc::mma_16bit_tmem_a(tmem + kTG, ra + 16, bx, idesc2, 1u);
           if constexpr (XLO)
-            tc::mma_bf16_tmem_a(tmem + kTG, ra, bx + (32768 >> 4), idesc2, 1u);
+            tc::mma_16bit_tmem_a(tmem + kTG, ra, bx + (32768 >> 4), idesc2, 1u);
         }
         tc::mma_commit(&bars->x_empty[s]);
         if (it + 2 < T) {
@@ -1077,8 +1047,8 @@ logreg_tc_pair_kernel(const __grid_constant__ CUtensorMap xmap, const float* __r
                   tc::smem_desc_sw128(bhi_a + kb * (CT * 128) + k * 32, 16, 1024);
               const uint64_t bl =
                   tc::smem_desc_sw128(blo_a + kb * (CT * 128) + k * 32, 16, 1024);
-              tc::mma_bf16(tz, a, bh, idesc1, (kb | k) ? 1u : 0u);
-              tc::mma_bf16(tz, a, bl, idesc1, 1u);
+              tc::mma_16bit(tz, a, bh, idesc1, (kb | k) ? 1u : 0u);
+              tc::mma_16bit(tz, a, bl, idesc1, 1u);
             }
           }
         }
@@ -1104,7 +1074,7 @@ logreg_tc_pair_kernel(const __grid_constant__ CUtensorMap xmap, const float* __r
           for (int ks = 0; ks < kRows / 16; ++ks) {
             const uint64_t a = tc::smem_desc_sw128(xa + mt * 32768 + ks * 2048, 16384, 1024);
             const uint64_t bd = tc::smem_desc_sw128(rs_a + ks * 2048, 16384, 1024);
-            tc::mma_bf16(tg + mt * CT, a, bd, idesc2, (it > 0 || ks > 0) ? 1u : 0u);
+            tc::mma_16bit(tg + mt * CT, a, bd, idesc2, (it > 0 || ks > 0) ? 1u : 0u);
           }
           tc::mma_commit(&bars->x_empty[it & 1][mt]);
         }
@@ -1345,25 +1315,6 @@ __global__ void lin_sum_kernel(const double* __restrict__ part, int nb, int D,
   lin[d] = acc;
 }
 
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*,
-                                  const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
-                                  const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-EncodeTiledFn encode_tiled() {
-  static EncodeTiledFn fn = nullptr;
-  if (!fn) {
-    void* p = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    GBM_CUDA(cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000,
-                                              cudaEnableDefault, &q));
-    if (q != cudaDriverEntryPointSuccess || !p)
-      throw CudaError{cudaErrorNotSupported, "cuTensorMapEncodeTiled entry point"};
-    fn = reinterpret_cast<EncodeTiledFn>(p);
-  }
-  return fn;
-}
-
 class LogregTc final : public Target {
  public:
   LogregTc(gbm_context* ctx, const void* X, int x_dtype, int64_t n, int64_t d, const float* y,
@@ -1434,8 +1385,8 @@ class LogregTc final : public Target {
       GBM_CUDA(cudaOccupancyMaxActiveClusters(&clusters, logreg_tc_pair_kernel, &cfg));
       grid_ = std::max(1, std::min(ctx->num_sms / 2, clusters));
     }
-    encode(&xmap_, xb_.ptr, Dp);
-    encode(&xlomap_, xlo_ ? xl_.ptr : xb_.ptr, Dp);
+    encode_rows(&xmap_, xb_.ptr, N_, Dp, kRows);
+    encode_rows(&xlomap_, xlo_ ? xl_.ptr : xb_.ptr, N_, Dp, kRows);
     const int attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
     if (kb_ == 2 && xlo_) {
       smem_ = TctLayout<true>::kBytes + 1024;
@@ -1508,20 +1459,6 @@ class LogregTc final : public Target {
   size_t smem_ = 0;
   float inv_var_ = 1.f;
   double log_norm_ = 0.0;
-  // Tensor map over a BF16 [N][Dp] matrix: boxes of 64 features x 128 rows,
-  // 128-byte swizzle, rows past N read as zeros.
-  void encode(CUtensorMap* map, void* base, int Dp) {
-    cuuint64_t dims[2] = {(cuuint64_t)Dp, (cuuint64_t)N_};
-    cuuint64_t strides[1] = {(cuuint64_t)Dp * 2};
-    cuuint32_t box[2] = {64, (cuuint32_t)kRows};
-    cuuint32_t estr[2] = {1, 1};
-    CUresult r = encode_tiled()(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, base, dims, strides,
-                                box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                                CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) throw CudaError{cudaErrorInvalidValue, "cuTensorMapEncodeTiled"};
-  }
-
   DeviceBuffer xb_, xl_, y_;
   DeviceBuffer ym_;    // y - 1/2, zero-padded to whole row tiles (chain-major kernel)
   DeviceBuffer lin_;   // X^T (y - 1/2), float64 [D]

@@ -239,6 +239,16 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&v)[16
       : "memory");
 }
 
+// 32 lanes x 32 bit, 8 consecutive columns written from each thread.
+__device__ __forceinline__ void tmem_st8(uint32_t taddr, const float (&v)[8]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(taddr),
+      "r"(__float_as_uint(v[0])), "r"(__float_as_uint(v[1])), "r"(__float_as_uint(v[2])),
+      "r"(__float_as_uint(v[3])), "r"(__float_as_uint(v[4])), "r"(__float_as_uint(v[5])),
+      "r"(__float_as_uint(v[6])), "r"(__float_as_uint(v[7]))
+      : "memory");
+}
+
 __device__ __forceinline__ void tmem_st_wait() {
   asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
 }
@@ -248,8 +258,9 @@ __device__ __forceinline__ void tmem_ld_wait() {
 }
 
 // ---- MMA ---------------------------------------------------------------------
-// D[tmem] (+)= A[smem] * B[smem], kind::f16 (BF16 inputs), FP32 accumulate.
-__device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc,
+// D[tmem] (+)= A[smem] * B[smem], kind::f16 (FP16 or BF16 inputs, as the
+// instruction descriptor says), FP32 accumulate.
+__device__ __forceinline__ void mma_16bit(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc,
                                          uint32_t idesc, uint32_t accumulate) {
   asm volatile(
       "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
@@ -258,9 +269,9 @@ __device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t adesc, uint64
       : "memory");
 }
 
-// D[tmem] (+)= A[tmem] * B[smem], kind::f16 (BF16 inputs), FP32 accumulate:
+// D[tmem] (+)= A[tmem] * B[smem], kind::f16, FP32 accumulate:
 // A (M x K) lives in TMEM, row m in lane m, two K elements per 32-bit column.
-__device__ __forceinline__ void mma_bf16_tmem_a(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc,
+__device__ __forceinline__ void mma_16bit_tmem_a(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc,
                                                 uint32_t idesc, uint32_t accumulate) {
   asm volatile(
       "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
@@ -316,6 +327,13 @@ __device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t addr, uint32_t lbo,
 __host__ __device__ constexpr uint32_t idesc_bf16_f32(int M, int N, bool a_mn, bool b_mn) {
   return (1u << 4) | (1u << 7) | (1u << 10) | ((a_mn ? 1u : 0u) << 15) |
          ((b_mn ? 1u : 0u) << 16) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
+}
+
+// The same with FP16 (format 0) or BF16 operands.
+__host__ __device__ constexpr uint32_t idesc_16bit_f32(int M, int N, bool a_mn, bool b_mn,
+                                                       bool bf16) {
+  return bf16 ? idesc_bf16_f32(M, N, a_mn, b_mn)
+              : idesc_bf16_f32(M, N, a_mn, b_mn) & ~((1u << 7) | (1u << 10));
 }
 
 // Byte offset of element (row, col) of a 128-byte-swizzled atom stack whose

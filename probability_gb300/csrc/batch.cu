@@ -10,20 +10,24 @@
 // launch per sampler step for all members), so a leaf of the sampler costs a
 // fixed number of launches however many posteriors are in flight.
 //
-// Gradient evaluation of the active chains is two persistent launches over a
-// tile list built on the device each leaf:
+// Gradient evaluation of the active chains is two persistent launches over
+// tile lists built on the device each leaf:
 //   schedule: for each member, its active chains are a contiguous run of the
 //             (sorted) active list; MVN members contribute
-//             ceil(active / ct) x ceil(D / 128) tiles, hierarchical members
-//             ceil(active / 8) tiles.
-//   phase 0:  MVN tiles form u = L^-1 (x - loc) for a block of 128 rows of u
-//             and that block's |u|^2; hierarchical tiles do all their work.
-//   phase 1:  MVN tiles form grad = -L^-T u for a block of 128 columns; the
-//             column-block-0 tile also sums the |u|^2 blocks (fixed order).
-// Each CTA walks the list with a stride of the grid, so large and small
-// members share the machine in one launch.  The chain-tile width ct (32 or
-// 64 chains) is chosen per size class of D by timing both at construction
-// (the autotuner).
+//             ceil(active / ct) x ceil(D / 64) tiles, hierarchical members
+//             ceil(active / 4) tiles, those with the longest sums first.
+//   phase 0:  MVN tiles form u = L^-1 (x - loc) for a block of 64 rows of u
+//             and its |u|^2; hierarchical tiles do all their work.
+//   phase 1:  MVN tiles form grad = -L^-T u for a block of 64 columns; the
+//             last column block's tile also adds the |u|^2 sums (fixed order).
+// CTAs take tiles from the list as they get done, so large and small members
+// share the machine in one launch.  The chain-tile width ct (32 or 64 chains) is
+// chosen per size class of D by timing both at construction (the autotuner).
+//
+// What bounds it: mvn_tile.cuh's tiles, and their longest sum where one large
+// member holds most of the work.  Twelve normals up to 2048 (497 chains) and
+// twelve hierarchical members: 517 us an evaluation with tiles of 128 outputs in
+// member order at a fixed stride, 208 now; members of at most 300: 83 and 48.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -32,6 +36,7 @@
 
 #include "engine.h"
 #include "gb300_mcmc.h"
+#include "mvn_tile.cuh"
 #include "nuts_chain.h"
 
 namespace gbm {
@@ -39,10 +44,9 @@ namespace {
 
 enum BatchFamily : int { kBatchMvn = 1, kBatchHier = 2 };   // the GBM_FAMILY_* values
 
-constexpr int kOB = 128;         // rows / columns of u or grad per MVN tile
-constexpr int kKc = 16;          // K chunk
-constexpr int kThreads = 256;
-constexpr int kHierChains = 8;   // chains per hierarchical tile (a warp each)
+constexpr int kOB = 64;          // rows / columns of u or grad per MVN tile
+constexpr int kThreads = 128;
+constexpr int kHierChains = 4;   // chains per hierarchical tile (a warp each)
 constexpr int kClasses = 4;      // size classes of D for the tile autotuner
 
 __host__ __device__ inline int size_class(int d) {
@@ -52,10 +56,8 @@ __host__ __device__ inline int size_class(int d) {
 struct BDesc {
   int family, dim, c_begin, c_end;
   long long p_begin;    // first |u|^2 partial of this member
-  int ct, nob;          // chain tile and 64-blocks of D (MVN)
-  const float* loc;
-  const float* linv;
-  double log_norm;
+  int ct;               // chain tile (MVN)
+  MvnFactor mvn;
   const float* y;
   const float* sigma;
   float mu_scale, tau_scale;
@@ -71,198 +73,77 @@ __device__ __forceinline__ int lower_bound_dev(const int* a, int n, int v) {
   return lo;
 }
 
-// Member index of tile `tile` given the exclusive prefix base[0..T].
-__device__ __forceinline__ int member_of(const int* base, int T, int tile) {
-  int lo = 0, hi = T;   // base[lo] <= tile < base[hi]
-  while (hi - lo > 1) {
-    const int m = (lo + hi) >> 1;
-    if (base[m] <= tile) lo = m; else hi = m;
-  }
-  return lo;
-}
-
-__global__ void batch_schedule_kernel(const BDesc* __restrict__ d, int T,
-                                      const int* __restrict__ act,
-                                      const int* __restrict__ act_count, int* __restrict__ a,
-                                      int* __restrict__ na, int* __restrict__ t1,
-                                      int* __restrict__ t2, int* __restrict__ base1,
-                                      int* __restrict__ base2) {
-  const int n = *act_count;
-  for (int t = threadIdx.x; t < T; t += blockDim.x) {
-    const int lo = lower_bound_dev(act, n, d[t].c_begin);
-    const int hi = lower_bound_dev(act, n, d[t].c_end);
-    const int m = hi - lo;
-    a[t] = lo;
-    na[t] = m;
-    if (d[t].family == kBatchMvn) {
-      const int tiles = (m + d[t].ct - 1) / d[t].ct * d[t].nob;
-      t1[t] = tiles;
-      t2[t] = tiles;
-    } else {
-      t1[t] = (m + kHierChains - 1) / kHierChains;
-      t2[t] = 0;
-    }
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    int s1 = 0, s2 = 0;
-    for (int t = 0; t < T; ++t) {
-      base1[t] = s1;
-      base2[t] = s2;
-      s1 += t1[t];
-      s2 += t2[t];
-    }
-    base1[T] = s1;
-    base2[T] = s2;
-  }
-}
-
-struct alignas(16) TileSmem {
-  float As[2][kKc][64 + 4];     // [stage][k][chain]
-  float Bs[2][kKc][kOB + 4];    // [stage][k][output]
-  double red[16][64];
-  long long cof[64];
-  int cid[64];
+// What a tile of the list works on: `group` of a phase's order, its k-th run of
+// chains.
+struct Group {
+  int member, ob;       // output block (MVN)
 };
 
-// One MVN tile: chains act[a0 .. a0 + nc) (nc <= CT) x outputs [o0, o0 + 128).
-//   PHASE 0: U[c][o] = sum_{k <= o} (x_c[k] - loc[k]) L^-1[o][k]; |U_c|^2 over
-//            the block -> part.
-//   PHASE 1: G[c][o] = -sum_{k >= o} U_c[k] L^-1[k][o]; block 0 also writes
-//            logp = -1/2 sum of the |U|^2 blocks + log_norm.
-// Thread (ty, tx) of the 16 x 16 layout accumulates chains ty*CPT .. +CPT-1
-// and outputs tx*4 .. +3 and 64 + tx*4 .. +3 in registers (each K step: one
-// shared load of the chains, two conflict-free 16-byte loads of the outputs,
-// 8·CPT FMAs).  K chunks of 16 are double-buffered in shared memory: the
-// next chunk's global loads are issued into registers before the current
-// chunk's FMAs and stored to the other stage after them.
-template <int PHASE, int CT>
-__device__ void mvn_tile(const BDesc& d, const int* __restrict__ act, int a0, int nc, int ob,
-                         const int64_t* __restrict__ coff, const float* __restrict__ X,
-                         float* __restrict__ out, double* __restrict__ part,
-                         double* __restrict__ logp, TileSmem& sm) {
-  constexpr int CPT = CT / 16;                  // chains per thread (4 or 2)
-  constexpr int AL = kKc * CT / kThreads;       // A values each thread loads per chunk
-  constexpr int BL = kKc * kOB / kThreads;      // B values each thread loads per chunk
-  static_assert(AL >= 1 && BL >= 1, "tile loads");
-  const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
-  const int D = d.dim, o0 = ob * kOB;
-  const float* M = d.linv;
-  __syncthreads();   // the previous tile is done with shared memory
-  if (tid < CT) {
-    const int c = tid < nc ? act[a0 + tid] : -1;
-    sm.cid[tid] = c;
-    sm.cof[tid] = c >= 0 ? coff[c] : 0;
+// Exclusive prefix sum over the block (1024 threads); the total in *total.
+__device__ int block_prefix(int v, int* total) {
+  __shared__ int warps[32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int x = v;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int y = __shfl_up_sync(~0u, x, o);
+    if (lane >= o) x += y;
+  }
+  __syncthreads();   // the last call's readers are done
+  if (lane == 31) warps[warp] = x;
+  __syncthreads();
+  if (warp == 0) {
+    int w = warps[lane];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(~0u, w, o);
+      if (lane >= o) w += y;
+    }
+    warps[lane] = w;
   }
   __syncthreads();
-  float acc[CPT][8];
-#pragma unroll
-  for (int i = 0; i < CPT; ++i)
-#pragma unroll
-    for (int j = 0; j < 8; ++j) acc[i][j] = 0.f;
-  const int k_begin = PHASE == 0 ? 0 : (o0 / kKc) * kKc;
-  const int k_end = PHASE == 0 ? min(D, o0 + kOB) : D;
-  const int chunks = (k_end - k_begin + kKc - 1) / kKc;
-  float ra[AL], rb[BL];
-  // Chunk loads: A(k, chain) with k fastest (a chain's state is contiguous);
-  // B(k, o) = M[o][k] (phase 0, k fastest) or M[k][o] (phase 1, o fastest).
-  auto load = [&](int k0) {
-#pragma unroll
-    for (int r = 0; r < AL; ++r) {
-      const int i = tid + r * kThreads, kk = i % kKc, cc = i / kKc, k = k0 + kk;
-      float v = 0.f;
-      if (cc < nc && k < D) {
-        v = X[sm.cof[cc] + k];
-        if (PHASE == 0) v -= d.loc[k];
-      }
-      ra[r] = v;
+  *total = warps[31];
+  return x - v + (warp > 0 ? warps[warp - 1] : 0);
+}
+
+// Block p writes phase p's tile list: {group, run of chains} of every tile in
+// the order of the groups, their number, and the counter that the phase takes
+// tiles from.  Block 0 also stores each member's run [a, a + na) of the active
+// list.
+__global__ void __launch_bounds__(1024)
+batch_schedule_kernel(const BDesc* __restrict__ d, int T, const int* __restrict__ act,
+                      const int* __restrict__ act_count, const Group* __restrict__ groups0,
+                      const Group* __restrict__ groups1, int n0, int n1, int* __restrict__ a,
+                      int* __restrict__ na, int2* __restrict__ tiles0, int2* __restrict__ tiles1,
+                      int* __restrict__ totals, int* __restrict__ next) {
+  const int n = *act_count, phase = blockIdx.x;
+  const Group* groups = phase == 0 ? groups0 : groups1;
+  int2* tiles = phase == 0 ? tiles0 : tiles1;
+  const int ng = phase == 0 ? n0 : n1;
+  if (phase == 0)
+    for (int t = threadIdx.x; t < T; t += blockDim.x) {
+      const int lo = lower_bound_dev(act, n, d[t].c_begin);
+      a[t] = lo;
+      na[t] = lower_bound_dev(act, n, d[t].c_end) - lo;
     }
-#pragma unroll
-    for (int r = 0; r < BL; ++r) {
-      const int i = tid + r * kThreads;
-      if (PHASE == 0) {
-        const int kk = i % kKc, oo = i / kKc, k = k0 + kk, o = o0 + oo;
-        rb[r] = (o < D && k < D && k <= o) ? M[(size_t)o * D + k] : 0.f;
-      } else {
-        const int oo = i % kOB, kk = i / kOB, k = k0 + kk, o = o0 + oo;
-        rb[r] = (o < D && k < D && k >= o) ? M[(size_t)k * D + o] : 0.f;
-      }
+  int done = 0;
+  for (int g0 = 0; g0 < ng; g0 += 1024) {
+    const int g = g0 + threadIdx.x;
+    int runs = 0;
+    if (g < ng) {
+      const BDesc& m = d[groups[g].member];
+      const int ct = m.family == kBatchMvn ? m.ct : kHierChains;
+      const int held = lower_bound_dev(act, n, m.c_end) - lower_bound_dev(act, n, m.c_begin);
+      runs = (held + ct - 1) / ct;
     }
-  };
-  auto store = [&](int st) {
-#pragma unroll
-    for (int r = 0; r < AL; ++r) {
-      const int i = tid + r * kThreads;
-      sm.As[st][i % kKc][i / kKc] = ra[r];
-    }
-#pragma unroll
-    for (int r = 0; r < BL; ++r) {
-      const int i = tid + r * kThreads;
-      if (PHASE == 0)
-        sm.Bs[st][i % kKc][i / kKc] = rb[r];
-      else
-        sm.Bs[st][i / kOB][i % kOB] = rb[r];
-    }
-  };
-  if (chunks > 0) {
-    load(k_begin);
-    store(0);
+    int total;
+    const int at = done + block_prefix(runs, &total);
+    for (int k = 0; k < runs; ++k) tiles[at + k] = make_int2(g, k);
+    done += total;
   }
-  __syncthreads();
-  for (int ch = 0; ch < chunks; ++ch) {
-    const int st = ch & 1;
-    const bool more = ch + 1 < chunks;
-    if (more) load(k_begin + (ch + 1) * kKc);
-#pragma unroll
-    for (int kk = 0; kk < kKc; ++kk) {
-      float aa[CPT];
-      if (CPT == 4) {
-        const float4 a4 = *reinterpret_cast<const float4*>(&sm.As[st][kk][ty * 4]);
-        aa[0] = a4.x; aa[1] = a4.y; aa[CPT > 2 ? 2 : 0] = a4.z; aa[CPT > 3 ? 3 : 0] = a4.w;
-      } else {
-        const float2 a2 = *reinterpret_cast<const float2*>(&sm.As[st][kk][ty * 2]);
-        aa[0] = a2.x; aa[1] = a2.y;
-      }
-      const float4 b0 = *reinterpret_cast<const float4*>(&sm.Bs[st][kk][tx * 4]);
-      const float4 b1 = *reinterpret_cast<const float4*>(&sm.Bs[st][kk][64 + tx * 4]);
-      const float bb[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
-#pragma unroll
-      for (int i = 0; i < CPT; ++i)
-#pragma unroll
-        for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(aa[i], bb[j], acc[i][j]);
-    }
-    if (more) store(st ^ 1);
-    __syncthreads();
-  }
-#pragma unroll
-  for (int i = 0; i < CPT; ++i) {
-    const int cc = ty * CPT + i;
-    double sq = 0.0;
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const int o = o0 + (j < 4 ? tx * 4 + j : 64 + tx * 4 + j - 4);
-      if (cc < nc && o < D) {
-        const float v = PHASE == 0 ? acc[i][j] : -acc[i][j];
-        out[sm.cof[cc] + o] = v;
-        sq += (double)v * (double)v;
-      }
-    }
-    if (PHASE == 0) sm.red[tx][cc] = sq;
-  }
-  if (PHASE == 0) {
-    __syncthreads();
-    if (tid < nc) {
-      double s = 0.0;
-      for (int t = 0; t < 16; ++t) s += sm.red[t][tid];
-      const int c = sm.cid[tid];
-      part[d.p_begin + (long long)(c - d.c_begin) * d.nob + ob] = s;
-    }
-  } else if (ob == 0 && tid < nc) {
-    const int c = sm.cid[tid];
-    const double* p = part + d.p_begin + (long long)(c - d.c_begin) * d.nob;
-    double s = 0.0;
-    for (int t = 0; t < d.nob; ++t) s += p[t];
-    logp[c] = -0.5 * s + d.log_norm;   // -1/2 |L^-1 (x - loc)|^2 + normaliser
+  if (threadIdx.x == 0) {
+    totals[phase] = done;
+    next[phase] = 0;
   }
 }
 
@@ -315,33 +196,71 @@ __device__ void hier_tile(const BDesc& d, const int* __restrict__ act, int a0, i
   }
 }
 
+// A phase's CTAs: phase 0 in groups of 128 threads, as many as fit an SM; phase 1
+// with four such groups a CTA, which share the k of a tile.
 template <int PHASE>
-__global__ void __launch_bounds__(kThreads, 2)
-batch_phase_kernel(const BDesc* __restrict__ desc, int T, const int* __restrict__ act,
+struct PhaseLaunch {
+  static constexpr int kGroups = PHASE == 0 ? 1 : 4;
+  static constexpr int kSmem =
+      (int)std::max(sizeof(MvnSmem<64, kOB, kGroups>), sizeof(MvnSmem<32, kOB, kGroups>));
+};
+
+template <int PHASE, int CT, int RO>
+__device__ void run_mvn(const BDesc& d, int o0, const int* __restrict__ act, int a0, int nc,
+                        const int64_t* __restrict__ coff, const float* __restrict__ X,
+                        float* __restrict__ out, double* __restrict__ part,
+                        double* __restrict__ logp, unsigned char* smem) {
+  constexpr int KG = PhaseLaunch<PHASE>::kGroups;
+  auto& sm = *reinterpret_cast<MvnSmem<CT, kOB, KG>*>(smem);
+  if (threadIdx.x < CT) {
+    const int i = threadIdx.x, c = i < nc ? act[a0 + i] : d.c_begin;
+    sm.id[i] = c;
+    sm.in[i] = sm.out[i] = coff[c];
+    sm.part[i] = d.p_begin + (long long)(c - d.c_begin) * mvn_parts(d.dim);
+  }
+  mvn_tile<PHASE, CT, kOB, 4, RO, KG>(d.mvn, nc, o0, X, out, part, logp, sm);
+}
+
+// Persistent CTAs.  The list begins with the longest tiles.  A CTA's first tile
+// is its place in it, every second stretch of the GPU's SMs counting backwards, so
+// that the CTAs that share an SM (as they are placed on an idle GPU: b, b + SMs,
+// ...) get about the same work in sum; then each takes the next one left.
+template <int PHASE>
+__global__ void __launch_bounds__(kThreads * PhaseLaunch<PHASE>::kGroups, PHASE == 0 ? 4 : 1)
+batch_phase_kernel(const BDesc* __restrict__ desc, const Group* __restrict__ groups,
+                   const int2* __restrict__ tiles, const int* __restrict__ total_dev,
+                   int* __restrict__ next, int sms, const int* __restrict__ act,
                    const int* __restrict__ a, const int* __restrict__ na,
-                   const int* __restrict__ base, const int64_t* __restrict__ coff,
-                   const float* __restrict__ q, float* __restrict__ u, float* __restrict__ grad,
-                   double* __restrict__ part, double* __restrict__ logp) {
-  __shared__ TileSmem sm;
-  const int total = base[T];
-  for (int tile = blockIdx.x; tile < total; tile += gridDim.x) {
-    const int t = member_of(base, T, tile);
-    const BDesc& d = desc[t];
-    const int local = tile - base[t];
+                   const int64_t* __restrict__ coff, const float* __restrict__ q,
+                   float* __restrict__ u, float* __restrict__ grad, double* __restrict__ part,
+                   double* __restrict__ logp) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  __shared__ int taken;
+  const int total = *total_dev, stretch = blockIdx.x / sms, place = blockIdx.x % sms;
+  int tile = stretch * sms + (stretch & 1 ? sms - 1 - place : place);
+  while (tile < total) {
+    const int2 at = tiles[tile];
+    const Group g = groups[at.x];
+    const BDesc& d = desc[g.member];
+    const int first = a[g.member], held = na[g.member];
     if (d.family == kBatchMvn) {
-      const int k = local / d.nob, ob = local % d.nob;
-      const int a0 = a[t] + k * d.ct;
-      const int nc = min(d.ct, na[t] - k * d.ct);
+      const int a0 = at.y * d.ct, nc = min(d.ct, held - a0);
       const float* X = PHASE == 0 ? q : u;
       float* out = PHASE == 0 ? u : grad;
       if (d.ct == 64)
-        mvn_tile<PHASE, 64>(d, act, a0, nc, ob, coff, X, out, part, logp, sm);
+        run_mvn<PHASE, 64, 8>(d, g.ob * kOB, act, first + a0, nc, coff, X, out, part, logp,
+                              smem);
       else
-        mvn_tile<PHASE, 32>(d, act, a0, nc, ob, coff, X, out, part, logp, sm);
+        run_mvn<PHASE, 32, 4>(d, g.ob * kOB, act, first + a0, nc, coff, X, out, part, logp,
+                              smem);
     } else if (PHASE == 0) {
-      const int a0 = a[t] + local * kHierChains;
-      hier_tile(d, act, a0, min(kHierChains, na[t] - local * kHierChains), coff, q, logp, grad);
+      const int a0 = at.y * kHierChains;
+      hier_tile(d, act, first + a0, min(kHierChains, held - a0), coff, q, logp, grad);
     }
+    if (threadIdx.x == 0) taken = (int)gridDim.x + atomicAdd(next, 1);
+    __syncthreads();
+    tile = taken;
+    __syncthreads();   // every thread has it, and is done with shared memory
   }
 }
 
@@ -368,21 +287,17 @@ class BatchTarget final : public Target {
       d.c_begin = chains;
       d.c_end = chains + (int)m[t].chains;
       d.ct = 64;
-      d.nob = (d.dim + kOB - 1) / kOB;
       d.p_begin = parts;
       owned_.emplace_back(new Owned());
       Owned& o = *owned_.back();
       if (d.family == kBatchMvn) {
         o.a.reserve(sizeof(float) * d.dim);
-        o.b.reserve(sizeof(float) * (size_t)d.dim * d.dim);
+        o.b.reserve(mvn_factor_bytes(d.dim));
         GBM_CUDA(cudaMemcpyAsync(o.a.ptr, m[t].loc, sizeof(float) * d.dim,
                                  cudaMemcpyDeviceToDevice, ctx->stream));
-        GBM_CUDA(cudaMemcpyAsync(o.b.ptr, m[t].scale_tril_inv, sizeof(float) * d.dim * d.dim,
-                                 cudaMemcpyDeviceToDevice, ctx->stream));
-        d.loc = o.a.as<float>();
-        d.linv = o.b.as<float>();
-        d.log_norm = m[t].log_normalizer;
-        parts += (int64_t)m[t].chains * d.nob;
+        d.mvn = mvn_factor(m[t].scale_tril_inv, o.a.as<float>(), d.dim, m[t].log_normalizer,
+                           o.b.as<float>(), ctx->stream);
+        parts += (int64_t)m[t].chains * mvn_parts(d.dim);
       } else {
         const int J = d.dim - 2;
         o.a.reserve(sizeof(float) * J);
@@ -427,16 +342,16 @@ class BatchTarget final : public Target {
     desc_.reserve(sizeof(BDesc) * T_);
     u_.reserve(sizeof(float) * (size_t)E_);
     part_.reserve(sizeof(double) * (size_t)std::max<int64_t>(parts, 1));
-    sched_.reserve(sizeof(int) * (size_t)(6 * (T_ + 1)));
+    make_order(0, &order_[0]);
+    make_order(1, &order_[1]);
+    sched_.reserve(sizeof(int) * (size_t)(2 * T_ + 4));
     all_.reserve(sizeof(int) * (size_t)(C_ + 1));
-    // Persistent CTAs: as many as are resident at once (a second wave would
-    // start its share of the tile list late).
-    int occ0 = 0, occ1 = 0;
-    GBM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ0, batch_phase_kernel<0>,
-                                                           kThreads, 0));
-    GBM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ1, batch_phase_kernel<1>,
-                                                           kThreads, 0));
-    grid_ = std::max(1, std::min(occ0, occ1)) * ctx->num_sms;
+    iota_kernel<<<(C_ + 255) / 256, 256, 0, ctx->stream>>>(all_.as<int>(), C_,
+                                                           all_.as<int>() + C_);
+    GBM_CUDA(cudaGetLastError());
+    sms_ = ctx->num_sms;
+    prepare_phase<0>();
+    prepare_phase<1>();
     upload();
     GBM_CUDA(cudaStreamSynchronize(ctx->stream));
     autotune();
@@ -456,25 +371,25 @@ class BatchTarget final : public Target {
   void eval(const float* q, int, const int*, int, double* logp, float* grad, int, void*,
             cudaStream_t s) override {
     int* idx = all_.as<int>();
-    iota_kernel<<<(C_ + 255) / 256, 256, 0, s>>>(idx, C_, idx + C_);
-    GBM_CUDA(cudaGetLastError());
     eval_active(q, idx, idx + C_, logp, grad, nullptr, s);
   }
 
   void eval_active(const float* q, const int* act, const int* act_count, double* logp,
                    float* grad, void*, cudaStream_t s) override {
-    int* w = sched_.as<int>();
-    const int T1 = T_ + 1;
-    int *a = w, *na = w + T1, *t1 = w + 2 * T1, *t2 = w + 3 * T1, *b1 = w + 4 * T1,
-        *b2 = w + 5 * T1;
+    int *a = sched_.as<int>(), *na = a + T_, *totals = a + 2 * T_, *next = totals + 2;
     const BDesc* d = desc_.as<BDesc>();
-    batch_schedule_kernel<<<1, 1024, 0, s>>>(d, T_, act, act_count, a, na, t1, t2, b1, b2);
-    batch_phase_kernel<0><<<grid_, kThreads, 0, s>>>(d, T_, act, a, na, b1, coff_.as<int64_t>(),
-                                                     q, u_.as<float>(), grad,
-                                                     part_.as<double>(), logp);
-    batch_phase_kernel<1><<<grid_, kThreads, 0, s>>>(d, T_, act, a, na, b2, coff_.as<int64_t>(),
-                                                     q, u_.as<float>(), grad,
-                                                     part_.as<double>(), logp);
+    const Group *g0 = order_[0].groups.as<Group>(), *g1 = order_[1].groups.as<Group>();
+    int2 *t0 = order_[0].tiles.as<int2>(), *t1 = order_[1].tiles.as<int2>();
+    batch_schedule_kernel<<<2, 1024, 0, s>>>(d, T_, act, act_count, g0, g1, order_[0].count,
+                                             order_[1].count, a, na, t0, t1, totals, next);
+    batch_phase_kernel<0><<<grid_[0], kThreads, PhaseLaunch<0>::kSmem, s>>>(
+        d, g0, t0, totals, next, sms_, act, a, na, coff_.as<int64_t>(), q, u_.as<float>(), grad,
+        part_.as<double>(), logp);
+    if (order_[1].count > 0)
+      batch_phase_kernel<1>
+          <<<grid_[1], kThreads * PhaseLaunch<1>::kGroups, PhaseLaunch<1>::kSmem, s>>>(
+              d, g1, t1, totals + 1, next + 1, sms_, act, a, na, coff_.as<int64_t>(), q,
+              u_.as<float>(), grad, part_.as<double>(), logp);
     GBM_CUDA(cudaGetLastError());
   }
 
@@ -505,6 +420,56 @@ class BatchTarget final : public Target {
   struct Owned {
     DeviceBuffer a, b;
   };
+
+  // As many CTAs as are resident at once, whole stretches of the SMs.
+  template <int PHASE>
+  void prepare_phase() {
+    constexpr int threads = kThreads * PhaseLaunch<PHASE>::kGroups;
+    GBM_CUDA(cudaFuncSetAttribute(batch_phase_kernel<PHASE>,
+                                  cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  PhaseLaunch<PHASE>::kSmem));
+    int per_sm = 0;
+    GBM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, batch_phase_kernel<PHASE>,
+                                                           threads, PhaseLaunch<PHASE>::kSmem));
+    grid_[PHASE] = std::max(1, per_sm) * sms_;
+  }
+
+  struct Order {
+    int count = 0;              // groups
+    DeviceBuffer groups, tiles;
+  };
+
+  // The groups of a phase, those with the longest sums first (hierarchical
+  // tiles, short, at the end of phase 0), and room for their tiles.
+  void make_order(int phase, Order* order) {
+    std::vector<Group> groups;
+    size_t tiles = 0;
+    for (int t = 0; t < T_; ++t) {
+      const BDesc& d = hdesc_[t];
+      const int chains = d.c_end - d.c_begin;
+      if (d.family == kBatchMvn) {
+        const int nob = (d.dim + kOB - 1) / kOB;
+        for (int ob = 0; ob < nob; ++ob) groups.push_back(Group{t, ob});
+        tiles += (size_t)nob * ((chains + 31) / 32);
+      } else if (phase == 0) {
+        groups.push_back(Group{t, 0});
+        tiles += (size_t)(chains + kHierChains - 1) / kHierChains;
+      }
+    }
+    auto length = [&](const Group& g) {
+      const BDesc& d = hdesc_[g.member];
+      if (d.family != kBatchMvn) return 0;
+      return phase == 0 ? std::min(d.dim, (g.ob + 1) * kOB) : d.dim - g.ob * kOB;
+    };
+    std::stable_sort(groups.begin(), groups.end(),
+                     [&](const Group& x, const Group& y) { return length(x) > length(y); });
+    order->count = (int)groups.size();
+    order->groups.reserve(sizeof(Group) * std::max<size_t>(groups.size(), 1));
+    order->tiles.reserve(sizeof(int2) * std::max<size_t>(tiles, 1));
+    GBM_CUDA(cudaMemcpyAsync(order->groups.ptr, groups.data(), sizeof(Group) * groups.size(),
+                             cudaMemcpyHostToDevice, ctx_->stream));
+    GBM_CUDA(cudaStreamSynchronize(ctx_->stream));   // the vector is this call's
+  }
 
   // The hierarchical members whose chains fit a warp's registers.
   void set_chain_models(gbm_context* ctx) {
@@ -588,10 +553,11 @@ class BatchTarget final : public Target {
   }
 
   gbm_context* ctx_;
-  int T_ = 0, C_ = 0, grid_ = 0;
+  int T_ = 0, C_ = 0, sms_ = 0, grid_[2] = {0, 0};
   int64_t E_ = 0;
   int chosen_[kClasses] = {0, 0, 0, 0};
   std::vector<BDesc> hdesc_;
+  Order order_[2];
   std::vector<std::unique_ptr<Owned>> owned_;
   DeviceBuffer desc_, coff_, cdim_, u_, part_, sched_, all_, models_, model_of_, table_;
   ChainModels chain_models_{};

@@ -7,9 +7,9 @@
 // caller (computed once from scale_tril).  Working with L^-1 keeps the
 // conditioning of L (the square root of the covariance's) -- multiplying by
 // the precision L^-T L^-1 in FP32 would square it.  Both products are
-// register-tiled triangular GEMMs over all chains on the CUDA cores; each CTA
-// of the first also forms its slice of |u|^2 and a third kernel sums the
-// slices in fixed order (deterministic).
+// triangular GEMMs over all chains on the CUDA cores (mvn_tile.cuh), one launch
+// each; the first also forms sums of u^2 over 32 outputs, which the second adds
+// in fixed order (deterministic).
 //
 // Non-centred hierarchical normal, the eight-schools pattern of
 // mcmc/eight_schools_hmc.py:41-58 with mu ~ N(0, s_mu), tau ~ HalfCauchy(0,
@@ -21,131 +21,78 @@
 #include <memory>
 
 #include "engine.h"
+#include "mvn_tile.cuh"
 #include "nuts_chain.h"
 
 namespace gbm {
 namespace {
 
-constexpr int kTile = 64;     // chains x features per CTA tile
-constexpr int kKc = 32;       // K chunk
-constexpr int kMvnThreads = 256;
+// Two launches over (chain tiles, output blocks), the blocks with the longest
+// sums first.  The tile is 32 x 64 at every size: 32 x 32 and 64 x 64 (4 x 8 a
+// thread) tiles were slower from 8 x 32 chains to 2048 x 512 (777 x 350, before
+// phase 1 was cut: 56, 51 and 83 us), and four groups halve phase 1.
+constexpr int kMvnCT = 32, kMvnOB = 64;
 
-// Two triangular GEMMs over all chains with M = L^-1 (lower triangular):
-//   MODE 0:  U[c][i] = sum_{k <= i} (Q[c][k] - mu[k]) M[i][k],
-//            part[c][itile] = sum_{i in tile} U[c][i]^2
-//   MODE 1:  G[c][j] = -sum_{i >= j} U[c][i] M[i][j]
-// K-chunks that lie entirely in the zero triangle are skipped.
-template <int MODE>
-__global__ void __launch_bounds__(kMvnThreads)
-mvn_tri_kernel(const float* __restrict__ A, int lda, const int* __restrict__ n_dev, int D,
-               const float* __restrict__ mu, const float* __restrict__ M,
-               float* __restrict__ out, int ldo, double* __restrict__ part, int dtiles) {
-  const int n = *n_dev;
-  const int c0 = blockIdx.y * kTile, o0 = blockIdx.x * kTile;
+template <int PHASE>
+struct MvnLaunch {
+  static constexpr int kGroups = PHASE == 0 ? 1 : 4;
+  static constexpr int kThreads = kMvnCT / 4 * (kMvnOB / 4) * kGroups;
+  using Smem = MvnSmem<kMvnCT, kMvnOB, kGroups>;
+};
+
+template <int PHASE>
+__global__ void __launch_bounds__(MvnLaunch<PHASE>::kThreads)
+mvn_tri_kernel(MvnFactor f, const float* __restrict__ A, int lda, const int* __restrict__ n_dev,
+               float* __restrict__ out, int ldo, double* __restrict__ part,
+               double* __restrict__ logp) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  auto& sm = *reinterpret_cast<typename MvnLaunch<PHASE>::Smem*>(smem);
+  const int n = *n_dev, c0 = blockIdx.x * kMvnCT;
   if (c0 >= n) return;
-  __shared__ float As[kKc][kTile + 4];   // [k][chain]
-  __shared__ float Bs[kKc][kTile + 4];   // [k][output column]
-  __shared__ double red[16][kTile];
-  const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
-  float acc[4][4] = {};
-  const int k_begin = MODE == 0 ? 0 : (o0 / kKc) * kKc;
-  const int k_end = MODE == 0 ? min(D, o0 + kTile) : D;
-  for (int k0 = k_begin; k0 < k_end; k0 += kKc) {
-    for (int i = tid; i < kKc * kTile; i += kMvnThreads) {
-      const int kk = i % kKc, cc = i / kKc;
-      const int c = c0 + cc, k = k0 + kk;
-      float a = 0.f;
-      if (c < n && k < D) a = MODE == 0 ? A[(size_t)c * lda + k] - mu[k] : A[(size_t)c * lda + k];
-      As[kk][cc] = a;
-      if (MODE == 0) {        // B(k, i) = M[i][k]: k contiguous in memory
-        const int oo = i / kKc, o = o0 + oo;
-        Bs[kk][oo] = (o < D && k < D && k <= o) ? M[(size_t)o * D + k] : 0.f;
-      } else {                // B(i, j) = M[i][j]: j contiguous in memory
-        const int oo = i % kTile, kr = i / kTile;
-        const int o = o0 + oo, k2 = k0 + kr;
-        Bs[kr][oo] = (o < D && k2 < D && k2 >= o) ? M[(size_t)k2 * D + o] : 0.f;
-      }
-    }
-    __syncthreads();
-#pragma unroll 8
-    for (int kk = 0; kk < kKc; ++kk) {
-      const float4 a4 = *reinterpret_cast<const float4*>(&As[kk][ty * 4]);
-      const float4 b4 = *reinterpret_cast<const float4*>(&Bs[kk][tx * 4]);
-      const float aa[4] = {a4.x, a4.y, a4.z, a4.w};
-      const float bb[4] = {b4.x, b4.y, b4.z, b4.w};
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(aa[i], bb[j], acc[i][j]);
-    }
-    __syncthreads();
+  const int ob = PHASE == 0 ? (int)(gridDim.y - 1 - blockIdx.y) : (int)blockIdx.y;
+  if (threadIdx.x < kMvnCT) {
+    const int c = c0 + threadIdx.x;
+    sm.in[threadIdx.x] = (long long)c * lda;
+    sm.out[threadIdx.x] = (long long)c * ldo;
+    sm.part[threadIdx.x] = (long long)c * mvn_parts(f.dim);
+    sm.id[threadIdx.x] = c;
   }
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int c = c0 + ty * 4 + i;
-    double sq = 0.0;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int o = o0 + tx * 4 + j;
-      if (c < n && o < D) {
-        const float v = MODE == 0 ? acc[i][j] : -acc[i][j];
-        out[(size_t)c * ldo + o] = v;
-        sq += (double)v * (double)v;
-      }
-    }
-    if (MODE == 0) red[tx][ty * 4 + i] = sq;
-  }
-  if (MODE == 0) {
-    __syncthreads();
-    if (tid < kTile && c0 + tid < n) {
-      double s = 0.0;
-      for (int t = 0; t < 16; ++t) s += red[t][tid];
-      part[(size_t)(c0 + tid) * dtiles + blockIdx.x] = s;
-    }
-  }
-}
-
-__global__ void mvn_finish_kernel(const double* __restrict__ part, int dtiles,
-                                  const int* __restrict__ n_dev, double log_norm,
-                                  double* __restrict__ logp) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= *n_dev) return;
-  double s = 0.0;
-  for (int t = 0; t < dtiles; ++t) s += part[(size_t)c * dtiles + t];
-  logp[c] = -0.5 * s + log_norm;   // -1/2 |L^-1 (x - mu)|^2
+  mvn_tile<PHASE, kMvnCT, kMvnOB, 4, 4, MvnLaunch<PHASE>::kGroups>(
+      f, min(kMvnCT, n - c0), ob * kMvnOB, A, out, part, logp, sm);
 }
 
 class Mvn final : public Target {
  public:
-  Mvn(gbm_context* ctx, const float* loc, const float* scale_tril_inv, int64_t d, double log_norm)
-      : log_norm_(log_norm) {
+  Mvn(gbm_context* ctx, const float* loc, const float* scale_tril_inv, int64_t d,
+      double log_norm) {
     dim = d;
     mu_.reserve(sizeof(float) * d);
-    m_.reserve(sizeof(float) * d * d);
+    m_.reserve(mvn_factor_bytes(d));
     GBM_CUDA(cudaMemcpyAsync(mu_.ptr, loc, sizeof(float) * d, cudaMemcpyDeviceToDevice,
                              ctx->stream));
-    GBM_CUDA(cudaMemcpyAsync(m_.ptr, scale_tril_inv, sizeof(float) * d * d,
-                             cudaMemcpyDeviceToDevice, ctx->stream));
-    dtiles_ = (int)((d + kTile - 1) / kTile);
+    factor_ = mvn_factor(scale_tril_inv, mu_.as<float>(), d, log_norm, m_.as<float>(),
+                         ctx->stream);
+    GBM_CUDA(cudaFuncSetAttribute(mvn_tri_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)sizeof(MvnLaunch<0>::Smem)));
+    GBM_CUDA(cudaFuncSetAttribute(mvn_tri_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)sizeof(MvnLaunch<1>::Smem)));
   }
   size_t workspace_bytes(int64_t cap) const override {
-    return sizeof(double) * (size_t)cap * dtiles_ + sizeof(float) * (size_t)cap * dim + 512;
+    return sizeof(double) * (size_t)cap * mvn_parts(dim) + sizeof(float) * (size_t)cap * dim + 512;
   }
   void eval(const float* q, int ldq, const int* n_dev, int cap, double* logp, float* grad,
             int ldg, void* ws, cudaStream_t s) override {
     double* part = static_cast<double*>(ws);
-    float* u = reinterpret_cast<float*>(part + (size_t)cap * dtiles_);
-    dim3 grid(dtiles_, (cap + kTile - 1) / kTile);
+    float* u = reinterpret_cast<float*>(part + (size_t)cap * mvn_parts(dim));
     const int D = (int)dim;
-    mvn_tri_kernel<0><<<grid, kMvnThreads, 0, s>>>(q, ldq, n_dev, D, mu_.as<float>(),
-                                                   m_.as<float>(), u, D, part, dtiles_);
-    mvn_tri_kernel<1><<<grid, kMvnThreads, 0, s>>>(u, D, n_dev, D, mu_.as<float>(),
-                                                   m_.as<float>(), grad, ldg, part, dtiles_);
-    GBM_CUDA(cudaGetLastError());
-    mvn_finish_kernel<<<(cap + 255) / 256, 256, 0, s>>>(part, dtiles_, n_dev, log_norm_, logp);
+    const dim3 grid((cap + kMvnCT - 1) / kMvnCT, (D + kMvnOB - 1) / kMvnOB);
+    mvn_tri_kernel<0><<<grid, MvnLaunch<0>::kThreads, sizeof(MvnLaunch<0>::Smem), s>>>(
+        factor_, q, ldq, n_dev, u, D, part, logp);
+    mvn_tri_kernel<1><<<grid, MvnLaunch<1>::kThreads, sizeof(MvnLaunch<1>::Smem), s>>>(
+        factor_, u, D, n_dev, grad, ldg, part, logp);
     GBM_CUDA(cudaGetLastError());
   }
-  int launches_per_eval(int64_t) const override { return 3; }
+  int launches_per_eval(int64_t) const override { return 2; }
   // Two triangular GEMMs: ~D^2 multiply-adds each per chain.
   double flops(int64_t n) const override { return 2.0 * (double)dim * dim * n; }
   double bytes(int64_t n) const override {
@@ -153,8 +100,7 @@ class Mvn final : public Target {
   }
 
  private:
-  double log_norm_;
-  int dtiles_ = 1;
+  MvnFactor factor_{};
   DeviceBuffer mu_, m_;
 };
 

@@ -1,0 +1,149 @@
+// X as FP16 hi + lo of scaled features, for gradient products on the tensor
+// cores: X' = X 2^(kF16Top - exponent of the column's largest), and residuals
+// as hi + lo of R' = kF16Scale R, so that a product of FP16 pairs carries a float
+// to 2^-24 of itself and gscale turns it back.
+#pragma once
+#include <cuda_fp16.h>
+#include <cuda_runtime.h>
+
+#include <cmath>
+#include <vector>
+
+#include "engine.h"
+#include "tc_common.cuh"
+
+namespace gbm {
+namespace {
+
+constexpr float kF16Scale = 32768.f;        // R' = 2^15 R
+constexpr int kF16Top = 14;                 // X' < 2^15
+
+__device__ __forceinline__ int float_exponent(unsigned bits) {
+  return (int)((bits >> 23) & 255u) - 127;
+}
+
+// Largest |x| of each column, as bits.
+__global__ void column_max_kernel(const float* __restrict__ X, int64_t N, int D, int64_t chunk,
+                                  unsigned* __restrict__ out) {
+  const int64_t r0 = (int64_t)blockIdx.x * chunk, r1 = r0 + chunk < N ? r0 + chunk : N;
+  for (int d = threadIdx.x; d < D; d += blockDim.x) {
+    unsigned m = 0;
+#pragma unroll 8
+    for (int64_t r = r0; r < r1; ++r) m = max(m, __float_as_uint(X[r * D + d]) & 0x7fffffffu);
+    if (m) atomicMax(&out[d], m);
+  }
+}
+
+// X [N][D] -> X' = X 2^(kF16Top - exponent of the column's largest) as FP16 hi
+// + lo [N][Dp], zero-padded; rows [b chunk, (b + 1) chunk) also sum X'^2 and
+// the square of what hi + lo leaves of it into part[b][d].
+__global__ void f16_pack_kernel(const float* __restrict__ X, int64_t N, int D, int Dp,
+                                int64_t chunk, const unsigned* __restrict__ max_bits,
+                                __half* __restrict__ hi, __half* __restrict__ lo,
+                                float2* __restrict__ part) {
+  const int64_t r0 = (int64_t)blockIdx.x * chunk, r1 = r0 + chunk < N ? r0 + chunk : N;
+  for (int d = threadIdx.x; d < Dp; d += blockDim.x) {
+    const int shift = d < D ? kF16Top - float_exponent(max_bits[d]) : 0;
+    float2 acc = make_float2(0.f, 0.f);
+#pragma unroll 4
+    for (int64_t r = r0; r < r1; ++r) {
+      const float v = d < D ? ldexpf(X[r * D + d], shift) : 0.f;
+      const __half h = __float2half_rn(v);
+      const float rest = v - __half2float(h);
+      const __half l = __float2half_rn(rest);
+      hi[r * Dp + d] = h;
+      lo[r * Dp + d] = l;
+      const float left = rest - __half2float(l);
+      acc.x = fmaf(v, v, acc.x);
+      acc.y = fmaf(left, left, acc.y);
+    }
+    if (d < D) part[(size_t)blockIdx.x * D + d] = acc;
+  }
+}
+
+// Sums of part over blocks: one block per feature, fixed order.
+__global__ void __launch_bounds__(128)
+column_rest_kernel(const float2* __restrict__ part, int nb, int D, double2* __restrict__ out) {
+  __shared__ double2 sh[128];
+  const int d = blockIdx.x, tid = threadIdx.x;
+  double2 acc = make_double2(0.0, 0.0);
+  for (int b = tid; b < nb; b += 128) {
+    acc.x += (double)part[(size_t)b * D + d].x;
+    acc.y += (double)part[(size_t)b * D + d].y;
+  }
+  sh[tid] = acc;
+  for (int o = 64; o > 0; o >>= 1) {
+    __syncthreads();
+    if (tid < o) {
+      sh[tid].x += sh[tid + o].x;
+      sh[tid].y += sh[tid + o].y;
+    }
+  }
+  if (tid == 0) out[d] = sh[0];
+}
+
+struct F16Rows {
+  DeviceBuffer mem;             // hi, lo [N][dp], gscale [D]
+  float* gscale = nullptr;      // from G' to G; zero for a column of zeros
+  CUtensorMap hi, lo;           // boxes of 64 features x box_rows rows
+
+  // False if X (or the labels, ym = y - 1/2) does not fit the form: infinities,
+  // NaN, exponents that the scaling cannot carry, or a range so wide that hi + lo
+  // leaves more than 2^-23 of a column in root mean square (a normal sample:
+  // 2^-25); a label so far outside [0, 1] that a residual, below |y - 1/2| + 1/2,
+  // could leave FP16's range (R' < 2^16); more than kMost elements (the form is as
+  // large as X in float32: beyond 16 GB the memory is the caller's).
+  bool prepare(gbm_context* ctx, const float* X, const float* ym, int64_t N, int D, int dp,
+               int box_rows) {
+    constexpr int64_t kMost = (int64_t)1 << 32;
+    if (N * dp > kMost) return false;
+    cudaStream_t s = ctx->stream;
+    const int nb = 8 * ctx->num_sms;
+    const int64_t chunk = (N + nb - 1) / nb;
+    const size_t off_part = (sizeof(unsigned) * (D + 1) + 255) / 256 * 256;
+    const size_t off_sum = off_part + (sizeof(float2) * (size_t)nb * D + 255) / 256 * 256;
+    DeviceBuffer buf;
+    buf.reserve(off_sum + sizeof(double2) * D);
+    unsigned* mx = buf.as<unsigned>();
+    float2* part = reinterpret_cast<float2*>(buf.as<char>() + off_part);
+    double2* sum = reinterpret_cast<double2*>(buf.as<char>() + off_sum);
+    const size_t bytes = sizeof(__half) * (size_t)N * dp;
+    mem.reserve(2 * bytes + sizeof(float) * D);
+    __half* h = mem.as<__half>();
+    __half* l = h + (size_t)N * dp;
+    gscale = reinterpret_cast<float*>(mem.as<char>() + 2 * bytes);
+    GBM_CUDA(cudaMemsetAsync(mx, 0, sizeof(unsigned) * (D + 1), s));
+    column_max_kernel<<<nb, 128, 0, s>>>(X, N, D, chunk, mx);
+    column_max_kernel<<<nb, 32, 0, s>>>(ym, N, 1, chunk, mx + D);
+    f16_pack_kernel<<<nb, 128, 0, s>>>(X, N, D, dp, chunk, mx, h, l, part);
+    column_rest_kernel<<<(unsigned)D, 128, 0, s>>>(part, nb, D, sum);
+    GBM_CUDA(cudaGetLastError());
+    std::vector<unsigned> hmax(D + 1);
+    std::vector<double2> hsum(D);
+    GBM_CUDA(cudaMemcpyAsync(hmax.data(), mx, sizeof(unsigned) * (D + 1), cudaMemcpyDeviceToHost,
+                             s));
+    GBM_CUDA(cudaMemcpyAsync(hsum.data(), sum, sizeof(double2) * D, cudaMemcpyDeviceToHost, s));
+    GBM_CUDA(cudaStreamSynchronize(s));
+    std::vector<float> gs(D, 0.f);
+    constexpr unsigned kLabelTop = 0x3fa00000u;   // 1.25f
+    bool fits = hmax[D] <= kLabelTop;
+    for (int i = 0; i < D; ++i) {
+      if (hmax[i] == 0) continue;
+      const int fexp = (int)((hmax[i] >> 23) & 255u) - 127;
+      fits = fits && fexp >= -60 && fexp <= 60 && hsum[i].y <= std::ldexp(hsum[i].x, -46);
+      gs[i] = std::ldexp(1.f, fexp - kF16Top - 15);
+    }
+    if (!fits) {
+      mem.release();
+      return false;
+    }
+    GBM_CUDA(cudaMemcpyAsync(gscale, gs.data(), sizeof(float) * D, cudaMemcpyHostToDevice, s));
+    GBM_CUDA(cudaStreamSynchronize(s));   // gs ends here
+    encode_rows(&hi, h, N, dp, box_rows);
+    encode_rows(&lo, l, N, dp, box_rows);
+    return true;
+  }
+};
+
+}  // namespace
+}  // namespace gbm

@@ -47,9 +47,9 @@
 #include <algorithm>
 #include <cmath>
 #include <memory>
-#include <vector>
 
 #include "engine.h"
+#include "f16_rows.cuh"
 #include "split_reduce.cuh"
 #include "tc_common.cuh"
 #include "tc_ptx.cuh"
@@ -395,8 +395,6 @@ logreg_f32_kernel(const float* __restrict__ X2, const float* __restrict__ ym, in
 // (344), 54 at 4 and 256 chains (72).
 // ---------------------------------------------------------------------------
 constexpr int kF32TcThreads = kF32Threads + 64;
-constexpr float kF16Scale = 32768.f;        // R' = 2^15 R
-constexpr int kF16Top = 14;                 // X' = X 2^(kF16Top - fexp) < 2^15
 constexpr int kHalf = kF32RT / 2;           // rows of a tile in each group
 constexpr int kRBox = kHalf * 128;          // [32 rows][128 B]: 64 chains
 constexpr int kXBox = 2 * kRBox;            // [2 tiles][32 rows][128 B]: 64 features
@@ -743,71 +741,6 @@ __global__ void f32_pack_kernel(const float* __restrict__ X, const float* __rest
   X2[((r >> 1) * Dp + d) * 2 + (r & 1)] = (r < N && d < D) ? X[r * D + d] : 0.f;
 }
 
-// ---- FP16 form of X ----
-__device__ __forceinline__ int float_exponent(unsigned bits) {
-  return (int)((bits >> 23) & 255u) - 127;
-}
-
-// Largest |x| of each column, as bits.
-__global__ void column_max_kernel(const float* __restrict__ X, int64_t N, int D, int64_t chunk,
-                                  unsigned* __restrict__ out) {
-  const int64_t r0 = (int64_t)blockIdx.x * chunk, r1 = r0 + chunk < N ? r0 + chunk : N;
-  for (int d = threadIdx.x; d < D; d += blockDim.x) {
-    unsigned m = 0;
-#pragma unroll 8
-    for (int64_t r = r0; r < r1; ++r) m = max(m, __float_as_uint(X[r * D + d]) & 0x7fffffffu);
-    if (m) atomicMax(&out[d], m);
-  }
-}
-
-// X [N][D] -> X' = X 2^(kF16Top - exponent of the column's largest) as FP16 hi
-// + lo [N][Dp], zero-padded; rows [b chunk, (b + 1) chunk) also sum X'^2 and
-// the square of what hi + lo leaves of it into part[b][d].
-__global__ void f16_pack_kernel(const float* __restrict__ X, int64_t N, int D, int Dp,
-                                int64_t chunk, const unsigned* __restrict__ max_bits,
-                                __half* __restrict__ hi, __half* __restrict__ lo,
-                                float2* __restrict__ part) {
-  const int64_t r0 = (int64_t)blockIdx.x * chunk, r1 = r0 + chunk < N ? r0 + chunk : N;
-  for (int d = threadIdx.x; d < Dp; d += blockDim.x) {
-    const int shift = d < D ? kF16Top - float_exponent(max_bits[d]) : 0;
-    float2 acc = make_float2(0.f, 0.f);
-#pragma unroll 4
-    for (int64_t r = r0; r < r1; ++r) {
-      const float v = d < D ? ldexpf(X[r * D + d], shift) : 0.f;
-      const __half h = __float2half_rn(v);
-      const float rest = v - __half2float(h);
-      const __half l = __float2half_rn(rest);
-      hi[r * Dp + d] = h;
-      lo[r * Dp + d] = l;
-      const float left = rest - __half2float(l);
-      acc.x = fmaf(v, v, acc.x);
-      acc.y = fmaf(left, left, acc.y);
-    }
-    if (d < D) part[(size_t)blockIdx.x * D + d] = acc;
-  }
-}
-
-// Sums of part over blocks: one block per feature, fixed order.
-__global__ void __launch_bounds__(128)
-column_rest_kernel(const float2* __restrict__ part, int nb, int D, double2* __restrict__ out) {
-  __shared__ double2 sh[128];
-  const int d = blockIdx.x, tid = threadIdx.x;
-  double2 acc = make_double2(0.0, 0.0);
-  for (int b = tid; b < nb; b += 128) {
-    acc.x += (double)part[(size_t)b * D + d].x;
-    acc.y += (double)part[(size_t)b * D + d].y;
-  }
-  sh[tid] = acc;
-  for (int o = 64; o > 0; o >>= 1) {
-    __syncthreads();
-    if (tid < o) {
-      sh[tid].x += sh[tid + o].x;
-      sh[tid].y += sh[tid + o].y;
-    }
-  }
-  if (tid == 0) out[d] = sh[0];
-}
-
 // lin[d] = sum_r (y_r - 1/2) X[r][d] in float64 and a fixed order: block b
 // sums rows [b chunk, (b + 1) chunk) into part[b][d]; blocks added in order.
 __global__ void f32_lin_partial(const float* __restrict__ X, const float* __restrict__ y,
@@ -882,7 +815,7 @@ class LogregF32 final : public Target {
     log_norm_ = -log((double)prior_scale) - 0.5 * log(2.0 * M_PI);
     grid_ = ctx->num_sms;
     err_dev_ = ctx->err_dev;
-    tc_ = n >= kTcMinRows && prepare_f16(ctx, X);
+    tc_ = n >= kTcMinRows && x16_.prepare(ctx, X, ym_.as<float>(), N_, (int)D_, dp_, kHalf);
     switch (kd_) {
       case 1: f32_set_smem<1>(); break;
       case 2: f32_set_smem<2>(); break;
@@ -914,7 +847,7 @@ class LogregF32 final : public Target {
 #define GBM_F32_LAUNCH(KD_)                                                                \
   if (tc_)                                                                                 \
     logreg_f32_tc_kernel<KD_><<<g, kF32TcThreads, F32TcLayout<KD_>::kBytes, s>>>(             \
-        himap_, lomap_, x2_.as<float>(), ym_.as<float>(), gscale_, N, D, qc, ldq,  \
+        x16_.hi, x16_.lo, x2_.as<float>(), ym_.as<float>(), x16_.gscale, N, D, qc, ldq,\
         n_dev, base, lim, g, lpart, gpart, err_dev_);                                        \
   else                                                                                     \
     logreg_f32_kernel<KD_><<<g, kF32Threads, F32Layout<KD_>::kBytes, s>>>(                    \
@@ -946,58 +879,6 @@ class LogregF32 final : public Target {
   }
 
  private:
-  // X as FP16 hi + lo of scaled features; false if a column does not fit that:
-  // infinities, NaN, exponents that the scaling cannot carry, or a range so
-  // wide that hi + lo leaves more than 2^-23 of it in root mean square (a normal
-  // sample: 2^-25); or if a label is so far outside [0, 1] that a residual,
-  // below |y - 1/2| + 1/2, could leave FP16's range (R' < 2^16).
-  bool prepare_f16(gbm_context* ctx, const float* X) {
-    cudaStream_t s = ctx->stream;
-    const int D = (int)D_, nb = 8 * ctx->num_sms;
-    const int64_t chunk = (N_ + nb - 1) / nb;
-    const size_t off_part = 1024;
-    const size_t off_sum = off_part + (sizeof(float2) * (size_t)nb * D + 255) / 256 * 256;
-    DeviceBuffer buf;
-    buf.reserve(off_sum + sizeof(double2) * D);
-    unsigned* mx = buf.as<unsigned>();
-    float2* part = reinterpret_cast<float2*>(buf.as<char>() + off_part);
-    double2* sum = reinterpret_cast<double2*>(buf.as<char>() + off_sum);
-    const size_t x16 = sizeof(__half) * (size_t)N_ * dp_;
-    x16_.reserve(2 * x16 + sizeof(float) * D);   // hi, lo (32-byte rows), scales
-    __half* hi = x16_.as<__half>();
-    __half* lo = hi + (size_t)N_ * dp_;
-    gscale_ = reinterpret_cast<float*>(x16_.as<char>() + 2 * x16);
-    GBM_CUDA(cudaMemsetAsync(mx, 0, sizeof(unsigned) * (D + 1), s));
-    column_max_kernel<<<nb, 128, 0, s>>>(X, N_, D, chunk, mx);
-    column_max_kernel<<<nb, 32, 0, s>>>(ym_.as<float>(), N_, 1, chunk, mx + D);
-    f16_pack_kernel<<<nb, 128, 0, s>>>(X, N_, D, dp_, chunk, mx, hi, lo, part);
-    column_rest_kernel<<<(unsigned)D, 128, 0, s>>>(part, nb, D, sum);
-    GBM_CUDA(cudaGetLastError());
-    std::vector<unsigned> hmax(D + 1);
-    std::vector<double2> hsum(D);
-    GBM_CUDA(cudaMemcpyAsync(hmax.data(), mx, sizeof(unsigned) * (D + 1), cudaMemcpyDeviceToHost, s));
-    GBM_CUDA(cudaMemcpyAsync(hsum.data(), sum, sizeof(double2) * D, cudaMemcpyDeviceToHost, s));
-    GBM_CUDA(cudaStreamSynchronize(s));
-    std::vector<float> gs(D, 0.f);   // from G' to G; a column of zeros stays zero
-    constexpr unsigned kLabelTop = 0x3fa00000u;   // 1.25f
-    bool fits = hmax[D] <= kLabelTop;
-    for (int i = 0; i < D; ++i) {
-      if (hmax[i] == 0) continue;
-      const int fexp = (int)((hmax[i] >> 23) & 255u) - 127;
-      fits = fits && fexp >= -60 && fexp <= 60 && hsum[i].y <= std::ldexp(hsum[i].x, -46);
-      gs[i] = std::ldexp(1.f, fexp - kF16Top - 15);
-    }
-    if (!fits) {
-      x16_.release();
-      return false;
-    }
-    GBM_CUDA(cudaMemcpyAsync(gscale_, gs.data(), sizeof(float) * D, cudaMemcpyHostToDevice, s));
-    GBM_CUDA(cudaStreamSynchronize(s));   // gs ends here
-    encode_rows(&himap_, hi, N_, dp_, kHalf);
-    encode_rows(&lomap_, lo, N_, dp_, kHalf);
-    return true;
-  }
-
   int64_t N_, D_, n2_ = 0;
   int kd_ = 1, dp_ = 16, grid_ = 0;
   float inv_var_ = 1.f;
@@ -1005,9 +886,7 @@ class LogregF32 final : public Target {
   int* err_dev_ = nullptr;
   DeviceBuffer x2_, ym_, lin_;
   bool tc_ = false;            // phase 2 on the tensor cores
-  DeviceBuffer x16_;
-  float* gscale_ = nullptr;    // within x16_
-  CUtensorMap himap_, lomap_;
+  F16Rows x16_;
 };
 
 }  // namespace

@@ -15,8 +15,11 @@
 // X_hi B_hi^T + X_hi B_lo^T (+ X_lo B_hi^T) and X_hi^T R_hi + X_hi^T R_lo
 // (+ X_lo^T R_hi) are accumulated in FP32 -- the residual correction of the
 // fused tensor-core kernels.  The hi and lo splits sit side by side as 2n
-// columns, so each contraction is one GEMM (plus one for X_lo).  FP32: both
-// GEMMs in FP32 (no TF32).
+// columns, so each contraction is one GEMM (plus one for X_lo).  FP32: Z in
+// FP32 (no TF32); X^T R from FP16 pairs on the tensor cores (grad_tc.cuh, whose
+// partials the split reduction adds), or in FP32 where the data do not fit those.
+// 12,289 x 601, 99 chains: 121 us with both GEMMs in FP32, 93 so;
+// 60,000 x 1000, 256 chains: 1238 and 718.
 //
 // This target evaluates all `cap` states of a call (the GEMM shapes are host
 // values): a sampler's inactive rows are computed and ignored.  Every GEMM
@@ -31,6 +34,7 @@
 #include <string>
 
 #include "engine.h"
+#include "grad_tc.cuh"
 #include "tc_ptx.cuh"
 
 namespace gbm {
@@ -40,6 +44,10 @@ constexpr size_t kCublasWs = 32u << 20;   // cuBLAS workspace inside the target 
 constexpr int kRowBlock = 2048;           // rows per epilogue block
 constexpr int kEpiThreads = 256;          // epilogue block size
 constexpr int kEpiRows = kRowBlock / kEpiThreads;
+// Rows from which the FP32 target's X^T R comes from FP16 pairs.  Faster below,
+// too (2001 x 300, 64 chains: 61 against 83 us), but there the FP32 GEMM, with few
+// additions, is the more exact one (1.5e-7 of the gradient against 1.8e-7).
+constexpr int64_t kTcMinRows = 4096;
 constexpr float kNegLog2eL = -1.4426950408889634f;
 constexpr float kLn2L = 0.6931471805599453f;
 
@@ -64,6 +72,14 @@ template <class T> __device__ __forceinline__ T from_float(float v);
 template <> __device__ __forceinline__ float from_float<float>(float v) { return v; }
 template <> __device__ __forceinline__ __nv_bfloat16 from_float<__nv_bfloat16>(float v) {
   return __float2bfloat16_rn(v);
+}
+
+// What a residual is stored as: its multiple and, for FP16 pairs, the negative
+// of the likelihood sums (the split reduction adds, large_finish subtracts).
+template <class TO> struct Stored { static constexpr float kScale = 1.f, kSign = 1.f; };
+template <> struct Stored<__half> { static constexpr float kScale = kF16Scale, kSign = -1.f; };
+template <> __device__ __forceinline__ __half from_float<__half>(float v) {
+  return __float2half_rn(v);
 }
 
 // X [N][D] (float32 or BF16) -> hi [Np][ld] (and lo for FP32 data in the
@@ -161,7 +177,7 @@ large_epilogue(const float* __restrict__ Z, const float* __restrict__ Zlo,
       const float u = 1.f + e;
       acc += fmaf(kLn2L, tc::lg2_approx(u), 0.5f * a);
       const float w = tc::rcp_approx(u) - 0.5f;
-      const float rv = zv[k] >= 0.f ? yv[k] - w : yv[k] + w;
+      const float rv = (zv[k] >= 0.f ? yv[k] - w : yv[k] + w) * Stored<TO>::kScale;
       const TO h = from_float<TO>(rv);
       Rhi[(size_t)c * ldz + r] = h;
       if (Rlo) Rlo[(size_t)c * ldz + r] = from_float<TO>(rv - (float)h);
@@ -173,7 +189,7 @@ large_epilogue(const float* __restrict__ Z, const float* __restrict__ Zlo,
     if (threadIdx.x == 0) {
       double s = 0.0;
       for (int w = 0; w < (int)(blockDim.x >> 5); ++w) s += red[w];
-      part[(size_t)blockIdx.x * n + c] = s;
+      part[(size_t)blockIdx.x * n + c] = (double)Stored<TO>::kSign * s;
     }
   }
 }
@@ -247,6 +263,12 @@ class LogregLarge final : public Target {
       GBM_CUDA(cudaGetLastError());
       GBM_CUDA(cudaStreamSynchronize(s));   // `part` is freed on scope exit
     }
+    sms_ = ctx->num_sms;
+    err_dev_ = ctx->err_dev;
+    dp_ = (int)((d + 15) / 16 * 16);
+    tc_ = !mixed && n >= kTcMinRows && x16_.prepare(ctx, static_cast<const float*>(X), ym_.as<float>(), N_, (int)D_,
+                                 dp_, kGradRT);
+    if (tc_) grad_tc_setup<true>();
     inv_var_ = 1.f / (prior_scale * prior_scale);
     log_norm_ = -log((double)prior_scale) - 0.5 * log(2.0 * M_PI);
   }
@@ -256,13 +278,13 @@ class LogregLarge final : public Target {
   // halves are added in FP32 by the epilogue (Z) and the finish (G).
   int sets() const { return mixed_ ? 2 : 1; }
 
-  // [B (sets x n rows) | Z (Np x sets n) | R | G (ld x sets n) | partials |
-  //  cuBLAS workspace]
+  // [B (sets x n rows) | Z (Np x sets n) | R | G (ld x sets n, or the gradient
+  //  partials) | partials | cuBLAS workspace]
   size_t workspace_bytes(int64_t cap) const override {
     const size_t el = mixed_ ? 2 : 4, w = (size_t)sets() * cap;
     const size_t nblk = (size_t)((N_ + kRowBlock - 1) / kRowBlock);
     return align256(el * w * ld_) + align256(4 * (size_t)ldz_ * w) +
-           align256(el * (size_t)ldz_ * w) + align256(4 * w * ld_) + align256(8 * nblk * cap) +
+           align256(el * (size_t)ldz_ * w) + align256(g_bytes(cap)) + align256(8 * nblk * cap) +
            kCublasWs;
   }
 
@@ -275,7 +297,7 @@ class LogregLarge final : public Target {
     unsigned char* B = p;          p += align256(el * (size_t)w * ld_);
     float* Z = reinterpret_cast<float*>(p);    p += align256(4 * (size_t)ldz_ * w);
     unsigned char* R = p;          p += align256(el * (size_t)ldz_ * w);
-    float* G = reinterpret_cast<float*>(p);    p += align256(4 * (size_t)w * ld_);
+    float* G = reinterpret_cast<float*>(p);    p += align256(g_bytes(cap));
     double* part = reinterpret_cast<double*>(p); p += align256(8 * (size_t)nblk * cap);
     void* cws = p;
     cublasHandle_t h = thread_handle(device_);
@@ -312,10 +334,24 @@ class LogregLarge final : public Target {
       large_epilogue<__nv_bfloat16><<<eg, kEpiThreads, 0, s>>>(
           Z, Zlo, ym_.as<float>(), N_, ldz_, n, reinterpret_cast<__nv_bfloat16*>(R),
           reinterpret_cast<__nv_bfloat16*>(R) + (size_t)n * ldz_, part);
+    else if (tc_)
+      large_epilogue<__half><<<eg, kEpiThreads, 0, s>>>(Z, nullptr, ym_.as<float>(), N_, ldz_, n,
+                                                reinterpret_cast<__half*>(R),
+                                                reinterpret_cast<__half*>(R) + (size_t)n * ldz_,
+                                                part);
     else
       large_epilogue<float><<<eg, kEpiThreads, 0, s>>>(Z, nullptr, ym_.as<float>(), N_, ldz_, n,
                                                reinterpret_cast<float*>(R), nullptr, part);
     GBM_CUDA(cudaGetLastError());
+    if (tc_) {
+      __half* r = reinterpret_cast<__half*>(R);
+      const int g = grad_tc_grid(sms_, n, N_, dp_);
+      launch_grad_tc<true>(x16_, r, r + (size_t)n * ldz_, ldz_, (int)N_, D, dp_, nullptr, 0, n, n,
+                           g, G, err_dev_, s);
+      launch_split_reduce(part, G, q, ldq, nullptr, 0, n, n, kGradCT, kGradRT, g, (int)N_, D,
+                          inv_var_, log_norm_, lin_.as<double>(), logp, grad, ldg, s, (int)nblk);
+      return;
+    }
     // G^T = X_hi^T [R_hi | R_lo] (+ X_lo^T R_hi into the first n columns):
     // column-major (ld x w) over all ld_ padded features (rows >= D come out
     // zero and are not read) and the Np padded rows (zero residuals).
@@ -332,15 +368,24 @@ class LogregLarge final : public Target {
     GBM_CUDA(cudaGetLastError());
   }
 
-  // split, epilogue, finish + the GEMMs (library kernels, not counted).
-  int launches_per_eval(int64_t) const override { return 3; }
+  // split, epilogue, finish (or gradient and reduction) + the GEMMs (library
+  // kernels, not counted).
+  int launches_per_eval(int64_t) const override { return tc_ ? 4 : 3; }
   double flops(int64_t n) const override { return 4.0 * (double)N_ * D_ * n; }
   double bytes(int64_t n) const override {
     return (mixed_ ? 2.0 : 4.0) * (double)N_ * D_ + 4.0 * N_ + 8.0 * (double)n * D_ + 8.0 * n;
   }
 
  private:
+  size_t g_bytes(int64_t cap) const {
+    return tc_ ? 4 * grad_tc_rows(sms_, cap, dp_) * (size_t)D_ : 4 * (size_t)sets() * cap * ld_;
+  }
+
   int64_t N_, D_;
+  bool tc_ = false;              // X^T R from FP16 pairs
+  int sms_ = 1, dp_ = 16;
+  int* err_dev_ = nullptr;
+  F16Rows x16_;
   bool mixed_, xlo_ = false;
   int device_ = 0, ld_ = 8;
   int64_t ldz_ = 8;   // leading dimension of Z and R: N rounded up to 8 rows

@@ -16,6 +16,10 @@
 // from HBM/L2 once per chain tile and Z/R never leave the SM.  Each CTA
 // writes one partial (logp, G); a second kernel sums the partials in fixed
 // split order (deterministic) and adds the prior.
+//
+// This is the form that needs no prepared copies of X: the allocation-free entry
+// point runs it at every size, and targets of 129 to 256 features whose data do not
+// fit FP16 pairs (logreg_wide.cu) or that have more than 2^22 rows.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -292,6 +296,7 @@ std::unique_ptr<Target> make_logreg_simt(gbm_context* ctx, const float* X, int64
                                          const float* y, float prior_scale) {
   if (d > 256) return nullptr;
   if (d <= 128) return make_logreg_f32(ctx, X, n, d, y, prior_scale);
+  if (auto t = make_logreg_wide(ctx, X, n, d, y, prior_scale)) return t;
   return std::unique_ptr<Target>(new LogregSimt(ctx, X, n, d, y, prior_scale));
 }
 

@@ -98,10 +98,10 @@ __global__ void __launch_bounds__(128 * kReduceGroups)
 split_reduce_kernel(const double* __restrict__ lpart, const float* __restrict__ gpart,
                     const float* __restrict__ Q, int ldq, const int* __restrict__ n_dev,
                     int c_base, int c_lim, int ct, int nt, int grid, int N, int D,
-                    float inv_var, double log_norm, const double* __restrict__ lin,
+                    float inv_var, double log_norm, const double* __restrict__ lin, int lparts,
                     double* __restrict__ logp, float* __restrict__ grad, int ldg) {
   __shared__ float range[kReduceGroups - 1][512];
-  const int n = chunk_count(*n_dev, c_base, c_lim);
+  const int n = n_dev ? chunk_count(*n_dev, c_base, c_lim) : c_lim;
   const int c = blockIdx.x;
   if (c >= n) return;
   const int S = split_count(n, ct, nt, grid, N);
@@ -110,37 +110,40 @@ split_reduce_kernel(const double* __restrict__ lpart, const float* __restrict__ 
   const float* q = Q + (size_t)c * ldq;
   const int groups = S <= kOrdered ? 1 : (int)(blockDim.x >> 7);
   const int group = threadIdx.x >> 7, first = threadIdx.x & 127;
-  if (group > 0) {
-    if (groups > 1) {
-      const int s0 = group * S / groups, s1 = (group + 1) * S / groups;
-      for (int d = first; d < D; d += 128) range[group - 1][d] = sum_splits(p + d, stride, s0, s1);
-      __syncthreads();
+  if (group > 0 && groups == 1) return;
+  const int s0 = groups > 1 ? group * S / groups : 0;
+  const int s1 = groups > 1 ? (group + 1) * S / groups : S;
+  for (int d0 = 0; d0 < D; d0 += 512) {
+    float acc[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int d = d0 + first + 128 * k;
+      if (d < D) {
+        acc[k] = sum_splits(p + d, stride, s0, s1);
+        if (group > 0) range[group - 1][first + 128 * k] = acc[k];
+      }
     }
-    return;
-  }
-  const int s1 = groups > 1 ? S / groups : S;
-  float acc[4];
+    if (groups > 1) {
+      __syncthreads();
 #pragma unroll
-  for (int k = 0; k < 4; ++k)
-    if (first + 128 * k < D) acc[k] = sum_splits(p + first + 128 * k, stride, 0, s1);
-  if (groups > 1) {
-    __syncthreads();
+      for (int k = 0; k < 4; ++k)
+        if (group == 0 && d0 + first + 128 * k < D)
+          for (int g = 0; g + 1 < groups; ++g) acc[k] += range[g][first + 128 * k];
+      if (d0 + 512 < D) __syncthreads();   // the ranges are written again
+    }
 #pragma unroll
-    for (int k = 0; k < 4; ++k)
-      if (first + 128 * k < D)
-        for (int g = 0; g + 1 < groups; ++g) acc[k] += range[g][first + 128 * k];
-  }
-#pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    const int d = first + 128 * k;
-    if (d < D) grad[(size_t)c * ldg + d] = acc[k] - q[d] * inv_var;
+    for (int k = 0; k < 4; ++k) {
+      const int d = d0 + first + 128 * k;
+      if (group == 0 && d < D) grad[(size_t)c * ldg + d] = acc[k] - q[d] * inv_var;
+    }
   }
   if (threadIdx.x >= 32) return;
   // Per-lane log-density terms: likelihood partials of splits lane, lane + 32,
   // ..., then lin . q - q.q / (2 s^2) over features lane, lane + 32, ...
   const int lane = threadIdx.x;
   double t = 0.0;
-  for (int j = lane; j < S; j += 32) t += lpart[(size_t)j * n + c];
+  const int rows = lparts > 0 ? lparts : S;
+  for (int j = lane; j < rows; j += 32) t += lpart[(size_t)j * n + c];
   double pr = 0.0, li = 0.0;
   for (int d = lane; d < D; d += 32) {
     const double qd = (double)q[d];
@@ -152,17 +155,19 @@ split_reduce_kernel(const double* __restrict__ lpart, const float* __restrict__ 
 }
 
 // Q, logp and grad point at chain c_base of the batch; `cap` bounds this
-// chunk's chains (<= c_lim); D <= 512.
+// chunk's chains (<= c_lim).  lparts: rows of lpart where they are not the
+// splits of the gradient; n_dev NULL: c_lim chains.
 void launch_split_reduce(const double* lpart, const float* gpart, const float* Q, int ldq,
                          const int* n_dev, int c_base, int c_lim, int cap, int ct, int nt,
                          int grid, int N, int D, float inv_var, double log_norm,
-                         const double* lin, double* logp, float* grad, int ldg, cudaStream_t s) {
+                         const double* lin, double* logp, float* grad, int ldg, cudaStream_t s,
+                         int lparts = 0) {
   // Few chains make many splits: several threads per feature.  (A sampler's
   // active chains are fewer than cap; one thread then adds more than kOrdered.)
   const int threads = split_count(cap, ct, nt, grid, N) <= kOrdered ? 128 : 128 * kReduceGroups;
   split_reduce_kernel<<<(unsigned)cap, threads, 0, s>>>(
-      lpart, gpart, Q, ldq, n_dev, c_base, c_lim, ct, nt, grid, N, D, inv_var, log_norm, lin, logp,
-      grad, ldg);
+      lpart, gpart, Q, ldq, n_dev, c_base, c_lim, ct, nt, grid, N, D, inv_var, log_norm, lin, lparts,
+      logp, grad, ldg);
   GBM_CUDA(cudaGetLastError());
 }
 

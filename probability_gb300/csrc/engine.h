@@ -108,6 +108,13 @@ struct Target {
   virtual const int* ragged_dims() const { return nullptr; }
   virtual int64_t ragged_chains() const { return 0; }
   virtual int64_t ragged_elements() const { return 0; }
+  // `steps` leapfrog steps of `chains` chains whole: from q, p [chains][ld], after
+  // each gradient but the last p += eps g, q += eps p; q, p, g and logp as they
+  // stand at the last gradient.  False: not held, nothing was launched.
+  virtual bool leapfrogs(float* q, float* p, float* g, double* logp, int ld, int chains,
+                         const float* eps, int per_chain, int steps, cudaStream_t s) {
+    return false;
+  }
   // Chains that run whole in one warp (nuts_chain.cu); nullptr: none.
   virtual const ChainModels* chain_models() const { return nullptr; }
   // Ragged evaluation in place: the chains act_idx[0 .. *act_count) (sorted),

@@ -50,6 +50,8 @@
 
 #include "engine.h"
 #include "f16_rows.cuh"
+#include "logreg_f32_math.cuh"
+#include "logreg_leapfrog.cuh"
 #include "split_reduce.cuh"
 #include "tc_common.cuh"
 #include "tc_ptx.cuh"
@@ -62,8 +64,6 @@ constexpr int kF32RT = 64;                  // rows per tile
 constexpr int kF32Threads = 256;
 constexpr uint64_t kF32WaitNs = 2000000000ull;   // 2 s bound on every wait
 constexpr int kF32TimeoutCode = 4;                // error word: bulk copy never landed
-constexpr float kNegLog2e = -1.4426950408889634f;
-constexpr float kLn2f = 0.6931471805599453f;
 
 template <int KD>
 struct F32Layout {
@@ -89,12 +89,6 @@ __host__ __device__ inline int f32_splits(int n, int grid, int row_tiles) {
 
 __device__ __forceinline__ float4 lds4(const float* p) {
   return *reinterpret_cast<const float4*>(p);
-}
-
-// -copysign(w, z): magnitude of w with the sign of -z.
-__device__ __forceinline__ float neg_copysign_f(float w, float z) {
-  return __int_as_float((__float_as_int(w) & 0x7fffffff) |
-                        (~__float_as_int(z) & (int)0x80000000));
 }
 
 // Phase 1 of one thread: z[i][c] = x_i . B_c over dk features (even) for its
@@ -196,26 +190,11 @@ __device__ __forceinline__ void f32_epilogue(const float (&z)[4][8], const float
   for (int i = 0; i < 4; ++i) {
     float r[8];
 #pragma unroll
-    for (int c = 0; c < 8; ++c) {
-      const float a = fabsf(z[i][c]);
-      const float e = tc::ex2_approx(a * kNegLog2e);       // e^-|z|
-      const float u1 = 1.f + e;
-      if (i < nvalid) {
-        sabs[c] += a;
-        prod[c] *= u1;
-      }
-      const float w = tc::rcp_approx(u1) - 0.5f;          // sigmoid(|z|) - 1/2
-      r[c] = yr[i] + neg_copysign_f(w, z[i][c]);
-    }
+    for (int c = 0; c < 8; ++c) f32_residual(z[i][c], yr[i], i < nvalid, sabs[c], prod[c], r[c]);
     store(i, r);
   }
 #pragma unroll
-  for (int c = 0; c < 8; ++c) {   // Kahan: lsum += -(sabs / 2 + ln prod)
-    const float v = -fmaf(kLn2f, tc::lg2_approx(prod[c]), 0.5f * sabs[c]) - lcomp[c];
-    const float t = lsum[c] + v;
-    lcomp[c] = (t - lsum[c]) - v;
-    lsum[c] = t;
-  }
+  for (int c = 0; c < 8; ++c) kahan_add(f32_like(sabs[c], prod[c]), lsum[c], lcomp[c]);
 }
 
 template <int KD>
@@ -868,6 +847,25 @@ class LogregF32 final : public Target {
                           kF32CT, kF32RT, g, N, D, inv_var_, log_norm_, lin_.as<double>(),
                           logp + base, grad + (size_t)base * ldg, ldg, s);
     }
+  }
+
+  // A trajectory of logreg_f32_kernel's gradients in one launch, while X and the
+  // chains fit the GPU's shared memory.
+  bool leapfrogs(float* q, float* p, float* g, double* logp, int ld, int chains, const float* eps,
+                 int per_chain, int steps, cudaStream_t s) override {
+    LeapShape h;
+    if (tc_ || !leap_shape(N_, (int)D_, chains, grid_, kF32CT, &h)) return false;
+    auto go = [&](auto launch) {
+      launch(h, x2_.as<float>(), ym_.as<float>(), (int)N_, dp_, chains, steps, eps, per_chain,
+             inv_var_, log_norm_, lin_.as<double>(), q, p, g, logp, ld, s);
+    };
+    if (h.G == 1)
+      go(launch_leapfrogs<1>);
+    else if (h.G == 2)
+      go(launch_leapfrogs<2>);
+    else
+      go(launch_leapfrogs<4>);
+    return true;
   }
 
   int launches_per_eval(int64_t cap) const override {

@@ -1309,11 +1309,13 @@ void hmc_step_launches(gbm_hmc* k, int64_t chains, const float* q, const double*
   const int wb = warp_blocks(chains);
   hmc_init_kernel<<<wb, 32 * kWarpsPerBlock, 0, s>>>(w, q, g, eps, per_chain, keyp);
   GBM_CUDA(cudaGetLastError());
-  for (int i = 0; i < num_leapfrog_steps; ++i) {
-    k->target->impl->eval(w.qw, w.D, w.count, w.C, w.lw, w.gw, w.D, k->target_ws.ptr, s);
-    if (i + 1 < num_leapfrog_steps)
-      hmc_kick_drift_kernel<<<wb, 32 * kWarpsPerBlock, 0, s>>>(w, eps, per_chain);
-  }
+  if (!k->target->impl->leapfrogs(w.qw, w.ph, w.gw, w.lw, w.D, w.C, eps, per_chain,
+                                  num_leapfrog_steps, s))
+    for (int i = 0; i < num_leapfrog_steps; ++i) {
+      k->target->impl->eval(w.qw, w.D, w.count, w.C, w.lw, w.gw, w.D, k->target_ws.ptr, s);
+      if (i + 1 < num_leapfrog_steps)
+        hmc_kick_drift_kernel<<<wb, 32 * kWarpsPerBlock, 0, s>>>(w, eps, per_chain);
+    }
   hmc_finish_kernel<<<wb, 32 * kWarpsPerBlock, 0, s>>>(w, q, l, g, eps, per_chain, keyp, out);
   GBM_CUDA(cudaGetLastError());
 }

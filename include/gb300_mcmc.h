@@ -221,6 +221,20 @@ GBM_API int gbm_hmc_one_step(gbm_hmc* kernel, int64_t chains, const float* state
                      double* log_acceptance_correction, double* log_accept_ratio,
                      uint8_t* is_accepted);
 
+/* gbm_hmc_one_step that also chooses, per chain, the accepted results' log
+ * acceptance correction and momenta: the proposal's where it was accepted, the
+ * previous results' elsewhere.  final_momentum must not be NULL here. */
+GBM_API int gbm_hmc_one_step_accepted(
+    gbm_hmc* kernel, int64_t chains, const float* state, const double* target_log_prob,
+    const float* grads, const float* step_size, int step_size_per_chain,
+    int32_t num_leapfrog_steps, const uint32_t seed[2], float* next_state, double* next_tlp,
+    float* next_grads, float* proposed_state, double* proposed_tlp, float* proposed_grads,
+    float* initial_momentum, float* final_momentum, double* log_acceptance_correction,
+    double* log_accept_ratio, uint8_t* is_accepted, const double* previous_correction,
+    const float* previous_initial_momentum, const float* previous_final_momentum,
+    double* accepted_correction, float* accepted_initial_momentum,
+    float* accepted_final_momentum);
+
 /* ---- NoUTurnSampler -------------------------------------------------- */
 
 /* NoUTurnSampler(target, step_size, max_tree_depth, max_energy_diff,

@@ -52,6 +52,8 @@ _SIGNATURES = {
     'gbm_hmc_create': ([P, I64, ctypes.POINTER(P)], ctypes.c_int),
     'gbm_hmc_destroy': ([P], ctypes.c_int),
     'gbm_hmc_one_step': ([P, I64, P, P, P, P, ctypes.c_int, I32, U32P] + [P] * 11, ctypes.c_int),
+    'gbm_hmc_one_step_accepted': (
+        [P, I64, P, P, P, P, ctypes.c_int, I32, U32P] + [P] * 17, ctypes.c_int),
     'gbm_nuts_create': ([P, I64, I32, F64, I32, ctypes.POINTER(P)], ctypes.c_int),
     'gbm_nuts_destroy': ([P], ctypes.c_int),
     'gbm_nuts_one_step': ([P, I64, P, P, P, P, ctypes.c_int, U32P] + [P] * 10, ctypes.c_int),
@@ -127,9 +129,7 @@ def check(status, what=''):
 
 def ptr(t):
   """Device pointer of a tensor (None -> NULL)."""
-  if t is None:
-    return None
-  return ctypes.c_void_p(t.data_ptr())
+  return None if t is None else t.data_ptr()
 
 
 def seed_words(seed):

@@ -17,6 +17,10 @@ def device():
 def as_tensor(x, dtype=None, dev=None):
   """Import any array (torch, DLPack producer such as TF/JAX, NumPy, Python
   scalars/lists) as a contiguous torch tensor on the engine's device."""
+  if (isinstance(x, torch.Tensor) and x.is_cuda and (dtype is None or x.dtype == dtype)
+      and x.is_contiguous()
+      and x.device.index == (torch.cuda.current_device() if dev is None else dev.index)):
+    return x                       # as it is
   dev = dev or device()
   if isinstance(x, torch.Tensor):
     t = x
@@ -42,6 +46,8 @@ def flatten_state(state):
     shapes = [p.shape for p in parts]
     return torch.cat(flat, 1).contiguous(), (sizes, shapes), True
   t = as_tensor(state, torch.float32)
+  if t.dim() == 2 and t.shape[0] > 0:
+    return t, ([t.shape[1]], [t.shape]), False
   if t.dim() == 1:
     return t.reshape(-1, 1).contiguous(), ([1], [t.shape]), False
   return t.reshape(t.shape[0], -1).contiguous(), ([t[0].numel()], [t.shape]), False
@@ -49,9 +55,11 @@ def flatten_state(state):
 
 def unflatten_state(flat, layout, is_list):
   sizes, shapes = layout
+  if not is_list:
+    return flat if flat.shape == shapes[0] else flat.reshape(shapes[0])
   parts = torch.split(flat, sizes, dim=1)
   parts = [p.reshape(s) for p, s in zip(parts, shapes)]
-  return list(parts) if is_list else parts[0]
+  return list(parts)
 
 
 def sanitize_seed(seed):

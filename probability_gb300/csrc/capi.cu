@@ -389,6 +389,29 @@ int gbm_hmc_destroy(gbm_hmc* k) {
   });
 }
 
+namespace {
+// One transition after the arguments' checks; `what` names the entry point.
+int run_hmc(const char* what, gbm_hmc* k, int64_t chains, const float* state,
+            const double* target_log_prob, const float* grads, const float* step_size,
+            int step_size_per_chain, int32_t num_leapfrog_steps, const uint32_t seed[2],
+            const gbm::HmcOutputs& out) {
+  if (!k || !state || !target_log_prob || !grads || !step_size || !seed || !out.next_state ||
+      !out.next_tlp || !out.next_grads || !out.log_accept_ratio || !out.is_accepted)
+    return invalid(std::string(what) + ": NULL argument");
+  if (chains <= 0 || chains > k->max_chains)
+    return invalid(std::string(what) + ": chains must be in [1, max_chains]");
+  if (num_leapfrog_steps < 1)
+    return invalid(std::string(what) + ": num_leapfrog_steps must be >= 1");
+  return guarded([&] {
+    DeviceGuard g(k->target->ctx->device);
+    gbm::check_device_error(k->target->ctx);
+    gbm::hmc_one_step(k, chains, state, target_log_prob, grads, step_size, step_size_per_chain,
+                      num_leapfrog_steps, make_uint2(seed[0], seed[1]), out);
+    return GBM_OK;
+  });
+}
+}  // namespace
+
 int gbm_hmc_one_step(gbm_hmc* k, int64_t chains, const float* state,
                      const double* target_log_prob, const float* grads,
                      const float* step_size, int step_size_per_chain,
@@ -398,22 +421,34 @@ int gbm_hmc_one_step(gbm_hmc* k, int64_t chains, const float* state,
                      float* initial_momentum, float* final_momentum,
                      double* log_acceptance_correction, double* log_accept_ratio,
                      uint8_t* is_accepted) {
-  if (!k || !state || !target_log_prob || !grads || !step_size || !seed || !next_state ||
-      !next_tlp || !next_grads || !log_accept_ratio || !is_accepted)
-    return invalid("gbm_hmc_one_step: NULL argument");
-  if (chains <= 0 || chains > k->max_chains)
-    return invalid("gbm_hmc_one_step: chains must be in [1, max_chains]");
-  if (num_leapfrog_steps < 1) return invalid("gbm_hmc_one_step: num_leapfrog_steps must be >= 1");
-  return guarded([&] {
-    DeviceGuard g(k->target->ctx->device);
-    gbm::check_device_error(k->target->ctx);
-    gbm::HmcOutputs out{next_state, next_tlp, next_grads, proposed_state, proposed_tlp,
-                        proposed_grads, initial_momentum, final_momentum,
-                        log_acceptance_correction, log_accept_ratio, is_accepted};
-    gbm::hmc_one_step(k, chains, state, target_log_prob, grads, step_size, step_size_per_chain,
-                      num_leapfrog_steps, make_uint2(seed[0], seed[1]), out);
-    return GBM_OK;
-  });
+  return run_hmc("gbm_hmc_one_step", k, chains, state, target_log_prob, grads, step_size,
+                 step_size_per_chain, num_leapfrog_steps, seed,
+                 gbm::HmcOutputs{next_state, next_tlp, next_grads, proposed_state, proposed_tlp,
+                                 proposed_grads, initial_momentum, final_momentum,
+                                 log_acceptance_correction, log_accept_ratio, is_accepted});
+}
+
+int gbm_hmc_one_step_accepted(
+    gbm_hmc* k, int64_t chains, const float* state, const double* target_log_prob,
+    const float* grads, const float* step_size, int step_size_per_chain,
+    int32_t num_leapfrog_steps, const uint32_t seed[2], float* next_state, double* next_tlp,
+    float* next_grads, float* proposed_state, double* proposed_tlp, float* proposed_grads,
+    float* initial_momentum, float* final_momentum, double* log_acceptance_correction,
+    double* log_accept_ratio, uint8_t* is_accepted, const double* previous_correction,
+    const float* previous_initial_momentum, const float* previous_final_momentum,
+    double* accepted_correction, float* accepted_initial_momentum,
+    float* accepted_final_momentum) {
+  if (!final_momentum || !previous_correction || !previous_initial_momentum || !previous_final_momentum ||
+      !accepted_correction || !accepted_initial_momentum || !accepted_final_momentum)
+    return invalid("gbm_hmc_one_step_accepted: NULL argument");
+  return run_hmc("gbm_hmc_one_step_accepted", k, chains, state, target_log_prob, grads, step_size,
+                 step_size_per_chain, num_leapfrog_steps, seed,
+                 gbm::HmcOutputs{next_state, next_tlp, next_grads, proposed_state, proposed_tlp,
+                                 proposed_grads, initial_momentum, final_momentum,
+                                 log_acceptance_correction, log_accept_ratio, is_accepted,
+                                 previous_correction, previous_initial_momentum,
+                                 previous_final_momentum, accepted_correction,
+                                 accepted_initial_momentum, accepted_final_momentum});
 }
 
 int gbm_nuts_create(gbm_target* target, int64_t max_chains, int32_t max_tree_depth,

@@ -713,11 +713,19 @@ __global__ void hmc_finish_kernel(HmcDev w, const float* __restrict__ q0,
   for (int d = lane; d < w.D; d += 32) {
     out.next_state[o + d] = acc ? w.qw[o + d] : q0[o + d];
     out.next_grads[o + d] = acc ? w.gw[o + d] : g0[o + d];
+    if (out.accepted_initial_momentum) {
+      out.accepted_initial_momentum[o + d] =
+          acc ? w.p0[o + d] : out.previous_initial_momentum[o + d];
+      out.accepted_final_momentum[o + d] =
+          acc ? out.final_momentum[o + d] : out.previous_final_momentum[o + d];
+    }
   }
   if (lane == 0) {
     out.next_tlp[c] = acc ? l1 : l0[c];
     if (out.proposed_tlp) out.proposed_tlp[c] = l1;
     if (out.log_acceptance_correction) out.log_acceptance_correction[c] = corr;
+    if (out.accepted_correction)
+      out.accepted_correction[c] = acc ? corr : out.previous_correction[c];
     out.log_accept_ratio[c] = lar;
     out.is_accepted[c] = acc ? 1 : 0;
   }

@@ -117,6 +117,14 @@ struct HmcOutputs {
   double* log_acceptance_correction;
   double* log_accept_ratio;
   uint8_t* is_accepted;
+  // Optional, with final_momentum: the proposal's correction and momenta where accepted
+  // and the previous results' elsewhere.
+  const double* previous_correction = nullptr;
+  const float* previous_initial_momentum = nullptr;
+  const float* previous_final_momentum = nullptr;
+  double* accepted_correction = nullptr;
+  float* accepted_initial_momentum = nullptr;
+  float* accepted_final_momentum = nullptr;
 };
 
 struct DaParams {

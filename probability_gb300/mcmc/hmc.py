@@ -29,6 +29,8 @@ def _step_size_tensor(step_size, chains, dev):
       raise ValueError('There should be exactly one `step_size` or it should '
                        'have same length as `current_state`.')
     step_size = step_size[0]
+  if isinstance(step_size, (int, float)):
+    return torch.full((1,), step_size, dtype=torch.float32, device=dev), 0
   s = _util.as_tensor(step_size, torch.float32, dev).reshape(-1)
   if s.numel() == 1:
     return s, 0
@@ -62,7 +64,11 @@ class _HmcEngine:
         pass
 
 
-def _hmc_transition(engine, state, target_log_prob, grads, step_size, num_leapfrog_steps, seed):
+def _hmc_transition(engine, state, target_log_prob, grads, step_size, num_leapfrog_steps, seed,
+                    previous=None):
+  """One transition.  `previous`: a results tuple whose correction and momenta the
+  engine chooses from for the accepted results (out['accepted'], None where it
+  can't: their form is not the state's)."""
   q, layout, is_list = _util.flatten_state(state)
   C, D = q.shape
   dev = q.device
@@ -75,16 +81,28 @@ def _hmc_transition(engine, state, target_log_prob, grads, step_size, num_leapfr
   out = dict(next_state=f32(), next_tlp=f64(), next_grads=f32(), proposed_state=f32(),
              proposed_tlp=f64(), proposed_grads=f32(), initial_momentum=f32(),
              final_momentum=f32(), corr=f64(), lar=f64(),
-             is_accepted=torch.empty(C, dtype=torch.uint8, device=dev))
+             # The engine writes 0 / 1 bytes.
+             is_accepted=torch.empty(C, dtype=torch.bool, device=dev))
   P = _native.ptr
-  _native.check(_native.lib().gbm_hmc_one_step(
-      engine.handle, C, P(q), P(l0), P(g0), P(eps), per_chain, int(num_leapfrog_steps),
-      _native.seed_words(seed), P(out['next_state']), P(out['next_tlp']),
-      P(out['next_grads']), P(out['proposed_state']), P(out['proposed_tlp']),
-      P(out['proposed_grads']), P(out['initial_momentum']), P(out['final_momentum']),
-      P(out['corr']), P(out['lar']), P(out['is_accepted'])), 'gbm_hmc_one_step')
+  args = (engine.handle, C, P(q), P(l0), P(g0), P(eps), per_chain, int(num_leapfrog_steps),
+          _native.seed_words(seed), P(out['next_state']), P(out['next_tlp']),
+          P(out['next_grads']), P(out['proposed_state']), P(out['proposed_tlp']),
+          P(out['proposed_grads']), P(out['initial_momentum']), P(out['final_momentum']),
+          P(out['corr']), P(out['lar']), P(out['is_accepted']))
+  out['accepted'] = None
+  if previous is not None and not is_list:
+    prev = (previous.log_acceptance_correction, previous.initial_momentum,
+            previous.final_momentum)
+    shapes = ((C,), layout[1][0], layout[1][0])
+    types = (torch.float64, torch.float32, torch.float32)
+    if all(isinstance(t, torch.Tensor) and t.shape == s and t.dtype == d and t.device == dev
+           and t.is_contiguous() for t, s, d in zip(prev, shapes, types)):
+      out['accepted'] = chosen = (f64(), f32(), f32())
+      _native.check(_native.lib().gbm_hmc_one_step_accepted(
+          *args, *[P(t) for t in prev], *[P(t) for t in chosen]), 'gbm_hmc_one_step_accepted')
+  if out['accepted'] is None:
+    _native.check(_native.lib().gbm_hmc_one_step(*args), 'gbm_hmc_one_step')
   unflat = lambda t: _util.unflatten_state(t, layout, is_list)
-  out['is_accepted'] = out['is_accepted'].bool()
   return out, unflat, is_list
 
 
@@ -178,16 +196,21 @@ class HamiltonianMonteCarlo(kernel_base.TransitionKernel):
     step_size, n = self._inner._params(prev)
     out, unflat, _ = _hmc_transition(
         self._inner._engine, current_state, prev.target_log_prob, prev.grads_target_log_prob,
-        step_size, int(n), seed)
+        step_size, int(n), seed, previous=prev)
     proposed = prev._replace(
         log_acceptance_correction=out['corr'], target_log_prob=out['proposed_tlp'],
         grads_target_log_prob=unflat(out['proposed_grads']),
         initial_momentum=unflat(out['initial_momentum']),
         final_momentum=unflat(out['final_momentum']), seed=_util.seed_tensor(seed))
     acc = out['is_accepted']
-    accepted = _choose(acc, proposed._replace(seed=[]), prev._replace(seed=[]))
+    if out['accepted'] is not None:
+      corr, p0, p1 = out['accepted']
+      accepted = proposed._replace(
+          log_acceptance_correction=corr, initial_momentum=unflat(p0), final_momentum=unflat(p1))
+    else:
+      accepted = _choose(acc, proposed, prev)
     accepted = accepted._replace(target_log_prob=out['next_tlp'],
-                                 grads_target_log_prob=unflat(out['next_grads']))
+                                 grads_target_log_prob=unflat(out['next_grads']), seed=[])
     kr = MetropolisHastingsKernelResults(
         accepted_results=accepted, is_accepted=acc, log_accept_ratio=out['lar'],
         proposed_state=unflat(out['proposed_state']), proposed_results=proposed, extra=[],

@@ -31,7 +31,11 @@ class Target:
     """Batched (log_prob float64 [C], grad float32 [C, D]) at ``state`` [C, D]."""
     q = _util.as_tensor(state, torch.float32)
     squeeze = q.dim() == 1
-    q = q.reshape(-1, self.dim).contiguous()
+    dim = self.__dict__.get('_dim')          # of the native target, which never changes
+    if dim is None:
+      dim = self._dim = self.dim
+    if q.dim() != 2 or q.shape[1] != dim:
+      q = q.reshape(-1, dim).contiguous()
     logp = torch.empty(q.shape[0], dtype=torch.float64, device=q.device)
     grad = torch.empty_like(q)
     _native.check(_native.lib().gbm_target_log_prob_and_grad(

@@ -126,7 +126,7 @@ grad_tc_kernel(const __grid_constant__ CUtensorMap rhi, const __grid_constant__ 
     __syncwarp();
   } else if (warp == 9) {
     // ---------------- MMAs ----------------
-    if (lane == 0) {
+    if (tc::elect_one()) {
       const uint32_t idesc = tc::idesc_16bit_f32(kGradCT, width, !K_MAJOR, true, false);
       bool ok = true;
       int halves = 0;               // halves whose MMAs were issued

@@ -478,7 +478,7 @@ logreg_f32_tc_kernel(const __grid_constant__ CUtensorMap himap,
 
   if (warp >= 8) {
     // ---------------- a group's loads and MMAs ----------------
-    if (lane == 0) {
+    if (tc::elect_one()) {
       // A turn's rows: 32 of each tile, X2 and y, and the FP16 form.
       auto load_x = [&](int j) {
         const int first = turn_first(group, j), count = turn_count(group, j, T);

@@ -242,7 +242,7 @@ logreg_tc_kernel(const __grid_constant__ CUtensorMap xmap,
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
-    if (lane == 0) {
+    if (tc::elect_one()) {
       constexpr uint32_t idesc1 = tc::idesc_bf16_f32(128, CT, false, false);  // K-major A, B
       constexpr uint32_t idesc2 = tc::idesc_bf16_f32(128, CT, true, true);    // MN-major A, B
       const uint32_t xs_a = tc::smem_u32(Xs), bhi_a = tc::smem_u32(Bhi);
@@ -670,7 +670,7 @@ logreg_tct_kernel(const __grid_constant__ CUtensorMap xmap,
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
-    if (lane == 0) {
+    if (tc::elect_one()) {
       const int nd = ksteps * 16;                                      // N of G^T
       constexpr uint32_t idesc1 = tc::idesc_bf16_f32(128, 128, false, false);
       const uint32_t idesc2 = tc::idesc_bf16_f32(128, nd, false, true);  // MN-major X
@@ -1017,7 +1017,7 @@ logreg_tc_pair_kernel(const __grid_constant__ CUtensorMap xmap, const float* __r
     __syncwarp();
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
-    if (lane == 0) {
+    if (tc::elect_one()) {
       constexpr uint32_t idesc1 = tc::idesc_bf16_f32(128, CT, false, false);
       constexpr uint32_t idesc2 = tc::idesc_bf16_f32(128, CT, true, true);
       const uint32_t xs_a = tc::smem_u32(Xs), bhi_a = tc::smem_u32(Bhi);

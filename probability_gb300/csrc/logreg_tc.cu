@@ -245,8 +245,12 @@ logreg_tc_kernel(const __grid_constant__ CUtensorMap xmap,
     if (tc::elect_one()) {
       constexpr uint32_t idesc1 = tc::idesc_bf16_f32(128, CT, false, false);  // K-major A, B
       constexpr uint32_t idesc2 = tc::idesc_bf16_f32(128, CT, true, true);    // MN-major A, B
-      const uint32_t xs_a = tc::smem_u32(Xs), bhi_a = tc::smem_u32(Bhi);
-      const uint32_t blo_a = tc::smem_u32(Blo), rs_a = tc::smem_u32(Rs);
+      const uint64_t xk = tc::smem_desc_sw128(tc::smem_u32(Xs), 16, 1024);       // K-major
+      const uint64_t xmn = tc::smem_desc_sw128(tc::smem_u32(Xs), 16384, 1024);   // MN-major
+      const uint64_t xlk = tc::smem_desc_sw128(tc::smem_u32(smem + L::kXlo), 16, 1024);
+      const uint64_t bhk = tc::smem_desc_sw128(tc::smem_u32(Bhi), 16, 1024);
+      const uint64_t blk = tc::smem_desc_sw128(tc::smem_u32(Blo), 16, 1024);
+      const uint64_t rmn = tc::smem_desc_sw128(tc::smem_u32(Rs), 16384, 1024);
       const uint32_t tg = tmem + 2 * CT;
       const int ksteps = (D + 15) >> 4;   // K-steps of 16 features holding data
       bool ok = true;
@@ -261,21 +265,19 @@ logreg_tc_kernel(const __grid_constant__ CUtensorMap xmap,
         }
         tc::tc_fence_after();
         const uint32_t tz = tmem + b * CT;
-        const uint32_t xa = xs_a + s * L::kXStage;
-        const uint32_t xla = tc::smem_u32(smem + L::kXlo);
+        const uint64_t xs = tc::desc_at(xk, s * L::kXStage);
 #pragma unroll
         for (int kb = 0; kb < KB; ++kb) {
 #pragma unroll
           for (int k = 0; k < 4; ++k) {
             if (kb * 4 + k >= ksteps) break;   // all-zero padding features
-            const uint64_t a = tc::smem_desc_sw128(xa + kb * 16384 + k * 32, 16, 1024);
-            const uint64_t bh = tc::smem_desc_sw128(bhi_a + kb * (CT * 128) + k * 32, 16, 1024);
-            const uint64_t bl = tc::smem_desc_sw128(blo_a + kb * (CT * 128) + k * 32, 16, 1024);
+            const uint64_t a = tc::desc_at(xs, kb * 16384 + k * 32);
+            const uint64_t bh = tc::desc_at(bhk, kb * (CT * 128) + k * 32);
+            const uint64_t bl = tc::desc_at(blk, kb * (CT * 128) + k * 32);
             tc::mma_16bit(tz, a, bh, idesc1, (kb | k) ? 1u : 0u);
             tc::mma_16bit(tz, a, bl, idesc1, 1u);
             if constexpr (XLO) {
-              const uint64_t al = tc::smem_desc_sw128(xla + kb * 16384 + k * 32, 16, 1024);
-              tc::mma_16bit(tz, al, bh, idesc1, 1u);
+              tc::mma_16bit(tz, tc::desc_at(xlk, kb * 16384 + k * 32), bh, idesc1, 1u);
             }
           }
         }
@@ -295,14 +297,14 @@ logreg_tc_kernel(const __grid_constant__ CUtensorMap xmap,
           break;
         }
         tc::tc_fence_after();
-        const uint32_t xa = xs_a + s * L::kXStage;
-        const uint32_t ra = rs_a + rb * L::kRBuf;
+        const uint64_t xs = tc::desc_at(xmn, s * L::kXStage);
+        const uint64_t rs = tc::desc_at(rmn, rb * L::kRBuf);
 #pragma unroll
         for (int mt = 0; mt < L::kMTiles; ++mt) {
 #pragma unroll
           for (int ks = 0; ks < kRows / 16; ++ks) {
-            const uint64_t a = tc::smem_desc_sw128(xa + mt * 32768 + ks * 2048, 16384, 1024);
-            const uint64_t bd = tc::smem_desc_sw128(ra + ks * 2048, 16384, 1024);
+            const uint64_t a = tc::desc_at(xs, mt * 32768 + ks * 2048);
+            const uint64_t bd = tc::desc_at(rs, ks * 2048);
             tc::mma_16bit(tg + mt * CT, a, bd, idesc2, (it > 0 || ks > 0) ? 1u : 0u);
           }
         }
@@ -838,30 +840,43 @@ logreg_tct_kernel(const __grid_constant__ CUtensorMap xmap,
 // One CTA cannot hold a 128-row X tile of 512 features (128 KB per stage)
 // beside the BF16 hi/lo chain states, so the features are split: CTA p of the
 // pair keeps features [256p, 256p + 256) of X and of the states and forms the
-// partial Z_p = X[:, F_p] B[:, F_p]^T in its TMEM.  Rows 64p .. 64p+63 belong
-// to CTA p: its "send" warps copy the partial of the other 64 rows into the
-// peer's exchange buffer (distributed shared memory), its "compute" warps add
-// the peer's partial to their own, run the epilogue and write R into both
-// CTAs' R tiles.  Each CTA then accumulates G for its own features,
-// G_p += X[:, F_p]^T R.  X is read from L2 once per chain tile, as in the
-// single-CTA kernel.  Every wait is bounded; a CTA that gives up also sets
-// its peer's abort flag.
+// partial Z_p = X[:, F_p] B[:, F_p]^T in its TMEM.  Chains 32p .. 32p+31 of the
+// tile belong to CTA p: each of its warps sends the partial of 32 rows x 8 of the
+// other chains into the peer's exchange buffer (distributed shared memory, a warp's
+// rows side by side; the bytes complete on the peer's barrier), adds the peer's
+// partial to 8 chains of its own, and writes their R into this CTA's half of its R
+// tile, from where one bulk copy per 32 rows takes it to the peer's.  Each CTA then
+// accumulates G for its own features, G_p += X[:, F_p]^T R.  One warp issues the
+// loads and the MMAs of Z, another those of G.  X is read from L2 once per chain
+// tile, as in the single-CTA kernel.  Every wait is bounded; a CTA that gives up
+// also sets its peer's abort flag.
+//
+// What bounds it: the chain Z -> exchange -> R -> G of a tile, two tiles in flight
+// (as many as X stages fit); the MMAs (48 of N = 64 a row tile at 48 clocks) are
+// 60% of it.  Chains are split between the CTAs rather than rows because a warp
+// reaches only its own quarter of TMEM's rows: by rows, half of the SM's quarters
+// did all of the epilogue.  1e6 x 512, 4096 chains: 28.1 ms with rows split, remote
+// stores and arrivals that wait for them, one issuing warp; 19.5 with chains split,
+// asynchronous exchange and two issuers; 14.8 with the MMAs issued by an elected
+// lane and every warp both sending and computing.
 // ---------------------------------------------------------------------------
 constexpr int kPairKB = 4;                  // 64-feature blocks per CTA
 constexpr int kPairCT = 64;                 // chains per tile
-constexpr int kPairEpi = 16;                // epilogue warps (8 compute + 8 send)
-constexpr int kZxStride = kPairCT * 4 + 16; // bytes per exchange row (bank-conflict pad)
+constexpr int kPairEpi = 16;                // epilogue warps
 
 struct PairLayout {
   static constexpr int kXStage = kPairKB * 16384;           // [4][128 rows][128 B]
   static constexpr int kBBytes = kPairKB * kPairCT * 128;   // [4][64 chains][128 B]
-  static constexpr int kRBuf = 16384;                       // [128 rows][64 chains] BF16
+  // R: two halves of 32 chains, [128 rows][64 B] BF16, 64-byte swizzle.
+  static constexpr int kRHalf = 8192;
+  static constexpr int kRBuf = 2 * kRHalf;
   static constexpr int kX = 0;                              // 2 stages
   static constexpr int kBhi = kX + 2 * kXStage;
   static constexpr int kBlo = kBhi + kBBytes;
   static constexpr int kR = kBlo + kBBytes;
-  static constexpr int kZx = kR + kRBuf;                    // [64 rows][kZxStride]
-  static constexpr int kCtl = kZx + 64 * kZxStride;
+  static constexpr int kZx = kR + kRBuf;                    // [8 chunks][128 rows][16 B]
+  static constexpr int kZxBytes = 8 * 128 * 16;
+  static constexpr int kCtl = kZx + kZxBytes;
   static constexpr int kBytes = kCtl + 256;
   static_assert(kBytes + 1024 <= 232448, "shared memory over the sm_103a limit");
 };
@@ -873,11 +888,12 @@ struct PairBars {
   // the tensor pipe instead of stalling the next tile's Z MMAs.
   uint64_t x_full[2][2], x_empty[2][2];   // [stage][half]
   uint64_t z_full[2], z_empty[2];
-  uint64_t zx_full;   // peer's partial for my rows has arrived (8 remote arrivals)
-  uint64_t zx_free;   // peer has read what I sent last (8 remote arrivals)
-  uint64_t r_full;    // R tile complete (8 local + 8 remote arrivals)
+  uint64_t zx_full;   // peer's partial for my chains has arrived (its 16 KB)
+  uint64_t zx_free;   // peer has read what I sent last (16 remote arrivals)
+  uint64_t r_full;    // R tile complete (16 local arrivals, 8 KB of the peer's copies)
   uint64_t r_free;    // both CTAs' GEMM2 done with R (2 multicast commits)
-  uint64_t g_done, drain;
+  uint64_t r_rows[4]; // per quarter: three of its warps have written their chains of R
+  uint64_t g_done, drain[2];
 };
 
 __device__ __forceinline__ bool wait_cluster_or_abort(uint64_t* bar, uint32_t parity,
@@ -932,7 +948,7 @@ logreg_tc_pair_kernel(const __grid_constant__ CUtensorMap xmap, const float* __r
   };
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  float lp_pub = 0.f;   // compute warps, lane j < 16: log-likelihood partial of chain 16 sub + j
+  float lp_pub = 0.f;   // epilogue warps, lane j < 8: log-likelihood partial of own chain j
   if (tid == 0) {
     for (int i = 0; i < 2; ++i) {
       for (int h = 0; h < 2; ++h) {
@@ -942,14 +958,17 @@ logreg_tc_pair_kernel(const __grid_constant__ CUtensorMap xmap, const float* __r
       tc::mbar_init(&bars->z_full[i], 1);
       tc::mbar_init(&bars->z_empty[i], kPairEpi);
     }
-    tc::mbar_init(&bars->zx_full, 8);
-    tc::mbar_init(&bars->zx_free, 8);
-    tc::mbar_init(&bars->r_full, 16);
+    tc::mbar_init(&bars->zx_full, 1);
+    tc::mbar_init(&bars->zx_free, kPairEpi);
+    tc::mbar_init(&bars->r_full, kPairEpi);
     tc::mbar_init(&bars->r_free, 2);
+    for (int i = 0; i < 4; ++i) tc::mbar_init(&bars->r_rows[i], 3);
     tc::mbar_init(&bars->g_done, 1);
-    tc::mbar_init(&bars->drain, 1);
+    tc::mbar_init(&bars->drain[0], 1);
+    tc::mbar_init(&bars->drain[1], 1);
     *abort_flag = 0;
     tc::fence_mbar_init();
+    if (T > 0) tc::mbar_arrive_expect_tx(&bars->zx_full, L::kZxBytes);
     tc::prefetch_tmap(&xmap);
   }
   if (warp == 1) tc::tmem_alloc(tmem_slot, 256);
@@ -985,20 +1004,25 @@ logreg_tc_pair_kernel(const __grid_constant__ CUtensorMap xmap, const float* __r
   tc::cluster_sync();
   const uint32_t tmem = *tmem_slot;
 
+  // Descriptors of X.
+  const uint64_t xk = tc::smem_desc_sw128(tc::smem_u32(Xs), 16, 1024);       // K-major
+  const uint64_t xmn = tc::smem_desc_sw128(tc::smem_u32(Xs), 16384, 1024);   // MN-major
   if (warp == 0) {
-    // ---------------- TMA producer: X[rows, F_p] ----------------
-    if (lane == 0) {
+    // ---------------- X[rows, F_p] by TMA, and the MMAs of Z ----------------
+    if (tc::elect_one()) {
+      constexpr uint32_t idesc1 = tc::idesc_bf16_f32(128, CT, false, false);
+      const uint64_t bhk = tc::smem_desc_sw128(tc::smem_u32(Bhi), 16, 1024);
+      const uint64_t blk = tc::smem_desc_sw128(tc::smem_u32(Blo), 16, 1024);
+      const int ksteps = (fD + 15) >> 4;        // K-steps of 16 features holding data
       // Half-stage fills in order: fill f is (tile f / 2, half f % 2).
       int nfill = 0;
-      bool stop = false;
-      for (int it = 0; it < T && !stop; ++it) {
+      bool ok = true;
+      auto load = [&](int it) -> bool {
         const int s = it & 1;
         for (int h = 0; h < 2; ++h) {
           if (!wait_or_abort(&bars->x_empty[s][h], ((uint32_t)(it >> 1) & 1) ^ 1, abort_flag)) {
             tc::record_error(err, kTcTimeoutTma);
-            abort_both();
-            stop = true;
-            break;
+            return false;
           }
           tc::mbar_arrive_expect_tx(&bars->x_full[s][h], L::kXStage / 2);
 #pragma unroll
@@ -1007,31 +1031,14 @@ logreg_tc_pair_kernel(const __grid_constant__ CUtensorMap xmap, const float* __r
                             (rt_begin + it) * kRows, &bars->x_full[s][h]);
           ++nfill;
         }
-      }
-      // Let the last fills land before the CTA can exit (each wait bounded).
-      for (int f = (nfill > 4 ? nfill - 4 : 0); f < nfill; ++f) {
-        const int j = f >> 1, h = f & 1;
-        tc::mbar_wait(&bars->x_full[j & 1][h], (uint32_t)((j >> 1) & 1), kWaitLimitNs);
-      }
-    }
-    __syncwarp();
-  } else if (warp == 1) {
-    // ---------------- MMA issuer ----------------
-    if (tc::elect_one()) {
-      constexpr uint32_t idesc1 = tc::idesc_bf16_f32(128, CT, false, false);
-      constexpr uint32_t idesc2 = tc::idesc_bf16_f32(128, CT, true, true);
-      const uint32_t xs_a = tc::smem_u32(Xs), bhi_a = tc::smem_u32(Bhi);
-      const uint32_t blo_a = tc::smem_u32(Blo), rs_a = tc::smem_u32(Rs);
-      const uint32_t tg = tmem + 2 * CT;
-      const int ksteps = (fD + 15) >> 4;        // K-steps of 16 features holding data
-      const int mtiles = (fD + 127) >> 7;       // 128-feature tiles of G
-      bool ok = true;
+        return true;
+      };
       auto gemm1 = [&](int it) -> bool {
         const int s = it & 1, b = it & 1;
         const uint32_t use = (uint32_t)(it >> 1) & 1;
         if (!wait_or_abort(&bars->z_empty[b], use ^ 1, abort_flag)) return false;
         const uint32_t tz = tmem + b * CT;
-        const uint32_t xa = xs_a + s * L::kXStage;
+        const uint64_t xs = tc::desc_at(xk, s * L::kXStage);
         // Half h holds K-steps 8h .. 8h + 7; a half without data (fD <= 128)
         // is neither waited for nor read.
         for (int h = 0; h < 2 && 8 * h < ksteps; ++h) {
@@ -1042,11 +1049,9 @@ logreg_tc_pair_kernel(const __grid_constant__ CUtensorMap xmap, const float* __r
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
               if (kb * 4 + k >= ksteps) break;
-              const uint64_t a = tc::smem_desc_sw128(xa + kb * 16384 + k * 32, 16, 1024);
-              const uint64_t bh =
-                  tc::smem_desc_sw128(bhi_a + kb * (CT * 128) + k * 32, 16, 1024);
-              const uint64_t bl =
-                  tc::smem_desc_sw128(blo_a + kb * (CT * 128) + k * 32, 16, 1024);
+              const uint64_t a = tc::desc_at(xs, kb * 16384 + k * 32);
+              const uint64_t bh = tc::desc_at(bhk, kb * (CT * 128) + k * 32);
+              const uint64_t bl = tc::desc_at(blk, kb * (CT * 128) + k * 32);
               tc::mma_16bit(tz, a, bh, idesc1, (kb | k) ? 1u : 0u);
               tc::mma_16bit(tz, a, bl, idesc1, 1u);
             }
@@ -1055,25 +1060,48 @@ logreg_tc_pair_kernel(const __grid_constant__ CUtensorMap xmap, const float* __r
         tc::mma_commit(&bars->z_full[b]);
         return true;
       };
-      if (T > 0) ok = gemm1(0);
+      // A stage is refilled when G of its tile is done, while Z of the next tile
+      // runs.
+      for (int it = 0; it < T && it < 2 && ok; ++it) ok = load(it);
       for (int it = 0; it < T && ok; ++it) {
-        if (it + 1 < T) {
-          ok = gemm1(it + 1);
-          if (!ok) break;
-        }
+        ok = gemm1(it);
+        if (ok && it > 0 && it + 1 < T) ok = load(it + 1);
+      }
+      if (!ok) {
+        tc::record_error(err, kTcTimeoutMma);
+        abort_both();
+      }
+      tc::mma_commit(&bars->drain[0]);
+      tc::mbar_wait(&bars->drain[0], 0, kWaitLimitNs);
+      // Let the last fills land before the CTA can exit (each wait bounded).
+      for (int f = (nfill > 4 ? nfill - 4 : 0); f < nfill; ++f) {
+        const int j = f >> 1, h = f & 1;
+        tc::mbar_wait(&bars->x_full[j & 1][h], (uint32_t)((j >> 1) & 1), kWaitLimitNs);
+      }
+    }
+    __syncwarp();
+  } else if (warp == 1) {
+    // ---------------- the MMAs of G ----------------
+    if (tc::elect_one()) {
+      constexpr uint32_t idesc2 = tc::idesc_bf16_f32(128, CT, true, true);
+      const uint64_t rmn = tc::smem_desc_sw64(tc::smem_u32(Rs), L::kRHalf, 512);
+      const uint32_t tg = tmem + 2 * CT;
+      const int mtiles = (fD + 127) >> 7;       // 128-feature tiles of G
+      bool ok = true;
+      for (int it = 0; it < T; ++it) {
         if (!wait_cluster_or_abort(&bars->r_full, (uint32_t)it & 1, abort_flag)) {
           ok = false;
           break;
         }
         tc::tc_fence_after();
-        const uint32_t xa = xs_a + (it & 1) * L::kXStage;
-        // M-tile mt reads half mt of the stage; each half is released as soon
-        // as the MMAs that read it (and every earlier one) complete.
+        const uint64_t xs = tc::desc_at(xmn, (it & 1) * L::kXStage);
+        // M-tile mt reads half mt of the stage; each half is released as soon as
+        // the MMAs that read it complete (those of Z have: R comes from it).
         for (int mt = 0; mt < mtiles; ++mt) {
 #pragma unroll
           for (int ks = 0; ks < kRows / 16; ++ks) {
-            const uint64_t a = tc::smem_desc_sw128(xa + mt * 32768 + ks * 2048, 16384, 1024);
-            const uint64_t bd = tc::smem_desc_sw128(rs_a + ks * 2048, 16384, 1024);
+            const uint64_t a = tc::desc_at(xs, mt * 32768 + ks * 2048);
+            const uint64_t bd = tc::desc_at(rmn, ks * 1024);
             tc::mma_16bit(tg + mt * CT, a, bd, idesc2, (it > 0 || ks > 0) ? 1u : 0u);
           }
           tc::mma_commit(&bars->x_empty[it & 1][mt]);
@@ -1086,116 +1114,132 @@ logreg_tc_pair_kernel(const __grid_constant__ CUtensorMap xmap, const float* __r
       } else {
         tc::record_error(err, kTcTimeoutMma);
         abort_both();
+        // A copy of the peer's may still be on its way: two seconds at most.
+        tc::mbar_wait(&bars->r_full, 0, kWaitLimitNs);
+        tc::mbar_wait(&bars->r_full, 1, kWaitLimitNs);
       }
-      tc::mma_commit(&bars->drain);
-      tc::mbar_wait(&bars->drain, 0, kWaitLimitNs);
+      tc::mma_commit(&bars->drain[1]);
+      tc::mbar_wait(&bars->drain[1], 0, kWaitLimitNs);
     }
     __syncwarp();
   } else {
-    // ---------------- epilogue: 8 compute + 8 send warps ----------------
+    // ---------------- epilogue ----------------
+    // A warp: 32 rows x 8 chains to send, then 8 of this CTA's own.
     // (waits are made warp-uniform so that no lane leaves a loop alone)
     const int quarter = warp & 3;                 // TMEM lanes (rows) 32*quarter ..
-    const int sub = (warp - 2) >> 2;              // chains [16 sub, 16 sub + 16)
-    const bool compute = (quarter >> 1) == (int)p;  // rows 64p .. 64p+63 are mine
+    const int sub = (warp - 2) >> 2;              // own chains 32p + 8 sub .. + 7
     const uint32_t lane_base = (uint32_t)(quarter * 32) << 16;
     const int r = quarter * 32 + lane;            // row of the tile (TMEM lane)
-    const int xrow = (quarter & 1) * 32 + lane;   // row in the 64-row exchange buffer
-    const uint32_t zx_peer = tc::map_to_rank(tc::smem_u32(Zx), peer) + xrow * kZxStride + sub * 64;
-    const uint32_t r_off = tc::sw128_offset(r, sub * 16);
-    const uint32_t r_off8 = tc::sw128_offset(r, sub * 16 + 8);
-    const uint32_t r_peer = tc::map_to_rank(tc::smem_u32(Rs), peer);
+    const int own = 32 * (int)p + 8 * sub, other = 32 * (int)peer + 8 * sub;
+    // Exchange buffer: chunk j (4 chains) of this warp's 8, row r.
+    const uint32_t zx_off = (uint32_t)(sub * 2 * 128 + r) * 16;
+    const uint32_t zx_peer = tc::map_to_rank(tc::smem_u32(Zx), peer) + zx_off;
+    unsigned char* Rmine = Rs + p * L::kRHalf;
+    const uint32_t r_off = tc::sw64_offset(r, sub);
+    unsigned char* r_block = Rmine + quarter * 2048;   // this quarter's 32 rows
+    const uint32_t r_peer = tc::map_to_rank(tc::smem_u32(r_block), peer);
     const uint32_t zx_full_peer = tc::map_to_rank(tc::smem_u32(&bars->zx_full), peer);
     const uint32_t zx_free_peer = tc::map_to_rank(tc::smem_u32(&bars->zx_free), peer);
     const uint32_t r_full_peer = tc::map_to_rank(tc::smem_u32(&bars->r_full), peer);
-    float sacc[16];
+    const bool first = warp == 4;                 // quarter 0, sub 0
+    float sacc[8];
 #pragma unroll
-    for (int c = 0; c < 16; ++c) sacc[c] = 0.f;
+    for (int c = 0; c < 8; ++c) sacc[c] = 0.f;
     bool ok = true;
     float y_next = 0.f;
-    if (compute) {
+    {
       const int row0 = rt_begin * kRows + r;
       if (T > 0 && row0 < N) y_next = y[row0];
     }
     for (int it = 0; it < T; ++it) {
       const int b = it & 1;
       const uint32_t ph = (uint32_t)it & 1;
-      if (!__all_sync(0xffffffffu, wait_or_abort(&bars->z_full[b], (uint32_t)(it >> 1) & 1, abort_flag))) {
+      if (!warp_wait(&bars->z_full[b], (uint32_t)(it >> 1) & 1, abort_flag)) {
         ok = false;
         break;
       }
       tc::tc_fence_after();
-      float h[16];
-      tc::tmem_ld16(tmem + b * CT + sub * 16 + lane_base, h);
+      float out[8], h[8];
+      tc::tmem_ld8(tmem + b * CT + other + lane_base, out);
+      tc::tmem_ld8(tmem + b * CT + own + lane_base, h);
       tc::tmem_ld_wait();
       tc::tc_fence_before();
       __syncwarp();
       if (lane == 0) tc::mbar_arrive(&bars->z_empty[b]);
-      if (!compute) {
-        // Send the partial of the peer's rows.
-        if (!__all_sync(0xffffffffu, wait_cluster_or_abort(&bars->zx_free, ph ^ 1, abort_flag))) {
-          ok = false;
-          break;
-        }
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-          tc::st_cluster_v4(zx_peer + 16 * j,
-                            make_uint4(__float_as_uint(h[4 * j]), __float_as_uint(h[4 * j + 1]),
-                                       __float_as_uint(h[4 * j + 2]),
-                                       __float_as_uint(h[4 * j + 3])));
-        // __syncwarp orders every lane's stores before lane 0's arrive, whose
-        // release (cluster scope) publishes them to the peer.
-        __syncwarp();
-        if (lane == 0) tc::mbar_arrive_cluster(zx_full_peer);
-        continue;
+      // The peer's chains' partial goes there, the peer's of mine comes here.
+      if (!__all_sync(0xffffffffu, wait_cluster_or_abort(&bars->zx_free, ph ^ 1, abort_flag))) {
+        ok = false;
+        break;
       }
-      // Compute warp: add the peer's partial for this row.
+#pragma unroll
+      for (int j = 0; j < 2; ++j)
+        tc::st_async_v4(zx_peer + 2048 * j,
+                        make_uint4(__float_as_uint(out[4 * j]), __float_as_uint(out[4 * j + 1]),
+                                   __float_as_uint(out[4 * j + 2]),
+                                   __float_as_uint(out[4 * j + 3])),
+                        zx_full_peer);
       if (!__all_sync(0xffffffffu, wait_cluster_or_abort(&bars->zx_full, ph, abort_flag))) {
         ok = false;
         break;
       }
-      const float4* zx = reinterpret_cast<const float4*>(Zx + xrow * kZxStride + sub * 64);
+      const float4* zx = reinterpret_cast<const float4*>(Zx + zx_off);
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const float4 v = zx[j];
+      for (int j = 0; j < 2; ++j) {
+        const float4 v = zx[128 * j];
         h[4 * j] += v.x;
         h[4 * j + 1] += v.y;
         h[4 * j + 2] += v.z;
         h[4 * j + 3] += v.w;
       }
-      __syncwarp();
-      if (lane == 0) tc::mbar_arrive_cluster(zx_free_peer);
       const int row = (rt_begin + it) * kRows + r;
       const bool valid = row < N;
       const float ym = (valid ? y_next : 0.f) - 0.5f;
       if (it + 1 < T && row + kRows < N) y_next = y[row + kRows];
-      uint32_t rp[8] = {0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
+      // R first: the MMAs wait for it; the rest waits for nobody.
+      uint32_t rp[4] = {0u, 0u, 0u, 0u};
       if (valid) {
 #pragma unroll
-        for (int j = 0; j < 16; ++j) {
-          const float a = fabsf(h[j]);
-          const float t = tc::ex2_approx(a * kNeg2Log2e);       // e^-|z|
-          sacc[j] += fmaf(kLn2, tc::lg2_approx(1.f + t), a);
-        }
-#pragma unroll
-        for (int j = 0; j < 8; ++j) rp[j] = residual_bf16x2(h[2 * j], h[2 * j + 1], ym);
+        for (int j = 0; j < 4; ++j) rp[j] = residual_bf16x2(h[2 * j], h[2 * j + 1], ym);
       }
       // Both CTAs' GEMM2 of the previous tile must be done with R.
       if (!__all_sync(0xffffffffu, wait_cluster_or_abort(&bars->r_free, ph ^ 1, abort_flag))) {
         ok = false;
         break;
       }
-      const uint4 v0 = make_uint4(rp[0], rp[1], rp[2], rp[3]);
-      const uint4 v1 = make_uint4(rp[4], rp[5], rp[6], rp[7]);
-      *reinterpret_cast<uint4*>(Rs + r_off) = v0;
-      *reinterpret_cast<uint4*>(Rs + r_off8) = v1;
-      tc::st_cluster_v4(r_peer + r_off, v0);
-      tc::st_cluster_v4(r_peer + r_off8, v1);
+      *reinterpret_cast<uint4*>(Rmine + r_off) = make_uint4(rp[0], rp[1], rp[2], rp[3]);
       tc::fence_proxy_async_smem();
-      tc::fence_proxy_async_cluster();
       __syncwarp();
+      if (sub != 0) {
+        if (lane == 0) {
+          tc::mbar_arrive(&bars->r_rows[quarter]);
+          tc::mbar_arrive(&bars->r_full);
+        }
+      } else {
+        // The quarter's first warp sends its 32 rows.
+        if (!warp_wait(&bars->r_rows[quarter], ph, abort_flag)) {
+          ok = false;
+          break;
+        }
+        if (lane == 0) {
+          tc::bulk_copy_cluster(r_peer, r_block, 2048, r_full_peer);
+          if (first)
+            tc::mbar_arrive_expect_tx(&bars->r_full, L::kRHalf);   // with the peer's copies
+          else
+            tc::mbar_arrive(&bars->r_full);
+        }
+      }
       if (lane == 0) {
-        tc::mbar_arrive(&bars->r_full);
-        tc::mbar_arrive_cluster(r_full_peer);
+        // One warp opens the next exchange (its bytes may be there before).
+        if (first && it + 1 < T) tc::mbar_arrive_expect_tx(&bars->zx_full, L::kZxBytes);
+        tc::mbar_arrive_cluster(zx_free_peer);
+      }
+      if (valid) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const float a = fabsf(h[j]);
+          const float t = tc::ex2_approx(a * kNeg2Log2e);       // e^-|z|
+          sacc[j] += fmaf(kLn2, tc::lg2_approx(1.f + t), a);
+        }
       }
     }
     if (ok && T > 0) ok = __all_sync(0xffffffffu, wait_or_abort(&bars->g_done, 0, abort_flag));
@@ -1219,25 +1263,22 @@ logreg_tc_pair_kernel(const __grid_constant__ CUtensorMap xmap, const float* __r
         }
       }
     }
-    if (compute) {
-      // Nonlinear log-likelihood partial of this warp's 32 rows, per chain,
-      // into red[p][quarter & 1][chain] of CTA 0 (the exchange buffer is idle
-      // after the loop; both CTAs have finished it at the cluster barrier).
+    // Nonlinear log-likelihood partial of this warp's 32 rows, per chain, into
+    // red[quarter][chain] of CTA 0 (the exchange buffer is idle after the loop; both
+    // CTAs have finished it at the cluster barrier).
 #pragma unroll
-      for (int j = 0; j < 16; ++j) {
-        float v = -sacc[j];
+    for (int j = 0; j < 8; ++j) {
+      float v = -sacc[j];
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-        if (j == lane) lp_pub = v;
-      }
+      for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+      if (j == lane) lp_pub = v;
     }
   }
   tc::tc_fence_before();
   __syncthreads();
   tc::cluster_sync();
-  if (warp >= 2 && ((warp & 3) >> 1) == (int)p && lane < 16) {
-    const int sub = (warp - 2) >> 2;
-    const int slot = ((int)p * 2 + (warp & 1)) * CT + sub * 16 + lane;
+  if (warp >= 2 && lane < 8) {
+    const int slot = (warp & 3) * CT + 32 * (int)p + 8 * ((warp - 2) >> 2) + lane;
     const uint32_t dst = tc::map_to_rank(tc::smem_u32(Zx), 0) + slot * 8;
     const double dv = (double)lp_pub;
     asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(dst), "d"(dv) : "memory");

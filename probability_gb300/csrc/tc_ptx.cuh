@@ -119,6 +119,26 @@ __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
                : "memory");
 }
 
+// 16 bytes to a CTA of the cluster, completing on that CTA's barrier.
+__device__ __forceinline__ void st_async_v4(uint32_t addr, uint4 v, uint32_t cluster_bar) {
+  asm volatile(
+      "st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, "
+      "[%5];" ::"r"(addr),
+      "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w), "r"(cluster_bar)
+      : "memory");
+}
+
+// Bulk copy from this CTA's shared memory to a CTA of the cluster (addresses and
+// size multiples of 16 bytes); the bytes complete on that CTA's barrier.
+__device__ __forceinline__ void bulk_copy_cluster(uint32_t dst, const void* src, uint32_t bytes,
+                                                  uint32_t cluster_bar) {
+  asm volatile(
+      "cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, "
+      "[%3];" ::"r"(dst),
+      "r"(smem_u32(src)), "r"(bytes), "r"(cluster_bar)
+      : "memory");
+}
+
 // try_wait with cluster-scope acquire (for phases completed by remote arrivals).
 __device__ __forceinline__ bool mbar_try_wait_cluster(uint64_t* bar, uint32_t parity) {
   uint32_t ok;
@@ -333,6 +353,19 @@ __device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t addr, uint32_t lbo,
   return d;
 }
 
+// The descriptor `bytes` further on.  Only its low word changes (start addresses
+// lie below 256 KB, so the 14-bit field holds the sum), which keeps an MMA's
+// descriptors at one addition each.
+__device__ __forceinline__ uint64_t desc_at(uint64_t desc, uint32_t bytes) {
+  return (desc & 0xffffffff00000000ull) | (uint32_t)((uint32_t)desc + (bytes >> 4));
+}
+
+// The same with 64-byte swizzle (mode 4): rows of 64 bytes (32 16-bit elements),
+// atoms of 8 rows.
+__device__ __forceinline__ uint64_t smem_desc_sw64(uint32_t addr, uint32_t lbo, uint32_t sbo) {
+  return (smem_desc_sw128(addr, lbo, sbo) & ~((uint64_t)7 << 61)) | (uint64_t)4 << 61;
+}
+
 // Instruction descriptor, kind::f16 with BF16 A/B and FP32 D: D format (bits
 // 4-5) = F32, A/B format (7-9, 10-12) = BF16, A/B major (15, 16: 0 = K-major,
 // 1 = MN-major), N >> 3 (17-22), M >> 4 (24-28).
@@ -354,6 +387,12 @@ __host__ __device__ constexpr uint32_t idesc_16bit_f32(int M, int N, bool a_mn, 
 __host__ __device__ __forceinline__ uint32_t sw128_offset(uint32_t row, uint32_t col_bf16) {
   const uint32_t chunk = (col_bf16 >> 3) ^ (row & 7u);
   return row * 128u + chunk * 16u + (col_bf16 & 7u) * 2u;
+}
+
+// Byte offset of 16-byte chunk `chunk` (0..3) of row `row` in a 64-byte-swizzled
+// block: the chunk index is XOR-ed with (row / 2) % 4.
+__host__ __device__ __forceinline__ uint32_t sw64_offset(uint32_t row, uint32_t chunk) {
+  return row * 64u + ((chunk ^ ((row >> 1) & 3u)) * 16u);
 }
 
 }  // namespace tc

@@ -42,8 +42,9 @@ namespace {
 
 constexpr size_t kCublasWs = 32u << 20;   // cuBLAS workspace inside the target workspace
 constexpr int kRowBlock = 2048;           // rows per epilogue block
-constexpr int kEpiThreads = 256;          // epilogue block size
-constexpr int kEpiRows = kRowBlock / kEpiThreads;
+constexpr int kEpiThreads = 64;           // epilogue block: a row block of one chain
+constexpr int kEpiRows = kRowBlock / 256;  // rows, 256 apart, of one FP32 sum
+constexpr int kEpiBatch = 4;              // of them loaded together
 // Rows from which the FP32 target's X^T R comes from FP16 pairs.  Faster below,
 // too (2001 x 300, 64 chains: 61 against 83 us), but there the FP32 GEMM, with few
 // additions, is the more exact one (1.5e-7 of the gradient against 1.8e-7).
@@ -136,85 +137,116 @@ __global__ void large_split_states(const float* __restrict__ q, int ldq, int n, 
   if (lo) lo[i] = from_float<TO>(v - (float)h);
 }
 
+// Four consecutive residuals, 8 or 16 bytes.
+__device__ __forceinline__ void store4(float* p, const float (&v)[4]) {
+  *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
+}
+template <class TO>
+__device__ __forceinline__ void store4(TO* p, const float (&v)[4]) {
+  TO t[4] = {from_float<TO>(v[0]), from_float<TO>(v[1]), from_float<TO>(v[2]),
+             from_float<TO>(v[3])};
+  *reinterpret_cast<uint2*>(p) = *reinterpret_cast<const uint2*>(t);
+}
+
 // Over Z [n columns][N rows] (column-major): per (row block, chain) the sum
 // of |z|/2 + ln(1 + e^-|z|) (float64 partial) and R = (y - 1/2) - sign(z)
 // (1/(1 + e^-|z|) - 1/2) (hi, and lo in the mixed form).
+//
+// What bounds it: memory (in the mixed form Z is as large as the L2 and R half of
+// that).  A thread takes four consecutive rows at a time, 16-byte loads, four rows'
+// batches in flight; the rows 256 apart that were one thread's when a thread took
+// one row stay one FP32 sum.  65,371 rows, 240 chains of hi and lo: 48 us with one
+// row a thread, 33 so; blocks of 256 threads and more loads in flight were slower.
 template <class TO>
-__global__ void __launch_bounds__(kEpiThreads)
+__global__ void __launch_bounds__(kEpiThreads, 16)
 large_epilogue(const float* __restrict__ Z, const float* __restrict__ Zlo,
                const float* __restrict__ ym, int64_t N, int64_t ldz, int n,
                TO* __restrict__ Rhi, TO* __restrict__ Rlo, double* __restrict__ part) {
-  __shared__ double red[8];
-  const int64_t r0 = (int64_t)blockIdx.x * kRowBlock;
+  __shared__ double red;
+  const int64_t r0 = (int64_t)blockIdx.x * kRowBlock + 4 * threadIdx.x;
   for (int c = blockIdx.y; c < n; c += gridDim.y) {   // grid.y is capped at 65535
-    const float* z = Z + (size_t)c * ldz;
-    const float* zl = Zlo ? Zlo + (size_t)c * ldz : nullptr;
-    // A thread's kEpiRows rows (stride blockDim): every load is issued before
-    // any use, so the block waits for memory once per chain, not per row.
-    float zv[kEpiRows], yv[kEpiRows];
+    const size_t col = (size_t)c * ldz;
+    float acc[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-    for (int k = 0; k < kEpiRows; ++k) {
-      const int64_t r = r0 + threadIdx.x + (int64_t)kEpiThreads * k;
-      zv[k] = 0.f;
-      yv[k] = 0.f;
-      if (r < N) {
-        zv[k] = zl ? z[r] + zl[r] : z[r];
-        yv[k] = ym[r];
+    for (int k0 = 0; k0 < kEpiRows; k0 += kEpiBatch) {
+      float4 zv[kEpiBatch], zl[kEpiBatch];
+#pragma unroll
+      for (int k = 0; k < kEpiBatch; ++k) {
+        const int64_t r = r0 + 256 * (k0 + k);
+        zv[k] = zl[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (r < ldz) {      // ldz is a multiple of 8: all four or none
+          zv[k] = __ldcs(reinterpret_cast<const float4*>(Z + col + r));
+          if (Zlo) zl[k] = __ldcs(reinterpret_cast<const float4*>(Zlo + col + r));
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < kEpiBatch; ++k) {
+        const int64_t r = r0 + 256 * (k0 + k);
+        if (r >= ldz) break;
+        const float4 y4 = *reinterpret_cast<const float4*>(ym + r);
+        const float yv[4] = {y4.x, y4.y, y4.z, y4.w};
+        float z[4] = {zv[k].x, zv[k].y, zv[k].z, zv[k].w};
+        if (Zlo) {
+          z[0] += zl[k].x;
+          z[1] += zl[k].y;
+          z[2] += zl[k].z;
+          z[3] += zl[k].w;
+        }
+        float hi[4], lo[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          hi[e] = lo[e] = 0.f;     // padding rows: zero residual, no likelihood term
+          if (r + e >= N) continue;
+          const float a = fabsf(z[e]);
+          const float t = tc::ex2_approx(a * kNegLog2eL);
+          const float u = 1.f + t;
+          acc[e] += fmaf(kLn2L, tc::lg2_approx(u), 0.5f * a);
+          const float w = tc::rcp_approx(u) - 0.5f;
+          hi[e] = (z[e] >= 0.f ? yv[e] - w : yv[e] + w) * Stored<TO>::kScale;
+          lo[e] = hi[e] - (float)from_float<TO>(hi[e]);
+        }
+        store4(Rhi + col + r, hi);
+        if (Rlo) store4(Rlo + col + r, lo);
       }
     }
-    float acc = 0.f;   // this thread's rows in FP32; float64 across threads
-#pragma unroll
-    for (int k = 0; k < kEpiRows; ++k) {
-      const int64_t r = r0 + threadIdx.x + (int64_t)kEpiThreads * k;
-      if (r >= ldz) break;
-      if (r >= N) {   // padding rows: zero residual, no likelihood term
-        Rhi[(size_t)c * ldz + r] = from_float<TO>(0.f);
-        if (Rlo) Rlo[(size_t)c * ldz + r] = from_float<TO>(0.f);
-        continue;
-      }
-      const float a = fabsf(zv[k]);
-      const float e = tc::ex2_approx(a * kNegLog2eL);
-      const float u = 1.f + e;
-      acc += fmaf(kLn2L, tc::lg2_approx(u), 0.5f * a);
-      const float w = tc::rcp_approx(u) - 0.5f;
-      const float rv = (zv[k] >= 0.f ? yv[k] - w : yv[k] + w) * Stored<TO>::kScale;
-      const TO h = from_float<TO>(rv);
-      Rhi[(size_t)c * ldz + r] = h;
-      if (Rlo) Rlo[(size_t)c * ldz + r] = from_float<TO>(rv - (float)h);
-    }
-    const double accd = warp_sum((double)acc);
-    __syncthreads();                                   // red[] of the previous chain is read
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = accd;
+    const double sum = warp_sum(((double)acc[0] + (double)acc[1]) +
+                                ((double)acc[2] + (double)acc[3]));
+    if (threadIdx.x == 32) red = sum;
     __syncthreads();
-    if (threadIdx.x == 0) {
-      double s = 0.0;
-      for (int w = 0; w < (int)(blockDim.x >> 5); ++w) s += red[w];
-      part[(size_t)blockIdx.x * n + c] = (double)Stored<TO>::kSign * s;
-    }
+    if (threadIdx.x == 0)
+      part[(size_t)blockIdx.x * n + c] = (double)Stored<TO>::kSign * (sum + red);
+    __syncthreads();                                   // red of this chain is read
   }
 }
 
-// One warp per chain: log-density from the partials (fixed order), the
-// linear term and the prior; gradient G - q / s^2.
-__global__ void large_finish(const double* __restrict__ part, int nblk, int n,
-                             const float* __restrict__ G, const float* __restrict__ Glo, int ld,
-                             const float* __restrict__ q, int ldq,
-                             const double* __restrict__ lin, int D, float inv_var,
-                             double log_norm, double* __restrict__ logp,
-                             float* __restrict__ grad, int ldg) {
-  const int c = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-  const int lane = threadIdx.x & 31;
-  if (c >= n) return;
+// One block per chain: log-density from the partials, the linear term and the
+// prior, in a fixed order; gradient G - q / s^2.  (A warp per chain waited for its
+// loads in turn: 15 us at 929 features, 240 chains, 8 so.)
+constexpr int kFinishThreads = 256;
+__global__ void __launch_bounds__(kFinishThreads)
+large_finish(const double* __restrict__ part, int nblk, int n, const float* __restrict__ G,
+             const float* __restrict__ Glo, int ld, const float* __restrict__ q, int ldq,
+             const double* __restrict__ lin, int D, float inv_var, double log_norm,
+             double* __restrict__ logp, float* __restrict__ grad, int ldg) {
+  __shared__ double red[kFinishThreads / 32];
+  const int c = blockIdx.x, tid = threadIdx.x;
   double t = 0.0;
-  for (int b = lane; b < nblk; b += 32) t -= part[(size_t)b * n + c];
-  for (int d = lane; d < D; d += 32) {
+#pragma unroll 4
+  for (int d = tid; d < D; d += kFinishThreads) {
     const float qv = q[(size_t)c * ldq + d];
     t += lin[d] * (double)qv - 0.5 * (double)inv_var * (double)qv * (double)qv;
     const float g = Glo ? G[(size_t)c * ld + d] + Glo[(size_t)c * ld + d] : G[(size_t)c * ld + d];
     grad[(size_t)c * ldg + d] = g - qv * inv_var;
   }
+  for (int b = tid; b < nblk; b += kFinishThreads) t -= part[(size_t)b * n + c];
   t = warp_sum(t);
-  if (lane == 0) logp[c] = t + (double)D * log_norm;
+  if ((tid & 31) == 0) red[tid >> 5] = t;
+  __syncthreads();
+  if (tid == 0) {
+    double s = 0.0;
+    for (int w = 0; w < kFinishThreads / 32; ++w) s += red[w];
+    logp[c] = s + (double)D * log_norm;
+  }
 }
 
 class LogregLarge final : public Target {
@@ -362,7 +394,7 @@ class LogregLarge final : public Target {
     };
     gemm_g(xh_.ptr, w, &zero);
     if (xlo_) gemm_g(xl_.ptr, n, &one);
-    large_finish<<<(unsigned)((n + 7) / 8), 256, 0, s>>>(
+    large_finish<<<(unsigned)n, kFinishThreads, 0, s>>>(
         part, (int)nblk, n, G, mixed_ ? G + (size_t)n * ld_ : nullptr, ld_, q, ldq,
         lin_.as<double>(), D, inv_var_, log_norm_, logp, grad, ldg);
     GBM_CUDA(cudaGetLastError());

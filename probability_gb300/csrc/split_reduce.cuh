@@ -4,19 +4,21 @@
 // Layout written by the partial kernels: lpart[S][n] (float64) and
 // gpart[S][n][D] (float32), where S = number of row splits for n chains:
 //   S = clamp(grid / ceil(n / ct), 1, ceil(N / nt)).
-// One block per chain: a thread of each 128 owns features thread + 128 k and
-// adds up to kOrdered splits in index order, 16 loads in flight; with more
-// splits, groups of 128 threads add a range of them each and the ranges are
-// added in order.  The log-density terms (likelihood partials, prior, linear
-// part) are combined per lane by the first warp and summed by one float64 warp
+// One block per chain and 128 features: a thread owns a feature and adds up to
+// kOrdered splits in index order, 16 loads in flight; with more splits, groups of
+// 128 threads add a range of them each and the ranges are added in order.  The
+// log-density terms (likelihood partials, prior, linear part) are combined per
+// lane by the last warp of a chain's first block and summed by one float64 warp
 // reduction.  The order depends only on S, D and the launch, so results are
 // reproducible.
 //
 // What bounds it: the latency of the partials' loads (L2), so the loads of a
 // chain are spread over threads instead of over rounds of one warp.  Measured
 // with the partial kernel: 12,007 x 173 BF16, 77 chains (94 splits) 37.2 us with
-// a warp per chain, 28.7 so; a leapfrog step of 1000 x 25, 64 chains 40.8 and
-// 38.2; 1024 chains (19 splits) the same (four groups there: 10 us more).
+// a warp per chain, 28.7 with a block, 26.3 so; 12,289 x 601 FP32, 99 chains (50
+// splits) 95.2 with a block for all features, 90.6 so; a leapfrog step of 1000 x
+// 25, 64 chains 40.8 with a warp and
+// 38.2 with a block; 1024 chains (19 splits) the same (four groups there: 10 us more).
 // `lin` (optional, float64 [D]) adds lin . q_c to each chain's log-density:
 // the tensor-core kernels leave the linear part sum_r (y_r - 1/2) z_rc of the
 // Bernoulli log-likelihood to this pass as (X^T (y - 1/2)) . q_c, exact in
@@ -100,58 +102,43 @@ split_reduce_kernel(const double* __restrict__ lpart, const float* __restrict__ 
                     int c_base, int c_lim, int ct, int nt, int grid, int N, int D,
                     float inv_var, double log_norm, const double* __restrict__ lin, int lparts,
                     double* __restrict__ logp, float* __restrict__ grad, int ldg) {
-  __shared__ float range[kReduceGroups - 1][512];
+  __shared__ float range[kReduceGroups - 1][128];
   const int n = n_dev ? chunk_count(*n_dev, c_base, c_lim) : c_lim;
   const int c = blockIdx.x;
   if (c >= n) return;
   const int S = split_count(n, ct, nt, grid, N);
-  const size_t stride = (size_t)n * D;
-  const float* p = gpart + (size_t)c * D;
   const float* q = Q + (size_t)c * ldq;
   const int groups = S <= kOrdered ? 1 : (int)(blockDim.x >> 7);
   const int group = threadIdx.x >> 7, first = threadIdx.x & 127;
-  if (group > 0 && groups == 1) return;
-  const int s0 = groups > 1 ? group * S / groups : 0;
-  const int s1 = groups > 1 ? (group + 1) * S / groups : S;
-  for (int d0 = 0; d0 < D; d0 += 512) {
-    float acc[4];
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const int d = d0 + first + 128 * k;
-      if (d < D) {
-        acc[k] = sum_splits(p + d, stride, s0, s1);
-        if (group > 0) range[group - 1][first + 128 * k] = acc[k];
-      }
+  const int d = blockIdx.y * 128 + first;
+  float acc = 0.f;
+  if (d < D && group < groups)
+    acc = sum_splits(gpart + (size_t)c * D + d, (size_t)n * D,
+                     groups > 1 ? group * S / groups : 0,
+                     groups > 1 ? (group + 1) * S / groups : S);
+  // Per-lane log-density terms, by the last warp beside the others' sums:
+  // likelihood partials lane, lane + 32, ..., then lin . q - q.q / (2 s^2) over
+  // features lane, lane + 32, ...
+  if (blockIdx.y == 0 && threadIdx.x + 32 >= blockDim.x) {
+    const int lane = threadIdx.x & 31, rows = lparts > 0 ? lparts : S;
+    double t = 0.0;
+    for (int j = lane; j < rows; j += 32) t += lpart[(size_t)j * n + c];
+    double pr = 0.0, li = 0.0;
+    for (int f = lane; f < D; f += 32) {
+      const double qd = (double)q[f];
+      pr += qd * qd;
+      if (lin) li += lin[f] * qd;
     }
-    if (groups > 1) {
-      __syncthreads();
-#pragma unroll
-      for (int k = 0; k < 4; ++k)
-        if (group == 0 && d0 + first + 128 * k < D)
-          for (int g = 0; g + 1 < groups; ++g) acc[k] += range[g][first + 128 * k];
-      if (d0 + 512 < D) __syncthreads();   // the ranges are written again
-    }
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const int d = d0 + first + 128 * k;
-      if (group == 0 && d < D) grad[(size_t)c * ldg + d] = acc[k] - q[d] * inv_var;
-    }
+    t = warp_sum(t + li - 0.5 * (double)inv_var * pr);
+    if (lane == 0) logp[c] = t + (double)D * log_norm;
   }
-  if (threadIdx.x >= 32) return;
-  // Per-lane log-density terms: likelihood partials of splits lane, lane + 32,
-  // ..., then lin . q - q.q / (2 s^2) over features lane, lane + 32, ...
-  const int lane = threadIdx.x;
-  double t = 0.0;
-  const int rows = lparts > 0 ? lparts : S;
-  for (int j = lane; j < rows; j += 32) t += lpart[(size_t)j * n + c];
-  double pr = 0.0, li = 0.0;
-  for (int d = lane; d < D; d += 32) {
-    const double qd = (double)q[d];
-    pr += qd * qd;
-    if (lin) li += lin[d] * qd;
+  if (groups > 1) {
+    if (group > 0) range[group - 1][first] = acc;
+    __syncthreads();
+    if (group == 0)
+      for (int g = 0; g + 1 < groups; ++g) acc += range[g][first];
   }
-  t = warp_sum(t + li - 0.5 * (double)inv_var * pr);
-  if (lane == 0) logp[c] = t + (double)D * log_norm;
+  if (group == 0 && d < D) grad[(size_t)c * ldg + d] = acc - q[d] * inv_var;
 }
 
 // Q, logp and grad point at chain c_base of the batch; `cap` bounds this
@@ -165,7 +152,8 @@ void launch_split_reduce(const double* lpart, const float* gpart, const float* Q
   // Few chains make many splits: several threads per feature.  (A sampler's
   // active chains are fewer than cap; one thread then adds more than kOrdered.)
   const int threads = split_count(cap, ct, nt, grid, N) <= kOrdered ? 128 : 128 * kReduceGroups;
-  split_reduce_kernel<<<(unsigned)cap, threads, 0, s>>>(
+  const dim3 blocks((unsigned)cap, (unsigned)((D + 127) / 128));
+  split_reduce_kernel<<<blocks, threads, 0, s>>>(
       lpart, gpart, Q, ldq, n_dev, c_base, c_lim, ct, nt, grid, N, D, inv_var, log_norm, lin, lparts,
       logp, grad, ldg);
   GBM_CUDA(cudaGetLastError());

@@ -16,9 +16,9 @@
 // chain are spread over threads instead of over rounds of one warp.  Measured
 // with the partial kernel: 12,007 x 173 BF16, 77 chains (94 splits) 37.2 us with
 // a warp per chain, 28.7 with a block, 26.3 so; 12,289 x 601 FP32, 99 chains (50
-// splits) 95.2 with a block for all features, 90.6 so; a leapfrog step of 1000 x
-// 25, 64 chains 40.8 with a warp and
-// 38.2 with a block; 1024 chains (19 splits) the same (four groups there: 10 us more).
+// splits) 95.2 with a block for all features, 90.6 so; a step of three launches at
+// 1000 x 25, 64 chains 40.8 with a warp, 38.2 with a block; 1024 chains (19 splits)
+// the same (four groups there: 10 us more).
 // `lin` (optional, float64 [D]) adds lin . q_c to each chain's log-density:
 // the tensor-core kernels leave the linear part sum_r (y_r - 1/2) z_rc of the
 // Bernoulli log-likelihood to this pass as (X^T (y - 1/2)) . q_c, exact in

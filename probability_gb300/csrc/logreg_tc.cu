@@ -321,6 +321,7 @@ logreg_tc_kernel(const __grid_constant__ CUtensorMap xmap,
       tc::mma_commit(&bars->drain);
       tc::mbar_wait(&bars->drain, 0, kWaitLimitNs);
     }
+    __syncwarp();   // the whole warp frees the TMEM below
   } else {
     // ---------------- epilogue (EPI warps) ----------------
     const int quarter = warp & 3;                 // TMEM lanes 32*quarter ..
@@ -748,6 +749,7 @@ logreg_tct_kernel(const __grid_constant__ CUtensorMap xmap,
       tc::mma_commit(&bars->drain);
       tc::mbar_wait(&bars->drain, 0, kWaitLimitNs);
     }
+    __syncwarp();   // the whole warp frees the TMEM below
   } else {
     // ---------------- epilogue (16 warps) ----------------
     // Kahan sum over tiles of sum_r (|h_r| + ln(1 + e^-|z_r|)) for this
@@ -1014,22 +1016,22 @@ logreg_tc_pair_kernel(const __grid_constant__ CUtensorMap xmap, const float* __r
       const uint64_t bhk = tc::smem_desc_sw128(tc::smem_u32(Bhi), 16, 1024);
       const uint64_t blk = tc::smem_desc_sw128(tc::smem_u32(Blo), 16, 1024);
       const int ksteps = (fD + 15) >> 4;        // K-steps of 16 features holding data
-      // Half-stage fills in order: fill f is (tile f / 2, half f % 2).
-      int nfill = 0;
+      const int halves = ksteps > 8 ? 2 : 1;    // half-stages that hold data
+      int loads = 0;                            // tiles whose loads were issued
       bool ok = true;
       auto load = [&](int it) -> bool {
         const int s = it & 1;
-        for (int h = 0; h < 2; ++h) {
+        for (int h = 0; h < halves; ++h) {
           if (!wait_or_abort(&bars->x_empty[s][h], ((uint32_t)(it >> 1) & 1) ^ 1, abort_flag)) {
             tc::record_error(err, kTcTimeoutTma);
             return false;
           }
+          loads = it + 1;
           tc::mbar_arrive_expect_tx(&bars->x_full[s][h], L::kXStage / 2);
 #pragma unroll
           for (int kb = 2 * h; kb < 2 * h + 2; ++kb)
             tc::tma_load_2d(Xs + s * L::kXStage + kb * 16384, &xmap, f0 + kb * 64,
                             (rt_begin + it) * kRows, &bars->x_full[s][h]);
-          ++nfill;
         }
         return true;
       };
@@ -1039,9 +1041,8 @@ logreg_tc_pair_kernel(const __grid_constant__ CUtensorMap xmap, const float* __r
         if (!wait_or_abort(&bars->z_empty[b], use ^ 1, abort_flag)) return false;
         const uint32_t tz = tmem + b * CT;
         const uint64_t xs = tc::desc_at(xk, s * L::kXStage);
-        // Half h holds K-steps 8h .. 8h + 7; a half without data (fD <= 128)
-        // is neither waited for nor read.
-        for (int h = 0; h < 2 && 8 * h < ksteps; ++h) {
+        // Half h holds K-steps 8h .. 8h + 7.
+        for (int h = 0; h < halves; ++h) {
           if (!wait_or_abort(&bars->x_full[s][h], use, abort_flag)) return false;
           tc::tc_fence_after();
 #pragma unroll
@@ -1073,11 +1074,10 @@ logreg_tc_pair_kernel(const __grid_constant__ CUtensorMap xmap, const float* __r
       }
       tc::mma_commit(&bars->drain[0]);
       tc::mbar_wait(&bars->drain[0], 0, kWaitLimitNs);
-      // Let the last fills land before the CTA can exit (each wait bounded).
-      for (int f = (nfill > 4 ? nfill - 4 : 0); f < nfill; ++f) {
-        const int j = f >> 1, h = f & 1;
-        tc::mbar_wait(&bars->x_full[j & 1][h], (uint32_t)((j >> 1) & 1), kWaitLimitNs);
-      }
+      // Let the last loads land before the CTA can exit (each wait bounded).
+      for (int j = (loads > 2 ? loads - 2 : 0); j < loads; ++j)
+        for (int h = 0; h < halves; ++h)
+          tc::mbar_wait(&bars->x_full[j & 1][h], (uint32_t)((j >> 1) & 1), kWaitLimitNs);
     }
     __syncwarp();
   } else if (warp == 1) {
@@ -1106,7 +1106,6 @@ logreg_tc_pair_kernel(const __grid_constant__ CUtensorMap xmap, const float* __r
           }
           tc::mma_commit(&bars->x_empty[it & 1][mt]);
         }
-        if (mtiles == 1) tc::mma_commit(&bars->x_empty[it & 1][1]);
         tc::mma_commit_multicast(&bars->r_free, (uint16_t)0x3);
       }
       if (ok) {
@@ -1243,6 +1242,11 @@ logreg_tc_pair_kernel(const __grid_constant__ CUtensorMap xmap, const float* __r
       }
     }
     if (ok && T > 0) ok = __all_sync(0xffffffffu, wait_or_abort(&bars->g_done, 0, abort_flag));
+    // Both CTAs' last release of R has arrived here: nothing of the peer's is on its
+    // way to this CTA when it exits.
+    if (ok && T > 0)
+      ok = __all_sync(0xffffffffu,
+                      wait_cluster_or_abort(&bars->r_free, (uint32_t)(T - 1) & 1, abort_flag));
     if (!ok) {
       tc::record_error(err, kTcTimeoutEpilogue);
       abort_both();

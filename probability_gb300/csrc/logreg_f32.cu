@@ -197,6 +197,33 @@ __device__ __forceinline__ void f32_epilogue(const float (&z)[4][8], const float
   for (int c = 0; c < 8; ++c) kahan_add(f32_like(sabs[c], prod[c]), lsum[c], lcomp[c]);
 }
 
+// The epilogue of four rows x four pairs of chains; `store` gets R of a row.
+template <class Store>
+__device__ __forceinline__ void f32_epilogue_pairs(const float2 (&z)[8][4], int first,
+                                                   const float (&yr)[4], int nvalid,
+                                                   float (&lsum)[8], float (&lcomp)[8],
+                                                   Store&& store) {
+  float2 sabs[4], prod[4];
+#pragma unroll
+  for (int c = 0; c < 4; ++c) {
+    sabs[c] = make_float2(0.f, 0.f);
+    prod[c] = make_float2(1.f, 1.f);
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    float2 r[4];
+#pragma unroll
+    for (int c = 0; c < 4; ++c)
+      r[c] = f32_residual2(z[first + i][c], yr[i], i < nvalid, sabs[c], prod[c]);
+    store(i, r);
+  }
+#pragma unroll
+  for (int c = 0; c < 4; ++c) {
+    kahan_add(f32_like(sabs[c].x, prod[c].x), lsum[2 * c], lcomp[2 * c]);
+    kahan_add(f32_like(sabs[c].y, prod[c].y), lsum[2 * c + 1], lcomp[2 * c + 1]);
+  }
+}
+
 template <int KD>
 __global__ void __launch_bounds__(kF32Threads, 1)
 logreg_f32_kernel(const float* __restrict__ X2, const float* __restrict__ ym, int N, int D,
@@ -369,7 +396,7 @@ logreg_f32_kernel(const float* __restrict__ X2, const float* __restrict__ ym, in
 //
 // What bounds it: the FMA pipe in phase 1, half of the kernel (107 of 128 FMAs a
 // clock and SM), and the issue of the epilogues.  An evaluation at 1e5 rows, 1024
-// chains: 523 us at 100 features (both phases on the CUDA cores: 849; this
+// chains: 516 us at 100 features (both phases on the CUDA cores: 849; this
 // kernel with one group of eight warps, epilogues together: 547), 221 at 25
 // (344), 54 at 4 and 256 chains (72).
 // ---------------------------------------------------------------------------
@@ -618,34 +645,28 @@ logreg_f32_tc_kernel(const __grid_constant__ CUtensorMap himap,
           if (t == 0) drain();
         }
         // ---- epilogue: log-likelihood sums, R' in FP16 hi + lo ----
-        float zt[4][8];
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-#pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            zt[i][2 * c] = z[4 * t + i][c].x;
-            zt[i][2 * c + 1] = z[4 * t + i][c].y;
-          }
         const float yr[4] = {yv[t].x, yv[t].y, yv[t].z, yv[t].w};
         const int nvalid = N - (rt_begin + it) * kF32RT - 4 * ty;   // rows of mine that exist
-        f32_epilogue(zt, yr, nvalid, lsum, lcomp, [&](int i, const float(&r)[8]) {
+        auto put = [&](int i, const float2(&r)[4]) {
           const uint32_t off = tc::sw128_offset(4 * gy + i, 4 * tx);
 #pragma unroll
           for (int b = 0; b < 2; ++b) {
             uint32_t hi[2], lo[2];
 #pragma unroll
             for (int e = 0; e < 2; ++e) {
-              const float v0 = r[4 * b + 2 * e] * kF16Scale, v1 = r[4 * b + 2 * e + 1] * kF16Scale;
-              const __half2 h = __floats2half2_rn(v0, v1);
+              const float2 v = __fmul2_rn(r[2 * b + e], make_float2(kF16Scale, kF16Scale));
+              const __half2 h = __float22half2_rn(v);
               const float2 hf = __half22float2(h);
-              const __half2 l = __floats2half2_rn(v0 - hf.x, v1 - hf.y);
+              const __half2 l =
+                  __float22half2_rn(__fadd2_rn(v, make_float2(-hf.x, -hf.y)));
               hi[e] = *reinterpret_cast<const uint32_t*>(&h);
               lo[e] = *reinterpret_cast<const uint32_t*>(&l);
             }
             *reinterpret_cast<uint2*>(R16 + b * kRBox + off) = make_uint2(hi[0], hi[1]);
             *reinterpret_cast<uint2*>(R16 + (2 + b) * kRBox + off) = make_uint2(lo[0], lo[1]);
           }
-        });
+        };
+        f32_epilogue_pairs(z, 4 * t, yr, nvalid, lsum, lcomp, put);
         tc::fence_proxy_async_smem();
         __syncwarp();
         if (lane == 0) tc::mbar_arrive(&bars->r_full);

@@ -30,6 +30,23 @@ __device__ __forceinline__ void f32_residual(float z, float yr, bool valid, floa
   r = yr + neg_copysign_f(w, z);
 }
 
+// The same for two chains, in packed arithmetic (the same roundings).
+__device__ __forceinline__ float2 f32_residual2(float2 z, float yr, bool valid, float2& sabs,
+                                                float2& prod) {
+  const float2 a = make_float2(fabsf(z.x), fabsf(z.y));
+  const float2 arg = __fmul2_rn(a, make_float2(kNegLog2e, kNegLog2e));
+  const float2 u = __fadd2_rn(make_float2(1.f, 1.f),
+                              make_float2(tc::ex2_approx(arg.x), tc::ex2_approx(arg.y)));
+  if (valid) {
+    sabs = __fadd2_rn(sabs, a);
+    prod = __fmul2_rn(prod, u);
+  }
+  const float2 w = __fadd2_rn(make_float2(tc::rcp_approx(u.x), tc::rcp_approx(u.y)),
+                              make_float2(-0.5f, -0.5f));
+  return __fadd2_rn(make_float2(yr, yr),
+                    make_float2(neg_copysign_f(w.x, z.x), neg_copysign_f(w.y, z.y)));
+}
+
 // -(sum |z|/2 + sum ln(1 + e^-|z|)) of four rows.
 __device__ __forceinline__ float f32_like(float sabs, float prod) {
   return -fmaf(kLn2f, tc::lg2_approx(prod), 0.5f * sabs);

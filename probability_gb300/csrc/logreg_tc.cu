@@ -65,36 +65,33 @@ __host__ __device__ inline int tc_splits(int n, int ct, int grid, int row_tiles)
   return s > row_tiles ? row_tiles : s;
 }
 
-// Shared memory of the row-major kernel (instantiated for 128 < D <= 256:
-// KB = 4, 64-chain tiles).  KB = 2 would give X_hi three stages, so that the
-// TMA refill of a stage (which can start only once GEMM2 has read it) runs a
-// full tile ahead of the GEMM1 that needs it, and a single R buffer.
-template <int KB, int CT, bool XLO>
+// The row-major kernel (128 < D <= 256): a tile is 128 rows x 64 chains.
+constexpr int kRowKB = 4;                   // 64-feature blocks of X
+constexpr int kRowCT = 64;                  // chains per tile
+constexpr int kRowEpi = 16;                 // epilogue warps
 struct TcLayout {
-  static constexpr int kStages = KB == 2 ? 3 : 2;      // X_hi stages
-  static constexpr int kRBufs = KB == 2 ? 1 : 2;       // R buffers
-  static constexpr int kXStage = KB * 16384;           // [KB][128 rows][128 B]
-  static constexpr int kBBytes = KB * CT * 128;        // [KB][CT rows][128 B]
-  static constexpr int kRBuf = (CT / 64) * 16384;      // [CT/64][128 rows][128 B]
+  static constexpr int kXStage = kRowKB * 16384;          // [KB][128 rows][128 B], 2 stages
+  static constexpr int kBBytes = kRowKB * kRowCT * 128;   // [KB][CT rows][128 B]
+  static constexpr int kRBuf = 16384;                     // [128 rows][128 B], 2 buffers
   static constexpr int kX = 0;
-  static constexpr int kBhi = kX + kStages * kXStage;
+  static constexpr int kBhi = kX + 2 * kXStage;
   static constexpr int kBlo = kBhi + kBBytes;
   static constexpr int kR = kBlo + kBBytes;
-  static constexpr int kXlo = kR + kRBufs * kRBuf;     // X residual, 1 stage (XLO only)
-  static constexpr int kCtl = kXlo + (XLO ? kXStage : 0);  // barriers + tmem slot + abort
+  static constexpr int kCtl = kR + 2 * kRBuf;             // barriers + tmem slot + abort
   // After the last MMA the R buffers are reused for the [4 quarters][CT]
   // double log-likelihood reduction.
   static constexpr int kRed = kR;
   static constexpr int kBytes = kCtl + 256;
-  static_assert(4 * CT * 8 <= kRBufs * kRBuf, "reduction scratch must fit the R buffers");
-  static constexpr int kMTiles = KB / 2;               // 128-feature tiles of G
-  static constexpr uint32_t kTmemCols = (2 * CT + kMTiles * CT) <= 256 ? 256 : 512;
+  static_assert(4 * kRowCT * 8 <= 2 * kRBuf, "reduction scratch must fit the R buffers");
+  static constexpr uint32_t kTmemCols = 256;              // two Z, two 128-feature tiles of G
   static_assert(kBytes + 1024 <= 232448, "shared memory over the sm_103a limit");
 };
 
 struct Bars {
-  uint64_t x_full[3], x_empty[3], z_full[2], z_empty[2], r_full[2], r_empty[2], g_done, drain;
-  uint64_t xlo_full, xlo_empty;
+  // X stages fill and drain in halves of 128 features: the G MMAs of the first
+  // free it while those of the second run.
+  uint64_t x_full[2][2], x_empty[2][2];   // [stage][half]
+  uint64_t z_full[2], z_empty[2], r_full[2], r_empty[2], g_done, drain[2];
 };
 
 __device__ __forceinline__ uint32_t pack_bf16x2(float a, float b) {
@@ -111,20 +108,22 @@ __device__ __forceinline__ uint32_t residual_bf16x2(float h0, float h1, float ym
   return pack_bf16x2(fmaf(-0.5f, tc::tanh_approx(h0), ym), fmaf(-0.5f, tc::tanh_approx(h1), ym));
 }
 
-// XLO: X is FP32 data stored as X_hi + X_lo (both BF16); GEMM1 adds the
-// X_lo B_hi product so Z keeps ~16 significant bits of the FP32 data.  The
-// gradient contraction uses X_hi.
-template <int KB, int CT, int EPI, bool XLO>
-__global__ void __launch_bounds__(tc_threads(EPI), 1)
-logreg_tc_kernel(const __grid_constant__ CUtensorMap xmap,
-                 const __grid_constant__ CUtensorMap xlomap, const float* __restrict__ y, int N,
+// One warp issues the loads of X and the MMAs of Z, another those of G, so that G
+// of a tile, ready when its R is, does not wait behind Z of the next tile for X.
+//
+// What bounds it: a tile's chain load, Z, R, G with two X stages in flight; MMAs of
+// N = 64 (2,000 clocks a tile at 200 features).  150,000 x 200, 200 chains: 81 us an
+// evaluation with eight epilogue warps, the likelihood before R and one thread that
+// issues all MMAs, 79 with sixteen and R first, 69 so.
+__global__ void __launch_bounds__(tc_threads(kRowEpi), 1)
+logreg_tc_kernel(const __grid_constant__ CUtensorMap xmap, const float* __restrict__ y, int N,
                  int D, const float* __restrict__ Q, int ldq, const int* __restrict__ n_dev,
                  int c_base, int c_lim, int grid, double* __restrict__ lpart,
                  float* __restrict__ gpart, int* __restrict__ err) {
-  using L = TcLayout<KB, CT, XLO>;
+  using L = TcLayout;
+  constexpr int KB = kRowKB, CT = kRowCT, EPI = kRowEpi;
   constexpr int kThreads = tc_threads(EPI);
   constexpr int kCW = CT * 4 / EPI;             // chains per epilogue warp
-  static_assert(kCW == 32 || kCW == 64, "epilogue width");
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>(
       (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -150,10 +149,11 @@ logreg_tc_kernel(const __grid_constant__ CUtensorMap xmap,
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if (tid == 0) {
-    for (int i = 0; i < 3; ++i) {
-      tc::mbar_init(&bars->x_full[i], 1);
-      tc::mbar_init(&bars->x_empty[i], 1);
-    }
+    for (int i = 0; i < 2; ++i)
+      for (int h = 0; h < 2; ++h) {
+        tc::mbar_init(&bars->x_full[i][h], 1);
+        tc::mbar_init(&bars->x_empty[i][h], 1);
+      }
     for (int i = 0; i < 2; ++i) {
       tc::mbar_init(&bars->z_full[i], 1);
       tc::mbar_init(&bars->z_empty[i], EPI);
@@ -161,9 +161,8 @@ logreg_tc_kernel(const __grid_constant__ CUtensorMap xmap,
       tc::mbar_init(&bars->r_empty[i], 1);
     }
     tc::mbar_init(&bars->g_done, 1);
-    tc::mbar_init(&bars->drain, 1);
-    tc::mbar_init(&bars->xlo_full, 1);
-    tc::mbar_init(&bars->xlo_empty, 1);
+    tc::mbar_init(&bars->drain[0], 1);
+    tc::mbar_init(&bars->drain[1], 1);
     *abort_flag = 0;
     tc::fence_mbar_init();
     tc::prefetch_tmap(&xmap);
@@ -200,132 +199,120 @@ logreg_tc_kernel(const __grid_constant__ CUtensorMap xmap,
   tc::tc_fence_after();
   const uint32_t tmem = *tmem_slot;
 
+  const uint64_t xk = tc::smem_desc_sw128(tc::smem_u32(Xs), 16, 1024);       // K-major
+  const uint64_t xmn = tc::smem_desc_sw128(tc::smem_u32(Xs), 16384, 1024);   // MN-major
   if (warp == 0) {
-    // ---------------- TMA producer ----------------
-    if (lane == 0) {
-      int it = 0;
-      for (; it < T; ++it) {
-        const int s = it % L::kStages;
-        const uint32_t use = (uint32_t)(it / L::kStages);
-        if (!wait_or_abort(&bars->x_empty[s], (use & 1) ^ 1, abort_flag)) {
-          tc::record_error(err,kTcTimeoutTma);
-          *abort_flag = 1;
-          break;
-        }
-        tc::mbar_arrive_expect_tx(&bars->x_full[s], L::kXStage);
-#pragma unroll
-        for (int kb = 0; kb < KB; ++kb)
-          tc::tma_load_2d(Xs + s * L::kXStage + kb * 16384, &xmap, kb * 64,
-                          (rt_begin + it) * kRows, &bars->x_full[s]);
-        if constexpr (XLO) {
-          // Single X_lo buffer: free once GEMM1 of the previous tile is done.
-          if (!wait_or_abort(&bars->xlo_empty, (uint32_t)(it & 1) ^ 1, abort_flag)) {
-            tc::record_error(err, kTcTimeoutTma);
-            *abort_flag = 1;
-            ++it;
-            break;
-          }
-          tc::mbar_arrive_expect_tx(&bars->xlo_full, L::kXStage);
-#pragma unroll
-          for (int kb = 0; kb < KB; ++kb)
-            tc::tma_load_2d(smem + L::kXlo + kb * 16384, &xlomap, kb * 64,
-                            (rt_begin + it) * kRows, &bars->xlo_full);
-        }
-      }
-      // Drain: every issued load has landed before the CTA can exit.
-      for (int j = (it > L::kStages ? it - L::kStages : 0); j < it; ++j)
-        tc::mbar_wait(&bars->x_full[j % L::kStages], (uint32_t)((j / L::kStages) & 1),
-                      kWaitLimitNs);
-      if constexpr (XLO) {
-        if (it > 0) tc::mbar_wait(&bars->xlo_full, (uint32_t)((it - 1) & 1), kWaitLimitNs);
-      }
-    }
-  } else if (warp == 1) {
-    // ---------------- MMA issuer ----------------
+    // ---------------- X by TMA, and the MMAs of Z ----------------
     if (tc::elect_one()) {
       constexpr uint32_t idesc1 = tc::idesc_bf16_f32(128, CT, false, false);  // K-major A, B
-      constexpr uint32_t idesc2 = tc::idesc_bf16_f32(128, CT, true, true);    // MN-major A, B
-      const uint64_t xk = tc::smem_desc_sw128(tc::smem_u32(Xs), 16, 1024);       // K-major
-      const uint64_t xmn = tc::smem_desc_sw128(tc::smem_u32(Xs), 16384, 1024);   // MN-major
-      const uint64_t xlk = tc::smem_desc_sw128(tc::smem_u32(smem + L::kXlo), 16, 1024);
       const uint64_t bhk = tc::smem_desc_sw128(tc::smem_u32(Bhi), 16, 1024);
       const uint64_t blk = tc::smem_desc_sw128(tc::smem_u32(Blo), 16, 1024);
-      const uint64_t rmn = tc::smem_desc_sw128(tc::smem_u32(Rs), 16384, 1024);
-      const uint32_t tg = tmem + 2 * CT;
-      const int ksteps = (D + 15) >> 4;   // K-steps of 16 features holding data
+      const int ksteps = (D + 15) >> 4;   // K-steps of 16 features holding data (> 8)
+      int loads = 0;                      // tiles whose loads were issued
       bool ok = true;
-      auto gemm1 = [&](int it) -> bool {
-        const int s = it % L::kStages, b = it & 1;
-        if (!wait_or_abort(&bars->x_full[s], (uint32_t)(it / L::kStages) & 1, abort_flag))
-          return false;
-        if (!wait_or_abort(&bars->z_empty[b], ((uint32_t)(it >> 1) & 1) ^ 1, abort_flag))
-          return false;
-        if constexpr (XLO) {
-          if (!wait_or_abort(&bars->xlo_full, (uint32_t)(it & 1), abort_flag)) return false;
+      auto load = [&](int it) -> bool {
+        const int s = it & 1;
+        for (int h = 0; h < 2; ++h) {
+          if (!wait_or_abort(&bars->x_empty[s][h], ((uint32_t)(it >> 1) & 1) ^ 1, abort_flag)) {
+            tc::record_error(err, kTcTimeoutTma);
+            return false;
+          }
+          loads = it + 1;
+          tc::mbar_arrive_expect_tx(&bars->x_full[s][h], L::kXStage / 2);
+#pragma unroll
+          for (int kb = 2 * h; kb < 2 * h + 2; ++kb)
+            tc::tma_load_2d(Xs + s * L::kXStage + kb * 16384, &xmap, kb * 64,
+                            (rt_begin + it) * kRows, &bars->x_full[s][h]);
         }
-        tc::tc_fence_after();
+        return true;
+      };
+      auto gemm1 = [&](int it) -> bool {
+        const int s = it & 1, b = it & 1;
+        const uint32_t use = (uint32_t)(it >> 1) & 1;
+        if (!wait_or_abort(&bars->z_empty[b], use ^ 1, abort_flag)) return false;
         const uint32_t tz = tmem + b * CT;
         const uint64_t xs = tc::desc_at(xk, s * L::kXStage);
+        for (int h = 0; h < 2; ++h) {
+          if (!wait_or_abort(&bars->x_full[s][h], use, abort_flag)) return false;
+          tc::tc_fence_after();
 #pragma unroll
-        for (int kb = 0; kb < KB; ++kb) {
+          for (int kb = 2 * h; kb < 2 * h + 2; ++kb) {
 #pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            if (kb * 4 + k >= ksteps) break;   // all-zero padding features
-            const uint64_t a = tc::desc_at(xs, kb * 16384 + k * 32);
-            const uint64_t bh = tc::desc_at(bhk, kb * (CT * 128) + k * 32);
-            const uint64_t bl = tc::desc_at(blk, kb * (CT * 128) + k * 32);
-            tc::mma_16bit(tz, a, bh, idesc1, (kb | k) ? 1u : 0u);
-            tc::mma_16bit(tz, a, bl, idesc1, 1u);
-            if constexpr (XLO) {
-              tc::mma_16bit(tz, tc::desc_at(xlk, kb * 16384 + k * 32), bh, idesc1, 1u);
+            for (int k = 0; k < 4; ++k) {
+              if (kb * 4 + k >= ksteps) break;   // all-zero padding features
+              const uint64_t a = tc::desc_at(xs, kb * 16384 + k * 32);
+              const uint64_t bh = tc::desc_at(bhk, kb * (CT * 128) + k * 32);
+              const uint64_t bl = tc::desc_at(blk, kb * (CT * 128) + k * 32);
+              tc::mma_16bit(tz, a, bh, idesc1, (kb | k) ? 1u : 0u);
+              tc::mma_16bit(tz, a, bl, idesc1, 1u);
             }
           }
         }
         tc::mma_commit(&bars->z_full[b]);
-        if constexpr (XLO) tc::mma_commit(&bars->xlo_empty);
         return true;
       };
-      if (T > 0) ok = gemm1(0);
+      // A stage is refilled when G of its tile is done, while Z of the next tile
+      // runs.
+      for (int it = 0; it < T && it < 2 && ok; ++it) ok = load(it);
       for (int it = 0; it < T && ok; ++it) {
-        if (it + 1 < T) {
-          ok = gemm1(it + 1);
-          if (!ok) break;
-        }
-        const int s = it % L::kStages, rb = it % L::kRBufs;
-        if (!wait_or_abort(&bars->r_full[rb], (uint32_t)(it / L::kRBufs) & 1, abort_flag)) {
+        ok = gemm1(it);
+        if (ok && it > 0 && it + 1 < T) ok = load(it + 1);
+      }
+      if (!ok) {
+        tc::record_error(err, kTcTimeoutMma);
+        *abort_flag = 1;
+      }
+      tc::mma_commit(&bars->drain[0]);
+      tc::mbar_wait(&bars->drain[0], 0, kWaitLimitNs);
+      // Let the last loads land before the CTA can exit (each wait bounded).
+      for (int j = (loads > 2 ? loads - 2 : 0); j < loads; ++j)
+        for (int h = 0; h < 2; ++h)
+          tc::mbar_wait(&bars->x_full[j & 1][h], (uint32_t)((j >> 1) & 1), kWaitLimitNs);
+    }
+    __syncwarp();
+  } else if (warp == 1) {
+    // ---------------- the MMAs of G ----------------
+    if (tc::elect_one()) {
+      constexpr uint32_t idesc2 = tc::idesc_bf16_f32(128, CT, true, true);    // MN-major A, B
+      const uint64_t rmn = tc::smem_desc_sw128(tc::smem_u32(Rs), 16384, 1024);
+      const uint32_t tg = tmem + 2 * CT;
+      bool ok = true;
+      for (int it = 0; it < T; ++it) {
+        const int rb = it & 1;
+        if (!wait_or_abort(&bars->r_full[rb], (uint32_t)(it >> 1) & 1, abort_flag)) {
           ok = false;
           break;
         }
         tc::tc_fence_after();
-        const uint64_t xs = tc::desc_at(xmn, s * L::kXStage);
+        const uint64_t xs = tc::desc_at(xmn, (it & 1) * L::kXStage);
         const uint64_t rs = tc::desc_at(rmn, rb * L::kRBuf);
 #pragma unroll
-        for (int mt = 0; mt < L::kMTiles; ++mt) {
+        for (int mt = 0; mt < KB / 2; ++mt) {
 #pragma unroll
           for (int ks = 0; ks < kRows / 16; ++ks) {
             const uint64_t a = tc::desc_at(xs, mt * 32768 + ks * 2048);
-            const uint64_t bd = tc::desc_at(rs, ks * 2048);
-            tc::mma_16bit(tg + mt * CT, a, bd, idesc2, (it > 0 || ks > 0) ? 1u : 0u);
+            tc::mma_16bit(tg + mt * CT, a, tc::desc_at(rs, ks * 2048), idesc2,
+                          (it > 0 || ks > 0) ? 1u : 0u);
           }
+          tc::mma_commit(&bars->x_empty[it & 1][mt]);
         }
-        tc::mma_commit(&bars->x_empty[s]);
         tc::mma_commit(&bars->r_empty[rb]);
       }
       if (ok) {
         tc::mma_commit(&bars->g_done);
       } else {
-        tc::record_error(err,kTcTimeoutMma);
+        tc::record_error(err, kTcTimeoutMma);
         *abort_flag = 1;
       }
       // Drain: all MMAs issued by this thread have completed.
-      tc::mma_commit(&bars->drain);
-      tc::mbar_wait(&bars->drain, 0, kWaitLimitNs);
+      tc::mma_commit(&bars->drain[1]);
+      tc::mbar_wait(&bars->drain[1], 0, kWaitLimitNs);
     }
     __syncwarp();   // the whole warp frees the TMEM below
   } else {
     // ---------------- epilogue (EPI warps) ----------------
     const int quarter = warp & 3;                 // TMEM lanes 32*quarter ..
-    const int half = (warp - 2) >> 2;             // chains [half*kCW, +kCW)
+    const int part = (warp - 2) >> 2;             // chains [part*kCW, +kCW)
     const uint32_t lane_base = (uint32_t)(quarter * 32) << 16;
     const int r = quarter * 32 + lane;            // row of the tile this thread owns
     // Per chain: softplus(z) = max(z, 0) + ln(1 + e^-|z|) and max(z, 0) =
@@ -345,60 +332,52 @@ logreg_tc_kernel(const __grid_constant__ CUtensorMap xmap,
       if (T > 0 && row0 < N) y_next = y[row0];
     }
     for (int it = 0; it < T; ++it) {
-      const int b = it & 1, rb = it % L::kRBufs;
-      if (!wait_or_abort(&bars->z_full[b], (uint32_t)(it >> 1) & 1, abort_flag)) {
+      const int b = it & 1, rb = it & 1;
+      if (!warp_wait(&bars->z_full[b], (uint32_t)(it >> 1) & 1, abort_flag)) {
         ok = false;
         break;
       }
       tc::tc_fence_after();
+      float h[kCW];
+      tc::tmem_ld16(tmem + b * CT + part * kCW + lane_base, h);
       const int row = (rt_begin + it) * kRows + r;
       const bool valid = row < N;
       const float ym = (valid ? y_next : 0.f) - 0.5f;
       if (it + 1 < T && row + kRows < N) y_next = y[row + kRows];
-      const uint32_t tz = tmem + b * CT + half * kCW;
       unsigned char* Rb = Rs + rb * L::kRBuf;
-      float h[kCW];
-#pragma unroll
-      for (int q = 0; q < kCW / 32; ++q) tc::tmem_ld32(tz + lane_base + q * 32, h + q * 32);
       tc::tmem_ld_wait();
-      bool r_free = false;
+      tc::tc_fence_before();
+      __syncwarp();
+      if (lane == 0) tc::mbar_arrive(&bars->z_empty[b]);
+      // R first: the MMAs wait for it; the likelihood terms wait for nobody.
+      uint32_t rp[kCW / 2];
 #pragma unroll
-      for (int g8 = 0; g8 < kCW / 8; ++g8) {
-        uint32_t rp[4] = {0u, 0u, 0u, 0u};                   // rows past N: R = 0
-        if (valid) {
-#pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            const float a = fabsf(h[g8 * 8 + j]);
-            const float t = tc::ex2_approx(a * kNeg2Log2e);     // e^-|z|
-            sacc[g8 * 8 + j] += fmaf(kLn2, tc::lg2_approx(1.f + t), a);
-          }
-#pragma unroll
-          for (int j = 0; j < 4; ++j)
-            rp[j] = residual_bf16x2(h[g8 * 8 + 2 * j], h[g8 * 8 + 2 * j + 1], ym);
-        }
-        if (g8 == 0) {
-          // GEMM2 of the tile that last used this R buffer must be done.
-          r_free = wait_or_abort(&bars->r_empty[rb], ((uint32_t)(it / L::kRBufs) & 1) ^ 1,
-                                 abort_flag);
-          if (!r_free) break;
-        }
-        const int c = half * kCW + g8 * 8;
-        *reinterpret_cast<uint4*>(Rb + (c >> 6) * 16384 + tc::sw128_offset(r, c & 63)) =
-            make_uint4(rp[0], rp[1], rp[2], rp[3]);
-      }
-      if (!r_free) {
+      for (int j = 0; j < kCW / 2; ++j)                      // rows past N: R = 0
+        rp[j] = valid ? residual_bf16x2(h[2 * j], h[2 * j + 1], ym) : 0u;
+      // GEMM2 of the tile that last used this R buffer must be done.
+      if (!warp_wait(&bars->r_empty[rb], ((uint32_t)(it >> 1) & 1) ^ 1, abort_flag)) {
         ok = false;
         break;
       }
-      tc::tc_fence_before();
+#pragma unroll
+      for (int g8 = 0; g8 < kCW / 8; ++g8) {
+        const int c = part * kCW + g8 * 8;
+        *reinterpret_cast<uint4*>(Rb + (c >> 6) * 16384 + tc::sw128_offset(r, c & 63)) =
+            make_uint4(rp[4 * g8], rp[4 * g8 + 1], rp[4 * g8 + 2], rp[4 * g8 + 3]);
+      }
       tc::fence_proxy_async_smem();
       __syncwarp();
-      if (lane == 0) {
-        tc::mbar_arrive(&bars->z_empty[b]);
-        tc::mbar_arrive(&bars->r_full[rb]);
+      if (lane == 0) tc::mbar_arrive(&bars->r_full[rb]);
+      if (valid) {
+#pragma unroll
+        for (int j = 0; j < kCW; ++j) {
+          const float a = fabsf(h[j]);
+          const float t = tc::ex2_approx(a * kNeg2Log2e);     // e^-|z|
+          sacc[j] += fmaf(kLn2, tc::lg2_approx(1.f + t), a);
+        }
       }
     }
-    if (ok && T > 0) ok = wait_or_abort(&bars->g_done, 0, abort_flag);
+    if (ok && T > 0) ok = warp_wait(&bars->g_done, 0, abort_flag);
     if (!ok) {
       tc::record_error(err,kTcTimeoutEpilogue);
       *abort_flag = 1;
@@ -406,17 +385,17 @@ logreg_tc_kernel(const __grid_constant__ CUtensorMap xmap,
       tc::tc_fence_after();
       // Gradient partials: TMEM lane = feature, column = chain.
 #pragma unroll
-      for (int mt = 0; mt < L::kMTiles; ++mt) {
+      for (int mt = 0; mt < KB / 2; ++mt) {
         const int d = mt * 128 + quarter * 32 + lane;
 #pragma unroll
         for (int ch = 0; ch < kCW / 16; ++ch) {
           float g[16];
-          tc::tmem_ld16(tmem + 2 * CT + mt * CT + half * kCW + lane_base + ch * 16, g);
+          tc::tmem_ld16(tmem + 2 * CT + mt * CT + part * kCW + lane_base + ch * 16, g);
           tc::tmem_ld_wait();
           if (d < D) {
 #pragma unroll
             for (int j = 0; j < 16; ++j) {
-              const int c = c0 + half * kCW + ch * 16 + j;
+              const int c = c0 + part * kCW + ch * 16 + j;
               if (c < n) gpart[((size_t)split * n + c) * D + d] = g[j];
             }
           }
@@ -430,7 +409,7 @@ logreg_tc_kernel(const __grid_constant__ CUtensorMap xmap,
         float v = -sacc[c];
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-        if (lane == 0) red[quarter * CT + half * kCW + c] = (double)v;
+        if (lane == 0) red[quarter * CT + part * kCW + c] = (double)v;
       }
     }
     named_barrier(1, 32 * EPI);
@@ -1442,9 +1421,8 @@ class LogregTc final : public Target {
       GBM_CUDA(cudaFuncSetAttribute(logreg_tct_kernel<false>, (cudaFuncAttribute)attr,
                                     (int)smem_));
     } else if (kb_ == 4) {
-      smem_ = TcLayout<4, 64, false>::kBytes + 1024;
-      GBM_CUDA(cudaFuncSetAttribute(logreg_tc_kernel<4, 64, 8, false>, (cudaFuncAttribute)attr,
-                                    (int)smem_));
+      smem_ = TcLayout::kBytes + 1024;
+      GBM_CUDA(cudaFuncSetAttribute(logreg_tc_kernel, (cudaFuncAttribute)attr, (int)smem_));
     }
   }
 
@@ -1466,22 +1444,19 @@ class LogregTc final : public Target {
       const float* qc = q + (size_t)base * ldq;
       // Work items of this launch (CTAs, or CTA pairs for the pair kernel).
       const int g = work_grid(grid_, std::min(lim, cap - base), ct_, N_, kMinSplitRows);
-#define GBM_TC_LAUNCH(KB_, CT_, EPI_, XLO_)                                               \
-  logreg_tc_kernel<KB_, CT_, EPI_, XLO_><<<g, tc_threads(EPI_), smem_, s>>>(              \
-      xmap_, xlomap_, y_.as<float>(), N, D, qc, ldq, n_dev, base, lim, g, lpart, gpart,     \
-      err_dev_)
 #define GBM_TCT_LAUNCH(XLO_)                                                              \
   logreg_tct_kernel<XLO_><<<g, tc_threads(kTctEpi), smem_, s>>>(                           \
       xmap_, xlomap_, ym_.as<float>(), N, D, qc, ldq, n_dev, base, lim, g, lpart, gpart,     \
       err_dev_)
       if (kb_ == 2 && xlo_) GBM_TCT_LAUNCH(true);
       else if (kb_ == 2) GBM_TCT_LAUNCH(false);
-      else if (kb_ == 4) GBM_TC_LAUNCH(4, 64, 8, false);
+      else if (kb_ == 4)
+        logreg_tc_kernel<<<g, tc_threads(kRowEpi), smem_, s>>>(
+            xmap_, y_.as<float>(), N, D, qc, ldq, n_dev, base, lim, g, lpart, gpart, err_dev_);
       else
         logreg_tc_pair_kernel<<<2 * g, tc_threads(kPairEpi), smem_, s>>>(
             xmap_, y_.as<float>(), N, D, qc, ldq, n_dev, base, lim, g, lpart, gpart,
             err_dev_);
-#undef GBM_TC_LAUNCH
 #undef GBM_TCT_LAUNCH
       GBM_CUDA(cudaGetLastError());
       launch_split_reduce(lpart, gpart, qc, ldq, n_dev, base, lim, std::min(lim, cap - base),

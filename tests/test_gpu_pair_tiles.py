@@ -1,5 +1,6 @@
-"""The mixed-precision kernel of 257 to 512 features (a pair of CTAs shares a tile
-of 64 chains: csrc/logreg_tc.cu) at the edges of its rows, features and chains.
+"""The mixed-precision kernels of 129 to 256 and of 257 to 512 features (there a
+pair of CTAs shares a tile of 64 chains: csrc/logreg_tc.cu) at the edges of their
+rows, features and chains.
 
 A chain's result does not depend on its place in the tile: with the chains in
 another order (other halves, other warps, the other CTA) the outputs are the same
@@ -24,6 +25,8 @@ def pg():
 
 
 @pytest.mark.parametrize('n,d,c', [
+    (1, 129, 1), (127, 130, 15), (128, 143, 16), (129, 144, 17), (256, 192, 33), (257, 193, 48),
+    (385, 255, 64), (9729, 256, 65), (19457, 200, 129), (40000, 160, 700),
     (1, 257, 1), (127, 258, 7), (128, 272, 8), (129, 273, 31), (255, 383, 32), (256, 384, 33),
     (257, 385, 40), (1000, 400, 56), (9728, 511, 63), (9729, 512, 64), (19457, 300, 65),
     (4000, 448, 129), (3000, 512, 700)])

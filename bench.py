@@ -521,10 +521,10 @@ def run_hmc(args, w):
   sm_max = (clk or {}).get('sm_max_mhz') or peaks.get('sm_max_mhz', 2070.0)
   peak, sms = fp32_peak_tflops(sm_max)
   achieved = flops / t_eval / 1e12
+  name = kernel_name(precision, X.shape[0], D)
   roofline = {'bound': 'fp32', 'achieved': achieved, 'peak': peak, 'unit': 'TFLOP/s',
-              'frac': achieved / peak, 'traffic': read_traffic(args.workload,
-                                                               kernel_name(precision, D)),
-              'kernel': kernel_name(precision, D),
+              'frac': achieved / peak, 'traffic': read_traffic(args.workload, name),
+              'kernel': name,
               'peak_source': 'nominal FP32 FMA rate: %d SMs x 128 lanes x 2 flop x %.0f MHz'
                              % (sms, sm_max),
               'eval_us': 1e6 * t_eval,
@@ -549,9 +549,10 @@ def run_hmc(args, w):
       'min_ess_note': 'min over dimensions of cross-chain ESS (diagnostic.py:203-337) of 500 '
                       'further draws, per draw, times the timed draws per second',
       'accept_rate': acc, 'e2e': e2e, 'roofline': roofline, 'cpu_baseline': cpu,
-      # per transition: momentum + half kick, L x (gradient kernel + split
-      # reduction), L - 1 kick-drift, MH finish, next step key
-      'gpu_launches': args.steps * (3 * w['leapfrogs'] + 2),
+      # per transition: next step key, momentum + half kick, MH finish, and the
+      # trajectory: one launch (FP32: X fits a cluster), or L x (gradient kernel +
+      # split reduction) and L - 1 kick-drifts
+      'gpu_launches': args.steps * (4 if precision == 'fp32' else 3 * w['leapfrogs'] + 2),
       'clocks': clk}), flush=True)
 
 
@@ -723,9 +724,10 @@ class Leg:
     return int(z[2].value)
 
 
-def kernel_name(precision, d):
+def kernel_name(precision, n, d):
   if precision == 'fp32':
-    return 'logreg_f32_kernel' if d <= 128 else 'logreg_partial_kernel'
+    return ('wide_products_kernel' if d > 128 else
+            'logreg_f32_tc_kernel' if n >= 4096 else 'logreg_f32_kernel')
   return ('logreg_tc_pair_kernel' if d > 256 else 'logreg_tc_kernel' if d > 128 else
           'logreg_tct_kernel')
 
@@ -737,7 +739,7 @@ def leg_roofline(leg, prof, workload, d, sm_max_mhz, measured_over):
   flops_per_grad, _ = leg.target.cost(1)
   eval_s = prof['eval_ms'] / 1000.0
   achieved = flops_per_grad * prof['lf'] / eval_s / 1e12 if eval_s > 0 else None
-  name = kernel_name(leg.target.precision, d)
+  name = kernel_name(leg.target.precision, leg.target.num_rows, d)
   if leg.target.precision == 'fp32':
     peak, sms = fp32_peak_tflops(sm_max_mhz)
     bound, src = 'fp32', ('nominal FP32 FMA rate: %d SMs x 128 lanes x 2 flop x %.0f MHz '

@@ -74,8 +74,10 @@ class LogisticRegression(Target):
   (spinoffs/inference_gym/inference_gym/targets/logistic_regression.py:88-103)
   with the intercept placed wherever the caller put it.
 
-  precision: 'fp32' (CUDA-core FP32, the plain form) or 'mixed' (BF16 tensor
-  cores with FP32 accumulation and hi/lo split residual correction).
+  precision: 'fp32' (the plain form: FP32 on the CUDA cores, the gradient's
+  products from FP16 pairs on the tensor cores where they lose nothing by it) or
+  'mixed' (BF16 tensor cores with FP32 accumulation and hi/lo split residual
+  correction).
   """
 
   def __init__(self, features, labels, prior_scale=1.0, precision='fp32'):

@@ -656,6 +656,7 @@ logreg_tct_kernel(const __grid_constant__ CUtensorMap xmap,
         tc::mbar_wait(&bars->x_full[j % L::kStages], (uint32_t)((j / L::kStages) & 1),
                       kWaitLimitNs);
     }
+    __syncwarp();
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
     if (tc::elect_one()) {

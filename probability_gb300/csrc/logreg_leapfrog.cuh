@@ -37,9 +37,10 @@ constexpr int kLeapMaxCluster = 8;
 // chains 25 us a step, three launches a step 34.  From there on those, which fill
 // the GPU, catch up.
 constexpr int kLeapWaves = 4;
-constexpr size_t kLeapSmem = 227 * 1024;
+constexpr int64_t kLeapSmem = 227 * 1024;
 
-// What a launch holds in shared memory, in floats.
+// What a launch holds in shared memory, in floats (64 bits: leap_shape asks for any
+// number of rows).
 struct LeapShape {
   int K, G;            // CTAs of a cluster, chains of a cluster
   int S, row_tiles;    // row splits of the whole, row tiles of the whole
@@ -47,16 +48,16 @@ struct LeapShape {
                        // neighbouring features without conflicts)
   int smax;            // most splits of a CTA
   int D;
-  __host__ __device__ int x() const { return 0; }
-  __host__ __device__ int y() const { return D * rowpad; }
-  __host__ __device__ int r() const { return y() + rowpad; }
-  __host__ __device__ int like() const { return r() + G * rowpad; }
-  __host__ __device__ int part() const { return like() + G * rowpad / 4; }
-  __host__ __device__ int q() const { return part() + 2 * smax * G * D; }
-  __host__ __device__ int p() const { return q() + G * D; }
-  __host__ __device__ int sums() const { return (p() + G * D + 1) / 2 * 2; }
-  __host__ __device__ size_t bytes() const {
-    return 4 * (size_t)(sums() + 2 * G * (1 + kLeapThreads / 32));
+  __host__ __device__ int64_t x() const { return 0; }
+  __host__ __device__ int64_t y() const { return (int64_t)D * rowpad; }
+  __host__ __device__ int64_t r() const { return y() + rowpad; }
+  __host__ __device__ int64_t like() const { return r() + (int64_t)G * rowpad; }
+  __host__ __device__ int64_t part() const { return like() + (int64_t)G * (rowpad / 4); }
+  __host__ __device__ int64_t q() const { return part() + (int64_t)2 * smax * G * D; }
+  __host__ __device__ int64_t p() const { return q() + (int64_t)G * D; }
+  __host__ __device__ int64_t sums() const { return (p() + (int64_t)G * D + 1) / 2 * 2; }
+  __host__ __device__ int64_t bytes() const {
+    return 4 * (sums() + 2 * G * (1 + kLeapThreads / 32));
   }
 };
 
@@ -316,7 +317,7 @@ void launch_leapfrogs(const LeapShape& h, const float* X2, const float* ym, int 
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)((C + G - 1) / G * h.K));
   cfg.blockDim = dim3(kLeapThreads);
-  cfg.dynamicSmemBytes = h.bytes();
+  cfg.dynamicSmemBytes = (size_t)h.bytes();
   cfg.stream = s;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;

@@ -1,7 +1,10 @@
 // X as FP16 hi + lo of scaled features, for gradient products on the tensor
 // cores: X' = X 2^(kF16Top - exponent of the column's largest), and residuals
-// as hi + lo of R' = kF16Scale R, so that a product of FP16 pairs carries a float
-// to 2^-24 of itself and gscale turns it back.
+// as hi + lo of R' = kF16Scale R; gscale turns a product of the two back.  hi + lo
+// carries a float to 2^-23 of itself, and not below 2^-25 (half of FP16's smallest
+// step): an entry 2^16 below its column's largest loses bits, one 2^39 below is gone.
+// prepare() measures what the entries lose and holds only columns that lose nothing
+// to speak of.
 #pragma once
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
@@ -34,52 +37,70 @@ __global__ void column_max_kernel(const float* __restrict__ X, int64_t N, int D,
   }
 }
 
+// What hi + lo leaves of a column's nonzero entries, each relative to the entry:
+// the largest, the sum of the others, and their number.
+struct ColumnLoss {
+  float rest, most;
+  unsigned entries;
+  __device__ __forceinline__ void add(float loss) {
+    rest += fminf(loss, most);
+    most = fmaxf(loss, most);
+  }
+};
+
 // X [N][D] -> X' = X 2^(kF16Top - exponent of the column's largest) as FP16 hi
-// + lo [N][Dp], zero-padded; rows [b chunk, (b + 1) chunk) also sum X'^2 and
-// the square of what hi + lo leaves of it into part[b][d].
+// + lo [N][Dp], zero-padded, and what rows [b chunk, (b + 1) chunk) lose by it in
+// part[b][d].
 __global__ void f16_pack_kernel(const float* __restrict__ X, int64_t N, int D, int Dp,
                                 int64_t chunk, const unsigned* __restrict__ max_bits,
                                 __half* __restrict__ hi, __half* __restrict__ lo,
-                                float2* __restrict__ part) {
+                                ColumnLoss* __restrict__ part) {
   const int64_t r0 = (int64_t)blockIdx.x * chunk, r1 = r0 + chunk < N ? r0 + chunk : N;
   for (int d = threadIdx.x; d < Dp; d += blockDim.x) {
     const int shift = d < D ? kF16Top - float_exponent(max_bits[d]) : 0;
-    float2 acc = make_float2(0.f, 0.f);
+    ColumnLoss loss{0.f, 0.f, 0u};
 #pragma unroll 4
     for (int64_t r = r0; r < r1; ++r) {
-      const float v = d < D ? ldexpf(X[r * D + d], shift) : 0.f;
+      const float x = d < D ? X[r * D + d] : 0.f;
+      const float v = ldexpf(x, shift);
       const __half h = __float2half_rn(v);
       const float rest = v - __half2float(h);
       const __half l = __float2half_rn(rest);
       hi[r * Dp + d] = h;
       lo[r * Dp + d] = l;
-      const float left = rest - __half2float(l);
-      acc.x = fmaf(v, v, acc.x);
-      acc.y = fmaf(left, left, acc.y);
+      const float left = fabsf(rest - __half2float(l));
+      // An entry that the scaling itself took to zero is lost whole.
+      if (x != 0.f) {
+        ++loss.entries;
+        loss.add(v != 0.f ? __fdividef(left, fabsf(v)) : 1.f);
+      }
     }
-    if (d < D) part[(size_t)blockIdx.x * D + d] = acc;
+    if (d < D) part[(size_t)blockIdx.x * D + d] = loss;
   }
 }
 
-// Sums of part over blocks: one block per feature, fixed order.
+// Losses of the columns from those of the blocks: one block per feature, fixed order.
 __global__ void __launch_bounds__(128)
-column_rest_kernel(const float2* __restrict__ part, int nb, int D, double2* __restrict__ out) {
-  __shared__ double2 sh[128];
+column_loss_kernel(const ColumnLoss* __restrict__ part, int nb, int D,
+                   ColumnLoss* __restrict__ out) {
+  __shared__ ColumnLoss sh[128];
   const int d = blockIdx.x, tid = threadIdx.x;
-  double2 acc = make_double2(0.0, 0.0);
-  for (int b = tid; b < nb; b += 128) {
-    acc.x += (double)part[(size_t)b * D + d].x;
-    acc.y += (double)part[(size_t)b * D + d].y;
-  }
-  sh[tid] = acc;
+  ColumnLoss sum{0.f, 0.f, 0u};
+  auto merge = [&](const ColumnLoss& c) {
+    sum.rest += c.rest;
+    sum.add(c.most);
+    sum.entries += c.entries;
+  };
+  for (int b = tid; b < nb; b += 128) merge(part[(size_t)b * D + d]);
+  sh[tid] = sum;
   for (int o = 64; o > 0; o >>= 1) {
     __syncthreads();
     if (tid < o) {
-      sh[tid].x += sh[tid + o].x;
-      sh[tid].y += sh[tid + o].y;
+      merge(sh[tid + o]);
+      sh[tid] = sum;
     }
   }
-  if (tid == 0) out[d] = sh[0];
+  if (tid == 0) out[d] = sum;
 }
 
 struct F16Rows {
@@ -89,24 +110,36 @@ struct F16Rows {
 
   // False if X (or the labels, ym = y - 1/2) does not fit the form: infinities,
   // NaN, exponents that the scaling cannot carry, or a range so wide that hi + lo
-  // leaves more than 2^-23 of a column in root mean square (a normal sample:
-  // 2^-25); a label so far outside [0, 1] that a residual, below |y - 1/2| + 1/2,
-  // could leave FP16's range (R' < 2^16); more than kMost elements (the form is as
-  // large as X in float32: beyond 16 GB the memory is the caller's).
+  // leaves more than kMostLoss of a column's nonzero entries on average, each relative
+  // to the entry; a label so far outside [0, 1] that a residual, below
+  // |y - 1/2| + 1/2, could leave FP16's range (R' < 2^16); more than kMost elements (the
+  // form is as large as X in float32: beyond 16 GB the memory is the caller's).
+  //
+  // The average is over entries and not over their squares because which rows count
+  // is the residuals' to say: where a fit has a large entry's row right, its residual
+  // is zero and the column's gradient is that of the small ones.  2^-23 is what one
+  // entry may lose with all of FP16's range above it, so a column without wide range
+  // always fits (a normal sample: 2^-25.5 at any length); one entry at 3000 times the
+  // others' scale fits, at 10^5 times not, exp(2 normal) fits and exp(3 normal) not.
+  // One entry (of 16 or more) may lose any amount: in a sample whose density does not
+  // vanish at zero the entry nearest to it, 2^-20 of the others, would otherwise
+  // turn one target of 150 away.
   bool prepare(gbm_context* ctx, const float* X, const float* ym, int64_t N, int D, int dp,
                int box_rows) {
     constexpr int64_t kMost = (int64_t)1 << 32;
+    constexpr double kMostLoss = 1.0 / (1 << 23);
+    constexpr unsigned kExempt = 16;
     if (N * dp > kMost) return false;
     cudaStream_t s = ctx->stream;
     const int nb = 8 * ctx->num_sms;
     const int64_t chunk = (N + nb - 1) / nb;
     const size_t off_part = (sizeof(unsigned) * (D + 1) + 255) / 256 * 256;
-    const size_t off_sum = off_part + (sizeof(float2) * (size_t)nb * D + 255) / 256 * 256;
+    const size_t off_sum = off_part + (sizeof(ColumnLoss) * (size_t)nb * D + 255) / 256 * 256;
     DeviceBuffer buf;
-    buf.reserve(off_sum + sizeof(double2) * D);
+    buf.reserve(off_sum + sizeof(ColumnLoss) * D);
     unsigned* mx = buf.as<unsigned>();
-    float2* part = reinterpret_cast<float2*>(buf.as<char>() + off_part);
-    double2* sum = reinterpret_cast<double2*>(buf.as<char>() + off_sum);
+    ColumnLoss* part = reinterpret_cast<ColumnLoss*>(buf.as<char>() + off_part);
+    ColumnLoss* loss = reinterpret_cast<ColumnLoss*>(buf.as<char>() + off_sum);
     const size_t bytes = sizeof(__half) * (size_t)N * dp;
     mem.reserve(2 * bytes + sizeof(float) * D);
     __half* h = mem.as<__half>();
@@ -116,13 +149,14 @@ struct F16Rows {
     column_max_kernel<<<nb, 128, 0, s>>>(X, N, D, chunk, mx);
     column_max_kernel<<<nb, 32, 0, s>>>(ym, N, 1, chunk, mx + D);
     f16_pack_kernel<<<nb, 128, 0, s>>>(X, N, D, dp, chunk, mx, h, l, part);
-    column_rest_kernel<<<(unsigned)D, 128, 0, s>>>(part, nb, D, sum);
+    column_loss_kernel<<<(unsigned)D, 128, 0, s>>>(part, nb, D, loss);
     GBM_CUDA(cudaGetLastError());
     std::vector<unsigned> hmax(D + 1);
-    std::vector<double2> hsum(D);
+    std::vector<ColumnLoss> hloss(D);
     GBM_CUDA(cudaMemcpyAsync(hmax.data(), mx, sizeof(unsigned) * (D + 1), cudaMemcpyDeviceToHost,
                              s));
-    GBM_CUDA(cudaMemcpyAsync(hsum.data(), sum, sizeof(double2) * D, cudaMemcpyDeviceToHost, s));
+    GBM_CUDA(cudaMemcpyAsync(hloss.data(), loss, sizeof(ColumnLoss) * D, cudaMemcpyDeviceToHost,
+                             s));
     GBM_CUDA(cudaStreamSynchronize(s));
     std::vector<float> gs(D, 0.f);
     constexpr unsigned kLabelTop = 0x3fa00000u;   // 1.25f
@@ -130,7 +164,9 @@ struct F16Rows {
     for (int i = 0; i < D; ++i) {
       if (hmax[i] == 0) continue;
       const int fexp = (int)((hmax[i] >> 23) & 255u) - 127;
-      fits = fits && fexp >= -60 && fexp <= 60 && hsum[i].y <= std::ldexp(hsum[i].x, -46);
+      const ColumnLoss& c = hloss[i];
+      const double lost = (double)c.rest + (c.entries >= kExempt ? 0.0 : (double)c.most);
+      fits = fits && fexp >= -60 && fexp <= 60 && lost <= kMostLoss * (double)c.entries;
       gs[i] = std::ldexp(1.f, fexp - kF16Top - 15);
     }
     if (!fits) {

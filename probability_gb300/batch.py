@@ -128,23 +128,17 @@ class TargetBatch(targets.Target):
     v = torch.as_tensor(per_member_values, dtype=dtype).to(dev)
     return torch.repeat_interleave(v, torch.as_tensor(self.member_chains, device=dev))
 
-  def _enter(self):
-    self.stream.wait_stream(torch.cuda.current_stream(self.stream.device))
-
-  def _leave(self):
-    torch.cuda.current_stream(self.stream.device).wait_stream(self.stream)
-
   def log_prob_and_grad(self, state):
     q = _util.as_tensor(state, torch.float32).reshape(-1)
     if q.numel() != self.elements:
       raise ValueError('state must hold %d elements (the ragged layout)' % self.elements)
     logp = torch.empty(self.chains, dtype=torch.float64, device=q.device)
     grad = torch.empty_like(q)
-    self._enter()
+    caller = self._enter()
     _native.check(_native.lib().gbm_target_log_prob_and_grad(
         self._handle, _native.ptr(q), self.chains, _native.ptr(logp), _native.ptr(grad)),
         'gbm_target_log_prob_and_grad')
-    self._leave()
+    self._leave(caller)
     return logp, grad
 
 
@@ -229,12 +223,12 @@ class BatchedNoUTurnSampler:
     lf = torch.empty(C, dtype=torch.int32, device=dev)
     acc, rmd, div = flag(), flag(), flag()
     Pt = _native.ptr
-    b._enter()
+    caller = b._enter()
     _native.check(_native.lib().gbm_nuts_one_step(
         self._handle, C, Pt(q), Pt(pkr.target_log_prob), Pt(pkr.grads_target_log_prob), Pt(eps),
         1, _native.seed_words(seed), Pt(nq), Pt(nl), Pt(ng), Pt(lar), Pt(lf), Pt(acc), Pt(rmd),
         Pt(div), Pt(energy), None), 'gbm_nuts_one_step')
-    b._leave()
+    b._leave(caller)
     return nq, NUTSKernelResults(
         target_log_prob=nl, grads_target_log_prob=ng, step_size=eps, log_accept_ratio=lar,
         leapfrogs_taken=lf, is_accepted=acc, reach_max_depth=rmd,
@@ -252,13 +246,8 @@ class BatchedNoUTurnSampler:
     b = self.batch
     q = _util.as_tensor(current_state, torch.float32).reshape(-1).contiguous()
     eps = self._eps(kernel_results.step_size).contiguous()
-    b._enter()
-    try:
-      run = run_free(self._handle, q, kernel_results, eps, 1, _util.sanitize_seed(seed),
-                     first_step, transitions_per_chain, max_leaf_iterations, (q.numel(),))
-    finally:
-      b._leave()
-    return run
+    return run_free(b, self._handle, q, kernel_results, eps, 1, _util.sanitize_seed(seed),
+                    first_step, transitions_per_chain, max_leaf_iterations, (q.numel(),))
 
 
 class MemberMassMatrixAdaptation:

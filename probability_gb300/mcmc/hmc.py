@@ -90,6 +90,7 @@ def _hmc_transition(engine, state, target_log_prob, grads, step_size, num_leapfr
           P(out['proposed_grads']), P(out['initial_momentum']), P(out['final_momentum']),
           P(out['corr']), P(out['lar']), P(out['is_accepted']))
   out['accepted'] = None
+  caller = engine.target._enter()
   if previous is not None and not is_list:
     prev = (previous.log_acceptance_correction, previous.initial_momentum,
             previous.final_momentum)
@@ -102,6 +103,7 @@ def _hmc_transition(engine, state, target_log_prob, grads, step_size, num_leapfr
           *args, *[P(t) for t in prev], *[P(t) for t in chosen]), 'gbm_hmc_one_step_accepted')
   if out['accepted'] is None:
     _native.check(_native.lib().gbm_hmc_one_step(*args), 'gbm_hmc_one_step')
+  engine.target._leave(caller)
   unflat = lambda t: _util.unflatten_state(t, layout, is_list)
   return out, unflat, is_list
 
@@ -154,7 +156,9 @@ class UncalibratedHamiltonianMonteCarlo(kernel_base.TransitionKernel):
 
   def bootstrap_results(self, init_state):
     q, layout, is_list = _util.flatten_state(init_state)
+    caller = self._target._enter()
     logp, grad = self._target.log_prob_and_grad(q)
+    self._target._leave(caller)
     unflat = lambda t: _util.unflatten_state(t, layout, is_list)
     zeros = torch.zeros_like(q)
     r = UncalibratedHamiltonianMonteCarloKernelResults(

@@ -73,9 +73,9 @@ FreeRun = collections.namedtuple(
     'FreeRun', ['all_states', 'trace', 'transitions_done', 'leaf_iterations'])
 
 
-def run_free(handle, q, kr, step_size, per_chain, seed, first_step, transitions_per_chain,
+def run_free(target, handle, q, kr, step_size, per_chain, seed, first_step, transitions_per_chain,
              max_leaf_iterations, state_shape):
-  """gbm_nuts_run_free for a sampler handle: q [elements] float32 on the
+  """gbm_nuts_run_free for a sampler handle of `target`: q [elements] float32 on the
   device, kr the results carrying target_log_prob / grads_target_log_prob.
   Returns FreeRun(all_states [K, *state_shape], trace of [K, C] tensors,
   transitions_done [C], leaf_iterations)."""
@@ -94,11 +94,15 @@ def run_free(handle, q, kr, step_size, per_chain, seed, first_step, transitions_
   g0 = _util.as_tensor(kr.grads_target_log_prob, torch.float32, dev).reshape(-1).contiguous()
   iters = ctypes.c_int64()
   P = _native.ptr
-  _native.check(_native.lib().gbm_nuts_run_free(
-      handle, C, P(q), P(l0), P(g0), P(step_size), per_chain, _native.seed_words(seed),
-      int(first_step), K, int(max_leaf_iterations), P(done), P(states),
-      P(tr['target_log_prob']), P(tr['log_accept_ratio']), P(tr['leapfrogs_taken']),
-      P(tr['is_accepted']), P(tr['has_divergence']), ctypes.byref(iters)), 'gbm_nuts_run_free')
+  caller = target._enter()
+  try:
+    _native.check(_native.lib().gbm_nuts_run_free(
+        handle, C, P(q), P(l0), P(g0), P(step_size), per_chain, _native.seed_words(seed),
+        int(first_step), K, int(max_leaf_iterations), P(done), P(states),
+        P(tr['target_log_prob']), P(tr['log_accept_ratio']), P(tr['leapfrogs_taken']),
+        P(tr['is_accepted']), P(tr['has_divergence']), ctypes.byref(iters)), 'gbm_nuts_run_free')
+  finally:
+    target._leave(caller)
   return FreeRun(states.reshape((K,) + tuple(state_shape)), tr, done, int(iters.value))
 
 
@@ -182,15 +186,12 @@ class NoUTurnSampler(kernel_base.TransitionKernel):
     lf = torch.empty(C, dtype=torch.int32, device=dev)
     acc, rmd, div = flag(), flag(), flag()
     P = _native.ptr
+    caller = self._target._enter()
     _native.check(_native.lib().gbm_nuts_one_step(
         self._handle, C, P(q), P(l0), P(g0), P(eps), per_chain, _native.seed_words(seed),
         P(nq), P(nl), P(ng), P(lar), P(lf), P(acc), P(rmd), P(div), P(energy), None),
         'gbm_nuts_one_step')
-    # The transition may still be running: a caller on another stream than the
-    # target's gets its buffers back only when it has ended.
-    ctx = self._target._ctx
-    if ctx.stream != torch.cuda.current_stream(dev):
-      ctx.synchronize()
+    self._target._leave(caller)
     unflat = lambda t: _util.unflatten_state(t, layout, is_list)
     kr = NUTSKernelResults(
         target_log_prob=nl, grads_target_log_prob=unflat(ng), step_size=pkr.step_size,
@@ -214,15 +215,16 @@ class NoUTurnSampler(kernel_base.TransitionKernel):
     C, D = q.shape
     self._ensure(C)
     eps, per_chain = _step_size_tensor(kernel_results.step_size, C, q.device)
-    run = run_free(self._handle, q.contiguous().reshape(-1), kernel_results, eps.contiguous(),
-                   per_chain, _util.sanitize_seed(seed), first_step, transitions_per_chain,
-                   max_leaf_iterations, (C, D))
-    return run
+    return run_free(self._target, self._handle, q.contiguous().reshape(-1), kernel_results,
+                    eps.contiguous(), per_chain, _util.sanitize_seed(seed), first_step,
+                    transitions_per_chain, max_leaf_iterations, (C, D))
 
   def bootstrap_results(self, init_state):
     """nuts.py:456-503 (one gradient evaluation; energy uses unit momenta)."""
     q, layout, is_list = _util.flatten_state(init_state)
+    caller = self._target._enter()
     logp, grad = self._target.log_prob_and_grad(q)
+    self._target._leave(caller)
     if isinstance(self.step_size, (list, tuple)) and len(self.step_size) != 1:
       raise ValueError('There should be exactly one `step_size` or it should '
                        'have same length as `current_state`.')

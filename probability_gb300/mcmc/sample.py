@@ -93,7 +93,9 @@ def run_chain(kernel, num_results, current_state, num_burnin_steps=0,
   dev = q.device
   is_hmc = isinstance(sampler, HamiltonianMonteCarlo)
   target = sampler._inner._target if is_hmc else sampler._target
+  caller = target._enter()
   logp, grad = target.log_prob_and_grad(q)
+  target._leave(caller)
   eps0 = sampler.step_size if step_size is None else step_size
   eps, per_chain = _step_size_tensor(eps0, C, dev)
   eps = eps.clone()
@@ -119,6 +121,7 @@ def run_chain(kernel, num_results, current_state, num_burnin_steps=0,
   args = (n_adapt, tap, float(dap.get('exploration_shrinkage', 0.05)),
           float(dap.get('step_count_smoothing', 10)), float(dap.get('decay_rate', 0.75)),
           P(da_state) if da is not None else None)
+  caller = target._enter()
   if is_hmc:
     eng = sampler._inner._engine
     eng.ensure(C)
@@ -142,6 +145,7 @@ def run_chain(kernel, num_results, current_state, num_burnin_steps=0,
           P(tr['has_divergence']), P(tr['step_size'])), 'gbm_nuts_sample_chain')
     finally:
       lib.gbm_nuts_set_free_running(sampler._handle, 0)
+  target._leave(caller)
   for k in ('is_accepted', 'has_divergence'):
     if k in tr:
       tr[k] = tr[k].bool()

@@ -27,6 +27,23 @@ class Target:
     _native.check(_native.lib().gbm_target_dim(self._handle, ctypes.byref(d)), 'gbm_target_dim')
     return int(d.value)
 
+  def _enter(self):
+    """Before a sampler's work for a caller: where the caller's stream is not the
+    target's, which runs it, the target's waits for what the caller has queued.
+    Returns the caller's stream then, else None, for _leave."""
+    stream = self._ctx.stream
+    caller = torch.cuda.current_stream(self._ctx.device)
+    if caller == stream:
+      return None
+    stream.wait_stream(caller)
+    return caller
+
+  def _leave(self, caller):
+    """After it: the caller's stream waits for the results, and with it whatever
+    reuses the memory of its arguments."""
+    if caller is not None:
+      caller.wait_stream(self._ctx.stream)
+
   def log_prob_and_grad(self, state):
     """Batched (log_prob float64 [C], grad float32 [C, D]) at ``state`` [C, D]."""
     q = _util.as_tensor(state, torch.float32)

@@ -212,7 +212,7 @@ class HamiltonianMonteCarlo(kernel_base.TransitionKernel):
       accepted = proposed._replace(
           log_acceptance_correction=corr, initial_momentum=unflat(p0), final_momentum=unflat(p1))
     else:
-      accepted = _choose(acc, proposed, prev)
+      accepted = _choose(acc, proposed._replace(seed=[]), prev._replace(seed=[]))
     accepted = accepted._replace(target_log_prob=out['next_tlp'],
                                  grads_target_log_prob=unflat(out['next_grads']), seed=[])
     kr = MetropolisHastingsKernelResults(

@@ -157,16 +157,29 @@ std::unique_ptr<Target> make_transformed(gbm_context* ctx, Target* inner, const 
 // one above 512.
 std::unique_ptr<Target> make_logreg_large(gbm_context* ctx, const void* X, int x_dtype, int64_t n,
                                           int64_t d, const float* y, float prior_scale,
-                                          bool mixed);
+                                          bool mixed, bool pairs = true);
 // FP32 target for up to 128 features (row-pair layout, bulk-copied tiles);
-// nullptr above that.
+// nullptr above that.  `pairs`: may keep FP16 pairs of X beside it (f16_rows.cuh).
 std::unique_ptr<Target> make_logreg_f32(gbm_context* ctx, const float* X, int64_t n, int64_t d,
-                                        const float* y, float prior_scale);
+                                        const float* y, float prior_scale, bool pairs = true);
 // FP32, 129 to 256 features; nullptr if the data do not fit its FP16 form.
 std::unique_ptr<Target> make_logreg_wide(gbm_context* ctx, const float* X, int64_t n, int64_t d,
                                          const float* y, float prior_scale);
 std::unique_ptr<Target> make_logreg_simt(gbm_context* ctx, const float* X, int64_t n,
-                                         int64_t d, const float* y, float prior_scale);
+                                         int64_t d, const float* y, float prior_scale,
+                                         bool pairs = true);
+
+// Device memory that a target takes at most, with the workspace of an evaluation of
+// `chains` states: what the constructors and workspace_bytes() reserve, before
+// there is a target to ask.
+size_t logreg_f32_bytes(int64_t n, int64_t d, int64_t chains, int num_sms, bool pairs);
+size_t logreg_wide_bytes(int64_t n, int64_t d, int64_t chains, int num_sms);  // 0: not its shape
+size_t logreg_simt_bytes(int64_t n, int64_t d, int64_t chains, int num_sms, bool pairs);
+size_t logreg_large_bytes(int64_t n, int64_t d, int64_t chains, int num_sms, bool mixed,
+                          int x_dtype, bool pairs);
+size_t logreg_tc_bytes(int64_t n, int64_t d, int64_t chains, int num_sms, int x_dtype);
+size_t mvn_bytes(int64_t d, int64_t chains);
+size_t hier_bytes(int64_t groups);
 
 }  // namespace gbm
 

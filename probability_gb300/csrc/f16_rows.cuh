@@ -108,12 +108,30 @@ struct F16Rows {
   float* gscale = nullptr;      // from G' to G; zero for a column of zeros
   CUtensorMap hi, lo;           // boxes of 64 features x box_rows rows
 
+  // Elements a form may have: beyond its 16 GB the memory is the caller's.
+  static constexpr int64_t kMost = (int64_t)1 << 32;
+
+  // Device memory of a form and of its making.
+  static int blocks(int num_sms) { return 8 * num_sms; }
+  static size_t parts_at(int D) { return (sizeof(unsigned) * (D + 1) + 255) / 256 * 256; }
+  static size_t losses_at(int D, int num_sms) {
+    return parts_at(D) + (sizeof(ColumnLoss) * (size_t)blocks(num_sms) * D + 255) / 256 * 256;
+  }
+  static size_t work_bytes(int D, int num_sms) {
+    return losses_at(D, num_sms) + sizeof(ColumnLoss) * D;
+  }
+  static size_t form_bytes(int64_t N, int D, int dp) {
+    return 2 * sizeof(__half) * (size_t)N * dp + sizeof(float) * D;
+  }
+  static size_t bytes(int64_t N, int D, int dp, int num_sms) {
+    return N * dp > kMost ? 0 : form_bytes(N, D, dp) + work_bytes(D, num_sms);
+  }
+
   // False if X (or the labels, ym = y - 1/2) does not fit the form: infinities,
   // NaN, exponents that the scaling cannot carry, or a range so wide that hi + lo
   // leaves more than kMostLoss of a column's nonzero entries on average, each relative
   // to the entry; a label so far outside [0, 1] that a residual, below
-  // |y - 1/2| + 1/2, could leave FP16's range (R' < 2^16); more than kMost elements (the
-  // form is as large as X in float32: beyond 16 GB the memory is the caller's).
+  // |y - 1/2| + 1/2, could leave FP16's range (R' < 2^16); more than kMost elements.
   //
   // The average is over entries and not over their squares because which rows count
   // is the residuals' to say: where a fit has a large entry's row right, its residual
@@ -126,25 +144,22 @@ struct F16Rows {
   // turn one target of 150 away.
   bool prepare(gbm_context* ctx, const float* X, const float* ym, int64_t N, int D, int dp,
                int box_rows) {
-    constexpr int64_t kMost = (int64_t)1 << 32;
     constexpr double kMostLoss = 1.0 / (1 << 23);
     constexpr unsigned kExempt = 16;
     if (N * dp > kMost) return false;
     cudaStream_t s = ctx->stream;
-    const int nb = 8 * ctx->num_sms;
+    const int nb = blocks(ctx->num_sms);
     const int64_t chunk = (N + nb - 1) / nb;
-    const size_t off_part = (sizeof(unsigned) * (D + 1) + 255) / 256 * 256;
-    const size_t off_sum = off_part + (sizeof(ColumnLoss) * (size_t)nb * D + 255) / 256 * 256;
     DeviceBuffer buf;
-    buf.reserve(off_sum + sizeof(ColumnLoss) * D);
+    buf.reserve(work_bytes(D, ctx->num_sms));
     unsigned* mx = buf.as<unsigned>();
-    ColumnLoss* part = reinterpret_cast<ColumnLoss*>(buf.as<char>() + off_part);
-    ColumnLoss* loss = reinterpret_cast<ColumnLoss*>(buf.as<char>() + off_sum);
-    const size_t bytes = sizeof(__half) * (size_t)N * dp;
-    mem.reserve(2 * bytes + sizeof(float) * D);
+    ColumnLoss* part = reinterpret_cast<ColumnLoss*>(buf.as<char>() + parts_at(D));
+    ColumnLoss* loss = reinterpret_cast<ColumnLoss*>(buf.as<char>() +
+                                                     losses_at(D, ctx->num_sms));
+    mem.reserve(form_bytes(N, D, dp));
     __half* h = mem.as<__half>();
     __half* l = h + (size_t)N * dp;
-    gscale = reinterpret_cast<float*>(mem.as<char>() + 2 * bytes);
+    gscale = reinterpret_cast<float*>(l + (size_t)N * dp);
     GBM_CUDA(cudaMemsetAsync(mx, 0, sizeof(unsigned) * (D + 1), s));
     column_max_kernel<<<nb, 128, 0, s>>>(X, N, D, chunk, mx);
     column_max_kernel<<<nb, 32, 0, s>>>(ym, N, 1, chunk, mx + D);

@@ -785,11 +785,10 @@ constexpr int64_t kTcMinRows = 4096;
 class LogregF32 final : public Target {
  public:
   LogregF32(gbm_context* ctx, const float* X, int64_t n, int64_t d, const float* y,
-            float prior_scale)
+            float prior_scale, bool pairs)
       : N_(n), D_(d) {
     dim = d;
-    kd_ = (int)((d + 15) / 16);
-    if (kd_ == 5) kd_ = 6;   // instantiated widths: 1 2 3 4 6 7 8
+    kd_ = width(d);
     dp_ = 16 * kd_;
     n2_ = (n + kF32RT - 1) / kF32RT * kF32RT;
     x2_.reserve(sizeof(float) * (size_t)n2_ * dp_);
@@ -815,7 +814,7 @@ class LogregF32 final : public Target {
     log_norm_ = -log((double)prior_scale) - 0.5 * log(2.0 * M_PI);
     grid_ = ctx->num_sms;
     err_dev_ = ctx->err_dev;
-    tc_ = n >= kTcMinRows && x16_.prepare(ctx, X, ym_.as<float>(), N_, (int)D_, dp_, kHalf);
+    tc_ = pairs && n >= kTcMinRows && x16_.prepare(ctx, X, ym_.as<float>(), N_, (int)D_, dp_, kHalf);
     switch (kd_) {
       case 1: f32_set_smem<1>(); break;
       case 2: f32_set_smem<2>(); break;
@@ -827,10 +826,15 @@ class LogregF32 final : public Target {
     }
   }
 
-  size_t workspace_bytes(int64_t cap) const override {
-    const size_t rows = (size_t)grid_ * kF32CT + (size_t)cap;
-    return rows * sizeof(double) + rows * (size_t)D_ * sizeof(float) + 256;
+  static int width(int64_t d) {      // in 16 features
+    const int kd = (int)((d + 15) / 16);
+    return kd == 5 ? 6 : kd;   // instantiated widths: 1 2 3 4 6 7 8
   }
+  static size_t work_bytes(int grid, int64_t cap, int64_t d) {
+    const size_t rows = (size_t)grid * kF32CT + (size_t)cap;
+    return rows * sizeof(double) + rows * (size_t)d * sizeof(float) + 256;
+  }
+  size_t workspace_bytes(int64_t cap) const override { return work_bytes(grid_, cap, D_); }
 
   // One launch covers at most grid_ * 128 chains (one work item per CTA);
   // larger batches run as consecutive chunks that share the workspace.
@@ -911,9 +915,17 @@ class LogregF32 final : public Target {
 }  // namespace
 
 std::unique_ptr<Target> make_logreg_f32(gbm_context* ctx, const float* X, int64_t n, int64_t d,
-                                        const float* y, float prior_scale) {
+                                        const float* y, float prior_scale, bool pairs) {
   if (d > 128) return nullptr;
-  return std::unique_ptr<Target>(new LogregF32(ctx, X, n, d, y, prior_scale));
+  return std::unique_ptr<Target>(new LogregF32(ctx, X, n, d, y, prior_scale, pairs));
+}
+
+size_t logreg_f32_bytes(int64_t n, int64_t d, int64_t chains, int num_sms, bool pairs) {
+  const int dp = 16 * LogregF32::width(d);
+  const size_t n2 = (size_t)((n + kF32RT - 1) / kF32RT * kF32RT);
+  return 4 * n2 * (dp + 1) + 8 * (size_t)d * (2 * num_sms + 1) +
+         (pairs && n >= kTcMinRows ? F16Rows::bytes(n, (int)d, dp, num_sms) : 0) +
+         LogregF32::work_bytes(num_sms, chains, d);
 }
 
 }  // namespace gbm

@@ -249,16 +249,43 @@ large_finish(const double* __restrict__ part, int nblk, int n, const float* __re
   }
 }
 
+// Sizes of a target's data and of its workspace.
+struct LargeShape {
+  int64_t N, D;
+  bool mixed;
+  int ld() const { return (int)((D + 7) / 8 * 8); }
+  // Leading dimension of Z and R: N rounded up to 8 rows.
+  int64_t ldz() const { return (N + 7) / 8 * 8; }
+  int dp() const { return (int)((D + 15) / 16 * 16); }
+  size_t el() const { return mixed ? 2 : 4; }
+  // Column sets: the mixed form stacks the hi and lo state (and residual)
+  // splits side by side, so each contraction is one GEMM of 2n columns whose
+  // halves are added in FP32 by the epilogue (Z) and the finish (G).
+  int sets() const { return mixed ? 2 : 1; }
+  // tc: X^T R from FP16 pairs.
+  size_t g_bytes(int64_t cap, bool tc, int sms) const {
+    return tc ? 4 * grad_tc_rows(sms, cap, dp()) * (size_t)D : 4 * (size_t)sets() * cap * ld();
+  }
+  // [B (sets x n rows) | Z (Np x sets n) | R | G (ld x sets n, or the gradient
+  //  partials) | partials | cuBLAS workspace]
+  size_t work_bytes(int64_t cap, bool tc, int sms) const {
+    const size_t w = (size_t)sets() * cap, nblk = (size_t)((N + kRowBlock - 1) / kRowBlock);
+    return align256(el() * w * ld()) + align256(4 * (size_t)ldz() * w) +
+           align256(el() * (size_t)ldz() * w) + align256(g_bytes(cap, tc, sms)) +
+           align256(8 * nblk * cap) + kCublasWs;
+  }
+};
+
 class LogregLarge final : public Target {
  public:
   LogregLarge(gbm_context* ctx, const void* X, int x_dtype, int64_t n, int64_t d, const float* y,
-              float prior_scale, bool mixed)
-      : N_(n), D_(d), mixed_(mixed), device_(ctx->device) {
+              float prior_scale, bool mixed, bool pairs)
+      : shape_{n, d, mixed}, N_(n), D_(d), mixed_(mixed), device_(ctx->device) {
     dim = d;
-    ld_ = (int)((d + 7) / 8 * 8);
-    ldz_ = (N_ + 7) / 8 * 8;
+    ld_ = shape_.ld();
+    ldz_ = shape_.ldz();
     xlo_ = mixed && x_dtype == 0;
-    const size_t el = mixed ? 2 : 4;
+    const size_t el = shape_.el();
     xh_.reserve(el * (size_t)ldz_ * ld_);
     if (xlo_) xl_.reserve(el * (size_t)ldz_ * ld_);
     ym_.reserve(sizeof(float) * (size_t)ldz_);
@@ -297,39 +324,29 @@ class LogregLarge final : public Target {
     }
     sms_ = ctx->num_sms;
     err_dev_ = ctx->err_dev;
-    dp_ = (int)((d + 15) / 16 * 16);
-    tc_ = !mixed && n >= kTcMinRows && x16_.prepare(ctx, static_cast<const float*>(X), ym_.as<float>(), N_, (int)D_,
-                                 dp_, kGradRT);
+    dp_ = shape_.dp();
+    tc_ = pairs && !mixed && n >= kTcMinRows &&
+          x16_.prepare(ctx, static_cast<const float*>(X), ym_.as<float>(), N_, (int)D_, dp_,
+                       kGradRT);
     if (tc_) grad_tc_setup<true>();
     inv_var_ = 1.f / (prior_scale * prior_scale);
     log_norm_ = -log((double)prior_scale) - 0.5 * log(2.0 * M_PI);
   }
 
-  // Column sets: the mixed form stacks the hi and lo state (and residual)
-  // splits side by side, so each contraction is one GEMM of 2n columns whose
-  // halves are added in FP32 by the epilogue (Z) and the finish (G).
-  int sets() const { return mixed_ ? 2 : 1; }
-
-  // [B (sets x n rows) | Z (Np x sets n) | R | G (ld x sets n, or the gradient
-  //  partials) | partials | cuBLAS workspace]
   size_t workspace_bytes(int64_t cap) const override {
-    const size_t el = mixed_ ? 2 : 4, w = (size_t)sets() * cap;
-    const size_t nblk = (size_t)((N_ + kRowBlock - 1) / kRowBlock);
-    return align256(el * w * ld_) + align256(4 * (size_t)ldz_ * w) +
-           align256(el * (size_t)ldz_ * w) + align256(g_bytes(cap)) + align256(8 * nblk * cap) +
-           kCublasWs;
+    return shape_.work_bytes(cap, tc_, sms_);
   }
 
   void eval(const float* q, int ldq, const int*, int cap, double* logp, float* grad, int ldg,
             void* ws, cudaStream_t s) override {
     const size_t el = mixed_ ? 2 : 4;
     const int64_t nblk = (N_ + kRowBlock - 1) / kRowBlock;
-    const int n = cap, w = sets() * cap, D = (int)D_;
+    const int n = cap, w = shape_.sets() * cap, D = (int)D_;
     unsigned char* p = static_cast<unsigned char*>(ws);
     unsigned char* B = p;          p += align256(el * (size_t)w * ld_);
     float* Z = reinterpret_cast<float*>(p);    p += align256(4 * (size_t)ldz_ * w);
     unsigned char* R = p;          p += align256(el * (size_t)ldz_ * w);
-    float* G = reinterpret_cast<float*>(p);    p += align256(g_bytes(cap));
+    float* G = reinterpret_cast<float*>(p);    p += align256(shape_.g_bytes(cap, tc_, sms_));
     double* part = reinterpret_cast<double*>(p); p += align256(8 * (size_t)nblk * cap);
     void* cws = p;
     cublasHandle_t h = thread_handle(device_);
@@ -409,10 +426,7 @@ class LogregLarge final : public Target {
   }
 
  private:
-  size_t g_bytes(int64_t cap) const {
-    return tc_ ? 4 * grad_tc_rows(sms_, cap, dp_) * (size_t)D_ : 4 * (size_t)sets() * cap * ld_;
-  }
-
+  LargeShape shape_;
   int64_t N_, D_;
   bool tc_ = false;              // X^T R from FP16 pairs
   int sms_ = 1, dp_ = 16;
@@ -420,7 +434,7 @@ class LogregLarge final : public Target {
   F16Rows x16_;
   bool mixed_, xlo_ = false;
   int device_ = 0, ld_ = 8;
-  int64_t ldz_ = 8;   // leading dimension of Z and R: N rounded up to 8 rows
+  int64_t ldz_ = 8;
   float inv_var_ = 1.f;
   double log_norm_ = 0.0;
   DeviceBuffer xh_, xl_, ym_, lin_;
@@ -430,9 +444,21 @@ class LogregLarge final : public Target {
 
 std::unique_ptr<Target> make_logreg_large(gbm_context* ctx, const void* X, int x_dtype, int64_t n,
                                           int64_t d, const float* y, float prior_scale,
-                                          bool mixed) {
+                                          bool mixed, bool pairs) {
   if (n >= ((int64_t)1 << 31) || d >= ((int64_t)1 << 20)) return nullptr;   // GEMM dimensions
-  return std::unique_ptr<Target>(new LogregLarge(ctx, X, x_dtype, n, d, y, prior_scale, mixed));
+  return std::unique_ptr<Target>(
+      new LogregLarge(ctx, X, x_dtype, n, d, y, prior_scale, mixed, pairs));
+}
+
+size_t logreg_large_bytes(int64_t n, int64_t d, int64_t chains, int num_sms, bool mixed,
+                          int x_dtype, bool pairs) {
+  const LargeShape h{n, d, mixed};
+  const bool tc = pairs && !mixed && n >= kTcMinRows;
+  const size_t x = h.el() * (size_t)h.ldz() * h.ld();
+  return x * (mixed && x_dtype == 0 ? 2 : 1) + 4 * (size_t)h.ldz() +
+         8 * (size_t)d * (2 * num_sms + 1) +
+         (tc ? F16Rows::bytes(n, (int)d, h.dp(), num_sms) : 0) +
+         std::max(h.work_bytes(chains, tc, num_sms), h.work_bytes(chains, false, num_sms));
 }
 
 }  // namespace gbm

@@ -225,10 +225,11 @@ class LogregSimt final : public Target {
     set_smem(kd_);
   }
 
-  size_t workspace_bytes(int64_t cap) const override {
-    const size_t rows = (size_t)grid_ * kCT + (size_t)cap;  // S * n <= grid * kCT + n
-    return rows * sizeof(double) + rows * (size_t)D_ * sizeof(float) + 256;
+  static size_t work_bytes(int grid, int64_t cap, int64_t d) {
+    const size_t rows = (size_t)grid * kCT + (size_t)cap;  // S * n <= grid * kCT + n
+    return rows * sizeof(double) + rows * (size_t)d * sizeof(float) + 256;
   }
+  size_t workspace_bytes(int64_t cap) const override { return work_bytes(grid_, cap, D_); }
 
   // One launch covers at most grid_ * kCT chains (one work item per CTA);
   // larger batches run as consecutive chunks that share the workspace.
@@ -293,11 +294,19 @@ namespace {
 } // namespace
 
 std::unique_ptr<Target> make_logreg_simt(gbm_context* ctx, const float* X, int64_t n, int64_t d,
-                                         const float* y, float prior_scale) {
+                                         const float* y, float prior_scale, bool pairs) {
   if (d > 256) return nullptr;
-  if (d <= 128) return make_logreg_f32(ctx, X, n, d, y, prior_scale);
-  if (auto t = make_logreg_wide(ctx, X, n, d, y, prior_scale)) return t;
+  if (d <= 128) return make_logreg_f32(ctx, X, n, d, y, prior_scale, pairs);
+  if (pairs)
+    if (auto t = make_logreg_wide(ctx, X, n, d, y, prior_scale)) return t;
   return std::unique_ptr<Target>(new LogregSimt(ctx, X, n, d, y, prior_scale));
+}
+
+size_t logreg_simt_bytes(int64_t n, int64_t d, int64_t chains, int num_sms, bool pairs) {
+  if (d <= 128) return logreg_f32_bytes(n, d, chains, num_sms, pairs);
+  const size_t plain = 4 * (size_t)n * ((d + 3) / 4 * 4 + 1) +
+                       LogregSimt::work_bytes(2 * num_sms, chains, d);
+  return std::max(plain, pairs ? logreg_wide_bytes(n, d, chains, num_sms) : 0);
 }
 
 }  // namespace gbm

@@ -1352,8 +1352,8 @@ class LogregTc final : public Target {
            float prior_scale)
       : N_(n), D_(d) {
     dim = d;
-    kb_ = d <= 128 ? 2 : d <= 256 ? 4 : 8;   // 8: the pair-cluster kernel
-    ct_ = kb_ == 2 ? 128 : 64;
+    kb_ = blocks64(d);   // 8: the pair-cluster kernel
+    ct_ = chain_tile(kb_);
     // FP32 data up to 128 features keeps a BF16 residual X_lo (see XLO).
     xlo_ = (x_dtype == 0 && kb_ == 2);
     const int Dp = kb_ * 64;
@@ -1433,10 +1433,13 @@ class LogregTc final : public Target {
     }
   }
 
-  size_t workspace_bytes(int64_t cap) const override {
-    const size_t rows = (size_t)grid_ * ct_ + (size_t)cap;
-    return rows * sizeof(double) + rows * (size_t)D_ * sizeof(float) + 256;
+  static int blocks64(int64_t d) { return d <= 128 ? 2 : d <= 256 ? 4 : 8; }
+  static int chain_tile(int kb) { return kb == 2 ? 128 : 64; }
+  static size_t work_bytes(int grid, int ct, int64_t cap, int64_t d) {
+    const size_t rows = (size_t)grid * ct + (size_t)cap;
+    return rows * sizeof(double) + rows * (size_t)d * sizeof(float) + 256;
   }
+  size_t workspace_bytes(int64_t cap) const override { return work_bytes(grid_, ct_, cap, D_); }
 
   void eval(const float* q, int ldq, const int* n_dev, int cap, double* logp, float* grad,
             int ldg, void* ws, cudaStream_t s) override {
@@ -1501,6 +1504,15 @@ std::unique_ptr<Target> make_logreg_tc(gbm_context* ctx, const void* X, int x_dt
                                        int64_t d, const float* y, float prior_scale) {
   if (d > 512) return nullptr;
   return std::unique_ptr<Target>(new LogregTc(ctx, X, x_dtype, n, d, y, prior_scale));
+}
+
+size_t logreg_tc_bytes(int64_t n, int64_t d, int64_t chains, int num_sms, int x_dtype) {
+  const int kb = LogregTc::blocks64(d);
+  const size_t x = 2 * (size_t)n * kb * 64;
+  const size_t ym = kb == 2 ? 4 * (size_t)((n + kRows - 1) / kRows * kRows) : 0;
+  return x * (kb == 2 && x_dtype == 0 ? 2 : 1) + 4 * (size_t)n + ym +
+         8 * (size_t)d * (2 * num_sms + 1) +
+         LogregTc::work_bytes(kb == 8 ? num_sms / 2 : num_sms, LogregTc::chain_tile(kb), chains, d);
 }
 
 }  // namespace gbm

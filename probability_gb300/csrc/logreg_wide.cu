@@ -201,19 +201,47 @@ wide_products_kernel(const float* __restrict__ xt, int64_t Np, const float* __re
   }
 }
 
+// Sizes of a target and of its launches.
+struct WideShape {
+  int64_t N, D;
+  int sms;
+  struct Layout {
+    int64_t cp;                    // chains rounded up to whole tiles
+    size_t gpart, lpart, qt, total;
+  };
+  int dp() const { return (int)((D + 15) / 16 * 16); }
+  int64_t np() const { return (N + kWideRT - 1) / kWideRT * kWideRT; }
+  // Chains of a launch: residuals of 1 GB at most, whole chain tiles.
+  int64_t lim() const {
+    const int64_t l = std::max<int64_t>(kGradCT, ((int64_t)1 << 30) / (4 * N) / kGradCT * kGradCT);
+    return std::min<int64_t>(l, (int64_t)sms * kGradCT);
+  }
+  // [residuals hi, lo | gradient partials | likelihood partials | Q^T]
+  Layout layout(int64_t chains) const {
+    const int64_t cap = std::min(chains, lim());
+    auto up = [](size_t b) { return (b + 255) / 256 * 256; };
+    Layout l;
+    l.cp = (cap + kWideCT - 1) / kWideCT * kWideCT;
+    l.gpart = up(4 * (size_t)N * l.cp);
+    l.lpart = l.gpart + up(sizeof(float) * grad_tc_rows(sms, cap, dp()) * (size_t)D);
+    l.qt = l.lpart + up(sizeof(double) * (size_t)(np() / kWideRT) * cap);
+    l.total = l.qt + up(sizeof(float) * (size_t)dp() * l.cp);
+    return l;
+  }
+};
+
 class LogregWide final : public Target {
  public:
-  LogregWide(gbm_context* ctx, int64_t n, int64_t d, float prior_scale) : N_(n), D_(d) {
+  LogregWide(gbm_context* ctx, int64_t n, int64_t d, float prior_scale)
+      : shape_{n, d, ctx->num_sms}, N_(n), D_(d) {
     dim = d;
-    dp_ = (int)((d + 15) / 16 * 16);
-    np_ = (n + kWideRT - 1) / kWideRT * kWideRT;
+    dp_ = shape_.dp();
+    np_ = shape_.np();
     sms_ = ctx->num_sms;
     err_dev_ = ctx->err_dev;
     inv_var_ = 1.f / (prior_scale * prior_scale);
     log_norm_ = -log((double)prior_scale) - 0.5 * log(2.0 * M_PI);
-    // Chains of a launch: residuals of 1 GB at most, whole chain tiles.
-    lim_ = std::max<int64_t>(kGradCT, ((int64_t)1 << 30) / (4 * n) / kGradCT * kGradCT);
-    lim_ = std::min<int64_t>(lim_, (int64_t)sms_ * kGradCT);
+    lim_ = shape_.lim();
   }
 
   // False if X or the labels do not fit FP16 pairs.
@@ -234,15 +262,12 @@ class LogregWide final : public Target {
     return true;
   }
 
-  // [residuals hi, lo | gradient partials | likelihood partials | Q^T]
-  size_t workspace_bytes(int64_t cap) const override {
-    return layout(std::min(cap, lim_)).total;
-  }
+  size_t workspace_bytes(int64_t cap) const override { return shape_.layout(cap).total; }
 
   void eval(const float* q, int ldq, const int* n_dev, int cap, double* logp, float* grad,
             int ldg, void* ws, cudaStream_t s) override {
     const int N = (int)N_, D = (int)D_, lim = (int)lim_;
-    const Layout l = layout(std::min<int64_t>(cap, lim_));
+    const WideShape::Layout l = shape_.layout(cap);
     char* w = static_cast<char*>(ws);
     __half* rhi = reinterpret_cast<__half*>(w);
     __half* rlo = rhi + (size_t)N_ * l.cp;
@@ -278,21 +303,7 @@ class LogregWide final : public Target {
   }
 
  private:
-  struct Layout {
-    int64_t cp;                    // chains rounded up to whole tiles
-    size_t gpart, lpart, qt, total;
-  };
-  Layout layout(int64_t cap) const {
-    auto up = [](size_t b) { return (b + 255) / 256 * 256; };
-    Layout l;
-    l.cp = (cap + kWideCT - 1) / kWideCT * kWideCT;
-    l.gpart = up(4 * (size_t)N_ * l.cp);
-    l.lpart = l.gpart + up(sizeof(float) * grad_tc_rows(sms_, cap, dp_) * (size_t)D_);
-    l.qt = l.lpart + up(sizeof(double) * (size_t)(np_ / kWideRT) * cap);
-    l.total = l.qt + up(sizeof(float) * (size_t)dp_ * l.cp);
-    return l;
-  }
-
+  WideShape shape_;
   int64_t N_, D_, np_ = 0, lim_ = 0;
   int dp_ = 16, sms_ = 1;
   float inv_var_ = 1.f;
@@ -304,14 +315,25 @@ class LogregWide final : public Target {
 
 }  // namespace
 
+// grid.y counts row tiles; residuals of a chain tile stay within 2 GB.
+static bool wide_holds(int64_t n, int64_t d) {
+  constexpr int64_t kMostRows = (int64_t)1 << 22;
+  return d > 128 && d <= 256 && n <= kMostRows;
+}
+
 std::unique_ptr<Target> make_logreg_wide(gbm_context* ctx, const float* X, int64_t n, int64_t d,
                                          const float* y, float prior_scale) {
-  // grid.y counts row tiles; residuals of a chain tile stay within 2 GB.
-  constexpr int64_t kMostRows = (int64_t)1 << 22;
-  if (d <= 128 || d > 256 || n > kMostRows) return nullptr;
+  if (!wide_holds(n, d)) return nullptr;
   auto t = std::make_unique<LogregWide>(ctx, n, d, prior_scale);
   if (!t->prepare(ctx, X, y)) return nullptr;
   return t;
+}
+
+size_t logreg_wide_bytes(int64_t n, int64_t d, int64_t chains, int num_sms) {
+  if (!wide_holds(n, d)) return 0;
+  const WideShape w{n, d, num_sms};
+  return 4 * (size_t)w.np() * (w.dp() + 1) + 4 * (size_t)n +
+         F16Rows::bytes(n, (int)d, w.dp(), num_sms) + w.layout(chains).total;
 }
 
 }  // namespace gbm

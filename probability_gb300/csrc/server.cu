@@ -49,6 +49,7 @@ struct Job {
   int error_code = GBM_OK;
   std::string error;
   size_t bytes = 0;
+  bool pairs = true;   // FP32 regression: may keep FP16 pairs of X beside it
   double t_submit = 0, t_start = 0, t_end = 0;
 };
 
@@ -61,24 +62,26 @@ int family_dim(const gbm_job_spec& s, int64_t* dim) {
   }
 }
 
-// Device memory a job needs (target data + workspaces + NUTS + loop buffers).
-size_t estimate_bytes(const gbm_job_spec& s, int num_sms) {
-  const double C = (double)s.chains, D = (double)s.dim;
-  double b = 0;
-  if (s.family == GBM_FAMILY_LOGISTIC_REGRESSION) {
-    const double N = (double)s.rows;
-    const double Dp = std::ceil(D / 64.0) * 64.0;
-    const bool mixed = s.precision == GBM_PRECISION_MIXED;
-    b += mixed ? N * Dp * 4.0 : N * (std::ceil(D / 16.0) * 16.0) * 4.0;
-    b += N * 8.0;
-    b += (2.0 * num_sms * 128.0 + C) * (8.0 + 4.0 * D);
-    if (D > (mixed ? 512.0 : 256.0))   // library-GEMM target: Z and R (hi, lo), B, G, cuBLAS
-      b += (N + 8.0) * C * (mixed ? 12.0 : 8.0) + C * Dp * 16.0 + (32u << 20);
-  } else if (s.family == GBM_FAMILY_MVN) {
-    b += 4.0 * D * D + 4.0 * D + C * (8.0 * std::ceil(D / 64.0) + 4.0 * D);
-  } else {
-    b += 8.0 * (double)s.groups;
+// Of a job's target, with its workspace (`pairs`: see Job).
+size_t target_bytes(const gbm_job_spec& s, int num_sms, bool pairs) {
+  const int64_t C = s.chains;
+  switch (s.family) {
+    case GBM_FAMILY_LOGISTIC_REGRESSION: {
+      const bool mixed = s.precision == GBM_PRECISION_MIXED;
+      if (s.features > (mixed ? 512 : 256))
+        return logreg_large_bytes(s.rows, s.features, C, num_sms, mixed, s.x_dtype, pairs);
+      return mixed ? logreg_tc_bytes(s.rows, s.features, C, num_sms, s.x_dtype)
+                   : logreg_simt_bytes(s.rows, s.features, C, num_sms, pairs);
+    }
+    case GBM_FAMILY_MVN: return mvn_bytes(s.dim, C);
+    default: return hier_bytes(s.groups);
   }
+}
+
+// Device memory a job needs (target data + workspace + NUTS + loop buffers).
+size_t estimate_bytes(const gbm_job_spec& s, int num_sms, bool pairs) {
+  const double C = (double)s.chains, D = (double)s.dim;
+  double b = (double)target_bytes(s, num_sms, pairs);
   const double vec = C * D;
   b += 4.0 * vec * (14.0 + 2.0 * s.max_tree_depth) + 160.0 * C;   // NUTS workspace
   b += 8.0 * vec + 64.0 * C;                                        // chain loop buffers
@@ -125,10 +128,11 @@ void run_job(gbm_context* ctx, Job* job) {
       t->impl = s.precision == GBM_PRECISION_MIXED
                     ? make_logreg_tc(ctx, s.x, s.x_dtype, s.rows, s.features, s.y, s.prior_scale)
                     : make_logreg_simt(ctx, static_cast<const float*>(s.x), s.rows, s.features,
-                                       s.y, s.prior_scale);
+                                       s.y, s.prior_scale, job->pairs);
       if (!t->impl)   // beyond the fused kernels' feature limits
         t->impl = make_logreg_large(ctx, s.x, s.x_dtype, s.rows, s.features, s.y,
-                                    s.prior_scale, s.precision == GBM_PRECISION_MIXED);
+                                    s.prior_scale, s.precision == GBM_PRECISION_MIXED,
+                                    job->pairs);
       break;
     case GBM_FAMILY_MVN:
       t->impl = make_mvn(ctx, s.loc, s.scale_tril_inv, s.dim, s.log_normalizer);
@@ -156,10 +160,9 @@ void run_job(gbm_context* ctx, Job* job) {
   da.reserve(256);
   GBM_CUDA(cudaMemcpyAsync(q.ptr, s.init_state, sizeof(float) * C * D, cudaMemcpyDeviceToDevice,
                            st));
-  t->ws.reserve(t->impl->workspace_bytes(C));
   set_count(t->count.as<int>(), (int)C, st);
   t->impl->eval(q.as<float>(), (int)D, t->count.as<int>(), (int)C, l.as<double>(), g.as<float>(),
-                (int)D, t->ws.ptr, st);
+                (int)D, k.target_ws.ptr, st);   // the sampler's: one workspace a job
   init_loop_state<<<1, 1, 0, st>>>(eps.as<float>(), da.as<double>(), s.step_size);
   GBM_CUDA(cudaGetLastError());
   DaConfig dac{s.num_adaptation_steps > 0 ? 1 : 0,
@@ -357,7 +360,11 @@ int gbm_server_submit(gbm_server* srv, const gbm_job_spec* spec, int64_t* job_id
   }
   std::unique_ptr<gbm::Job> job(new gbm::Job());
   job->spec = s;
-  job->bytes = gbm::estimate_bytes(s, srv->num_sms);
+  job->bytes = gbm::estimate_bytes(s, srv->num_sms, true);
+  if (job->bytes > srv->budget) {   // X alone may fit where X and its pairs do not
+    job->pairs = false;
+    job->bytes = gbm::estimate_bytes(s, srv->num_sms, false);
+  }
   if (job->bytes > srv->budget) {
     gbm::set_error("gbm_server_submit: job needs more device memory than the server budget");
     return GBM_ENOMEM;

@@ -77,9 +77,10 @@ class Mvn final : public Target {
     GBM_CUDA(cudaFuncSetAttribute(mvn_tri_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)sizeof(MvnLaunch<1>::Smem)));
   }
-  size_t workspace_bytes(int64_t cap) const override {
-    return sizeof(double) * (size_t)cap * mvn_parts(dim) + sizeof(float) * (size_t)cap * dim + 512;
+  static size_t work_bytes(int64_t cap, int64_t d) {
+    return sizeof(double) * (size_t)cap * mvn_parts(d) + sizeof(float) * (size_t)cap * d + 512;
   }
+  size_t workspace_bytes(int64_t cap) const override { return work_bytes(cap, dim); }
   void eval(const float* q, int ldq, const int* n_dev, int cap, double* logp, float* grad,
             int ldg, void* ws, cudaStream_t s) override {
     double* part = static_cast<double*>(ws);
@@ -188,6 +189,15 @@ class Hier final : public Target {
 };
 
 }  // namespace
+
+size_t mvn_bytes(int64_t d, int64_t chains) {
+  return sizeof(float) * (size_t)d + mvn_factor_bytes(d) + Mvn::work_bytes(chains, d);
+}
+
+size_t hier_bytes(int64_t groups) {
+  return 2 * sizeof(float) * (size_t)groups + sizeof(double) * chain_log_table().size() +
+         sizeof(HierModel) + 256;
+}
 
 std::unique_ptr<Target> make_mvn(gbm_context* ctx, const float* loc, const float* scale_tril_inv,
                                  int64_t d, double log_norm) {

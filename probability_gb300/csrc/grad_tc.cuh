@@ -1,7 +1,8 @@
 // Gradient partials of a logistic regression on the tensor cores, from residuals
 // in memory: G^T[c][d] = sum_r R[r][c] X[r][d] with R and X as FP16 hi + lo
 // (f16_rows.cuh), for the FP32 targets whose features are too many for a kernel
-// that also forms Z.
+// that also forms Z.  R is held as multiples of 2^-15, or of a power of two for each
+// 128 rows of a chain, which then goes into the sums.
 //
 // A CTA owns 128 chains x 256 features (M x N of its MMAs) and a stretch of rows,
 // and writes one partial.  TMA brings 64 rows of R and X into one of two stages;
@@ -44,13 +45,14 @@ struct GradBars {
 
 // R: boxes of 64 chains x 64 rows of [N][chains] (K_MAJOR false), or of 64 rows x
 // 128 chains of [chains][rows].  grid = split stretches x chain tiles at most,
-// times feature tiles.
+// times feature tiles.  rscale (K_MAJOR false): what 2^15 R of a chain's 128 rows is
+// of what is stored, [rows / 128][cp].
 template <bool K_MAJOR>
 __global__ void __launch_bounds__(kGradThreads, 1)
 grad_tc_kernel(const __grid_constant__ CUtensorMap rhi, const __grid_constant__ CUtensorMap rlo,
                const __grid_constant__ CUtensorMap xhi, const __grid_constant__ CUtensorMap xlo,
-               const float* __restrict__ gscale, int N, int D, int dp,
-               const int* __restrict__ n_dev, int c_base, int c_lim, int grid, int ftiles,
+               const float* __restrict__ gscale, const float* __restrict__ rscale, int cp, int N,
+               int D, int dp, const int* __restrict__ n_dev, int c_base, int c_lim, int grid, int ftiles,
                float* __restrict__ gpart, int* __restrict__ err) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>(
@@ -179,8 +181,12 @@ grad_tc_kernel(const __grid_constant__ CUtensorMap rhi, const __grid_constant__ 
 #pragma unroll
     for (int i = 0; i < 128; ++i) sum[i] = 0.f;
     bool ok = true;
+    const int chain = c0 + (warp & 3) * 32 + lane;
+    float scale = 1.f;
     for (int u = 0; u < 2 * U; ++u) {      // half stages
       const int s = u & 1;
+      if (!K_MAJOR && s == 0 && chain < cp)
+        scale = rscale[(size_t)((u0 + (u >> 1)) >> 1) * cp + chain];
       if (!warp_wait(&bars->acc_full[s], (uint32_t)(u >> 1) & 1, abort_flag)) {
         ok = false;
         break;
@@ -193,7 +199,8 @@ grad_tc_kernel(const __grid_constant__ CUtensorMap rhi, const __grid_constant__ 
         tc::tmem_ld16(tmem + s * kGradFT + quarter + col + 16 * j, v);
         tc::tmem_ld_wait();
 #pragma unroll
-        for (int e = 0; e < 16; ++e) sum[16 * j + e] += v[e];
+        for (int e = 0; e < 16; ++e)
+          sum[16 * j + e] = K_MAJOR ? sum[16 * j + e] + v[e] : fmaf(v[e], scale, sum[16 * j + e]);
       }
       tc::tc_fence_before();
       __syncwarp();
@@ -253,9 +260,9 @@ void grad_tc_setup() {
 }
 
 // Partials of chains [c_base, c_base + cap) whose residuals are at r (hi, then lo
-// at r_lo): [N][ldr] chains, or [chains][ldr] rows.
+// at r_lo): [N][ldr] chains with rscale, or [chains][ldr] rows.
 template <bool K_MAJOR>
-void launch_grad_tc(const F16Rows& x, __half* r, __half* r_lo, int64_t ldr, int N, int D, int dp,
+void launch_grad_tc(const F16Rows& x, __half* r, __half* r_lo, const float* rscale, int64_t ldr, int N, int D, int dp,
                     const int* n_dev, int c_base, int c_lim, int cap, int grid, float* gpart,
                     int* err, cudaStream_t s) {
   CUtensorMap hi, lo;
@@ -268,7 +275,7 @@ void launch_grad_tc(const F16Rows& x, __half* r, __half* r_lo, int64_t ldr, int 
   }
   const int ft = grad_tc_ftiles(dp);
   grad_tc_kernel<K_MAJOR><<<(unsigned)(grid * ft), kGradThreads, kGradSmem, s>>>(
-      hi, lo, x.hi, x.lo, x.gscale, N, D, dp, n_dev, c_base, c_lim, grid, ft, gpart, err);
+      hi, lo, x.hi, x.lo, x.gscale, rscale, (int)ldr, N, D, dp, n_dev, c_base, c_lim, grid, ft, gpart, err);
   GBM_CUDA(cudaGetLastError());
 }
 

@@ -6,7 +6,9 @@
 //   products  a CTA (128 threads, 8 rows x 8 chains each) forms Z of 128 rows x
 //             64 chains from X^T and Q^T, 16 features a stage, four stages of
 //             16-byte asynchronous copies; then the log-likelihood sums and the
-//             residuals, FP16 hi + lo, to memory [rows][chains];
+//             residuals, FP16 hi + lo, to memory [rows][chains], scaled by a power
+//             of two of the largest of a chain's 128 (rows that are all but
+//             fitted leave residuals far below FP16's range);
 //   gradient  grad_tc.cuh.
 // Z is one chain of FMAs in ascending features and the log-likelihood is added by
 // fours of rows in FP32, then in float64: logreg_simt.cu's bits.
@@ -33,7 +35,7 @@ constexpr int kWideRT = 128, kWideCT = 64, kWideK = 16, kWideRing = 4;
 constexpr int kWideThreads = 128;
 constexpr int kWideStage = kWideK * (kWideRT + kWideCT);          // floats
 constexpr int kWideSmem = kWideRing * kWideStage * 4;
-static_assert(kWideSmem >= 16 * kWideCT * 8, "likelihood sums fit the stages");
+static_assert(kWideSmem >= 16 * kWideCT * 8 + 4 * kWideCT * 4, "sums and maxima fit the stages");
 
 __device__ __forceinline__ void wide_copy16(float* dst, const float* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
@@ -81,10 +83,9 @@ __global__ void wide_states_kernel(const float* __restrict__ Q, int ldq,
 
 __global__ void __launch_bounds__(kWideThreads, 3)
 wide_products_kernel(const float* __restrict__ xt, int64_t Np, const float* __restrict__ y,
-                     const float* __restrict__ ym, int N, int Dp, const float* __restrict__ qt,
-                     int cp, const int* __restrict__ n_dev, int c_base, int c_lim,
+                     int N, int Dp, const float* __restrict__ qt, int cp, const int* __restrict__ n_dev, int c_base, int c_lim,
                      double* __restrict__ lpart, __half* __restrict__ rhi,
-                     __half* __restrict__ rlo) {
+                     __half* __restrict__ rlo, float* __restrict__ rscale) {
   extern __shared__ __align__(16) float stages[];
   const int n = chunk_count(*n_dev, c_base, c_lim);
   const int c0 = blockIdx.x * kWideCT;
@@ -142,10 +143,14 @@ wide_products_kernel(const float* __restrict__ xt, int64_t Np, const float* __re
           z[i][j] = __ffma2_rn(make_float2(xa[i], xa[i]), qa[j], z[i][j]);
     }
   }
-  // Log-likelihood (by fours of rows in FP32) and residuals.
+  // Log-likelihood (by fours of rows in FP32) and residuals, in the place of z.
   double ll[8];
+  float most[8];       // largest residual of each chain
 #pragma unroll
-  for (int c = 0; c < 8; ++c) ll[c] = 0.0;
+  for (int c = 0; c < 8; ++c) {
+    ll[c] = 0.0;
+    most[c] = 0.f;
+  }
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
     float four[8];
@@ -155,44 +160,85 @@ wide_products_kernel(const float* __restrict__ xt, int64_t Np, const float* __re
     for (int i = 0; i < 4; ++i) {
       const int64_t row = r0 + 64 * h + 4 * ty + i;
       if (row < N) {
-        const float yv = y[row], yc = ym[row];
-        uint32_t hi[4], lo[4];
+        const float yv = y[row];
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-          float rv[2];
 #pragma unroll
           for (int e = 0; e < 2; ++e) {
-            const float zv = e ? z[4 * h + i][j].y : z[4 * h + i][j].x;
+            float& at = e ? z[4 * h + i][j].y : z[4 * h + i][j].x;
+            const float zv = at;
             const float t = expf(-fabsf(zv)), l = log1pf(t);
             // bernoulli.py:126-140: -softplus(z) (1 - y) - softplus(-z) y
             const float up = fmaxf(zv, 0.f) + l, down = fmaxf(-zv, 0.f) + l;
             four[2 * j + e] += -up * (1.f - yv) - down * yv;
-            const float w = tc::rcp_approx(1.f + t) - 0.5f;   // sigmoid(|z|) - 1/2
-            rv[e] = (zv >= 0.f ? yc - w : yc + w) * kF16Scale;
+            // y - sigmoid(z) from w = sigmoid(-|z|): a row that is all but fitted
+            // keeps its residual's bits, whichever its label.  1 - v is exact, and
+            // better than the product while it has bits enough.
+            const float v = tc::rcp_approx(1.f + t);
+            const float w = t > 0x1p-7f ? 1.f - v : t * v;
+            at = zv >= 0.f ? (yv - 1.f) + w : yv - w;
+            most[2 * j + e] = fmaxf(most[2 * j + e], fabsf(at));
           }
-          const __half2 a = __floats2half2_rn(rv[0], rv[1]);
-          const float2 af = __half22float2(a);
-          const __half2 b = __floats2half2_rn(rv[0] - af.x, rv[1] - af.y);
-          hi[j] = *reinterpret_cast<const uint32_t*>(&a);
-          lo[j] = *reinterpret_cast<const uint32_t*>(&b);
         }
-        const size_t at = (size_t)row * cp + c0 + 4 * tx;
-        *reinterpret_cast<uint2*>(rhi + at) = make_uint2(hi[0], hi[1]);
-        *reinterpret_cast<uint2*>(rhi + at + 32) = make_uint2(hi[2], hi[3]);
-        *reinterpret_cast<uint2*>(rlo + at) = make_uint2(lo[0], lo[1]);
-        *reinterpret_cast<uint2*>(rlo + at + 32) = make_uint2(lo[2], lo[3]);
       }
     }
 #pragma unroll
     for (int c = 0; c < 8; ++c) ll[c] += (double)four[c];
   }
+#pragma unroll
+  for (int c = 0; c < 8; ++c) {
+    most[c] = fmaxf(most[c], __shfl_xor_sync(~0u, most[c], 8));
+    most[c] = fmaxf(most[c], __shfl_xor_sync(~0u, most[c], 16));
+  }
   asm volatile("cp.async.wait_group 0;" ::: "memory");
   __syncthreads();   // every thread is done with the stages
-  double* red = reinterpret_cast<double*>(stages);   // [16][64]
+  double* red = reinterpret_cast<double*>(stages);             // [16][64]
+  float* tops = reinterpret_cast<float*>(red + 16 * kWideCT);  // [4 warps][64]
+  auto chain_of = [&](int c) { return c < 4 ? 4 * tx + c : 32 + 4 * tx + c - 4; };
 #pragma unroll
-  for (int c = 0; c < 8; ++c)
-    red[ty * kWideCT + (c < 4 ? 4 * tx + c : 32 + 4 * tx + c - 4)] = ll[c];
+  for (int c = 0; c < 8; ++c) {
+    red[ty * kWideCT + chain_of(c)] = ll[c];
+    if (lane < 8) tops[(tid >> 5) * kWideCT + chain_of(c)] = most[c];
+  }
   __syncthreads();
+  // A chain's 128 residuals are stored as multiples of the power of two that takes
+  // the largest of them below 2^15; gradient sums are in multiples of 2^-15.
+  float up[8], back[8];
+#pragma unroll
+  for (int c = 0; c < 8; ++c) {
+    float m = 0.f;
+#pragma unroll
+    for (int w = 0; w < kWideThreads / 32; ++w) m = fmaxf(m, tops[w * kWideCT + chain_of(c)]);
+    const int e = max(float_exponent(__float_as_uint(m)), -100);
+    up[c] = __int_as_float((kF16Top - e + 127) << 23);
+    back[c] = __int_as_float((15 - kF16Top + e + 127) << 23);
+  }
+  if (ty == 0) {
+    float* s = rscale + (size_t)blockIdx.y * cp + c0 + 4 * tx;
+    *reinterpret_cast<float4*>(s) = make_float4(back[0], back[1], back[2], back[3]);
+    *reinterpret_cast<float4*>(s + 32) = make_float4(back[4], back[5], back[6], back[7]);
+  }
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int64_t row = r0 + 64 * (i >> 2) + 4 * ty + (i & 3);
+    if (row < N) {
+      uint32_t hi[4], lo[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float rx = z[i][j].x * up[2 * j], ry = z[i][j].y * up[2 * j + 1];
+        const __half2 a = __floats2half2_rn(rx, ry);
+        const float2 af = __half22float2(a);
+        const __half2 b = __floats2half2_rn(rx - af.x, ry - af.y);
+        hi[j] = *reinterpret_cast<const uint32_t*>(&a);
+        lo[j] = *reinterpret_cast<const uint32_t*>(&b);
+      }
+      const size_t at = (size_t)row * cp + c0 + 4 * tx;
+      *reinterpret_cast<uint2*>(rhi + at) = make_uint2(hi[0], hi[1]);
+      *reinterpret_cast<uint2*>(rhi + at + 32) = make_uint2(hi[2], hi[3]);
+      *reinterpret_cast<uint2*>(rlo + at) = make_uint2(lo[0], lo[1]);
+      *reinterpret_cast<uint2*>(rlo + at + 32) = make_uint2(lo[2], lo[3]);
+    }
+  }
   if (tid < kWideCT && c0 + tid < n) {
     double s = 0.0;
 #pragma unroll
@@ -207,7 +253,7 @@ struct WideShape {
   int sms;
   struct Layout {
     int64_t cp;                    // chains rounded up to whole tiles
-    size_t gpart, lpart, qt, total;
+    size_t gpart, lpart, qt, rscale, total;
   };
   int dp() const { return (int)((D + 15) / 16 * 16); }
   int64_t np() const { return (N + kWideRT - 1) / kWideRT * kWideRT; }
@@ -216,7 +262,7 @@ struct WideShape {
     const int64_t l = std::max<int64_t>(kGradCT, ((int64_t)1 << 30) / (4 * N) / kGradCT * kGradCT);
     return std::min<int64_t>(l, (int64_t)sms * kGradCT);
   }
-  // [residuals hi, lo | gradient partials | likelihood partials | Q^T]
+  // [residuals hi, lo | gradient partials | likelihood partials | Q^T | scales of R]
   Layout layout(int64_t chains) const {
     const int64_t cap = std::min(chains, lim());
     auto up = [](size_t b) { return (b + 255) / 256 * 256; };
@@ -225,7 +271,8 @@ struct WideShape {
     l.gpart = up(4 * (size_t)N * l.cp);
     l.lpart = l.gpart + up(sizeof(float) * grad_tc_rows(sms, cap, dp()) * (size_t)D);
     l.qt = l.lpart + up(sizeof(double) * (size_t)(np() / kWideRT) * cap);
-    l.total = l.qt + up(sizeof(float) * (size_t)dp() * l.cp);
+    l.rscale = l.qt + up(sizeof(float) * (size_t)dp() * l.cp);
+    l.total = l.rscale + up(sizeof(float) * (size_t)(np() / kWideRT) * l.cp);
     return l;
   }
 };
@@ -274,6 +321,7 @@ class LogregWide final : public Target {
     float* gpart = reinterpret_cast<float*>(w + l.gpart);
     double* lpart = reinterpret_cast<double*>(w + l.lpart);
     float* qt = reinterpret_cast<float*>(w + l.qt);
+    float* rscale = reinterpret_cast<float*>(w + l.rscale);
     const int rtiles = (int)(np_ / kWideRT), cp = (int)l.cp;
     for (int base = 0; base < cap; base += lim) {
       const int here = std::min(lim, cap - base);
@@ -282,11 +330,11 @@ class LogregWide final : public Target {
       wide_states_kernel<<<dim3((unsigned)(ctiles * 2), (unsigned)((dp_ + 31) / 32)), dim3(32, 8),
                            0, s>>>(qc, ldq, n_dev, base, lim, D, dp_, cp, qt);
       wide_products_kernel<<<dim3((unsigned)ctiles, (unsigned)rtiles), kWideThreads, kWideSmem,
-                             s>>>(xt_.as<float>(), np_, y_.as<float>(), ym_.as<float>(), N, dp_,
-                                  qt, cp, n_dev, base, lim, lpart, rhi, rlo);
+                             s>>>(xt_.as<float>(), np_, y_.as<float>(), N, dp_, qt, cp, n_dev,
+                                  base, lim, lpart, rhi, rlo, rscale);
       GBM_CUDA(cudaGetLastError());
       const int g = grad_tc_grid(sms_, here, N_, dp_);
-      launch_grad_tc<false>(x16_, rhi, rlo, cp, N, D, dp_, n_dev, base, lim, here, g, gpart,
+      launch_grad_tc<false>(x16_, rhi, rlo, rscale, cp, N, D, dp_, n_dev, base, lim, here, g, gpart,
                             err_dev_, s);
       launch_split_reduce(lpart, gpart, qc, ldq, n_dev, base, lim, here, kGradCT, kGradRT, g, N, D,
                           inv_var_, log_norm_, nullptr, logp + base, grad + (size_t)base * ldg,

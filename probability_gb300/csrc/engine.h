@@ -50,18 +50,32 @@ struct DeviceBuffer {
     bytes = 0;
   }
   void reserve(size_t b) {
-    if (b <= bytes) return;
-    release();
-    if (b == 0) return;
-    stream = alloc_stream();
-    if (stream) {
-      GBM_CUDA(cudaMallocAsync(&ptr, b, stream));
-    } else {
-      GBM_CUDA(cudaMalloc(&ptr, b));
+    const cudaError_t e = allocate(b);
+    if (e != cudaSuccess) throw CudaError{e, "device allocation"};
+  }
+  // reserve() for what can be done without: false where there is no memory.
+  bool try_reserve(size_t b) {
+    const cudaError_t e = allocate(b);
+    if (e == cudaErrorMemoryAllocation) {
+      cudaGetLastError();   // not the next launch's
+      return false;
     }
-    bytes = b;
+    if (e != cudaSuccess) throw CudaError{e, "device allocation"};
+    return true;
   }
   template <class T> T* as() const { return static_cast<T*>(ptr); }
+
+ private:
+  cudaError_t allocate(size_t b) {
+    if (b <= bytes) return cudaSuccess;
+    release();
+    if (b == 0) return cudaSuccess;
+    stream = alloc_stream();
+    const cudaError_t e = stream ? cudaMallocAsync(&ptr, b, stream) : cudaMalloc(&ptr, b);
+    if (e == cudaSuccess) bytes = b;
+    else ptr = nullptr;
+    return e;
+  }
 };
 
 // A non-centred hierarchical normal whose whole chains a warp can run

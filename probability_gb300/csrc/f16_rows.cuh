@@ -131,7 +131,7 @@ struct F16Rows {
   // NaN, exponents that the scaling cannot carry, or a range so wide that hi + lo
   // leaves more than kMostLoss of a column's nonzero entries on average, each relative
   // to the entry; a label so far outside [0, 1] that a residual, below
-  // |y - 1/2| + 1/2, could leave FP16's range (R' < 2^16); more than kMost elements.
+  // |y - 1/2| + 1/2, could leave FP16's range (R' < 2^16); more than kMost elements, or no memory for it.
   //
   // The average is over entries and not over their squares because which rows count
   // is the residuals' to say: where a fit has a large entry's row right, its residual
@@ -151,12 +151,12 @@ struct F16Rows {
     const int nb = blocks(ctx->num_sms);
     const int64_t chunk = (N + nb - 1) / nb;
     DeviceBuffer buf;
-    buf.reserve(work_bytes(D, ctx->num_sms));
+    if (!buf.try_reserve(work_bytes(D, ctx->num_sms)) || !mem.try_reserve(form_bytes(N, D, dp)))
+      return false;
     unsigned* mx = buf.as<unsigned>();
     ColumnLoss* part = reinterpret_cast<ColumnLoss*>(buf.as<char>() + parts_at(D));
     ColumnLoss* loss = reinterpret_cast<ColumnLoss*>(buf.as<char>() +
                                                      losses_at(D, ctx->num_sms));
-    mem.reserve(form_bytes(N, D, dp));
     __half* h = mem.as<__half>();
     __half* l = h + (size_t)N * dp;
     gscale = reinterpret_cast<float*>(l + (size_t)N * dp);

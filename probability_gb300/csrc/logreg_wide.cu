@@ -291,11 +291,12 @@ class LogregWide final : public Target {
     lim_ = shape_.lim();
   }
 
-  // False if X or the labels do not fit FP16 pairs.
+  // False if X or the labels do not fit FP16 pairs, or there is no memory for them.
   bool prepare(gbm_context* ctx, const float* X, const float* y) {
-    ym_.reserve(sizeof(float) * (size_t)np_);
-    y_.reserve(sizeof(float) * (size_t)N_);
-    xt_.reserve(sizeof(float) * (size_t)np_ * dp_);
+    if (!ym_.try_reserve(sizeof(float) * (size_t)np_) ||
+        !y_.try_reserve(sizeof(float) * (size_t)N_) ||
+        !xt_.try_reserve(sizeof(float) * (size_t)np_ * dp_))
+      return false;
     wide_pack_kernel<<<dim3((unsigned)(np_ / 32), (unsigned)((dp_ + 31) / 32)), dim3(32, 8), 0,
                        ctx->stream>>>(X, y, N_, np_, (int)D_, dp_, xt_.as<float>(),
                                       ym_.as<float>());

@@ -15,7 +15,8 @@
 //   schedule: for each member, its active chains are a contiguous run of the
 //             (sorted) active list; MVN members contribute
 //             ceil(active / ct) x ceil(D / 64) tiles, hierarchical members
-//             ceil(active / 4) tiles, those with the longest sums first.
+//             ceil(active / 4) (more chains a tile where there are very many),
+//             those with the longest sums first.
 //   phase 0:  MVN tiles form u = L^-1 (x - loc) for a block of 64 rows of u
 //             and its |u|^2; hierarchical tiles do all their work.
 //   phase 1:  MVN tiles form grad = -L^-T u for a block of 64 columns; the
@@ -46,7 +47,15 @@ enum BatchFamily : int { kBatchMvn = 1, kBatchHier = 2 };   // the GBM_FAMILY_* 
 
 constexpr int kOB = 64;          // rows / columns of u or grad per MVN tile
 constexpr int kThreads = 128;
-constexpr int kHierChains = 4;   // chains per hierarchical tile (a warp each)
+// Chains of a hierarchical tile, a multiple of its four warps: four, and up to 32 of
+// short vectors where the batch's hierarchical chains still make 16 tiles for each
+// SM and more (taking a tile costs about as much as a short chain, and the warps of
+// one wait for each other).
+inline int hier_tile_chains(int64_t all_chains, int dim, int num_sms) {
+  int ct = 4;
+  while (ct < 32 && 2 * ct * dim <= 2048 && all_chains >= (int64_t)2 * ct * 16 * num_sms) ct *= 2;
+  return ct;
+}
 constexpr int kClasses = 4;      // size classes of D for the tile autotuner
 
 __host__ __device__ inline int size_class(int d) {
@@ -56,7 +65,7 @@ __host__ __device__ inline int size_class(int d) {
 struct BDesc {
   int family, dim, c_begin, c_end;
   long long p_begin;    // first |u|^2 partial of this member
-  int ct;               // chain tile (MVN)
+  int ct;               // chain tile
   MvnFactor mvn;
   const float* y;
   const float* sigma;
@@ -106,21 +115,28 @@ __device__ int block_prefix(int v, int* total) {
   return x - v + (warp > 0 ? warps[warp - 1] : 0);
 }
 
-// Block p writes phase p's tile list: {group, run of chains} of every tile in
-// the order of the groups, their number, and the counter that the phase takes
-// tiles from.  Block 0 also stores each member's run [a, a + na) of the active
-// list.
+// Blocks (p, *) write phase p's tile list: {group, run of chains} of every tile in
+// the order of the groups; block (p, 0) also their number and the counter that the
+// phase takes tiles from, block (0, 0) each member's run [a, a + na) of the active
+// list.  Groups may have any number of tiles (a member of 2^20 chains: 2^18), so the
+// tiles and not the groups are shared out among the threads, each of which looks up
+// its tile's group, and among as many blocks as make about 8 tiles a thread.  2^20
+// chains of one member (two groups): 5200 us an evaluation with a group's tiles
+// written by one thread, 2750 so, 2330 with larger tiles (hier_tile_chains); 65,536
+// chains 352, 202 and 175.
 __global__ void __launch_bounds__(1024)
 batch_schedule_kernel(const BDesc* __restrict__ d, int T, const int* __restrict__ act,
                       const int* __restrict__ act_count, const Group* __restrict__ groups0,
                       const Group* __restrict__ groups1, int n0, int n1, int* __restrict__ a,
                       int* __restrict__ na, int2* __restrict__ tiles0, int2* __restrict__ tiles1,
                       int* __restrict__ totals, int* __restrict__ next) {
+  __shared__ int first[1024];        // tile of the batch of groups that is its group's first
   const int n = *act_count, phase = blockIdx.x;
+  const bool lead = blockIdx.y == 0;
   const Group* groups = phase == 0 ? groups0 : groups1;
   int2* tiles = phase == 0 ? tiles0 : tiles1;
   const int ng = phase == 0 ? n0 : n1;
-  if (phase == 0)
+  if (phase == 0 && lead)
     for (int t = threadIdx.x; t < T; t += blockDim.x) {
       const int lo = lower_bound_dev(act, n, d[t].c_begin);
       a[t] = lo;
@@ -132,67 +148,77 @@ batch_schedule_kernel(const BDesc* __restrict__ d, int T, const int* __restrict_
     int runs = 0;
     if (g < ng) {
       const BDesc& m = d[groups[g].member];
-      const int ct = m.family == kBatchMvn ? m.ct : kHierChains;
+      const int ct = m.ct;
       const int held = lower_bound_dev(act, n, m.c_end) - lower_bound_dev(act, n, m.c_begin);
       runs = (held + ct - 1) / ct;
     }
     int total;
-    const int at = done + block_prefix(runs, &total);
-    for (int k = 0; k < runs; ++k) tiles[at + k] = make_int2(g, k);
+    first[threadIdx.x] = block_prefix(runs, &total);
+    __syncthreads();
+    for (int i = blockIdx.y * 1024 + threadIdx.x; i < total; i += gridDim.y * 1024) {
+      int lo = 0;                    // the last group whose first tile is not past i
+#pragma unroll
+      for (int step = 512; step > 0; step >>= 1)
+        if (first[lo + step] <= i) lo += step;
+      tiles[done + i] = make_int2(g0 + lo, i - first[lo]);
+    }
+    __syncthreads();
     done += total;
   }
-  if (threadIdx.x == 0) {
+  if (threadIdx.x == 0 && lead) {
     totals[phase] = done;
     next[phase] = 0;
   }
 }
 
-// One hierarchical tile: a warp per chain (targets_misc.cu hier_kernel).
+// One hierarchical tile: a warp per chain (targets_misc.cu hier_kernel), every fourth
+// of the tile's chains.
 __device__ void hier_tile(const BDesc& d, const int* __restrict__ act, int a0, int nc,
                           const int64_t* __restrict__ coff, const float* __restrict__ Q,
                           double* __restrict__ logp, float* __restrict__ Gout) {
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (w >= nc) return;
-  const int c = act[a0 + w];
-  const float* x = Q + coff[c];
-  float* G = Gout + coff[c];
-  const int J = d.dim - 2;
-  const float mu = x[0], eta = x[1];
-  const float tau = expf(eta);
-  float lp = 0.f, gmu = 0.f, geta = 0.f;
-  // Four groups per lane per pass: their loads are issued before any use, so
-  // a pass waits for memory once instead of four times.
-  for (int j0 = lane; j0 < J; j0 += 128) {
-    float z[4], sg[4], yy[4];
+  for (int i = w; i < nc; i += kThreads / 32) {
+    const int c = act[a0 + i];
+    const float* x = Q + coff[c];
+    float* G = Gout + coff[c];
+    const int J = d.dim - 2;
+    const float mu = x[0], eta = x[1];
+    const float tau = expf(eta);
+    float lp = 0.f, gmu = 0.f, geta = 0.f;
+    // Four groups per lane per pass: their loads are issued before any use, so
+    // a pass waits for memory once instead of four times.
+    for (int j0 = lane; j0 < J; j0 += 128) {
+      float z[4], sg[4], yy[4];
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const int j = j0 + 32 * u;
-      z[u] = j < J ? x[2 + j] : 0.f;
-      sg[u] = j < J ? d.sigma[j] : 1.f;
-      yy[u] = j < J ? d.y[j] : 0.f;
-    }
+      for (int u = 0; u < 4; ++u) {
+        const int j = j0 + 32 * u;
+        z[u] = j < J ? x[2 + j] : 0.f;
+        sg[u] = j < J ? d.sigma[j] : 1.f;
+        yy[u] = j < J ? d.y[j] : 0.f;
+      }
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const int j = j0 + 32 * u;
-      if (j >= J) break;
-      const float res = (yy[u] - (mu + tau * z[u])) / sg[u];
-      const float r = res / sg[u];
-      lp += -0.5f * z[u] * z[u] - 0.5f * res * res;
-      gmu += r;
-      geta += r * z[u];
-      G[2 + j] = -z[u] + tau * r;
+      for (int u = 0; u < 4; ++u) {
+        const int j = j0 + 32 * u;
+        if (j >= J) break;
+        const float res = (yy[u] - (mu + tau * z[u])) / sg[u];
+        const float r = res / sg[u];
+        lp += -0.5f * z[u] * z[u] - 0.5f * res * res;
+        gmu += r;
+        geta += r * z[u];
+        G[2 + j] = -z[u] + tau * r;
+      }
     }
-  }
-  double lpd = warp_sum((double)lp);
-  gmu = warp_sum(gmu);
-  geta = warp_sum(geta);
-  if (lane == 0) {
-    const float t = tau / d.tau_scale;
-    lpd += -0.5 * (double)(mu / d.mu_scale) * (double)(mu / d.mu_scale) - log1p((double)t * t) +
-           (double)eta + d.hconst;
-    logp[c] = lpd;
-    G[0] = -mu / (d.mu_scale * d.mu_scale) + gmu;
-    G[1] = -2.f * t * t / (1.f + t * t) + 1.f + tau * geta;
+    double lpd = warp_sum((double)lp);
+    gmu = warp_sum(gmu);
+    geta = warp_sum(geta);
+    if (lane == 0) {
+      const float t = tau / d.tau_scale;
+      lpd += -0.5 * (double)(mu / d.mu_scale) * (double)(mu / d.mu_scale) - log1p((double)t * t) +
+             (double)eta + d.hconst;
+      logp[c] = lpd;
+      G[0] = -mu / (d.mu_scale * d.mu_scale) + gmu;
+      G[1] = -2.f * t * t / (1.f + t * t) + 1.f + tau * geta;
+    }
   }
 }
 
@@ -235,14 +261,15 @@ batch_phase_kernel(const BDesc* __restrict__ desc, const Group* __restrict__ gro
                    float* __restrict__ u, float* __restrict__ grad, double* __restrict__ part,
                    double* __restrict__ logp) {
   extern __shared__ __align__(16) unsigned char smem[];
-  __shared__ int taken;
+  __shared__ int taken[2];   // the next tile, of even and odd turns
   const int total = *total_dev, stretch = blockIdx.x / sms, place = blockIdx.x % sms;
   int tile = stretch * sms + (stretch & 1 ? sms - 1 - place : place);
-  while (tile < total) {
+  for (int turn = 0; tile < total; turn ^= 1) {
     const int2 at = tiles[tile];
     const Group g = groups[at.x];
     const BDesc& d = desc[g.member];
     const int first = a[g.member], held = na[g.member];
+    int ahead = -1;
     if (d.family == kBatchMvn) {
       const int a0 = at.y * d.ct, nc = min(d.ct, held - a0);
       const float* X = PHASE == 0 ? q : u;
@@ -254,13 +281,15 @@ batch_phase_kernel(const BDesc* __restrict__ desc, const Group* __restrict__ gro
         run_mvn<PHASE, 32, 4>(d, g.ob * kOB, act, first + a0, nc, coff, X, out, part, logp,
                               smem);
     } else if (PHASE == 0) {
-      const int a0 = at.y * kHierChains;
-      hier_tile(d, act, first + a0, min(kHierChains, held - a0), coff, q, logp, grad);
+      const int a0 = at.y * d.ct;
+      // These tiles are short, and last in the list: the next one is asked for first.
+      if (threadIdx.x == 0) ahead = atomicAdd(next, 1);
+      hier_tile(d, act, first + a0, min(d.ct, held - a0), coff, q, logp, grad);
     }
-    if (threadIdx.x == 0) taken = (int)gridDim.x + atomicAdd(next, 1);
-    __syncthreads();
-    tile = taken;
-    __syncthreads();   // every thread has it, and is done with shared memory
+    if (threadIdx.x == 0)
+      taken[turn] = (int)gridDim.x + (ahead >= 0 ? ahead : atomicAdd(next, 1));
+    __syncthreads();   // every thread is done with shared memory
+    tile = taken[turn];
   }
 }
 
@@ -279,6 +308,9 @@ class BatchTarget final : public Target {
     hdesc_.resize(T_);
     int64_t elems = 0, parts = 0;
     int chains = 0, dmax = 0;
+    int64_t hier_chains = 0;
+    for (int t = 0; t < T_; ++t)
+      if (m[t].family != kBatchMvn) hier_chains += m[t].chains;
     for (int t = 0; t < T_; ++t) {
       BDesc& d = hdesc_[t];
       d = BDesc{};
@@ -286,7 +318,7 @@ class BatchTarget final : public Target {
       d.dim = (int)(m[t].family == kBatchMvn ? m[t].dim : m[t].dim + 2);
       d.c_begin = chains;
       d.c_end = chains + (int)m[t].chains;
-      d.ct = 64;
+      d.ct = d.family == kBatchMvn ? 64 : hier_tile_chains(hier_chains, d.dim, ctx->num_sms);
       d.p_begin = parts;
       owned_.emplace_back(new Owned());
       Owned& o = *owned_.back();
@@ -380,7 +412,7 @@ class BatchTarget final : public Target {
     const BDesc* d = desc_.as<BDesc>();
     const Group *g0 = order_[0].groups.as<Group>(), *g1 = order_[1].groups.as<Group>();
     int2 *t0 = order_[0].tiles.as<int2>(), *t1 = order_[1].tiles.as<int2>();
-    batch_schedule_kernel<<<2, 1024, 0, s>>>(d, T_, act, act_count, g0, g1, order_[0].count,
+    batch_schedule_kernel<<<dim3(2, sched_blocks_), 1024, 0, s>>>(d, T_, act, act_count, g0, g1, order_[0].count,
                                              order_[1].count, a, na, t0, t1, totals, next);
     batch_phase_kernel<0><<<grid_[0], kThreads, PhaseLaunch<0>::kSmem, s>>>(
         d, g0, t0, totals, next, sms_, act, a, na, coff_.as<int64_t>(), q, u_.as<float>(), grad,
@@ -453,7 +485,7 @@ class BatchTarget final : public Target {
         tiles += (size_t)nob * ((chains + 31) / 32);
       } else if (phase == 0) {
         groups.push_back(Group{t, 0});
-        tiles += (size_t)(chains + kHierChains - 1) / kHierChains;
+        tiles += (size_t)(chains + d.ct - 1) / d.ct;
       }
     }
     auto length = [&](const Group& g) {
@@ -464,6 +496,8 @@ class BatchTarget final : public Target {
     std::stable_sort(groups.begin(), groups.end(),
                      [&](const Group& x, const Group& y) { return length(x) > length(y); });
     order->count = (int)groups.size();
+    const int blocks = (int)std::min<size_t>((tiles + 8191) / 8192, (size_t)ctx_->num_sms / 2);
+    sched_blocks_ = std::max(sched_blocks_, blocks);
     order->groups.reserve(sizeof(Group) * std::max<size_t>(groups.size(), 1));
     order->tiles.reserve(sizeof(int2) * std::max<size_t>(tiles, 1));
     GBM_CUDA(cudaMemcpyAsync(order->groups.ptr, groups.data(), sizeof(Group) * groups.size(),
@@ -553,7 +587,7 @@ class BatchTarget final : public Target {
   }
 
   gbm_context* ctx_;
-  int T_ = 0, C_ = 0, sms_ = 0, grid_[2] = {0, 0};
+  int T_ = 0, C_ = 0, sms_ = 0, grid_[2] = {0, 0}, sched_blocks_ = 1;
   int64_t E_ = 0;
   int chosen_[kClasses] = {0, 0, 0, 0};
   std::vector<BDesc> hdesc_;

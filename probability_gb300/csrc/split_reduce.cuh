@@ -4,7 +4,8 @@
 // Layout written by the partial kernels: lpart[S][n] (float64) and
 // gpart[S][n][D] (float32), where S = number of row splits for n chains:
 //   S = clamp(grid / ceil(n / ct), 1, ceil(N / nt)).
-// One block per chain and 128 features: a thread owns a feature and adds up to
+// One block per chain and 128 features (or several chains of up to 64 features, where
+// there are many): a thread owns a feature and adds up to
 // kOrdered splits in index order, 16 loads in flight; with more splits, groups of
 // 128 threads add a range of them each and the ranges are added in order.  The
 // log-density terms (likelihood partials, prior, linear part) are combined per
@@ -34,6 +35,11 @@ namespace gbm {
 
 constexpr int kOrdered = 32;               // splits one thread adds
 constexpr int kReduceGroups = 4;           // groups of 128 threads when there may be more
+// Chains from which a block takes several of up to 64 features: those of fewer are
+// all in flight at once whatever the block, and more wait for issue and the FP64
+// pipe, which idle warps take their share of (50 x 4, 19,456 chains: 39.5 us an
+// evaluation with a block a chain, 31 so; 1000 x 25, 4096: 37.5 and 35.4).
+constexpr int kPackedChains = 2048;
 
 // Chains of one launch.  A launch covers at most grid * ct chains (one work
 // item per CTA); larger batches are evaluated as consecutive chunks of
@@ -72,10 +78,10 @@ __host__ __device__ __forceinline__ int split_count(int n, int ct, int nt, int g
   return s > row_tiles ? row_tiles : s;
 }
 
-// Sum of p[s * stride], s in [s0, s1), in order.
+// Sum of p[s * stride], s in [s0, s1), in order, U loads in flight.
+template <int U>
 __device__ __forceinline__ float sum_splits(const float* __restrict__ p, size_t stride, int s0,
                                             int s1) {
-  constexpr int U = 16;
   float acc = 0.f;
   int s = s0;
   for (; s + U <= s1; s += U) {
@@ -96,41 +102,48 @@ __device__ __forceinline__ float sum_splits(const float* __restrict__ p, size_t 
   return acc;
 }
 
-__global__ void __launch_bounds__(128 * kReduceGroups)
+// F threads a chain: 128, of which there may be several groups, or 32 or 64 of a block
+// of 128.
+template <int F>
+__global__ void __launch_bounds__(F == 128 ? 128 * kReduceGroups : 128)
 split_reduce_kernel(const double* __restrict__ lpart, const float* __restrict__ gpart,
                     const float* __restrict__ Q, int ldq, const int* __restrict__ n_dev,
                     int c_base, int c_lim, int ct, int nt, int grid, int N, int D,
-                    float inv_var, double log_norm, const double* __restrict__ lin, int lparts,
+                    float inv_var, double half_inv_var, double dims, double log_norm,
+                    const double* __restrict__ lin, int lparts,
                     double* __restrict__ logp, float* __restrict__ grad, int ldg) {
-  __shared__ float range[kReduceGroups - 1][128];
+  __shared__ float range[F == 128 ? kReduceGroups - 1 : 1][F];
   const int n = n_dev ? chunk_count(*n_dev, c_base, c_lim) : c_lim;
-  const int c = blockIdx.x;
+  const int c = F == 128 ? (int)blockIdx.x : (int)(blockIdx.x * (128 / F) + threadIdx.x / F);
   if (c >= n) return;
+  const int threads = F == 128 ? (int)blockDim.x : F;               // of this chain
+  const int thread = F == 128 ? (int)threadIdx.x : (int)threadIdx.x % F;
   const int S = split_count(n, ct, nt, grid, N);
   const float* q = Q + (size_t)c * ldq;
-  const int groups = S <= kOrdered ? 1 : (int)(blockDim.x >> 7);
-  const int group = threadIdx.x >> 7, first = threadIdx.x & 127;
+  const int groups = S <= kOrdered ? 1 : max(1, threads >> 7);
+  const int group = thread >> 7, first = thread & 127;
   const int d = blockIdx.y * 128 + first;
   float acc = 0.f;
   if (d < D && group < groups)
-    acc = sum_splits(gpart + (size_t)c * D + d, (size_t)n * D,
+    acc = sum_splits<F == 128 ? 16 : 4>(gpart + (size_t)c * D + d, (size_t)n * D,
                      groups > 1 ? group * S / groups : 0,
                      groups > 1 ? (group + 1) * S / groups : S);
   // Per-lane log-density terms, by the last warp beside the others' sums:
   // likelihood partials lane, lane + 32, ..., then lin . q - q.q / (2 s^2) over
   // features lane, lane + 32, ...
-  if (blockIdx.y == 0 && threadIdx.x + 32 >= blockDim.x) {
+  if (blockIdx.y == 0 && thread + 32 >= threads) {
     const int lane = threadIdx.x & 31, rows = lparts > 0 ? lparts : S;
-    double t = 0.0;
+    double t = 0.0, pr = 0.0, li = 0.0;
+#pragma unroll 1
     for (int j = lane; j < rows; j += 32) t += lpart[(size_t)j * n + c];
-    double pr = 0.0, li = 0.0;
+#pragma unroll(F == 128 ? 4 : 1)
     for (int f = lane; f < D; f += 32) {
       const double qd = (double)q[f];
       pr += qd * qd;
       if (lin) li += lin[f] * qd;
     }
-    t = warp_sum(t + li - 0.5 * (double)inv_var * pr);
-    if (lane == 0) logp[c] = t + (double)D * log_norm;
+    t = warp_sum(t + li - half_inv_var * pr);
+    if (lane == 0) logp[c] = t + dims * log_norm;
   }
   if (groups > 1) {
     if (group > 0) range[group - 1][first] = acc;
@@ -152,10 +165,18 @@ void launch_split_reduce(const double* lpart, const float* gpart, const float* Q
   // Few chains make many splits: several threads per feature.  (A sampler's
   // active chains are fewer than cap; one thread then adds more than kOrdered.)
   const int threads = split_count(cap, ct, nt, grid, N) <= kOrdered ? 128 : 128 * kReduceGroups;
-  const dim3 blocks((unsigned)cap, (unsigned)((D + 127) / 128));
-  split_reduce_kernel<<<blocks, threads, 0, s>>>(
-      lpart, gpart, Q, ldq, n_dev, c_base, c_lim, ct, nt, grid, N, D, inv_var, log_norm, lin, lparts,
-      logp, grad, ldg);
+  auto go = [&](auto kernel, int per_block) {
+    const dim3 blocks((unsigned)((cap + per_block - 1) / per_block), (unsigned)((D + 127) / 128));
+    kernel<<<blocks, threads, 0, s>>>(lpart, gpart, Q, ldq, n_dev, c_base, c_lim, ct, nt, grid, N,
+                                      D, inv_var, 0.5 * (double)inv_var, (double)D, log_norm, lin,
+                                      lparts, logp, grad, ldg);
+  };
+  if (threads == 128 && D <= 32 && cap >= kPackedChains)
+    go(split_reduce_kernel<32>, 4);
+  else if (threads == 128 && D <= 64 && cap >= kPackedChains)
+    go(split_reduce_kernel<64>, 2);
+  else
+    go(split_reduce_kernel<128>, 1);
   GBM_CUDA(cudaGetLastError());
 }
 

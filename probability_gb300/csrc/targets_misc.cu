@@ -27,44 +27,70 @@
 namespace gbm {
 namespace {
 
-// Two launches over (chain tiles, output blocks), the blocks with the longest
-// sums first.  The tile is 32 x 64 at every size: 32 x 32 and 64 x 64 (4 x 8 a
-// thread) tiles were slower from 8 x 32 chains to 2048 x 512 (777 x 350, before
-// phase 1 was cut: 56, 51 and 83 us), and four groups halve phase 1.
-constexpr int kMvnCT = 32, kMvnOB = 64;
-
-template <int PHASE>
+// Two launches over (chain tiles, output blocks), the blocks with the longest sums
+// first.
+template <int PHASE, int CT, int OB, int RO, int KG>
 struct MvnLaunch {
-  static constexpr int kGroups = PHASE == 0 ? 1 : 4;
-  static constexpr int kThreads = kMvnCT / 4 * (kMvnOB / 4) * kGroups;
-  using Smem = MvnSmem<kMvnCT, kMvnOB, kGroups>;
+  static constexpr int kGroups = PHASE == 0 ? 1 : KG;
+  static constexpr int kThreads = CT / 4 * (OB / RO) * kGroups;
+  using Smem = MvnSmem<CT, OB, kGroups>;
 };
 
-template <int PHASE>
-__global__ void __launch_bounds__(MvnLaunch<PHASE>::kThreads)
+template <int PHASE, int CT, int OB, int RO, int KG>
+__global__ void __launch_bounds__(MvnLaunch<PHASE, CT, OB, RO, KG>::kThreads)
 mvn_tri_kernel(MvnFactor f, const float* __restrict__ A, int lda, const int* __restrict__ n_dev,
                float* __restrict__ out, int ldo, double* __restrict__ part,
                double* __restrict__ logp) {
+  using L = MvnLaunch<PHASE, CT, OB, RO, KG>;
   extern __shared__ __align__(16) unsigned char smem[];
-  auto& sm = *reinterpret_cast<typename MvnLaunch<PHASE>::Smem*>(smem);
-  const int n = *n_dev, c0 = blockIdx.x * kMvnCT;
+  auto& sm = *reinterpret_cast<typename L::Smem*>(smem);
+  const int n = *n_dev, c0 = blockIdx.x * CT;
   if (c0 >= n) return;
   const int ob = PHASE == 0 ? (int)(gridDim.y - 1 - blockIdx.y) : (int)blockIdx.y;
-  if (threadIdx.x < kMvnCT) {
+  if (threadIdx.x < CT) {
     const int c = c0 + threadIdx.x;
     sm.in[threadIdx.x] = (long long)c * lda;
     sm.out[threadIdx.x] = (long long)c * ldo;
     sm.part[threadIdx.x] = (long long)c * mvn_parts(f.dim);
     sm.id[threadIdx.x] = c;
   }
-  mvn_tile<PHASE, kMvnCT, kMvnOB, 4, 4, MvnLaunch<PHASE>::kGroups>(
-      f, min(kMvnCT, n - c0), ob * kMvnOB, A, out, part, logp, sm);
+  mvn_tile<PHASE, CT, OB, 4, RO, L::kGroups>(f, min(CT, n - c0), ob * OB, A, out, part, logp, sm);
 }
+
+// The tiles of a target's evaluations, MvnLaunch's parameters.
+template <int CT, int OB, int RO, int KG>
+struct MvnTiles {
+  template <int PHASE>
+  static void set_smem() {
+    GBM_CUDA(cudaFuncSetAttribute(mvn_tri_kernel<PHASE, CT, OB, RO, KG>,
+                                  cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)sizeof(typename MvnLaunch<PHASE, CT, OB, RO, KG>::Smem)));
+  }
+  static void prepare() {
+    set_smem<0>();
+    set_smem<1>();
+  }
+  template <int PHASE>
+  static void launch(const MvnFactor& f, const float* a, int lda, const int* n_dev, int cap,
+                     float* out, int ldo, double* part, double* logp, cudaStream_t s) {
+    using L = MvnLaunch<PHASE, CT, OB, RO, KG>;
+    const dim3 grid((cap + CT - 1) / CT, (f.dim + OB - 1) / OB);
+    mvn_tri_kernel<PHASE, CT, OB, RO, KG><<<grid, L::kThreads, sizeof(typename L::Smem), s>>>(
+        f, a, lda, n_dev, out, ldo, part, logp);
+    GBM_CUDA(cudaGetLastError());
+  }
+  static void eval(const MvnFactor& f, const float* q, int ldq, const int* n_dev, int cap,
+                   float* u, float* grad, int ldg, double* part, double* logp, cudaStream_t s) {
+    launch<0>(f, q, ldq, n_dev, cap, u, f.dim, part, logp, s);
+    launch<1>(f, u, f.dim, n_dev, cap, grad, ldg, part, logp, s);
+  }
+};
 
 class Mvn final : public Target {
  public:
   Mvn(gbm_context* ctx, const float* loc, const float* scale_tril_inv, int64_t d,
-      double log_norm) {
+      double log_norm)
+      : sms_(ctx->num_sms) {
     dim = d;
     mu_.reserve(sizeof(float) * d);
     m_.reserve(mvn_factor_bytes(d));
@@ -72,10 +98,8 @@ class Mvn final : public Target {
                              ctx->stream));
     factor_ = mvn_factor(scale_tril_inv, mu_.as<float>(), d, log_norm, m_.as<float>(),
                          ctx->stream);
-    GBM_CUDA(cudaFuncSetAttribute(mvn_tri_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)sizeof(MvnLaunch<0>::Smem)));
-    GBM_CUDA(cudaFuncSetAttribute(mvn_tri_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)sizeof(MvnLaunch<1>::Smem)));
+    for (int64_t chains : {(int64_t)1, kMany * sms_ * 64})
+      tiles(chains, [](auto t) { decltype(t)::prepare(); });
   }
   static size_t work_bytes(int64_t cap, int64_t d) {
     return sizeof(double) * (size_t)cap * mvn_parts(d) + sizeof(float) * (size_t)cap * d + 512;
@@ -86,12 +110,9 @@ class Mvn final : public Target {
     double* part = static_cast<double*>(ws);
     float* u = reinterpret_cast<float*>(part + (size_t)cap * mvn_parts(dim));
     const int D = (int)dim;
-    const dim3 grid((cap + kMvnCT - 1) / kMvnCT, (D + kMvnOB - 1) / kMvnOB);
-    mvn_tri_kernel<0><<<grid, MvnLaunch<0>::kThreads, sizeof(MvnLaunch<0>::Smem), s>>>(
-        factor_, q, ldq, n_dev, u, D, part, logp);
-    mvn_tri_kernel<1><<<grid, MvnLaunch<1>::kThreads, sizeof(MvnLaunch<1>::Smem), s>>>(
-        factor_, u, D, n_dev, grad, ldg, part, logp);
-    GBM_CUDA(cudaGetLastError());
+    tiles(cap, [&](auto t) {
+      decltype(t)::eval(factor_, q, ldq, n_dev, cap, u, grad, ldg, part, logp, s);
+    });
   }
   int launches_per_eval(int64_t) const override { return 2; }
   // Two triangular GEMMs: ~D^2 multiply-adds each per chain.
@@ -101,6 +122,33 @@ class Mvn final : public Target {
   }
 
  private:
+  // The tiles for `chains` chains, passed to `use`.  32 x 64 is the fastest of all
+  // tiles up to 2048 x 512 (64 x 64, 4 x 8 a thread: 777 x 350 51 against 56 us before
+  // phase 1 was cut, 300 x 2000 41.4 against 38.7).  From kMany tiles an SM on, what
+  // counts is the work done, and 64 x 64 does more with a shared load: 1000 x 5000 366
+  // us with 32 x 64, 314 so; 65 x 20,000 62 and 50; 1000 x 2000 (under the line) 152
+  // and 156.  Vectors of at most 32 have one block of 32 outputs: 2 x 100,000 99 us
+  // with 32 x 64, 34 so, and as long as before at any few chains.  Phase 1 cuts k into
+  // as many stretches as an output has 32s, at most four: a stretch less is a group
+  // of threads less that waits (64 x 20,000 40 us with four, 35 with two), and the
+  // sums are the same.
+  static constexpr int64_t kMany = 4;
+  template <class Use>
+  void tiles(int64_t chains, Use&& use) const {
+    const bool many = (chains + 63) / 64 * ((dim + 63) / 64) >= kMany * sms_;
+    if (dim <= 32)
+      use(MvnTiles<64, 32, 4, 1>());
+    else if (dim <= 64 && many)
+      use(MvnTiles<64, 64, 8, 2>());
+    else if (dim <= 64)
+      use(MvnTiles<32, 64, 4, 2>());
+    else if (many)
+      use(MvnTiles<64, 64, 8, 4>());
+    else
+      use(MvnTiles<32, 64, 4, 4>());
+  }
+
+  int sms_ = 1;
   MvnFactor factor_{};
   DeviceBuffer mu_, m_;
 };

@@ -55,6 +55,18 @@ def test_single(pg, d, c):
   _check(t, x, *t.log_prob_and_grad(x))
 
 
+@pytest.mark.parametrize('d,c', [(1, 40000), (8, 38848), (20, 70003), (32, 39001), (33, 38848),
+                                 (40, 38847), (64, 45001), (65, 19456), (130, 13001), (300, 8001)])
+def test_many_chains(pg, d, c):
+  """Past the number of chains from which tiles are 64 x 64; bits as in a small call."""
+  t, x = _normal(pg, d, c)
+  lp, g = t.log_prob_and_grad(x)
+  _check(t, x, lp, g)
+  few = torch.arange(c - 100, c, device='cuda')
+  lp1, g1 = t.log_prob_and_grad(x[few])
+  assert torch.equal(lp[few], lp1) and torch.equal(g[few], g1)
+
+
 def test_batch_gives_the_same_bits(pg):
   rng = np.random.default_rng(5)
   made = [_normal(pg, d, c) for d, c in SIZES]

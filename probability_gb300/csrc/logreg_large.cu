@@ -221,8 +221,10 @@ large_epilogue(const float* __restrict__ Z, const float* __restrict__ Zlo,
 
 // One block per chain: log-density from the partials, the linear term and the
 // prior, in a fixed order; gradient G - q / s^2.  (A warp per chain waited for its
-// loads in turn: 15 us at 929 features, 240 chains, 8 so.)
-constexpr int kFinishThreads = 256;
+// loads in turn: 15 us at 929 features, 240 chains, 8 so; a block of 256 threads leaves
+// the GPU short of chains where they are many: 300 x 300, 20,000 of them 366 us an
+// evaluation, 328 so.)
+constexpr int kFinishThreads = 128;
 __global__ void __launch_bounds__(kFinishThreads)
 large_finish(const double* __restrict__ part, int nblk, int n, const float* __restrict__ G,
              const float* __restrict__ Glo, int ld, const float* __restrict__ q, int ldq,

@@ -273,7 +273,7 @@ GBM_API int gbm_nuts_one_step(gbm_nuts* kernel, int64_t chains, const float* sta
  * states (float32, [state elements] each), target log-probs, log-accept
  * ratios (float64 [chains]), leapfrogs taken (int32), accepted and
  * divergence flags (uint8).  leaf_iterations (host, may be NULL): the
- * iterations run. */
+ * iterations, as gbm_nuts_last_leaf_iterations counts them. */
 GBM_API int gbm_nuts_run_free(gbm_nuts* kernel, int64_t chains, const float* state,
                               const double* target_log_prob, const float* grads_target_log_prob,
                               const float* step_size, int step_size_per_chain,
@@ -284,12 +284,17 @@ GBM_API int gbm_nuts_run_free(gbm_nuts* kernel, int64_t chains, const float* sta
                               int32_t* trace_leapfrogs_taken, uint8_t* trace_is_accepted,
                               uint8_t* trace_has_divergence, int64_t* leaf_iterations);
 
-/* Number of leaf iterations (batched gradient evaluations) the last
- * gbm_nuts_one_step (or gbm_nuts_run_free) launched. */
+/* Number of leaf iterations (batched gradient evaluations) of the last
+ * gbm_nuts_one_step (or gbm_nuts_run_free).  Chains of hierarchical normals of up to
+ * 1024 elements run whole trajectories in one launch; they count as the
+ * iterations that their longest trajectory takes leaf by leaf, so that the number
+ * does not depend on how a chain was run.  Waits for that step. */
 GBM_API int gbm_nuts_last_leaf_iterations(const gbm_nuts* kernel, int64_t* out);
 
-/* Profiling of NUTS transitions.  When enabled, CUDA events on the context
- * stream bracket every batched target evaluation.  gbm_nuts_read_profile
+/* Profiling of NUTS transitions.  When enabled, every chain runs leaf by leaf
+ * (hierarchical normals too, whose whole trajectories are one launch otherwise:
+ * there are no evaluations in it to bracket; the results are the same) and CUDA
+ * events on the context stream bracket every batched target evaluation.  gbm_nuts_read_profile
  * synchronizes the stream and returns, since the previous read, the summed
  * device time of those evaluations (ms), their count, and the number of
  * kernels this handle launched (targets' kernels included), then resets. */

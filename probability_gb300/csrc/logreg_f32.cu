@@ -29,7 +29,7 @@
 // into a double-buffered shared-memory stage.  X is read from HBM once per
 // chain tile (L2 serves the other chain tiles of the same rows).
 //
-// From kTcMinRows rows on, phase 2 runs on the tensor cores instead
+// From kPairRows rows on, phase 2 runs on the tensor cores instead
 // (logreg_f32_tc_kernel), beside phase 1 of the next tile: the residuals go to
 // shared memory as FP16 hi + lo (of R 2^15) and X is kept as FP16 hi + lo
 // (of each feature scaled to the top of FP16's range) beside its FP32 form,
@@ -774,13 +774,12 @@ void f32_set_smem() {
                                 F32TcLayout<KD>::kBytes));
 }
 
-// Rows from which phase 2 runs on the tensor cores.  It is the faster one from
+// From kPairRows rows on phase 2 runs on the tensor cores.  It is the faster one from
 // there on: 4096 rows x 10 features x 64 chains 26.2 us an evaluation (27.7 on
 // the CUDA cores), x 100 30.1 (35.2), 8192 x 4 x 1024 31.3 (35.0).  Below, where
 // an evaluation is launch latency for the most part (2000 x 100 x 64: 36
 // against 43 us), the gradient keeps its FP32 summation order: a sampler run
 // over a small data set repeats to the digit.
-constexpr int64_t kTcMinRows = 4096;
 
 class LogregF32 final : public Target {
  public:
@@ -814,7 +813,7 @@ class LogregF32 final : public Target {
     log_norm_ = -log((double)prior_scale) - 0.5 * log(2.0 * M_PI);
     grid_ = ctx->num_sms;
     err_dev_ = ctx->err_dev;
-    tc_ = pairs && n >= kTcMinRows && x16_.prepare(ctx, X, ym_.as<float>(), N_, (int)D_, dp_, kHalf);
+    tc_ = pairs && n >= kPairRows && x16_.prepare(ctx, X, ym_.as<float>(), N_, (int)D_, dp_, kHalf);
     switch (kd_) {
       case 1: f32_set_smem<1>(); break;
       case 2: f32_set_smem<2>(); break;
@@ -924,7 +923,7 @@ size_t logreg_f32_bytes(int64_t n, int64_t d, int64_t chains, int num_sms, bool 
   const int dp = 16 * LogregF32::width(d);
   const size_t n2 = (size_t)((n + kF32RT - 1) / kF32RT * kF32RT);
   return 4 * n2 * (dp + 1) + 8 * (size_t)d * (2 * num_sms + 1) +
-         (pairs && n >= kTcMinRows ? F16Rows::bytes(n, (int)d, dp, num_sms) : 0) +
+         (pairs && n >= kPairRows ? F16Rows::bytes(n, (int)d, dp, num_sms) : 0) +
          LogregF32::work_bytes(num_sms, chains, d);
 }
 

@@ -45,10 +45,9 @@ constexpr int kRowBlock = 2048;           // rows per epilogue block
 constexpr int kEpiThreads = 64;           // epilogue block: a row block of one chain
 constexpr int kEpiRows = kRowBlock / 256;  // rows, 256 apart, of one FP32 sum
 constexpr int kEpiBatch = 4;              // of them loaded together
-// Rows from which the FP32 target's X^T R comes from FP16 pairs.  Faster below,
+// From kPairRows rows on the FP32 target's X^T R comes from FP16 pairs.  Faster below,
 // too (2001 x 300, 64 chains: 61 against 83 us), but there the FP32 GEMM, with few
 // additions, is the more exact one (1.5e-7 of the gradient against 1.8e-7).
-constexpr int64_t kTcMinRows = 4096;
 constexpr float kNegLog2eL = -1.4426950408889634f;
 constexpr float kLn2L = 0.6931471805599453f;
 
@@ -327,7 +326,7 @@ class LogregLarge final : public Target {
     sms_ = ctx->num_sms;
     err_dev_ = ctx->err_dev;
     dp_ = shape_.dp();
-    tc_ = pairs && !mixed && n >= kTcMinRows &&
+    tc_ = pairs && !mixed && n >= kPairRows &&
           x16_.prepare(ctx, static_cast<const float*>(X), ym_.as<float>(), N_, (int)D_, dp_,
                        kGradRT);
     if (tc_) grad_tc_setup<true>();
@@ -455,7 +454,7 @@ std::unique_ptr<Target> make_logreg_large(gbm_context* ctx, const void* X, int x
 size_t logreg_large_bytes(int64_t n, int64_t d, int64_t chains, int num_sms, bool mixed,
                           int x_dtype, bool pairs) {
   const LargeShape h{n, d, mixed};
-  const bool tc = pairs && !mixed && n >= kTcMinRows;
+  const bool tc = pairs && !mixed && n >= kPairRows;
   const size_t x = h.el() * (size_t)h.ldz() * h.ld();
   return x * (mixed && x_dtype == 0 ? 2 : 1) + 4 * (size_t)h.ldz() +
          8 * (size_t)d * (2 * num_sms + 1) +

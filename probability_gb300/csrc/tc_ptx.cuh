@@ -103,12 +103,6 @@ __device__ __forceinline__ uint32_t map_to_rank(uint32_t smem_addr, uint32_t ran
   return r;
 }
 
-__device__ __forceinline__ void st_cluster_v4(uint32_t addr, uint4 v) {
-  asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(v.x),
-               "r"(v.y), "r"(v.z), "r"(v.w)
-               : "memory");
-}
-
 __device__ __forceinline__ void st_cluster_u32(uint32_t addr, uint32_t v) {
   asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
 }
@@ -149,13 +143,6 @@ __device__ __forceinline__ bool mbar_try_wait_cluster(uint64_t* bar, uint32_t pa
       : "r"(smem_u32(bar)), "r"(parity)
       : "memory");
   return ok != 0;
-}
-
-__device__ __forceinline__ void fence_acq_rel_cluster() {
-  asm volatile("fence.acq_rel.cluster;" ::: "memory");
-}
-__device__ __forceinline__ void fence_proxy_async_cluster() {
-  asm volatile("fence.proxy.async.shared::cluster;" ::: "memory");
 }
 
 // Whole-cluster barrier (every thread of every CTA of the cluster).

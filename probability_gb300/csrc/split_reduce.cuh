@@ -134,8 +134,17 @@ split_reduce_kernel(const double* __restrict__ lpart, const float* __restrict__ 
   if (blockIdx.y == 0 && thread + 32 >= threads) {
     const int lane = threadIdx.x & 31, rows = lparts > 0 ? lparts : S;
     double t = 0.0, pr = 0.0, li = 0.0;
+    constexpr int U = F == 128 ? 8 : 1;       // loads in flight
 #pragma unroll 1
-    for (int j = lane; j < rows; j += 32) t += lpart[(size_t)j * n + c];
+    for (int j = lane; j < rows; j += 32 * U) {
+      double v[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        v[u] = u == 0 || j + 32 * u < rows ? lpart[(size_t)(j + 32 * u) * n + c] : 0.0;
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (u == 0 || j + 32 * u < rows) t += v[u];
+    }
 #pragma unroll(F == 128 ? 4 : 1)
     for (int f = lane; f < D; f += 32) {
       const double qd = (double)q[f];

@@ -2,7 +2,7 @@
 // in memory: G^T[c][d] = sum_r R[r][c] X[r][d] with R and X as FP16 hi + lo
 // (f16_rows.cuh), for the FP32 targets whose features are too many for a kernel
 // that also forms Z.  R is held as multiples of 2^-15, or of a power of two for each
-// 128 rows of a chain, which then goes into the sums.
+// 32 rows of a chain, which then goes into the sums.
 //
 // A CTA owns 128 chains x 256 features (M x N of its MMAs) and a stretch of rows,
 // and writes one partial.  TMA brings 64 rows of R and X into one of two stages;
@@ -45,8 +45,8 @@ struct GradBars {
 
 // R: boxes of 64 chains x 64 rows of [N][chains] (K_MAJOR false), or of 64 rows x
 // 128 chains of [chains][rows].  grid = split stretches x chain tiles at most,
-// times feature tiles.  rscale (K_MAJOR false): what 2^15 R of a chain's 128 rows is
-// of what is stored, [rows / 128][cp].
+// times feature tiles.  rscale (K_MAJOR false): what 2^15 R of a chain's 32 rows is
+// of what is stored, [rows / 32][cp].
 template <bool K_MAJOR>
 __global__ void __launch_bounds__(kGradThreads, 1)
 grad_tc_kernel(const __grid_constant__ CUtensorMap rhi, const __grid_constant__ CUtensorMap rlo,
@@ -182,11 +182,24 @@ grad_tc_kernel(const __grid_constant__ CUtensorMap rhi, const __grid_constant__ 
     for (int i = 0; i < 128; ++i) sum[i] = 0.f;
     bool ok = true;
     const int chain = c0 + (warp & 3) * 32 + lane;
-    float scale = 1.f;
+    // Of a stage's two halves, and of the next stage's, which are loaded a stage ahead.
+    const bool scaled = !K_MAJOR && chain < cp;
+    float scale[2] = {1.f, 1.f}, next[2] = {1.f, 1.f};
+    auto load_scales = [&](int unit) {
+      if (scaled && unit < U) {
+        const float* sc = rscale + (size_t)(2 * (u0 + unit)) * cp + chain;
+        next[0] = sc[0];
+        next[1] = sc[cp];
+      }
+    };
+    load_scales(0);
     for (int u = 0; u < 2 * U; ++u) {      // half stages
       const int s = u & 1;
-      if (!K_MAJOR && s == 0 && chain < cp)
-        scale = rscale[(size_t)((u0 + (u >> 1)) >> 1) * cp + chain];
+      if (s == 0) {
+        scale[0] = next[0];
+        scale[1] = next[1];
+        load_scales((u >> 1) + 1);
+      }
       if (!warp_wait(&bars->acc_full[s], (uint32_t)(u >> 1) & 1, abort_flag)) {
         ok = false;
         break;
@@ -200,7 +213,7 @@ grad_tc_kernel(const __grid_constant__ CUtensorMap rhi, const __grid_constant__ 
         tc::tmem_ld_wait();
 #pragma unroll
         for (int e = 0; e < 16; ++e)
-          sum[16 * j + e] = K_MAJOR ? sum[16 * j + e] + v[e] : fmaf(v[e], scale, sum[16 * j + e]);
+          sum[16 * j + e] = K_MAJOR ? sum[16 * j + e] + v[e] : fmaf(v[e], s ? scale[1] : scale[0], sum[16 * j + e]);
       }
       tc::tc_fence_before();
       __syncwarp();

@@ -7,7 +7,7 @@
 //             64 chains from X^T and Q^T, 16 features a stage, four stages of
 //             16-byte asynchronous copies; then the log-likelihood sums and the
 //             residuals, FP16 hi + lo, to memory [rows][chains], scaled by a power
-//             of two of the largest of a chain's 128 (rows that are all but
+//             of two of the largest of a chain's 32 (rows that are all but
 //             fitted leave residuals far below FP16's range);
 //   gradient  grad_tc.cuh.
 // Z is one chain of FMAs in ascending features and the log-likelihood is added by
@@ -16,8 +16,8 @@
 // What bounds it: FMA issue of the products (an 8 x 8 thread's shared loads take
 // as long as its FMAs: 107 of 128 FMAs a clock and SM).  30,011 x 237, 192 chains:
 // 359 us an evaluation by logreg_simt.cu (4 x 4 a thread, unpipelined, G on the
-// CUDA cores), 111 so: products 65, gradient 27, reduction 15; 300 x 130, 16 chains
-// 61 and 40.
+// CUDA cores), 108 so: products 65 (two of them for the residuals' scales and small
+// bits), gradient 26, reduction 11; 300 x 130, 16 chains 61 and 38.
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
@@ -35,7 +35,7 @@ constexpr int kWideRT = 128, kWideCT = 64, kWideK = 16, kWideRing = 4;
 constexpr int kWideThreads = 128;
 constexpr int kWideStage = kWideK * (kWideRT + kWideCT);          // floats
 constexpr int kWideSmem = kWideRing * kWideStage * 4;
-static_assert(kWideSmem >= 16 * kWideCT * 8 + 4 * kWideCT * 4, "sums and maxima fit the stages");
+static_assert(kWideSmem >= 16 * kWideCT * 8, "likelihood sums fit the stages");
 
 __device__ __forceinline__ void wide_copy16(float* dst, const float* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
@@ -92,7 +92,8 @@ wide_products_kernel(const float* __restrict__ xt, int64_t Np, const float* __re
   if (c0 >= n) return;
   const int64_t r0 = (int64_t)blockIdx.y * kWideRT;
   const int tid = threadIdx.x, lane = tid & 31;
-  const int ty = (tid >> 5) * 4 + (lane >> 3);   // rows 4 ty.., 64 + 4 ty..
+  // A warp has 32 rows: this thread's are ry.. and ry + 16..
+  const int ty = (tid >> 5) * 4 + (lane >> 3), ry = (tid >> 5) * 32 + (lane >> 3) * 4;
   const int tx = lane & 7;                       // chains 4 tx.., 32 + 4 tx..
   const float* xsrc = xt + r0;
   const float* qsrc = qt + c0;
@@ -125,12 +126,12 @@ wide_products_kernel(const float* __restrict__ xt, int64_t Np, const float* __re
     asm volatile("cp.async.wait_group %0;" ::"n"(kWideRing - 2) : "memory");
     __syncthreads();   // this stage is complete, the last one is free
     copy(ch + kWideRing - 1);
-    const float* xs = stages + (ch % kWideRing) * kWideStage + 4 * ty;
+    const float* xs = stages + (ch % kWideRing) * kWideStage + ry;
     const float* qs = stages + (ch % kWideRing) * kWideStage + kWideK * kWideRT + 4 * tx;
 #pragma unroll
     for (int k = 0; k < kWideK; ++k) {
       const float4 x0 = *reinterpret_cast<const float4*>(xs + k * kWideRT);
-      const float4 x1 = *reinterpret_cast<const float4*>(xs + k * kWideRT + 64);
+      const float4 x1 = *reinterpret_cast<const float4*>(xs + k * kWideRT + 16);
       const float4 q0 = *reinterpret_cast<const float4*>(qs + k * kWideCT);
       const float4 q1 = *reinterpret_cast<const float4*>(qs + k * kWideCT + 32);
       const float xa[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
@@ -158,7 +159,7 @@ wide_products_kernel(const float* __restrict__ xt, int64_t Np, const float* __re
     for (int c = 0; c < 8; ++c) four[c] = 0.f;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      const int64_t row = r0 + 64 * h + 4 * ty + i;
+      const int64_t row = r0 + ry + 16 * h + i;
       if (row < N) {
         const float yv = y[row];
 #pragma unroll
@@ -185,42 +186,25 @@ wide_products_kernel(const float* __restrict__ xt, int64_t Np, const float* __re
 #pragma unroll
     for (int c = 0; c < 8; ++c) ll[c] += (double)four[c];
   }
-#pragma unroll
-  for (int c = 0; c < 8; ++c) {
-    most[c] = fmaxf(most[c], __shfl_xor_sync(~0u, most[c], 8));
-    most[c] = fmaxf(most[c], __shfl_xor_sync(~0u, most[c], 16));
-  }
-  asm volatile("cp.async.wait_group 0;" ::: "memory");
-  __syncthreads();   // every thread is done with the stages
-  double* red = reinterpret_cast<double*>(stages);             // [16][64]
-  float* tops = reinterpret_cast<float*>(red + 16 * kWideCT);  // [4 warps][64]
-  auto chain_of = [&](int c) { return c < 4 ? 4 * tx + c : 32 + 4 * tx + c - 4; };
-#pragma unroll
-  for (int c = 0; c < 8; ++c) {
-    red[ty * kWideCT + chain_of(c)] = ll[c];
-    if (lane < 8) tops[(tid >> 5) * kWideCT + chain_of(c)] = most[c];
-  }
-  __syncthreads();
-  // A chain's 128 residuals are stored as multiples of the power of two that takes
+  // A chain's 32 residuals are stored as multiples of the power of two that takes
   // the largest of them below 2^15; gradient sums are in multiples of 2^-15.
   float up[8], back[8];
 #pragma unroll
   for (int c = 0; c < 8; ++c) {
-    float m = 0.f;
-#pragma unroll
-    for (int w = 0; w < kWideThreads / 32; ++w) m = fmaxf(m, tops[w * kWideCT + chain_of(c)]);
-    const int e = max(float_exponent(__float_as_uint(m)), -100);
+    most[c] = fmaxf(most[c], __shfl_xor_sync(~0u, most[c], 8));
+    most[c] = fmaxf(most[c], __shfl_xor_sync(~0u, most[c], 16));
+    const int e = max(float_exponent(__float_as_uint(most[c])), -100);
     up[c] = __int_as_float((kF16Top - e + 127) << 23);
     back[c] = __int_as_float((15 - kF16Top + e + 127) << 23);
   }
-  if (ty == 0) {
-    float* s = rscale + (size_t)blockIdx.y * cp + c0 + 4 * tx;
+  if (lane < 8) {
+    float* s = rscale + ((size_t)blockIdx.y * (kWideRT / 32) + (tid >> 5)) * cp + c0 + 4 * tx;
     *reinterpret_cast<float4*>(s) = make_float4(back[0], back[1], back[2], back[3]);
     *reinterpret_cast<float4*>(s + 32) = make_float4(back[4], back[5], back[6], back[7]);
   }
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
-    const int64_t row = r0 + 64 * (i >> 2) + 4 * ty + (i & 3);
+    const int64_t row = r0 + ry + 16 * (i >> 2) + (i & 3);
     if (row < N) {
       uint32_t hi[4], lo[4];
 #pragma unroll
@@ -239,6 +223,13 @@ wide_products_kernel(const float* __restrict__ xt, int64_t Np, const float* __re
       *reinterpret_cast<uint2*>(rlo + at + 32) = make_uint2(lo[2], lo[3]);
     }
   }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  __syncthreads();   // every thread is done with the stages
+  double* red = reinterpret_cast<double*>(stages);   // [16][64]
+#pragma unroll
+  for (int c = 0; c < 8; ++c)
+    red[ty * kWideCT + (c < 4 ? 4 * tx + c : 32 + 4 * tx + c - 4)] = ll[c];
+  __syncthreads();
   if (tid < kWideCT && c0 + tid < n) {
     double s = 0.0;
 #pragma unroll
@@ -272,7 +263,7 @@ struct WideShape {
     l.lpart = l.gpart + up(sizeof(float) * grad_tc_rows(sms, cap, dp()) * (size_t)D);
     l.qt = l.lpart + up(sizeof(double) * (size_t)(np() / kWideRT) * cap);
     l.rscale = l.qt + up(sizeof(float) * (size_t)dp() * l.cp);
-    l.total = l.rscale + up(sizeof(float) * (size_t)(np() / kWideRT) * l.cp);
+    l.total = l.rscale + up(sizeof(float) * (size_t)(np() / 32) * l.cp);
     return l;
   }
 };

@@ -137,6 +137,12 @@ def seed_words(seed):
   return arr
 
 
+# Handle of the current stream of a device: torch's own call for it where there is one
+# (0.1 us; the stream object 1 to 3).
+raw_stream = getattr(torch._C, '_cuda_getCurrentRawStream', None) or (
+    lambda device: torch.cuda.current_stream(device).cuda_stream)
+
+
 class Context:
   """One engine context per (device, stream); streams are torch's."""
   _cache = {}
@@ -144,6 +150,7 @@ class Context:
   def __init__(self, device, stream):
     self.device = device
     self.stream = stream
+    self.raw_stream = stream.cuda_stream
     h = P()
     check(lib().gbm_context_create(device, P(stream.cuda_stream), ctypes.byref(h)),
           'gbm_context_create')

@@ -31,11 +31,11 @@ class Target:
     """Before a sampler's work for a caller: where the caller's stream is not the
     target's, which runs it, the target's waits for what the caller has queued.
     Returns the caller's stream then, else None, for _leave."""
-    stream = self._ctx.stream
-    caller = torch.cuda.current_stream(self._ctx.device)
-    if caller == stream:
+    ctx = self._ctx
+    if _native.raw_stream(ctx.device) == ctx.raw_stream:
       return None
-    stream.wait_stream(caller)
+    caller = torch.cuda.current_stream(ctx.device)
+    ctx.stream.wait_stream(caller)
     return caller
 
   def _leave(self, caller):

@@ -823,6 +823,11 @@ class LogregF32 final : public Target {
       case 7: f32_set_smem<7>(); break;
       default: f32_set_smem<8>(); break;
     }
+    if (!tc_) {
+      prepare_leapfrogs<1>();
+      prepare_leapfrogs<2>();
+      prepare_leapfrogs<4>();
+    }
   }
 
   static int width(int64_t d) {      // in 16 features

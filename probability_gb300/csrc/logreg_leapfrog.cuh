@@ -307,13 +307,18 @@ inline bool leap_shape(int64_t N, int D, int C, int grid_max, int chain_tile, Le
   return false;
 }
 
+// Once before the launches.
+template <int G>
+void prepare_leapfrogs() {
+  GBM_CUDA(cudaFuncSetAttribute(logreg_leapfrog_kernel<G>,
+                                cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kLeapSmem));
+}
+
 template <int G>
 void launch_leapfrogs(const LeapShape& h, const float* X2, const float* ym, int N, int Dp, int C,
                       int steps, const float* eps, int per_chain, float inv_var, double log_norm,
                       const double* lin, float* q, float* p, float* g, double* logp, int ld,
                       cudaStream_t s) {
-  GBM_CUDA(cudaFuncSetAttribute(logreg_leapfrog_kernel<G>,
-                                cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kLeapSmem));
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)((C + G - 1) / G * h.K));
   cfg.blockDim = dim3(kLeapThreads);

@@ -220,10 +220,11 @@ large_epilogue(const float* __restrict__ Z, const float* __restrict__ Zlo,
 
 // One block per chain: log-density from the partials, the linear term and the
 // prior, in a fixed order; gradient G - q / s^2.  (A warp per chain waited for its
-// loads in turn: 15 us at 929 features, 240 chains, 8 so; a block of 256 threads leaves
-// the GPU short of chains where they are many: 300 x 300, 20,000 of them 366 us an
-// evaluation, 328 so.)
-constexpr int kFinishThreads = 128;
+// loads in turn: 15 us at 929 features, 240 chains, 8 with 256 threads; from
+// kManyChains on, where that leaves the GPU short of chains, 128: 300 x 300, 20,000 of
+// them 366 and 328 us an evaluation.)
+constexpr int kManyChains = 2048;
+template <int kFinishThreads>
 __global__ void __launch_bounds__(kFinishThreads)
 large_finish(const double* __restrict__ part, int nblk, int n, const float* __restrict__ G,
              const float* __restrict__ Glo, int ld, const float* __restrict__ q, int ldq,
@@ -412,9 +413,16 @@ class LogregLarge final : public Target {
     };
     gemm_g(xh_.ptr, w, &zero);
     if (xlo_) gemm_g(xl_.ptr, n, &one);
-    large_finish<<<(unsigned)n, kFinishThreads, 0, s>>>(
-        part, (int)nblk, n, G, mixed_ ? G + (size_t)n * ld_ : nullptr, ld_, q, ldq,
-        lin_.as<double>(), D, inv_var_, log_norm_, logp, grad, ldg);
+    auto finish = [&](auto kernel, int threads) {
+      kernel<<<(unsigned)n, threads, 0, s>>>(part, (int)nblk, n, G,
+                                             mixed_ ? G + (size_t)n * ld_ : nullptr, ld_, q, ldq,
+                                             lin_.as<double>(), D, inv_var_, log_norm_, logp, grad,
+                                             ldg);
+    };
+    if (n >= kManyChains)
+      finish(large_finish<128>, 128);
+    else
+      finish(large_finish<256>, 256);
     GBM_CUDA(cudaGetLastError());
   }
 

@@ -134,7 +134,7 @@ split_reduce_kernel(const double* __restrict__ lpart, const float* __restrict__ 
   if (blockIdx.y == 0 && thread + 32 >= threads) {
     const int lane = threadIdx.x & 31, rows = lparts > 0 ? lparts : S;
     double t = 0.0, pr = 0.0, li = 0.0;
-    constexpr int U = F == 128 ? 8 : 1;       // loads in flight
+    constexpr int U = F == 128 ? 8 : 1, V = F == 128 ? 4 : 1;   // steps whose loads are in flight
 #pragma unroll 1
     for (int j = lane; j < rows; j += 32 * U) {
       double v[U];
@@ -145,11 +145,23 @@ split_reduce_kernel(const double* __restrict__ lpart, const float* __restrict__ 
       for (int u = 0; u < U; ++u)
         if (u == 0 || j + 32 * u < rows) t += v[u];
     }
-#pragma unroll(F == 128 ? 4 : 1)
-    for (int f = lane; f < D; f += 32) {
-      const double qd = (double)q[f];
-      pr += qd * qd;
-      if (lin) li += lin[f] * qd;
+#pragma unroll 1
+    for (int f = lane; f < D; f += 32 * V) {
+      float qv[V];
+      double lv[V];
+#pragma unroll
+      for (int u = 0; u < V; ++u) {
+        const bool held = u == 0 || f + 32 * u < D;
+        qv[u] = held ? q[f + 32 * u] : 0.f;
+        lv[u] = held && lin ? lin[f + 32 * u] : 0.0;
+      }
+#pragma unroll
+      for (int u = 0; u < V; ++u)
+        if (u == 0 || f + 32 * u < D) {
+          const double qd = (double)qv[u];
+          pr += qd * qd;
+          if (lin) li += lv[u] * qd;
+        }
     }
     t = warp_sum(t + li - half_inv_var * pr);
     if (lane == 0) logp[c] = t + dims * log_norm;

@@ -27,8 +27,8 @@
 //
 // What bounds it: mvn_tile.cuh's tiles, and their longest sum where one large
 // member holds most of the work.  Twelve normals up to 2048 (497 chains) and
-// twelve hierarchical members: 517 us an evaluation with tiles of 128 outputs in
-// member order at a fixed stride, 208 now; members of at most 300: 83 and 48.
+// twelve hierarchical members: 521 us an evaluation with tiles of 128 outputs in
+// member order at a fixed stride, 207 now; members of at most 300: 66 and 41.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -505,7 +505,7 @@ class BatchTarget final : public Target {
     GBM_CUDA(cudaStreamSynchronize(ctx_->stream));   // the vector is this call's
   }
 
-  // The hierarchical members whose chains fit a warp's registers.
+  // The hierarchical members whose chains a warp holds (kChainMaxDim elements).
   void set_chain_models(gbm_context* ctx) {
     const std::vector<double> table = chain_log_table();
     table_.reserve(sizeof(double) * table.size());

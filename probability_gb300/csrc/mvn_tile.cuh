@@ -26,8 +26,8 @@
 // clocks a step with one warp on each SM quarter (issue, and shared-memory latency
 // that a lone warp cannot hide).  One tile of 64 x 64 a CTA with two stages filled
 // through registers took 105.  Measured, whole evaluations: 777 x 350 chains 146 us
-// before, 48 so; 2048 x 512 446 and 169; 300 x 300 70 and 27; the ragged batch
-// below 517 and 208.
+// before, 52 so; 2048 x 512 446 and 175; 300 x 300 70 and 29; the ragged batch
+// below 521 and 207.
 #pragma once
 #include <cuda_runtime.h>
 

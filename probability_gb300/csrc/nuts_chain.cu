@@ -10,7 +10,8 @@
 // chain's trajectories to the end: position, momentum, gradient and momentum
 // sum of the growing end stay on the SM (a register a lane up to 32 elements,
 // shared memory above), the scalars are warp-uniform registers, and only the
-// far end, the candidates and the later U-turn slots are in memory.  A warp that is done leaves its place to the next chain's block.
+// far end, the candidates and the later U-turn slots are in memory.  A warp that is
+// done leaves its place to the next chain's block.
 //
 // The arithmetic, its order within a lane and the draws are those of the
 // batched kernels (samplers.cu, targets_misc.cu, batch.cu), but for the
@@ -21,7 +22,7 @@
 // work is kept to the ~45 instructions that the energies need.  Measured: one
 // transition of 256 eight-schools chains 1.18 ms -> 0.15 (kernel 0.14, ~2,000
 // clocks a leaf of the longest chain); 4 free-running transitions of 16
-// members (4,300 chains, up to 512 groups) 60.6 ms -> 10.9.
+// members (4,300 chains, up to 512 groups) 71.5 ms -> 12.3.
 #include <cuda_runtime.h>
 
 #include <algorithm>

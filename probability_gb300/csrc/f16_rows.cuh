@@ -136,7 +136,8 @@ struct F16Rows {
   // NaN, exponents that the scaling cannot carry, or a range so wide that hi + lo
   // leaves more than kMostLoss of a column's nonzero entries on average, each relative
   // to the entry; a label so far outside [0, 1] that a residual, below
-  // |y - 1/2| + 1/2, could leave FP16's range (R' < 2^16); more than kMost elements, or no memory for it.
+  // |y - 1/2| + 1/2, could leave FP16's range (R' < 2^16); more than kMost
+  // elements, or no memory for it.
   //
   // The average is over entries and not over their squares because which rows count
   // is the residuals' to say: where a fit has a large entry's row right, its residual

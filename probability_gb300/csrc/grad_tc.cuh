@@ -52,8 +52,8 @@ __global__ void __launch_bounds__(kGradThreads, 1)
 grad_tc_kernel(const __grid_constant__ CUtensorMap rhi, const __grid_constant__ CUtensorMap rlo,
                const __grid_constant__ CUtensorMap xhi, const __grid_constant__ CUtensorMap xlo,
                const float* __restrict__ gscale, const float* __restrict__ rscale, int cp, int N,
-               int D, int dp, const int* __restrict__ n_dev, int c_base, int c_lim, int grid, int ftiles,
-               float* __restrict__ gpart, int* __restrict__ err) {
+               int D, int dp, const int* __restrict__ n_dev, int c_base, int c_lim, int grid,
+               int ftiles, float* __restrict__ gpart, int* __restrict__ err) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>(
       (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -212,8 +212,10 @@ grad_tc_kernel(const __grid_constant__ CUtensorMap rhi, const __grid_constant__ 
         tc::tmem_ld16(tmem + s * kGradFT + quarter + col + 16 * j, v);
         tc::tmem_ld_wait();
 #pragma unroll
-        for (int e = 0; e < 16; ++e)
-          sum[16 * j + e] = K_MAJOR ? sum[16 * j + e] + v[e] : fmaf(v[e], s ? scale[1] : scale[0], sum[16 * j + e]);
+        for (int e = 0; e < 16; ++e) {
+          float& at = sum[16 * j + e];
+          at = K_MAJOR ? at + v[e] : fmaf(v[e], s ? scale[1] : scale[0], at);
+        }
       }
       tc::tc_fence_before();
       __syncwarp();
@@ -275,9 +277,9 @@ void grad_tc_setup() {
 // Partials of chains [c_base, c_base + cap) whose residuals are at r (hi, then lo
 // at r_lo): [N][ldr] chains with rscale, or [chains][ldr] rows.
 template <bool K_MAJOR>
-void launch_grad_tc(const F16Rows& x, __half* r, __half* r_lo, const float* rscale, int64_t ldr, int N, int D, int dp,
-                    const int* n_dev, int c_base, int c_lim, int cap, int grid, float* gpart,
-                    int* err, cudaStream_t s) {
+void launch_grad_tc(const F16Rows& x, __half* r, __half* r_lo, const float* rscale, int64_t ldr,
+                    int N, int D, int dp, const int* n_dev, int c_base, int c_lim, int cap,
+                    int grid, float* gpart, int* err, cudaStream_t s) {
   CUtensorMap hi, lo;
   if (K_MAJOR) {
     encode_rows(&hi, r, cap, (int)ldr, kGradCT);
@@ -288,7 +290,8 @@ void launch_grad_tc(const F16Rows& x, __half* r, __half* r_lo, const float* rsca
   }
   const int ft = grad_tc_ftiles(dp);
   grad_tc_kernel<K_MAJOR><<<(unsigned)(grid * ft), kGradThreads, kGradSmem, s>>>(
-      hi, lo, x.hi, x.lo, x.gscale, rscale, (int)ldr, N, D, dp, n_dev, c_base, c_lim, grid, ft, gpart, err);
+      hi, lo, x.hi, x.lo, x.gscale, rscale, (int)ldr, N, D, dp, n_dev, c_base, c_lim, grid, ft,
+      gpart, err);
   GBM_CUDA(cudaGetLastError());
 }
 

@@ -35,8 +35,8 @@
 // (of each feature scaled to the top of FP16's range) beside its FP32 form,
 //   G^T = R_lo^T X_hi + R_hi^T X_lo + R_hi^T X_hi  (M = 128 chains, K = 64 rows).
 // hi + lo carries a float to 2^-23 of itself at worst (f16_rows.cuh says for which
-// columns); what is left out (lo.lo) is as small.  The tensor cores truncate every addition to their FP32 accumulator,
-// so a turn of at most two tiles starts from zero, the small terms of a tile
+// columns); what is left out (lo.lo) is as small.  The tensor cores truncate every
+// addition to their FP32 accumulator, so a turn of at most two tiles starts from zero, the small terms of a tile
 // first, and is then added in FP32 to the sum of the turns before: gradient
 // error against 64 bits 1.4e-7 at 1e5 x 100 x 1024 chains (phase 2 on the CUDA
 // cores: 2.9e-7).  Z, and with it the log-density, is phase 1's, bit for bit.

@@ -397,8 +397,8 @@ class LogregLarge final : public Target {
     if (tc_) {
       __half* r = reinterpret_cast<__half*>(R);
       const int g = grad_tc_grid(sms_, n, N_, dp_);
-      launch_grad_tc<true>(x16_, r, r + (size_t)n * ldz_, nullptr, ldz_, (int)N_, D, dp_, nullptr, 0, n, n,
-                           g, G, err_dev_, s);
+      launch_grad_tc<true>(x16_, r, r + (size_t)n * ldz_, nullptr, ldz_, (int)N_, D, dp_,
+                           nullptr, 0, n, n, g, G, err_dev_, s);
       launch_split_reduce(part, G, q, ldq, nullptr, 0, n, n, kGradCT, kGradRT, g, (int)N_, D,
                           inv_var_, log_norm_, lin_.as<double>(), logp, grad, ldg, s, (int)nblk);
       return;

@@ -83,7 +83,8 @@ __global__ void wide_states_kernel(const float* __restrict__ Q, int ldq,
 
 __global__ void __launch_bounds__(kWideThreads, 3)
 wide_products_kernel(const float* __restrict__ xt, int64_t Np, const float* __restrict__ y,
-                     int N, int Dp, const float* __restrict__ qt, int cp, const int* __restrict__ n_dev, int c_base, int c_lim,
+                     int N, int Dp, const float* __restrict__ qt, int cp,
+                     const int* __restrict__ n_dev, int c_base, int c_lim,
                      double* __restrict__ lpart, __half* __restrict__ rhi,
                      __half* __restrict__ rlo, float* __restrict__ rscale) {
   extern __shared__ __align__(16) float stages[];

@@ -16,8 +16,8 @@
 // What bounds it: FMA issue of the products (an 8 x 8 thread's shared loads take
 // as long as its FMAs: 107 of 128 FMAs a clock and SM).  30,011 x 237, 192 chains:
 // 359 us an evaluation by logreg_simt.cu (4 x 4 a thread, unpipelined, G on the
-// CUDA cores), 108 so: products 65 (two of them for the residuals' scales and small
-// bits), gradient 26, reduction 11; 300 x 130, 16 chains 61 and 38.
+// CUDA cores), 106 so: products 63, gradient 25, reduction 10; 300 x 130, 16 chains
+// 61 and 38.
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
@@ -153,21 +153,25 @@ wide_products_kernel(const float* __restrict__ xt, int64_t Np, const float* __re
     ll[c] = 0.0;
     most[c] = 0.f;
   }
+  constexpr int kTurn = 2;
+  float four[8];
 #pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    float four[8];
+  for (int c = 0; c < 8; ++c) four[c] = 0.f;
+  // Two rows an iteration of a rolled loop, in which z turns: unrolled over its eight
+  // rows this runs once, from a cold instruction cache (2000 x 200, 64 chains: 21.7 us
+  // for the kernel, 16.9 so).
+#pragma unroll 1
+  for (int k = 0; k < 8; k += kTurn) {
 #pragma unroll
-    for (int c = 0; c < 8; ++c) four[c] = 0.f;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int64_t row = r0 + ry + 16 * h + i;
+    for (int b = 0; b < kTurn; ++b) {
+      const int64_t row = r0 + ry + 16 * (k >> 2) + ((k + b) & 3);
       if (row < N) {
         const float yv = y[row];
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
 #pragma unroll
           for (int e = 0; e < 2; ++e) {
-            float& at = e ? z[4 * h + i][j].y : z[4 * h + i][j].x;
+            float& at = e ? z[b][j].y : z[b][j].x;
             const float zv = at;
             const float t = expf(-fabsf(zv)), l = log1pf(t);
             // bernoulli.py:126-140: -softplus(z) (1 - y) - softplus(-z) y
@@ -184,8 +188,27 @@ wide_products_kernel(const float* __restrict__ xt, int64_t Np, const float* __re
         }
       }
     }
+    if (((k + kTurn) & 3) == 0) {
 #pragma unroll
-    for (int c = 0; c < 8; ++c) ll[c] += (double)four[c];
+      for (int c = 0; c < 8; ++c) {
+        ll[c] += (double)four[c];
+        four[c] = 0.f;
+      }
+    }
+    // The rows turn: after eight they are in their places again.
+    float2 done[kTurn][4];
+#pragma unroll
+    for (int b = 0; b < kTurn; ++b)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) done[b][j] = z[b][j];
+#pragma unroll
+    for (int m = 0; m < 8 - kTurn; ++m)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) z[m][j] = z[m + kTurn][j];
+#pragma unroll
+    for (int b = 0; b < kTurn; ++b)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) z[8 - kTurn + b][j] = done[b][j];
   }
   // A chain's 32 residuals are stored as multiples of the power of two that takes
   // the largest of them below 2^15; gradient sums are in multiples of 2^-15.

@@ -62,9 +62,10 @@ template <int CT, int OB, int RO, int KG>
 struct MvnTiles {
   template <int PHASE>
   static void set_smem() {
-    GBM_CUDA(cudaFuncSetAttribute(mvn_tri_kernel<PHASE, CT, OB, RO, KG>,
-                                  cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)sizeof(typename MvnLaunch<PHASE, CT, OB, RO, KG>::Smem)));
+    constexpr int bytes = (int)sizeof(typename MvnLaunch<PHASE, CT, OB, RO, KG>::Smem);
+    if (bytes > 48 * 1024)    // up to there a launch may ask for it as it is
+      GBM_CUDA(cudaFuncSetAttribute(mvn_tri_kernel<PHASE, CT, OB, RO, KG>,
+                                    cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
   }
   static void prepare() {
     set_smem<0>();
